@@ -1006,15 +1006,37 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qrows_kernel(const RowsParams
                     const int tgf_lo = (int)((int64_t)p.total * b_lo / gridDim.x) / upt;
                     const float *src = p.part + (size_t)warp * 256 + lane;
                     const float *first = src + b_lo * cta_stride + (size_t)(tg - tgf_lo) * kRowsWarps * 256;
+                    // entry 32 i + lane of the tile's 16 x 16: (row, activation row).  The eight entries of a piece, their
+                    // residuals and scales are requested together, so a fold waits for L2 about once per kFold pieces and not once
+                    // per entry and piece.  What bounds a narrow launch is this chain of latencies: 4096 x 4096 Q4_K with
+                    // 16 rows (up to ten pieces a tile) took 21 us with the loads one after another and takes 16.  More than
+                    // three pieces at a time spill at the 96 registers of 544 threads.
+                    constexpr int kFold = 3;
+                    float sum[8], res[8];
+                    const int tok = lane & 15;
+                    const float inv = tok < p.m ? __ldg(p.inv_scale + tok) : 0.f;
+                    const bool live = tok < p.m;
 #pragma unroll
-                    for (int i = 0; i < 8; i++) {               // entry 32 i + lane of the tile's 16 x 16: (row, activation row)
-                        const int idx = 32 * i + lane, rt = idx >> 4, tok = idx & 15, row = tile16 * 16 + rt;
-                        float sum = __ldcg(first + 32 * i);
-                        for (int cta = b_lo + 1; cta <= b_hi; cta++) sum += __ldcg(src + cta * cta_stride + 32 * i);
-                        if (tok < p.m && row < p.n[wi]) {
-                            const float res = p.resid ? __ldg(p.resid + (size_t)tok * p.n[wi] + row) : 0.f;
-                            p.out[wi][(size_t)tok * p.n[wi] + row] = res + sum * __ldg(p.inv_scale + tok);
-                        }
+                    for (int i = 0; i < 8; i++) {
+                        const int row = tile16 * 16 + 2 * i + (lane >> 4);
+                        sum[i] = __ldcg(first + 32 * i);
+                        res[i] = p.resid && live && row < p.n[wi] ? __ldg(p.resid + (size_t)tok * p.n[wi] + row) : 0.f;
+                    }
+                    for (int cta = b_lo + 1; cta <= b_hi; cta += kFold) {
+                        float v[kFold][8];
+#pragma unroll
+                        for (int q = 0; q < kFold; q++)
+#pragma unroll
+                            for (int i = 0; i < 8; i++) v[q][i] = cta + q <= b_hi ? __ldcg(src + (cta + q) * cta_stride + 32 * i) : 0.f;
+#pragma unroll
+                        for (int q = 0; q < kFold; q++)
+#pragma unroll
+                            for (int i = 0; i < 8; i++) sum[i] += v[q][i];
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const int row = tile16 * 16 + 2 * i + (lane >> 4);
+                        if (live && row < p.n[wi]) p.out[wi][(size_t)tok * p.n[wi] + row] = res[i] + sum[i] * inv;
                     }
                 }
             }
