@@ -28,10 +28,14 @@ __device__ __forceinline__ float warp_sum(float v)
 
 // ================================================================ one row
 constexpr int kMvThreads = 256, kMvWarps = kMvThreads / 32, kMvRows = 4, kMvChunk = 256;
+constexpr int kMvDepth = 3;                                                   // weight chunks a warp has on their way
+constexpr size_t kMvStage = (size_t)kMvRows * kMvThreads * 16;
+constexpr int kMvVec = 8;                                                     // float4 per thread of a row held in registers: up to 8192 inputs
 
 struct DenseMvParams {
     const __nv_bfloat16 *w;
     int n, k, ld, nch;                 // nch: chunks of 256 columns
+    int depth;                         // weight chunks a warp has on their way: kMvDepth, or 1 beside a very long row
     const float *bias;
     const float *x;
     const __nv_bfloat16 *emb;
@@ -64,6 +68,13 @@ struct DenseMvParams {
 // eight (two 16-byte reads) are read without bank conflicts.
 __device__ __forceinline__ int xs_at(int e) { return (e & ~255) + ((e & 4) << 5) + ((e & 255) >> 3) * 4 + (e & 3); }
 
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool in)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 template <int NV>
 __device__ __forceinline__ void block_sums(float (&v)[NV], float *red)
 {
@@ -88,7 +99,8 @@ __global__ void __launch_bounds__(kMvThreads, 4) dense_matvec_kernel(const Dense
 {
     constexpr int GROUPS = kMvWarps / WK, TILE = GROUPS * kMvRows;
     constexpr bool GNORM = PRO == DPRO_GNORM, EXPERT = PRO == DPRO_EXPERT, EXPERTS = PRO == DPRO_EXPERTS;
-    extern __shared__ __align__(16) float xs[];
+    extern __shared__ __align__(16) float mv_smem[];
+    float *xs = mv_smem + p.depth * (kMvStage / sizeof(float));
     __shared__ float red[GNORM ? 2 * kMaxNormGroups : kMvWarps * 3];
     __shared__ float fold[2][GROUPS][WK][kMvRows];
     __shared__ int s_sel[EXPERT ? kMaxTop : 1];
@@ -96,20 +108,50 @@ __global__ void __launch_bounds__(kMvThreads, 4) dense_matvec_kernel(const Dense
     __shared__ const __nv_bfloat16 *s_base[EXPERTS ? kMaxTop + 1 : 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wk = warp % WK, wg = warp / WK;
 
-    // what the first tile reads does not depend on the launch before: ask L2 for it before waiting
+    // The weights do not depend on the launch before, so a warp has its first chunks copied to shared memory, and asks L2 for
+    // the rest of its first tile, before it waits.  A thread reads only what it copied itself: no barrier.
+    const uint32_t ring = smem_u32(mv_smem) + (uint32_t)tid * 16;
+    const __nv_bfloat16 *wbase = p.w;
+    int pf_tile = blockIdx.x, pf_c = wk, pf_slot = 0;
+    auto issue = [&] {
+        if (pf_tile < p.tiles) {
+            const int r0 = pf_tile * TILE + wg * kMvRows;
+            const __nv_bfloat16 *base = wbase;
+            int ld = p.ld, col = pf_c * kMvChunk + lane * 8;
+            if constexpr (EXPERTS) {
+                const int seg = min(pf_c / p.seg_nch, p.route.top);
+                base = s_base[seg];
+                col -= seg * p.seg_nch * kMvChunk;
+                ld = seg < p.route.top ? p.ld : p.shared_ld;
+            }
+            const bool in = col < ld;
+#pragma unroll
+            for (int r = 0; r < kMvRows; r++)
+                cp_async16(ring + (uint32_t)((pf_slot * kMvRows + r) * kMvThreads * 16), base + (size_t)min(r0 + r, p.n - 1) * ld + (in ? col : 0), in);
+            if ((pf_c += WK) >= p.nch) { pf_c = wk; pf_tile += gridDim.x; }
+        }
+        cp_async_commit();
+        if (++pf_slot == p.depth) pf_slot = 0;
+    };
+    auto fill = [&] {
+        for (int i = 0; i < p.depth; i++) issue();
+    };
     if (!EXPERT) {
         const int r0 = blockIdx.x * TILE + wg * kMvRows;
         const __nv_bfloat16 *w0 = EXPERTS ? p.shared_w : p.w;         // which experts' rows is not known yet
         const int ld = EXPERTS ? p.shared_ld : p.ld, nch = EXPERTS ? (p.shared_ld + kMvChunk - 1) / kMvChunk : p.nch;
+        if (!EXPERTS) fill();
         for (int r = 0; r < kMvRows && w0; r++) {
             const int row = min(r0 + r, p.n - 1);
             const __nv_bfloat16 *src = w0 + (size_t)row * ld;
-            for (int c = wk + (lane >> 2) * WK; c < nch; c += 8 * WK) {
+            for (int c = wk + ((EXPERTS ? 0 : p.depth) + (lane >> 2)) * WK; c < nch; c += 8 * WK) {
                 const int e = c * kMvChunk + (lane & 3) * 64;
                 if (e < ld) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + e));
             }
         }
     }
+    if (PRO == DPRO_NORM)
+        for (int e = tid * 32; e < p.k; e += kMvThreads * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.norm_w + e));
     if (GNORM) {
         for (int e = tid * 32; e < p.k; e += kMvThreads * 32) {
             asm volatile("prefetch.global.L2 [%0];" ::"l"(p.norm_w + e));
@@ -120,17 +162,50 @@ __global__ void __launch_bounds__(kMvThreads, 4) dense_matvec_kernel(const Dense
     pdl_launch_dependents();
 
     const int kp = p.nch * kMvChunk;
-    const __nv_bfloat16 *wbase = p.w;
     float *actp = p.act_out;
+    // a row of whole float4 is requested at once and stays in registers until its statistics are known
+    constexpr bool VEC = PRO == DPRO_PLAIN || EXPERT || PRO == DPRO_NORM || PRO == DPRO_POLY;
+    const bool vec = VEC && !p.emb && p.k % 4 == 0 && kp <= kMvVec * 4 * kMvThreads && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0;
+    float4 xv[VEC ? kMvVec : 1];
+    if (VEC && vec) {
+#pragma unroll
+        for (int i = 0; i < kMvVec; i++) {
+            const int e = (tid + i * kMvThreads) * 4;
+            xv[i] = e < p.k ? __ldcg(reinterpret_cast<const float4 *>(p.x + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
     if (PRO == DPRO_PLAIN || EXPERT) {
-        for (int e = tid; e < kp; e += kMvThreads) xs[xs_at(e)] = e < p.k ? __ldcg(p.x + e) : 0.f;
+        if (vec) {
+#pragma unroll
+            for (int i = 0; i < kMvVec; i++)
+                if ((tid + i * kMvThreads) * 4 < kp) *reinterpret_cast<float4 *>(xs + xs_at((tid + i * kMvThreads) * 4)) = xv[i];
+        } else {
+            for (int e = tid; e < kp; e += kMvThreads) xs[xs_at(e)] = e < p.k ? __ldcg(p.x + e) : 0.f;
+        }
         if (EXPERT) {
             route_token(p.logits, p.route, xs + kp, s_sel, s_weight);
             const int slot = blockIdx.y;
             wbase += (size_t)s_sel[slot] * p.n * p.ld;
+            fill();
             actp += (size_t)slot * (p.n / 2);
             if (blockIdx.x == 0 && slot == 0)
                 for (int i = tid; i < p.route.top; i += kMvThreads) { p.sel[i] = s_sel[i]; p.weight[i] = s_weight[i]; }
+        }
+    } else if (PRO == DPRO_NORM && vec) {
+        float ss[1] = {0.f};
+#pragma unroll
+        for (int i = 0; i < kMvVec; i++) ss[0] += (xv[i].x * xv[i].x + xv[i].y * xv[i].y) + (xv[i].z * xv[i].z + xv[i].w * xv[i].w);
+        block_sums(ss, red);
+        const float inv = 1.f / sqrtf(ss[0] / (float)p.k + p.eps);
+#pragma unroll
+        for (int i = 0; i < kMvVec; i++) {
+            const int e = (tid + i * kMvThreads) * 4;
+            if (e >= kp) continue;
+            const bool in = e < p.k;                     // xv is zero beyond
+            float4 o;
+            o.x = xv[i].x * inv * ((in ? p.norm_w[e] : 0.f) + p.norm_offset); o.y = xv[i].y * inv * ((in ? p.norm_w[e + 1] : 0.f) + p.norm_offset);
+            o.z = xv[i].z * inv * ((in ? p.norm_w[e + 2] : 0.f) + p.norm_offset); o.w = xv[i].w * inv * ((in ? p.norm_w[e + 3] : 0.f) + p.norm_offset);
+            *reinterpret_cast<float4 *>(xs + xs_at(e)) = o;
         }
     } else if (PRO == DPRO_NORM) {
         const __nv_bfloat16 *er = p.emb ? p.emb + (size_t)*p.token * p.emb_ld : nullptr;
@@ -241,6 +316,7 @@ __global__ void __launch_bounds__(kMvThreads, 4) dense_matvec_kernel(const Dense
             s_base[s] = s < top ? p.w + (size_t)__ldcg(p.sel + s) * p.n * p.ld : p.shared_w;
         }
         __syncthreads();
+        fill();
         for (int s = 0; s < top; s++) {
             const float w = s_weight[s];
             const float *x = p.x + (size_t)s * p.ldx;
@@ -252,45 +328,50 @@ __global__ void __launch_bounds__(kMvThreads, 4) dense_matvec_kernel(const Dense
         for (int e = tid; e < kp - first; e += kMvThreads) xs[first + xs_at(e)] = e < p.shared_k ? w * __ldcg(p.shared_x + e) : 0.f;
     } else {
         float ss[3] = {0.f, 0.f, 0.f};
-        for (int e = tid; e < p.k; e += kMvThreads) {
-            const float v = __ldcg(p.x + e), v2 = v * v;
-            xs[xs_at(e)] = v;
-            ss[0] += v2; ss[1] += v2 * v2; ss[2] += v2 * v2 * v2;
+        auto add = [&](float v) { const float v2 = v * v; ss[0] += v2; ss[1] += v2 * v2; ss[2] += v2 * v2 * v2; };
+        if (vec) {
+#pragma unroll
+            for (int i = 0; i < kMvVec; i++) { add(xv[i].x); add(xv[i].y); add(xv[i].z); add(xv[i].w); }
+        } else {
+            for (int e = tid; e < p.k; e += kMvThreads) {
+                const float v = __ldcg(p.x + e);
+                xs[xs_at(e)] = v;
+                add(v);
+            }
         }
         block_sums(ss, red);
         const float inv_n = 1.f / (float)p.k;
         const float a = p.poly[0] / sqrtf(ss[0] * inv_n + p.eps), b = p.poly[1] / sqrtf(ss[1] * inv_n + p.eps),
                     c = p.poly[2] / sqrtf(ss[2] * inv_n + p.eps), d = p.poly[3];
-        for (int e = tid; e < kp; e += kMvThreads) {
-            float *s = xs + xs_at(e);
-            const float z = *s;
-            *s = e < p.k ? z * (a + z * (b + z * c)) + d : 0.f;
+        auto act = [&](float z) { return z * (a + z * (b + z * c)) + d; };
+        if (vec) {
+#pragma unroll
+            for (int i = 0; i < kMvVec; i++) {
+                const int e = (tid + i * kMvThreads) * 4;
+                if (e >= kp) continue;
+                const float4 v = xv[i];
+                *reinterpret_cast<float4 *>(xs + xs_at(e)) = e < p.k ? make_float4(act(v.x), act(v.y), act(v.z), act(v.w)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        } else {
+            for (int e = tid; e < kp; e += kMvThreads) {
+                float *s = xs + xs_at(e);
+                *s = e < p.k ? act(*s) : 0.f;
+            }
         }
     }
     __syncthreads();
 
-    int flip = 0;
+    int flip = 0, slot = 0;
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x, flip ^= 1) {
         const int r0 = tile * TILE + wg * kMvRows;
-        const uint4 *rows[kMvRows];
-#pragma unroll
-        for (int r = 0; r < kMvRows; r++) rows[r] = reinterpret_cast<const uint4 *>(wbase + (size_t)min(r0 + r, p.n - 1) * p.ld) + lane;
         float acc[kMvRows] = {0.f, 0.f, 0.f, 0.f};
-        auto load = [&](int c, uint4 (&v)[kMvRows]) {
-            if constexpr (EXPERTS) {
-                const int seg = min(c / p.seg_nch, p.route.top), col = (c - seg * p.seg_nch) * kMvChunk + lane * 8, ld = seg < p.route.top ? p.ld : p.shared_ld;
-                const bool in = c < p.nch && col < ld;
+        for (int c = wk; c < p.nch; c += WK) {
+            if (p.depth == kMvDepth) cp_async_wait<kMvDepth - 1>();
+            else cp_async_wait<0>();
+            uint4 v[kMvRows];
 #pragma unroll
-                for (int r = 0; r < kMvRows; r++)
-                    v[r] = in ? __ldcs(reinterpret_cast<const uint4 *>(s_base[seg] + (size_t)min(r0 + r, p.n - 1) * ld + col)) : make_uint4(0u, 0u, 0u, 0u);
-            } else {
-                const bool in = c < p.nch && c * kMvChunk + lane * 8 < p.ld;
-#pragma unroll
-                for (int r = 0; r < kMvRows; r++) v[r] = in ? __ldcs(rows[r] + c * (kMvChunk / 8)) : make_uint4(0u, 0u, 0u, 0u);
-            }
-        };
-        auto mul = [&](int c, const uint4 (&v)[kMvRows]) {
-            if (c >= p.nch) return;
+            for (int r = 0; r < kMvRows; r++) v[r] = lds128(ring + (uint32_t)((slot * kMvRows + r) * kMvThreads * 16));
+            if (++slot == p.depth) slot = 0;
             const float4 xa = *reinterpret_cast<const float4 *>(xs + c * kMvChunk + lane * 4);
             const float4 xb = *reinterpret_cast<const float4 *>(xs + c * kMvChunk + 128 + lane * 4);
 #pragma unroll
@@ -302,13 +383,7 @@ __global__ void __launch_bounds__(kMvThreads, 4) dense_matvec_kernel(const Dense
                 s = fmaf(bf_lo(v[r].w), xb.z, s); s = fmaf(bf_hi(v[r].w), xb.w, s);
                 acc[r] = s;
             }
-        };
-        for (int c = wk; c < p.nch; c += 2 * WK) {
-            uint4 va[kMvRows], vb[kMvRows];
-            load(c, va);
-            load(c + WK, vb);
-            mul(c, va);
-            mul(c + WK, vb);
+            issue();                                     // into the slot just read
         }
 #pragma unroll
         for (int r = 0; r < kMvRows; r++) acc[r] = warp_sum(acc[r]);
@@ -711,10 +786,12 @@ tlb_status launched(const char *what)
 }
 
 template <int PRO, int WK>
-tlb_status run_matvec(const DenseMvParams &p, bool pdl)
+tlb_status run_matvec(DenseMvParams p, bool pdl)
 {
     Context *c = ctx();
-    const size_t smem = ((size_t)p.nch * kMvChunk + (PRO == DPRO_EXPERT ? route_scratch_floats(p.route) : 0)) * sizeof(float);
+    const size_t row = ((size_t)p.nch * kMvChunk + (PRO == DPRO_EXPERT ? route_scratch_floats(p.route) : 0)) * sizeof(float);
+    p.depth = row + kMvDepth * kMvStage + 2048 <= c->smem_optin ? kMvDepth : 1;
+    const size_t smem = row + p.depth * kMvStage;
     static size_t allowed = 40 << 10;      // with the static part, under the 48 KB that need no asking
     if (smem > allowed) {
         TLB_CUDA(cudaFuncSetAttribute(dense_matvec_kernel<PRO, WK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
