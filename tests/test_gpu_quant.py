@@ -184,6 +184,25 @@ def test_qgemm_matches_oracle(orc, t, n, k, m):
         assert relerr(got, emu) < GEMM_EMU_TOL
 
 
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("n,k,m", [(128, 256, 129), (300, 512, 256), (257, 768, 257), (1000, 2304, 333), (640, 1024, 384), (129, 4096, 385), (2000, 512, 769)])
+def test_qgemm_pairs_of_ctas(orc, t, n, k, m):
+    """More than 128 rows run on pairs of CTAs: an odd number of row tiles, one and two accumulators, token tiles that end
+    inside either CTA's half or before it begins, K ranges of unequal length."""
+    rng = np.random.default_rng(5100 + t + n + m)
+    w = synth.random_quant(t, n, k, rng)
+    x = rng.standard_normal((m, k), dtype=np.float32)
+    x[m // 2] *= 300.0
+    q = tl.QTensor.from_gguf_bytes(t, n, k, w)
+    got = tl.Tensor.from_numpy(x).matmul_quantized(q).numpy()
+    again = tl.Tensor.from_numpy(x).matmul_quantized(q).numpy()
+    np.testing.assert_array_equal(got.view(np.uint32), again.view(np.uint32))
+    ref = x.astype(np.float64) @ q.dequantize().numpy().astype(np.float64).T
+    assert got.shape == (m, n)
+    for i in range(m):
+        assert relerr(got[i], ref[i]) < GEMM_TOL, i
+
+
 @pytest.mark.parametrize("t,n,k", [(synth.Q4_K, 4096, 4096), (synth.Q6_K, 16384, 4096), (synth.Q4_0, 2048, 5632), (synth.Q8_0, 2048, 2048)])
 def test_qgemm_full_size_agrees_with_matvec(t, n, k):
     """Model-sized weights, 512 rows: sampled rows of the GEMM against the streaming matvec on the same rows."""

@@ -50,6 +50,7 @@ constexpr int kTmemCols = 512;
 constexpr int kTmemA0 = 256;
 constexpr int kStageACols = kGemmBK / 2;
 constexpr int kGemmAStages = 8;
+constexpr int kTmemWideA0 = 384, kGemmWideStages = 4;   // two accumulators of up to 192 columns side by side: four weight stages above them
 // Shared memory: the activation ring.  One barrier pair per K step in flight: slot kt % slots, slots = max(8, ring depth)
 constexpr int kGemmBBytes = 192 * 1024;
 constexpr int kGemmMaxSlots = 16;
@@ -68,6 +69,7 @@ struct GemmParams {
     int nt;                 // activation rows per CTA (MMA N)
     int nb;                 // depth of the activation ring (stages)
     int gs;                 // 64-wide K groups per stage: 1, or 4 (a whole 256-wide unit per barrier round) for tiles of up to 64 rows
+    int pair;               // two CTAs (adjacent row tiles) share a token tile: half of it each
     int kt_total;           // K / 64
     int unit_bytes;
     const float *inv_scale; // [m]
@@ -152,11 +154,13 @@ __device__ __forceinline__ void q4k_scales4(const uint4 &h, bool upper, uint32_t
 }
 // store4 parameters of one sub-block: (1024 + q) * sc - 1024 sc = q sc exactly, then * d - dmin m
 struct Q4KSub { uint32_t sc, c, ndm; };
-__device__ __forceinline__ Q4KSub q4k_sub(uint32_t scw, uint32_t mw, int byte, uint32_t dmin2)
+// high: the quants enter as 1024 + 16 q, the scale as sc / 16 (exact)
+__device__ __forceinline__ Q4KSub q4k_sub(uint32_t scw, uint32_t mw, int byte, uint32_t dmin2, bool high)
 {
     Q4KSub o;
     o.sc = byte_h2(scw, byte);
-    o.c = hmul2u(o.sc, 0xE400E400u);                             // -1024 sc, exact
+    if (high) o.sc = hmul2u(o.sc, 0x2C002C00u);
+    o.c = hmul2u(o.sc, 0xE400E400u);                             // -1024 sc (-64 sc for high nibbles), exact
     o.ndm = hmul2u(byte_h2(mw, byte), dmin2) ^ 0x80008000u;      // -(dmin m), rounded once
     return o;
 }
@@ -197,12 +201,15 @@ __device__ __forceinline__ void unit_emit(const Q4KRegs &u, int g, AFrag &f)
         uint32_t scw, mw;
         q4k_scales4(u.h[rs], g >= 2, scw, mw);
         const uint32_t d2 = prmt(u.h[rs].x, 0u, 0x1010u), dmin2 = prmt(u.h[rs].x, 0u, 0x3232u);
-        const Q4KSub lo = q4k_sub(scw, mw, (2 * g) & 3, dmin2), hi = q4k_sub(scw, mw, (2 * g + 1) & 3, dmin2);
+        const Q4KSub lo = q4k_sub(scw, mw, (2 * g) & 3, dmin2, false), hi = q4k_sub(scw, mw, (2 * g + 1) & 3, dmin2, true);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const Q4KSub &q = (j >> 1) ? hi : lo;
-            const uint32_t wd = word_of(u.q[g & 1], rs * 2 + (j & 1));   // bytes 16 (j & 1) + 4c .. of the group's 32
-            store4(f, j, rs, (wd >> (4 * (j >> 1))) & 0x0F0F0F0Fu, q.sc, q.c, d2, q.ndm);
+            const uint32_t wd = word_of(u.q[g & 1], rs * 2 + (j & 1)), w8 = wd >> 8;   // bytes 16 (j & 1) + 4c .. of the group's 32
+            // one LOP3 makes a pair 1024 + q of low nibbles, or 1024 + 16 q of high ones in place (their scale is sc / 16)
+            const uint32_t mask = (j >> 1) ? 0x00F000F0u : 0x000F000Fu;
+            f.v[4 * j + 2 * rs] = hfma2u(hfma2u(and_or(wd, mask, 0x64006400u), q.sc, q.c), d2, q.ndm);
+            f.v[4 * j + 2 * rs + 1] = hfma2u(hfma2u(and_or(w8, mask, 0x64006400u), q.sc, q.c), d2, q.ndm);
         }
     }
 }
@@ -322,11 +329,11 @@ template <> struct UnitRegs<8> { using type = Q80Regs; };
 // (the warp's 16 lanes, first column) of weight stage 0.  A stage holds gs 64-wide groups (gs = 1: K step = group, the
 // warp fills every other pair of K steps; gs = 4: K step = unit, both warps of a row tile fill the same stage).
 // Barrier slot of K step kt: kt % slots; weight stage: kt % na.
-template <int FMT, int HALF, int GS>
+template <int FMT, int HALF, int GS, int PAIR>
 __device__ __forceinline__ bool produce(const GemmParams &p, const uint8_t *ub, bool have, int lane, uint32_t dst, int slots,
                                         uint32_t full0, uint32_t empty0, volatile int *abort_flag, int u0, int units)
 {
-    constexpr int na = GS == 4 ? 3 : kGemmAStages;
+    constexpr int na = GS == 4 ? 3 : PAIR == 2 ? kGemmWideStages : kGemmAStages;
     typename UnitRegs<FMT>::type cur, nxt;
     ub += (size_t)u0 * p.unit_bytes;          // this CTA's K range starts at unit u0
     // Registers hold one unit ahead; one lane of the pair's first warp asks L2 for the units kAhead further on, so
@@ -360,7 +367,10 @@ __device__ __forceinline__ bool produce(const GemmParams &p, const uint8_t *ub, 
             if (!wide || gg == 1) {
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(full0 + 8u * (uint32_t)(kt % slots));
+                if (lane == 0) {                                      // full0: the even CTA's barriers where two CTAs share a tile
+                    if (PAIR) mbar_arrive_cluster(full0 + 8u * (uint32_t)(kt % slots));
+                    else mbar_arrive(full0 + 8u * (uint32_t)(kt % slots));
+                }
             }
         }
     }
@@ -368,7 +378,8 @@ __device__ __forceinline__ bool produce(const GemmParams &p, const uint8_t *ub, 
 }
 
 // ---- the kernel
-template <int FMT, int GS>
+// PAIR: 0 one CTA per tile; 1 two CTAs share a token tile of up to 256; 2 ... of up to 384, as two accumulators
+template <int FMT, int GS, int PAIR>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
 {
@@ -382,10 +393,12 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
     // gs = 4 (token tiles of up to 64 rows): a stage is a whole 256-wide unit - four TMA boxes, sixteen MMAs, one barrier
     // round - because with so little tensor work per group the round itself (arrive, wait, commit, wait) sets the pace.
     // The accumulator then takes columns [0, 64) and three weight stages of 128 columns follow from column 128.
-    constexpr int gs = GS, na = GS == 4 ? 3 : kGemmAStages;
-    constexpr uint32_t tmem_a0 = GS == 4 ? 128u : (uint32_t)kTmemA0;
+    constexpr int gs = GS, na = GS == 4 ? 3 : PAIR == 2 ? kGemmWideStages : kGemmAStages;
+    constexpr int kAcc = PAIR == 2 ? 2 : 1;
+    constexpr uint32_t tmem_a0 = GS == 4 ? 128u : PAIR == 2 ? (uint32_t)kTmemWideA0 : (uint32_t)kTmemA0;
     const int nb = p.nb, slots = max(na, nb);
-    const uint32_t group_b = (uint32_t)p.nt * 128u;                // bytes of one 64-wide activation box (multiple of 2048)
+    const uint32_t box_rows = (uint32_t)p.nt / (PAIR ? 2u : 1u);   // activation rows this CTA brings
+    const uint32_t group_b = box_rows * 128u;                      // bytes of one 64-wide piece of them (multiple of 1024)
     const uint32_t stage_b = group_b * (uint32_t)gs;
     const uint32_t bars = sB + (uint32_t)nb * stage_b;
     // Slot kt % slots serves K step kt.  full: eight producer warps + the TMA thread's expect_tx; empty: the commit
@@ -406,10 +419,11 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
     const int rt = (int)blockIdx.x - (wi ? p.rt_end[wi - 1] : 0);   // 128-row tile inside weight wi
     const int n_rows = p.n[wi];
 
+    const uint32_t rank = PAIR ? cluster_rank() : 0u;             // 0: the CTA that issues the MMAs and owns the full barriers
     if (tid == 0) {
         abort_word = 0;
         for (int i = 0; i < slots; i++) {
-            mbar_init(full_bar(i), gs == 4 ? 17 : 9);    // the producer warps of a stage + the TMA thread's expect_tx
+            mbar_init(full_bar(i), gs == 4 || PAIR ? 17 : 9);    // the producer warps of a stage (of both CTAs) + the TMA thread's expect_tx
             mbar_init(empty_bar(i), 1);
         }
         mbar_init(accum_bar, 1);
@@ -417,13 +431,20 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == kGemmProducers + 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(kTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(kTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(kTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync();               // the other CTA's barriers are there
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    const uint32_t full_lead = PAIR ? cluster_addr(full_bar(0), 0) : full_bar(0);
 
     if (warp < kGemmProducers) {
         // ------------------------------------------------ dequantise the weight tile, stage by stage
@@ -431,11 +452,11 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
         // w + 4 take the two halves of quarter w % 4, and w + 8, w + 12 the same rows' other two 64-groups.
         const int sub = 2 * (warp & 3) + ((warp >> 2) & 1);
         const int tile16 = rt * 8 + sub;
-        const bool have = tile16 < p.n_tiles16[wi];
+        const bool have = tile16 < p.n_tiles16[wi];       // false throughout for the CTA that fills up the last pair
         const uint8_t *ub = p.w[wi] + (size_t)(have ? tile16 : 0) * p.upt * p.unit_bytes;
         const uint32_t dst = tmem + ((uint32_t)(sub * 16) << 16) + tmem_a0;
-        const bool ok = warp < 8 ? produce<FMT, 0, GS>(p, ub, have, lane, dst, slots, full_bar(0), empty_bar(0), abort_flag, u0, u1 - u0)
-                                 : produce<FMT, 1, GS>(p, ub, have, lane, dst, slots, full_bar(0), empty_bar(0), abort_flag, u0, u1 - u0);
+        const bool ok = warp < 8 ? produce<FMT, 0, GS, PAIR>(p, ub, have, lane, dst, slots, full_lead, empty_bar(0), abort_flag, u0, u1 - u0)
+                                 : produce<FMT, 1, GS, PAIR>(p, ub, have, lane, dst, slots, full_lead, empty_bar(0), abort_flag, u0, u1 - u0);
         // ------------------------------------------------ epilogue: tensor memory -> Y[token][row]
         if (ok && mbar_wait(accum_bar, 0, abort_flag, p.err, 22)) {
             tc_fence_after();
@@ -478,23 +499,37 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
                     if (!mbar_wait(empty_bar(bslot), (uint32_t)bround & 1u, abort_flag, p.err, 23)) break;
                     if (++bslot == slots) { bslot = 0; bround++; }
                 }
-                mbar_expect_tx(full_bar(slot), stage_b);
-                for (int j = 0; j < gs; j++)
-                    tma_load_2d(sB + (uint32_t)st * stage_b + (uint32_t)j * group_b, &xmap, (kt_base + kt * gs + j) * kGemmBK, tok0, full_bar(slot));
+                if (PAIR) {
+                    if (rank == 0) mbar_expect_tx(full_bar(slot), 2 * stage_b);      // both CTAs' halves
+#pragma unroll
+                    for (int h = 0; h < kAcc; h++)           // this CTA's half of each accumulator's columns
+                        tma_load_2d_pair(sB + (uint32_t)st * stage_b + (uint32_t)h * (group_b / kAcc), &xmap, (kt_base + kt) * kGemmBK,
+                                         tok0 + h * (p.nt / kAcc) + (int)(rank * (box_rows / kAcc)), full_lead + 8u * (uint32_t)slot);
+                } else {
+                    mbar_expect_tx(full_bar(slot), stage_b);
+                    for (int j = 0; j < gs; j++)
+                        tma_load_2d(sB + (uint32_t)st * stage_b + (uint32_t)j * group_b, &xmap, (kt_base + kt * gs + j) * kGemmBK, tok0, full_bar(slot));
+                }
                 issued = kt + 1;
                 if (++st == nb) st = 0;
                 if (++slot == slots) slot = 0;
             }
             if (*abort_flag) {
-                // let copies that were already requested land before the CTA gives its shared memory back
-                for (int kt = max(0, issued - nb); kt < issued; kt++)
-                    mbar_wait_drain(full_bar(kt % slots), (uint32_t)(kt / slots) & 1u);
+                // let copies that were already requested land before the CTA gives its shared memory back; those of the odd
+                // CTA report to the other one's barriers, so it gives them a millisecond, far more than a copy takes
+                if (PAIR && rank != 0) {
+                    const unsigned long long t0 = global_ns();
+                    while (global_ns() - t0 < 1000000ull) {}
+                } else {
+                    for (int kt = max(0, issued - nb); kt < issued; kt++)
+                        mbar_wait_drain(full_bar(kt % slots), (uint32_t)(kt / slots) & 1u);
+                }
             }
         }
     } else {
         // ------------------------------------------------ MMA issue
-        if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(p.nt >> 3) << 17) | ((uint32_t)(kGemmRows >> 4) << 24);   // f32 D, f16 A/B, K-major both
+        if (lane == 0 && rank == 0) {
+            const uint32_t idesc = (1u << 4) | ((uint32_t)((p.nt / kAcc) >> 3) << 17) | ((uint32_t)((PAIR ? 2 : 1) * kGemmRows >> 4) << 24);   // f32 D, f16 A/B, K-major both
             bool ok = true;
             int st = 0, slot = 0, round = 0;
             for (int kt = 0; kt < KT; kt++) {
@@ -505,21 +540,30 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
                     const uint32_t ta = tmem + tmem_a0 + (uint32_t)((kt % na) * (kStageACols * gs) + j * kStageACols);
 #pragma unroll
                     for (int k16 = 0; k16 < kGemmBK / 16; k16++)   // 16 f16: 8 columns of tensor memory, 32 bytes along the swizzle row
-                        umma_f16_ts(tmem, ta + 8u * k16, bd + 2u * k16, idesc, (kt | j | k16) != 0);
+                        if (PAIR) {
+                            umma_f16_ts_pair(tmem, ta + 8u * k16, bd + 2u * k16, idesc, (kt | j | k16) != 0);
+                            if (kAcc == 2) umma_f16_ts_pair(tmem + (uint32_t)(p.nt / 2), ta + 8u * k16, bd + (group_b >> 5) + 2u * k16, idesc, (kt | k16) != 0);
+                        } else {
+                            umma_f16_ts(tmem, ta + 8u * k16, bd + 2u * k16, idesc, (kt | j | k16) != 0);
+                        }
                 }
-                umma_commit(empty_bar(slot));   // arrives when the MMAs above have read both stages
+                if (PAIR) umma_commit_pair(empty_bar(slot));
+                else umma_commit(empty_bar(slot));   // arrives when the MMAs above have read both stages
                 if (++st == nb) st = 0;
                 if (++slot == slots) { slot = 0; round++; }
             }
-            umma_commit(accum_bar);
+            if (PAIR) umma_commit_pair(accum_bar);
+            else umma_commit(accum_bar);
             if (!ok) mbar_wait_drain(accum_bar, 0);   // MMAs already issued finish before the tensor memory is freed
         }
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync();               // neither CTA's memory goes while the other's MMAs, copies or arrivals may reach it
     if (warp == kGemmProducers + 1) {
         __syncwarp();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
     }
 }
 
@@ -1159,15 +1203,40 @@ __global__ void __launch_bounds__(NT) x_to_f16_kernel(const float *__restrict__ 
     if (threadIdx.x == 0) inv_scale[blockIdx.x] = inv;
 }
 
-// Activation rows per CTA: up to 128 rows one tile; above, 256-row tiles if they give every SM work, else 128-row
-// ones (more, smaller CTAs).
-int pick_token_tile(int64_t m, int64_t n, int sms)
+// How a GEMM is cut: tiles of nt activation rows, by one CTA or a pair, and `splits` ranges of K.
+struct GemmPlan { int nt, pair, splits; };
+
+// Up to 128 rows: one tile.  Above: pairs of CTAs, whose tiles may have up to 384 rows.  With few rows per tile its time is
+// its K length - the dequantising warps set the pace, 0.47 to 0.49 us for a 64-wide step of up to 256 rows, and with two
+// accumulators, beside which fewer weight stages fit, 0.67 us for up to 384 - so fewer, wider tiles do the same work in fewer
+// steps, until they leave SMs idle; splitting K fills those, at the price of a second pass over splits x m x n partial sums.
+// The plan is the cheapest by this model (a pure function of its arguments).
+GemmPlan plan_gemm(int64_t m, int64_t row_tiles, int64_t units, int64_t n_all, int sms)
 {
-    const int64_t row_tiles = (n + kGemmRows - 1) / kGemmRows;
-    if (m <= 128) return (int)((m + 15) / 16 * 16);
-    const int64_t ctas256 = row_tiles * ((m + 255) / 256);
-    if (ctas256 >= sms) return 256;
-    return 128;
+    auto us = [&](int64_t tok_tiles, int nt, int pair, int s) {
+        const int64_t ctas = row_tiles * tok_tiles * s, waves = (ctas + sms - 1) / sms, len = (units + s - 1) / s;
+        const double step = nt > 256 ? 0.67 : 0.45 + nt * 0.00016;
+        double t = (double)waves * ((double)len * 4.0 * step + 2.0 + nt * 0.008) + (pair ? 1.0 : 0.0);   // + fill and drain, the read-back
+        if (s > 1) t += 5.0 + (double)(s * m * n_all) * 8.0 / 2.5e6;      // the summing launch: its latency + partials written and read
+        return t;
+    };
+    GemmPlan best = {};
+    double best_us = 1e30;
+    auto consider = [&](int64_t tok_tiles, int nt, int pair, int s) {
+        const double t = us(tok_tiles, nt, pair, s);
+        if (t < best_us * 0.97) { best_us = t; best = {nt, pair, s}; }
+    };
+    if (m <= 128) {
+        const int nt = (int)((m + 15) / 16 * 16);
+        for (int s = 1; s <= 16 && (s == 1 || (s * 4 <= units && units >= 8)); s++) consider(1, nt, 0, s);
+        return best;
+    }
+    for (int64_t t = (m + 383) / 384; t <= (m + 95) / 96 && t <= (m + 383) / 384 + 3; t++) {
+        int nt = (int)(((m + t - 1) / t + 31) / 32 * 32);       // MMAs over two CTAs take their columns in steps of 32, two of them 64
+        if (nt > 256) nt = (nt + 63) / 64 * 64;
+        for (int s = 1; s <= 8 && (s == 1 || s * 4 <= units); s++) consider((m + nt - 1) / nt, nt, 1, s);
+    }
+    return best;
 }
 
 }  // namespace
@@ -1175,42 +1244,36 @@ int pick_token_tile(int64_t m, int64_t n, int sms)
 bool qgemm_supported(int type) { return type == 12 || type == 14 || type == 2 || type == 8; }
 
 namespace {
-template <int FMT, int GS>
+template <int FMT, int GS, int PAIR>
 tlb_status launch_fmt_gemm_gs(dim3 grid, size_t smem, cudaStream_t stream, const CUtensorMap &map, const GemmParams &p)
 {
     static bool attr_set = false;
     if (!attr_set) {
-        TLB_CUDA(cudaFuncSetAttribute(qgemm_kernel<FMT, GS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemMax));
+        TLB_CUDA(cudaFuncSetAttribute(qgemm_kernel<FMT, GS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemMax));
         attr_set = true;
     }
-    qgemm_kernel<FMT, GS><<<grid, kGemmThreads, smem, stream>>>(map, p);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = PAIR ? 1 : 0;
+    TLB_CUDA(cudaLaunchKernelEx(&cfg, qgemm_kernel<FMT, GS, PAIR>, map, p));
     return TLB_OK;
 }
 template <int FMT>
 tlb_status launch_fmt_gemm(dim3 grid, size_t smem, cudaStream_t stream, const CUtensorMap &map, const GemmParams &p)
 {
-    return p.gs == 4 ? launch_fmt_gemm_gs<FMT, 4>(grid, smem, stream, map, p) : launch_fmt_gemm_gs<FMT, 1>(grid, smem, stream, map, p);
+    if (p.gs == 4) return launch_fmt_gemm_gs<FMT, 4, 0>(grid, smem, stream, map, p);
+    if (!p.pair) return launch_fmt_gemm_gs<FMT, 1, 0>(grid, smem, stream, map, p);
+    return p.nt > 256 ? launch_fmt_gemm_gs<FMT, 1, 2>(grid, smem, stream, map, p) : launch_fmt_gemm_gs<FMT, 1, 1>(grid, smem, stream, map, p);
 }
 }  // namespace
-
-// K-splits for m activation rows on `tiles` 128-row tiles of `units` 256-wide K units, n_all output columns in all.
-// With few token rows a tile's time is its K length (the dequantising warps set the pace), so the launch costs
-// waves x units-per-split; a split count is worth its second pass over s x m x n_all partial sums when it evens out
-// the last wave or fills idle SMs.  Returns the count with the least estimated time (1 = no split).
-int qgemm_k_splits(int64_t m, int64_t tiles, int64_t units, int64_t n_all, int sm_count)
-{
-    if (m > 64 || units < 8) return 1;
-    const double us_per_unit = 1.8;                                         // 4 K steps of ~0.45 us
-    int best = 1;
-    double best_us = 1e30;
-    for (int s = 1; s <= 16 && s * 4 <= units; s++) {
-        const int64_t waves = (tiles * s + sm_count - 1) / sm_count, len = (units + s - 1) / s;
-        double us = (double)(waves * len) * us_per_unit + (double)waves * 2.0;   // + fill and drain of every wave
-        if (s > 1) us += 4.0 + (double)(s * m * n_all) * 8.0 / 3.0e6;       // the summing launch: its latency + partials written and read
-        if (us < best_us - 0.5) { best_us = us; best = s; }
-    }
-    return best;
-}
 
 tlb_status qgemm_prepare(GemmAct *a, const float *x, const float *x2, int64_t m, int64_t k, const float *norm_w, float eps)
 {
@@ -1359,12 +1422,12 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
     if (!qgemm_supported(w0->type)) return fail(TLB_ERR_TYPE, "tensor-core GEMM: GGML type %d is not supported", w0->type);
     if (qrows_rows(a.m)) return qrows_run(ws, n_w, a, outs, resid);
     GemmParams p;
-    int64_t row_tiles = 0, n_max = 0;
+    int64_t row_tiles = 0;
     for (int i = 0; i < kGemmMaxW; i++) {
         const tlb_qtensor *w = i < n_w ? ws[i] : nullptr;
         if (w && (w->type != w0->type || w->k != a.k || w->n > INT32_MAX))
             return fail(TLB_ERR_SHAPE, "tensor-core GEMM: weight K %lld vs activation K %lld, or mixed types", (long long)w->k, (long long)a.k);
-        if (w) { row_tiles += (w->n + kGemmRows - 1) / kGemmRows; n_max = std::max(n_max, row_tiles * kGemmRows); }
+        if (w) row_tiles += (w->n + kGemmRows - 1) / kGemmRows;
         p.w[i] = w ? w->dev() : nullptr;
         p.out[i] = w ? outs[i] : nullptr;
         p.n[i] = w ? (int)w->n : 0;
@@ -1374,11 +1437,15 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
     auto encode = tensor_map_encoder();
     if (!encode) return fail(TLB_ERR_DEVICE, "cuTensorMapEncodeTiled is not available from this driver");
     const int64_t m = a.m;
-    const int nt = pick_token_tile(m, n_max, c->sm_count);
+    int64_t n_all = 0;
+    for (int i = 0; i < kGemmMaxW; i++) { p.col0[i] = (int)n_all; n_all += p.n[i]; }
+    const GemmPlan plan = plan_gemm(m, row_tiles, w0->upt, n_all, c->sm_count);
+    const int nt = plan.nt, splits = plan.splits;
+    const bool pair = plan.pair;
     CUtensorMap map;
     const cuuint64_t dims[2] = {(cuuint64_t)a.k, (cuuint64_t)m};
     const cuuint64_t strides[1] = {(cuuint64_t)a.k * sizeof(__half)};
-    const cuuint32_t box[2] = {(cuuint32_t)kGemmBK, (cuuint32_t)nt};
+    const cuuint32_t box[2] = {(cuuint32_t)kGemmBK, (cuuint32_t)(!pair ? nt : nt > 256 ? nt / 4 : nt / 2)};
     const cuuint32_t estr[2] = {1, 1};
     CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.xh->ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1388,19 +1455,18 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
     p.upt = w0->upt;
     p.m = (int)m;
     p.nt = nt;
-    p.gs = nt <= 64 ? 4 : 1;
-    p.nb = std::max(p.gs == 4 ? 3 : 4, std::min(kGemmMaxSlots, kGemmBBytes / (nt * 128 * p.gs)));
+    p.pair = pair;
+    p.gs = !pair && nt <= 64 ? 4 : 1;
+    const int stage_b = (pair ? nt / 2 : nt) * 128 * p.gs;
+    p.nb = std::max(p.gs == 4 ? 3 : 4, std::min(kGemmMaxSlots, kGemmBBytes / stage_b));
     p.kt_total = (int)(a.k / kGemmBK);
     p.unit_bytes = qformat(w0->type)->unit_bytes;
     p.inv_scale = (const float *)a.inv->ptr;
     p.resid = resid;
     p.err = c->err_flag;
 
-    const size_t smem = (size_t)p.nb * nt * 128 * p.gs + (kGemmSmemMax - kGemmBBytes);
+    const size_t smem = (size_t)p.nb * stage_b + (kGemmSmemMax - kGemmBBytes);
     const int64_t tok_tiles = (m + nt - 1) / nt;
-    int64_t n_all = 0;
-    for (int i = 0; i < kGemmMaxW; i++) { p.col0[i] = (int)n_all; n_all += p.n[i]; }
-    const int splits = qgemm_k_splits(m, row_tiles * tok_tiles, p.upt, n_all, c->sm_count);
     Storage *part = nullptr;
     if (splits > 1) {
         part = storage_alloc((size_t)splits * m * n_all * sizeof(float));
@@ -1409,7 +1475,7 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
     p.splits = splits;
     p.part = part ? (float *)part->ptr : nullptr;
     p.n_all = (int)n_all;
-    dim3 grid((unsigned)row_tiles, (unsigned)tok_tiles, (unsigned)splits);
+    dim3 grid((unsigned)(pair ? (row_tiles + 1) / 2 * 2 : row_tiles), (unsigned)tok_tiles, (unsigned)splits);
     tlb_status ls;
     switch (w0->type) {
         case 12: ls = launch_fmt_gemm<12>(grid, smem, c->stream, map, p); break;

@@ -125,9 +125,6 @@ namespace tlb {
 // in tensor memory; up to 16 rows: a streaming kernel on mma.sync)
 bool qgemm_supported(int ggml_type);
 tlb_status launch_qgemm(const tlb_qtensor *w, const float *x, int64_t m, float *out);
-// K-splits the tensor-core GEMM uses for m activation rows on `tiles` row tiles of `units` 256-wide K units each and
-// n_all output columns (1 = none)
-int qgemm_k_splits(int64_t m, int64_t tiles, int64_t units, int64_t n_all, int sm_count);
 // activation row counts that qgemm_run_multi hands to its streaming kernel for few rows instead of the tensor-memory GEMM
 bool qrows_rows(int64_t m);
 // the same in steps, so that several weights can share one conversion of the activations:
