@@ -277,7 +277,6 @@ tlb_status enqueue_head(tlb_decoder *d, const float *ssq_parts, const float *x =
         j.prologue = PRO_ADD_NORM; j.x = x ? x : d->xb; j.x2 = x2; j.x_out = x_out;
         j.ssq_parts = ssq_parts; j.n_parts = ssq_parts ? (dm + 15) / 16 : 0;
         j.norm_w = d->out_norm->f32(); j.eps = c.eps;
-        j.last_of_chain = true;
         j.pdl = d->pdl && (!x2 || d->tp_pdl_ar);     // behind an NCCL collective: a plain stream dependency
         j.dry_run = d->dry;
         TLB_TRY(launch_qmatvec(j));
@@ -1139,7 +1138,6 @@ tlb_status tlb_decoder_time_kernel(tlb_decoder *d, const char *which, int copies
             j.n_w = 1; set_w(j, 0, lw.down, o); j.type = lw.down->type; j.k = F; bytes = lw.down->nbytes();
         } else {
             j.n_w = 1; set_w(j, 0, d->head, o); j.type = d->head->type; j.k = dm; bytes = d->head->nbytes();
-            j.last_of_chain = true;
         }
         j.pdl = d->pdl;   // as in the decode chain: a launch's set-up overlaps its predecessor
         st = launch_qmatvec(j);

@@ -43,8 +43,6 @@ namespace tlb {
 
 constexpr int kWarps = 16;
 constexpr int kThreads = kWarps * 32;
-constexpr int kCtasPerSm = 1;       // CTAs a launch brings per SM
-constexpr int kResidentPerSm = 1;   // CTAs the register and shared-memory budgets allow per SM
 
 struct ItemRef {
     const uint8_t *src;   // first unit of the item
@@ -58,7 +56,7 @@ struct ItemCursor { int slice, tile; };
 __device__ __forceinline__ ItemCursor cursor_at(const MvParams &p, int item)
 {
     ItemCursor c;
-    c.slice = item / p.tiles;
+    c.slice = p.div_tiles(item);
     c.tile = item - c.slice * p.tiles;
     return c;
 }
@@ -148,10 +146,15 @@ __device__ __forceinline__ float tp_sum_tile(const MvParams &p, unsigned seq, in
     return a;
 }
 
-template <int FMT>
-__global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const __grid_constant__ MvParams p)
+// ONE: one activation row.  What bounds a short launch is the 900 or so instructions a warp issues outside its units, 16 warps
+// deep; with the row count known at compile time and the divisions replaced (Divider) a decode step of the TinyLlama shapes
+// (111 launches) takes 761 us instead of 848, one of eight Llama-3-8B layers and head 510 instead of 551, a lone
+// 2048 x 2048 call 12.3 instead of 13.4.
+template <int FMT, bool ONE>
+__global__ void __launch_bounds__(kThreads, 1) qmatvec_kernel(const __grid_constant__ MvParams p)
 {
     extern __shared__ __align__(128) uint8_t smem[];
+    const int M = ONE ? 1 : p.m, NL = ONE ? 3 : p.nl;      // activation rows and int8 levels of each
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     MvShared *sh = reinterpret_cast<MvShared *>(smem + p.off_misc);
     const int spw = p.spw;
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const
     const int wu1 = local ? cta_units * (warp + 1) / kWarps : (nci * (warp + 1) / kWarps) * p.upi;
     const int n_units = wu1 - wu0;
     // activation blocks the CTA's items cover
-    const int s_first = nci > 0 ? ci0 / p.tiles : 0, s_last = nci > 0 ? (ci1 - 1) / p.tiles : 0;
+    const int s_first = nci > 0 ? p.div_tiles(ci0) : 0, s_last = nci > 0 ? p.div_tiles(ci1 - 1) : 0;
     const int blk0 = s_first * p.upi, nb = nci > 0 ? (s_last + 1) * p.upi - blk0 : 0;
 
     // Ring set-up, one lane per stage so that it takes one round of latencies instead of `spw`:
@@ -186,7 +189,7 @@ __global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         if (lane < n_first) {
-            const int g = wu0 + lane, it = g / p.upi, uo = g - it * p.upi;
+            const int g = wu0 + lane, it = p.div_upi(g), uo = g - it * p.upi;
             first_src = item_ref(p, cursor_at(p, ci0 + it)).src + (size_t)uo * p.unit_bytes;
             if (lane < kEarly) {
                 mbar_expect_tx(bars + lane * 8, p.unit_bytes);
@@ -202,7 +205,7 @@ __global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const
     const uint8_t *pf_src = nullptr;
     ItemCursor pf_cur;
     {
-        const int g = wu0 + n_first, it = g / p.upi, uo = g - it * p.upi;
+        const int g = wu0 + n_first, it = p.div_upi(g), uo = g - it * p.upi;
         pf_cur = cursor_at(p, ci0 + it);
         if (uo && pf_remaining > 0) {   // in the middle of an item
             pf_src = item_ref(p, pf_cur).src + (size_t)uo * p.unit_bytes;
@@ -228,7 +231,7 @@ __global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const
     }
     const unsigned tp_seq = p.tp_reduce ? ld_volatile_u32(p.tp.seq) : 0u;   // the launch before has completed: its exchange is over
     __syncthreads();               // abort_flag initialised; also keeps the CTA together for the prologue
-    build_activation<FMT>(p, sh, smem, tid, kThreads, blk0, nb, wgt_first, [&](float dep) {
+    build_activation<FMT, ONE>(p, sh, smem, tid, kThreads, blk0, nb, wgt_first, [&](float dep) {
         // the rest of the ring's first round; the test on `dep` only ties the requests to the arrival of the loads
         if (lane >= kEarly && lane < n_first && __float_as_uint(dep) != 0x7fedcba9u) {
             mbar_expect_tx(bars + lane * 8, p.unit_bytes);
@@ -237,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const
     });
     volatile int *abortp = &sh->abort_flag;
 
-    const int ncols = p.m * p.nl;
+    const int ncols = M * NL;
     LaneCtx L;
     L.lane = lane; L.r = lane >> 2; L.c = lane & 3;
     {
@@ -245,18 +248,18 @@ __global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const
         const int colr = r < ncols ? r : 0, c0 = 2 * c < ncols ? 2 * c : 0, c1 = 2 * c + 1 < ncols ? 2 * c + 1 : 0;
         L.xq_b = smem_u32(smem + p.off_xq) + colr * p.col_stride;
         L.alam_b = smem_u32(smem + p.off_alam) + 2 * c * 4;
-        L.xsum_b = smem_u32(smem + p.off_xsum) + ((r < 2 * p.m) ? r : (r & 1)) * (p.nb_max * 8) * 2;
+        L.xsum_b = smem_u32(smem + p.off_xsum) + ((r < 2 * M) ? r : (r & 1)) * (p.nb_max * 8) * 2;
         L.sa_b = smem_u32(smem + p.off_sa) + colr * 32;
         L.sa_c0 = smem_u32(smem + p.off_sa) + c0 * 4;
         L.sa_c1 = smem_u32(smem + p.off_sa) + c1 * 4;
-        L.minv_b = smem_u32(smem + p.off_minv) + (c < p.m ? c : 0) * 4;
+        L.minv_b = smem_u32(smem + p.off_minv) + (c < M ? c : 0) * 4;
     }
     float *segbuf = reinterpret_cast<float *>(smem + p.off_seg);   // local mode: [warp][run][16 * m] partial results
 
     int stage = 0, phase = 0, consumed = 0;
     bool ok = true;
     int remaining = n_units, seg = 0;
-    const int it0 = wu0 / p.upi;
+    const int it0 = p.div_upi(wu0);
     int uo0 = wu0 - it0 * p.upi;          // the first run may start inside an item (local mode)
     ItemCursor cur = cursor_at(p, ci0 + it0);
     while (remaining > 0 && ok) {
@@ -301,10 +304,10 @@ __global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const
         // Fold the level columns of each activation row (they sit in the four lanes of a quad).  The
         // Q4_K min term of activation row mi lives in lane c == mi.  The 16 * m partial results of the run
         // go to this warp's slot in shared memory (local mode) or to the item's slot of the slice scratch.
-        float *part = local ? segbuf + ((size_t)warp * p.max_seg + seg) * (16 * p.m)
-                            : p.part + ((size_t)ir.slice * p.tiles + ir.tile) * (16 * p.m);
-        for (int mi = 0; mi < p.m; mi++) {
-            const int lo = mi * p.nl, hi = lo + p.nl, cA = 2 * L.c, cB = 2 * L.c + 1;
+        float *part = local ? segbuf + ((size_t)warp * p.max_seg + seg) * (16 * M)
+                            : p.part + ((size_t)ir.slice * p.tiles + ir.tile) * (16 * M);
+        for (int mi = 0; mi < M; mi++) {
+            const int lo = mi * NL, hi = lo + NL, cA = 2 * L.c, cB = 2 * L.c + 1;
             const bool inA = cA >= lo && cA < hi, inB = cB >= lo && cB < hi;
             float v0 = (inA ? master[0] : 0.f) + (inB ? master[1] : 0.f);   // row r
             float v1 = (inA ? master[2] : 0.f) + (inB ? master[3] : 0.f);   // row r + 8
@@ -346,9 +349,9 @@ __global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const
                 for (int w = 0; w < kWarps; w++) {
                     const int b0 = cta_units * w / kWarps, b1 = cta_units * (w + 1) / kWarps;
                     if (b1 <= a0 || b0 >= a1 || b1 == b0) continue;
-                    const float *sp = segbuf + ((size_t)w * p.max_seg + (tl - b0 / p.upi)) * (16 * p.m);
-                    if (lane < 16 * p.m) acc0 += sp[lane];
-                    if (lane + 32 < 16 * p.m) acc1 += sp[lane + 32];
+                    const float *sp = segbuf + ((size_t)w * p.max_seg + (tl - p.div_upi(b0))) * (16 * M);
+                    if (lane < 16 * M) acc0 += sp[lane];
+                    if (lane + 32 < 16 * M) acc1 += sp[lane + 32];
                 }
                 ItemCursor cf;
                 cf.slice = 0;
@@ -360,8 +363,8 @@ __global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const
                     float *out = p.out[fr.wi];
                     const int nrows = p.n_rows[fr.wi];
                     const int g = fr.row0 + (lane & 15);
-                    if (lane < 16 * p.m && g < nrows) out[(size_t)(lane >> 4) * nrows + g] = acc0;
-                    if (lane + 32 < 16 * p.m && g < nrows) out[(size_t)((lane >> 4) + 2) * nrows + g] = acc1;
+                    if (lane < 16 * M && g < nrows) out[(size_t)(lane >> 4) * nrows + g] = acc0;
+                    if (lane + 32 < 16 * M && g < nrows) out[(size_t)((lane >> 4) + 2) * nrows + g] = acc1;
                 } else {
                     finish_rows(fr, acc0);
                 }
@@ -378,12 +381,12 @@ __global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const
                 }
             }
         }
-    } else if (ok && wu1 > wu0 && p.fold_poll) {
+    } else if (ONE && ok && wu1 > wu0 && p.fold_poll) {
         // One activation row.  The slice scratch rests at kFoldEmpty between launches, so a value that is not kFoldEmpty is
         // a slice that has arrived: the warp that owns slice 0 of a tile reads the tile's slices (all requested at once,
         // re-read while some are missing; bounded), adds them in slice order, puts kFoldEmpty back and writes the rows.
         // No fence, counter or atomic: a 4-byte store is indivisible, and the next launch starts after this one is over.
-        const int i0 = ci0 + it0, i1 = ci0 + wu1 / p.upi;
+        const int i0 = ci0 + it0, i1 = ci0 + p.div_upi(wu1);
         const size_t sstride = (size_t)p.tiles * 16;
         for (int item = i0; item < i1 && item < p.tiles; item++) {     // items below `tiles` are slice 0
             ItemCursor cf;
@@ -436,7 +439,7 @@ __global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const
         // item j); the warp that completes a tile's last K-slice adds the slices in index order and
         // writes the output rows, so the sum is the same whichever warp does it.  It also clears the
         // tile's counter for the next launch on this stream.
-        const int i0 = ci0 + it0, i1 = ci0 + wu1 / p.upi;
+        const int i0 = ci0 + it0, i1 = ci0 + p.div_upi(wu1);
         __threadfence();                                      // our slices are visible before the counts say so
         __syncwarp();
         for (int base = i0; base < i1; base += 32) {
@@ -454,10 +457,10 @@ __global__ void __launch_bounds__(kThreads, kResidentPerSm) qmatvec_kernel(const
                 const ItemRef fr = item_ref(p, cf);
                 float *out = p.out[fr.wi];
                 const int nrows = p.n_rows[fr.wi];
-                const float *src = p.part + (size_t)fr.tile * (16 * p.m);
-                const size_t sstride = (size_t)p.tiles * (16 * p.m);
+                const float *src = p.part + (size_t)fr.tile * (16 * M);
+                const size_t sstride = (size_t)p.tiles * (16 * M);
                 if (p.finish == FIN_PLAIN && !tpr) {
-                    for (int e = lane; e < 16 * p.m; e += 32) {
+                    for (int e = lane; e < 16 * M; e += 32) {
                         float a = __ldcg(src + e);
                         for (int s = 1; s < p.kb; s++) a += __ldcg(src + s * sstride + e);
                         const int mi = e >> 4, g = fr.row0 + (e & 15);
@@ -549,7 +552,7 @@ static double slice_cost(int type, int m, int64_t tiles, int upt, int upi, int s
 {
     const int kb = upt / upi;
     const int64_t n_items = tiles * kb;
-    const int grid = (int)std::min<int64_t>((int64_t)sm_count * kCtasPerSm, n_items);
+    const int grid = (int)std::min<int64_t>(sm_count, n_items);
     const int64_t ipc = (n_items + grid - 1) / grid, ipw = (ipc + kWarps - 1) / kWarps;
     const int nb = blocks_per_cta(n_items, grid, tiles, upi, upt);
     const double unit = type == TLB_GGML_Q6_K ? 300.0 : type == TLB_GGML_Q8_0 ? 150.0 : 210.0;
@@ -584,8 +587,8 @@ int qmatvec_plan_slices(int type, int64_t k, int m, int64_t tiles, int max_slice
     return best;
 }
 
-template <int FMT>
-static tlb_status launch_fmt(const MvParams &p, int grid, size_t smem, bool pdl)
+template <int FMT, bool ONE>
+static tlb_status launch_fmt_rows(const MvParams &p, int grid, size_t smem, bool pdl)
 {
     // Function attributes are set once, to their final values, before the first launch: a graph whose
     // kernel nodes were captured while the limit was still growing replayed 25 % slower than the same
@@ -593,8 +596,8 @@ static tlb_status launch_fmt(const MvParams &p, int grid, size_t smem, bool pdl)
     // that SMs do not re-partition between launches.
     static bool prepared = false;
     if (!prepared) {
-        TLB_CUDA(cudaFuncSetAttribute(qmatvec_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx()->smem_optin));
-        TLB_CUDA(cudaFuncSetAttribute(qmatvec_kernel<FMT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        TLB_CUDA(cudaFuncSetAttribute((qmatvec_kernel<FMT, ONE>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx()->smem_optin));
+        TLB_CUDA(cudaFuncSetAttribute((qmatvec_kernel<FMT, ONE>), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         prepared = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -611,9 +614,15 @@ static tlb_status launch_fmt(const MvParams &p, int grid, size_t smem, bool pdl)
     }
     cfg.attrs = at;
     cfg.numAttrs = na;
-    TLB_CUDA(cudaLaunchKernelEx(&cfg, qmatvec_kernel<FMT>, p));
+    TLB_CUDA(cudaLaunchKernelEx(&cfg, (qmatvec_kernel<FMT, ONE>), p));
     count_launch();
     return TLB_OK;
+}
+
+template <int FMT>
+static tlb_status launch_fmt(const MvParams &p, int grid, size_t smem, bool pdl)
+{
+    return p.m == 1 ? launch_fmt_rows<FMT, true>(p, grid, smem, pdl) : launch_fmt_rows<FMT, false>(p, grid, smem, pdl);
 }
 
 tlb_status launch_qmatvec(const MatvecJob &job)
@@ -659,20 +668,16 @@ tlb_status launch_qmatvec(const MatvecJob &job)
     p.tile_cnt = c->mv_cnt;
     p.tiles = (int)tiles;
     p.n_items = (int)(tiles * p.kb);
+    p.div_tiles = Divider((uint32_t)p.tiles);
+    p.div_upi = Divider((uint32_t)p.upi);
     p.unit_bytes = f->unit_bytes;
     p.stage_bytes = stage_bytes_of(f);
-    const int grid = (int)std::min<int64_t>((int64_t)c->sm_count * kCtasPerSm, p.n_items);
+    const int grid = (int)std::min<int64_t>(c->sm_count, p.n_items);
     p.ipc_q = p.n_items / grid;
     p.ipc_r = p.n_items % grid;
     p.nb_max = blocks_per_cta(p.n_items, grid, tiles, p.upi, p.upt);
     const SmemPlan sp = plan_smem(job.type, job.m, p.nl, p.nb_max);
-    // Shared memory per CTA: a third of the SM (1 KB per CTA is reserved by the system), so that a CTA of
-    // the next kernel can be resident beside this launch's two; a launch nothing worthwhile follows may
-    // take half, and a shape whose tables need more takes what it needs.
-    const size_t sm_total = c->smem_optin + 1024;
-    size_t budget = sm_total / (job.last_of_chain ? kCtasPerSm : kResidentPerSm) - 1024;
-    if (sp.fixed + 128 + 2 * (size_t)kWarps * (p.stage_bytes + 8) > budget) budget = sm_total / kCtasPerSm - 1024;
-    if (sp.fixed + 128 + 2 * (size_t)kWarps * (p.stage_bytes + 8) > budget) budget = c->smem_optin;
+    const size_t budget = c->smem_optin;                  // one CTA per SM
     const size_t per_stage = (size_t)kWarps * (p.stage_bytes + 8);
     if (sp.fixed + 128 + 2 * per_stage > budget)
         return fail(TLB_ERR_SHAPE, "K = %lld with %d rows needs more shared memory than one SM has (max K %zu)",

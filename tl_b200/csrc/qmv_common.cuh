@@ -156,6 +156,19 @@ __device__ __forceinline__ void imma16832(int (&d)[4], uint32_t a0, uint32_t a1,
 
 // ---------------------------------------------------------------- kernel parameters
 
+// Division by a launch constant without the division: exact for 0 <= n < 2^31 (Granlund and Montgomery, "Division by invariant
+// integers using multiplication", 1994).  A warp of a short launch did eight divisions of some 25 instructions each.
+struct Divider {
+    uint32_t mul = 0, shift = 0;
+    Divider() = default;
+    explicit Divider(uint32_t d)
+    {
+        while ((1ull << shift) < d) shift++;
+        mul = (uint32_t)((((1ull << shift) - d) << 32) / d + 1);
+    }
+    __device__ __forceinline__ int operator()(int n) const { return (int)((__umulhi((uint32_t)n, mul) + (uint32_t)n) >> shift); }
+};
+
 struct MvParams {
     const uint8_t *w[3];
     float *out[3];            // [m][n_rows] per tensor
@@ -179,6 +192,7 @@ struct MvParams {
     int kb;                   // K-slices = output slices = upt / upi
     int tiles;                // tiles of the launch (all tensors)
     int n_items;              // kb * tiles
+    Divider div_tiles, div_upi;
     int ipc_q, ipc_r;         // n_items = grid * ipc_q + ipc_r: CTA b takes ipc_q (+1 if b < ipc_r) consecutive items
     int nb_max;               // 256-blocks of activation a CTA may need: the shared tables are sized for it
     int unit_bytes, stage_bytes;

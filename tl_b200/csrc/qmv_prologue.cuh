@@ -31,10 +31,11 @@ __device__ __forceinline__ float warp_absmax(const float4 v)
     return mx;
 }
 
-template <int FMT>
+template <int FMT, bool ONE>
 __device__ __forceinline__ void quantise_block(const MvParams &p, uint8_t *smem, const float amax, const float4 v,
                                                int mrow, int lb, int j, int lane)
 {
+    const int M = ONE ? 1 : p.m, NL = ONE ? 3 : p.nl;
     // blocks whose largest magnitude is below 2^-100 (or not finite) quantise to zero levels: their
     // contribution is below f32 resolution of any realistic result, and 1 / alpha stays finite
     const float alpha = (amax > 7.9e-31f && amax < 3.0e38f) ? amax * (1.f / 127.f) : 1.f;
@@ -44,7 +45,7 @@ __device__ __forceinline__ void quantise_block(const MvParams &p, uint8_t *smem,
     float lsum[3] = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int l = 0; l < 3; l++) {
-        if (l < p.nl) {
+        if (l < NL) {
             uint32_t tb[4];
 #pragma unroll
             for (int e = 0; e < 4; e++) {
@@ -66,15 +67,15 @@ __device__ __forceinline__ void quantise_block(const MvParams &p, uint8_t *smem,
     const int off = lb * 256 + G * 64 + (t & 3) * 16 + (t >> 3) * 8 + ((t >> 2) & 1) * 4;
 #pragma unroll
     for (int l = 0; l < 3; l++)
-        if (l < p.nl) *reinterpret_cast<uint32_t *>(smem + p.off_xq + (size_t)(mrow * p.nl + l) * p.col_stride + off) = words[l];
+        if (l < NL) *reinterpret_cast<uint32_t *>(smem + p.off_xq + (size_t)(mrow * NL + l) * p.col_stride + off) = words[l];
     if (j < kMaxCols) {   // alam[lb][0..7]: this row's levels; other rows' columns are written by their own groups
-        const int col = j, l = col - mrow * p.nl;
+        const int col = j, l = col - mrow * NL;
         float *alam = reinterpret_cast<float *>(smem + p.off_alam);
-        if (l >= 0 && l < p.nl) {
+        if (l >= 0 && l < NL) {
             float a = alpha;
             for (int i = 0; i < l; i++) a *= (1.f / 254.f);
             alam[lb * kMaxCols + col] = a;
-        } else if (col >= p.m * p.nl && mrow == 0) {
+        } else if (col >= M * NL && mrow == 0) {
             alam[lb * kMaxCols + col] = 0.f;   // unused columns
         }
     }
@@ -103,23 +104,23 @@ __device__ __forceinline__ void quantise_block(const MvParams &p, uint8_t *smem,
         __half *sa = reinterpret_cast<__half *>(smem + p.off_sa);
 #pragma unroll
         for (int l = 0; l < 3; l++)
-            if (l < p.nl) {
+            if (l < NL) {
                 float s = lsum[l];
                 s += __shfl_xor_sync(0xffffffffu, s, 1);
                 s += __shfl_xor_sync(0xffffffffu, s, 2);
-                if ((lane & 3) == 0) sa[((size_t)lb * kMaxCols + mrow * p.nl + l) * 16 + (j >> 2)] = __float2half_rn(s);
+                if ((lane & 3) == 0) sa[((size_t)lb * kMaxCols + mrow * NL + l) * 16 + (j >> 2)] = __float2half_rn(s);
             }
     }
     if (FMT == TLB_GGML_Q4_0) {   // level sums over blocks of 32 = 8 consecutive lanes, int32; [lb*8 + j/8][8 cols]
         int *sa = reinterpret_cast<int *>(smem + p.off_sa);
 #pragma unroll
         for (int l = 0; l < 3; l++)
-            if (l < p.nl) {
+            if (l < NL) {
                 float s = lsum[l];
                 s += __shfl_xor_sync(0xffffffffu, s, 1);
                 s += __shfl_xor_sync(0xffffffffu, s, 2);
                 s += __shfl_xor_sync(0xffffffffu, s, 4);
-                if ((lane & 7) == 0) sa[(size_t)(lb * 8 + (j >> 3)) * kMaxCols + mrow * p.nl + l] = __float2int_rn(s);
+                if ((lane & 7) == 0) sa[(size_t)(lb * 8 + (j >> 3)) * kMaxCols + mrow * NL + l] = __float2int_rn(s);
             }
     }
 }
@@ -151,13 +152,14 @@ __device__ __forceinline__ void load_norm_weights(const MvParams &p, int tid, in
     }
 }
 
-template <int FMT, typename AfterLoads>
+// ONE: one activation row (three levels); its blocks are the items, no division tells them apart.
+template <int FMT, bool ONE, typename AfterLoads>
 __device__ void build_activation(const MvParams &p, MvShared *sh, uint8_t *smem, int tid, int nthreads, int blk0, int nb,
                                  const float4 (&wgt_first)[kKeep], AfterLoads after_loads)
 {
     const int lane = tid & 31, warp = tid >> 5, nwarps = nthreads >> 5;
     const int ngroups = nthreads >> 6, grp = tid >> 6, j = tid & 63;
-    const int nblk = p.k / 256, n_mine = p.m * nb;
+    const int nblk = p.k / 256, n_mine = (ONE ? 1 : p.m) * nb;
     const bool norm = p.prologue == PRO_ADD_NORM;
     const float *emb = nullptr;
     if (norm && p.token) emb = p.emb_table + (size_t)__ldg(p.token) * p.k;
@@ -216,7 +218,7 @@ __device__ void build_activation(const MvParams &p, MvShared *sh, uint8_t *smem,
         for (int i = 0; i < kKeep; i++) {
             const int item = first + grp + i * ngroups;
             if (item < n_mine) {
-                const int mrow = item / nb, lb = item - mrow * nb, k4 = (blk0 + lb) * 64 + j;
+                const int mrow = ONE ? 0 : item / nb, lb = item - mrow * nb, k4 = (blk0 + lb) * 64 + j;
                 keep[i] = attn ? attn_value(lb) : prologue_value(p, emb, mrow, k4, 0.f);
                 if (norm) wgt[i] = first == 0 ? wgt_first[i] : __ldg(reinterpret_cast<const float4 *>(p.norm_w) + k4);
             }
@@ -293,8 +295,8 @@ __device__ void build_activation(const MvParams &p, MvShared *sh, uint8_t *smem,
         for (int i = 0; i < kKeep; i++) {
             const int item = first + grp + i * ngroups;
             if (item < n_mine) {
-                const int mrow = item / nb, lb = item - mrow * nb;
-                quantise_block<FMT>(p, smem, fmaxf(pair_max[2 * i], pair_max[2 * i + 1]), keep[i], mrow, lb, j, lane);
+                const int mrow = ONE ? 0 : item / nb, lb = item - mrow * nb;
+                quantise_block<FMT, ONE>(p, smem, fmaxf(pair_max[2 * i], pair_max[2 * i + 1]), keep[i], mrow, lb, j, lane);
             }
         }
         if (first + grp < n_mine && first + ngroups * kKeep < n_mine) named_bar(2 + grp, 64);   // pair_max is reused by the next pass

@@ -225,7 +225,6 @@ struct MatvecJob {
     const float *resid = nullptr;
     float *ssq_out = nullptr;
     bool dry_run = false;            // validate and plan only: tells whether the launch would be accepted
-    bool last_of_chain = false;      // no matvec follows closely: take half an SM's shared memory instead of a third
 };
 tlb_status launch_qmatvec(const MatvecJob &job);
 // K-slices the kernel wants for a launch of `tiles` 16-row tiles (all tensors) over inner dimension k,
