@@ -89,6 +89,22 @@ def test_qmatvec_matches_oracle(orc, t, n, k, m):
     assert relerr(got, ref) < (MATVEC_TOL if m <= 4 else GEMM_TOL)
 
 
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("n,k,rows", [(2368, 2048, (1,)), (2384, 2048, (1,)), (40, 256, (1, 3)), (14336, 1024, (3, 4)), (6000, 2304, (3, 4)), (2400, 14336, (1, 2))])
+def test_qmatvec_warps_and_slices(orc, t, n, k, rows):
+    """Both sides of the rules that choose a launch's warps (8 units per SM on 148 SMs) and its K-slices (three rows on, and
+    rows too long to be quantised whole)."""
+    rng = np.random.default_rng(5200 + t + n)
+    q = tl.QTensor.from_gguf_bytes(t, n, k, synth.random_quant(t, n, k, rng))
+    w = q.dequantize().numpy().astype(np.float64)
+    for m in rows:
+        x = rng.standard_normal((m, k), dtype=np.float32)
+        got = tl.Tensor.from_numpy(x).matmul_quantized(q).numpy()
+        ref = x.astype(np.float64) @ w.T
+        for i in range(m):
+            assert relerr(got[i], ref[i]) < 1e-4, (m, i)
+
+
 @pytest.mark.parametrize("t,n,k", [(synth.Q4_K, 4096, 4096), (synth.Q4_K, 4096, 14336), (synth.Q6_K, 8192, 4096),
                                    (synth.Q8_0, 2048, 2048), (synth.Q4_0, 5632, 2048)])
 def test_qmatvec_model_shapes(orc, t, n, k):

@@ -397,6 +397,18 @@ tlb_status enqueue_step_tp(tlb_decoder *d)
     return enqueue_head(d, nullptr, d->xa, d->part, d->xb);   // xb = xa + sum: the residual before output_norm
 }
 
+// Whether every linear layer of a step has so few units (16 rows x 256 weights) per SM that its launch is made of fixed costs.
+bool short_launches(const tlb_decoder *d)
+{
+    const int64_t most = 48 * (int64_t)ctx()->sm_count;
+    auto units = [](const tlb_qtensor *w) { return (int64_t)w->n_tiles * w->upt; };
+    for (int l = 0; l < d->cfg.n_layers; l++) {
+        const LayerW &w = d->layers[l];
+        if (units(w.q) + units(w.k) + units(w.v) > most || units(w.o) > most || units(w.gu) > most || units(w.down) > most) return false;
+    }
+    return true;
+}
+
 tlb_status enqueue_step(tlb_decoder *d)
 {
     if (d->lay) {
@@ -413,6 +425,7 @@ tlb_status enqueue_step(tlb_decoder *d)
     const tlb_decoder_cfg &c = d->cfg;
     const int dm = c.d_model, qd = d->H * c.head_dim, kvd = d->KVH * c.head_dim, F = d->F;
     const int L = c.n_layers;
+    const bool few = short_launches(d);
     for (int l = 0; l < L; l++) {
         const LayerW &w = d->layers[l];
         {   // K1: q | k | v in one launch when they share a type, else one launch per type
@@ -434,7 +447,7 @@ tlb_status enqueue_step(tlb_decoder *d)
                 if (l == 0 && first) { j.emb_table = d->emb->f32(); j.token = d->state; j.x_out = d->xb; }
                 else if (l == 0) { j.x = d->xb; }
                 else { j.x = d->xb; j.ssq_parts = d->ssq_d; j.n_parts = (dm + 15) / 16; }
-                j.pdl = d->pdl;
+                j.few = few; j.pdl = d->pdl;
                 j.dry_run = d->dry;
                 TLB_TRY(launch_qmatvec(j));
                 first = false;
@@ -462,7 +475,7 @@ tlb_status enqueue_step(tlb_decoder *d)
             j.att_rep = c.n_heads / c.n_kv_heads; j.att_dim = c.head_dim; j.att_keys = kAttnKeysPerSplit;
             j.finish = FIN_RESID; j.resid = d->xb; j.ssq_out = d->ssq_o;   // xa = xb + o_proj(attn)
             j.tp_reduce = tpr;
-            j.pdl = d->pdl;
+            j.few = few; j.pdl = d->pdl;
             j.dry_run = d->dry;
             TLB_TRY(launch_qmatvec(j));
         }
@@ -474,7 +487,7 @@ tlb_status enqueue_step(tlb_decoder *d)
             j.prologue = PRO_ADD_NORM; j.x = d->xa; j.ssq_parts = d->ssq_o; j.n_parts = (dm + 15) / 16;
             j.norm_w = w.ffn_norm->f32(); j.eps = c.eps;
             j.finish = FIN_SILU;
-            j.pdl = d->pdl;
+            j.few = few; j.pdl = d->pdl;
             j.dry_run = d->dry;
             TLB_TRY(launch_qmatvec(j));
         }
@@ -486,7 +499,7 @@ tlb_status enqueue_step(tlb_decoder *d)
             j.prologue = PRO_PLAIN; j.x = d->hbuf;
             j.finish = FIN_RESID; j.resid = d->xa; j.ssq_out = d->ssq_d;   // xb = xa + down(h)
             j.tp_reduce = tpr;
-            j.pdl = d->pdl;
+            j.few = few; j.pdl = d->pdl;
             j.dry_run = d->dry;
             TLB_TRY(launch_qmatvec(j));
         }

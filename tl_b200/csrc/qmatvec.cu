@@ -41,8 +41,8 @@
 
 namespace tlb {
 
-constexpr int kWarps = 16;
-constexpr int kThreads = kWarps * 32;
+constexpr int kWarps = 16;          // warps of a CTA
+constexpr int kFewWarps = 8;        // ... of a launch with few units (warps_for)
 
 struct ItemRef {
     const uint8_t *src;   // first unit of the item
@@ -150,8 +150,8 @@ __device__ __forceinline__ float tp_sum_tile(const MvParams &p, unsigned seq, in
 // deep; with the row count known at compile time and the divisions replaced (Divider) a decode step of the TinyLlama shapes
 // (111 launches) takes 761 us instead of 848, one of eight Llama-3-8B layers and head 510 instead of 551, a lone
 // 2048 x 2048 call 12.3 instead of 13.4.
-template <int FMT, bool ONE>
-__global__ void __launch_bounds__(kThreads, 1) qmatvec_kernel(const __grid_constant__ MvParams p)
+template <int FMT, int NW, bool ONE>
+__global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_constant__ MvParams p)
 {
     extern __shared__ __align__(128) uint8_t smem[];
     const int M = ONE ? 1 : p.m, NL = ONE ? 3 : p.nl;      // activation rows and int8 levels of each
@@ -169,8 +169,8 @@ __global__ void __launch_bounds__(kThreads, 1) qmatvec_kernel(const __grid_const
     const int ci0 = b * p.ipc_q + min(b, p.ipc_r), nci = p.ipc_q + (b < p.ipc_r ? 1 : 0), ci1 = ci0 + nci;
     const bool local = p.kb == 1;
     const int cta_units = nci * p.upi;
-    const int wu0 = local ? cta_units * warp / kWarps : (nci * warp / kWarps) * p.upi;
-    const int wu1 = local ? cta_units * (warp + 1) / kWarps : (nci * (warp + 1) / kWarps) * p.upi;
+    const int wu0 = local ? cta_units * warp / NW : (nci * warp / NW) * p.upi;
+    const int wu1 = local ? cta_units * (warp + 1) / NW : (nci * (warp + 1) / NW) * p.upi;
     const int n_units = wu1 - wu0;
     // activation blocks the CTA's items cover
     const int s_first = nci > 0 ? p.div_tiles(ci0) : 0, s_last = nci > 0 ? p.div_tiles(ci1 - 1) : 0;
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmatvec_kernel(const __grid_const
     };
 
     float4 wgt_first[kKeep];       // static inputs of the prologue, fetched while the previous kernel finishes
-    load_norm_weights(p, tid, kThreads, blk0, nb, wgt_first);
+    load_norm_weights(p, tid, NW * 32, blk0, nb, wgt_first);
     if (p.use_pdl) {
         pdl_wait();                // everything below may read what the previous kernel wrote
         // Released only after our own wait: a dependent's early part then runs with every kernel
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmatvec_kernel(const __grid_const
     }
     const unsigned tp_seq = p.tp_reduce ? ld_volatile_u32(p.tp.seq) : 0u;   // the launch before has completed: its exchange is over
     __syncthreads();               // abort_flag initialised; also keeps the CTA together for the prologue
-    build_activation<FMT, ONE>(p, sh, smem, tid, kThreads, blk0, nb, wgt_first, [&](float dep) {
+    build_activation<FMT, ONE>(p, sh, smem, tid, NW * 32, blk0, nb, wgt_first, [&](float dep) {
         // the rest of the ring's first round; the test on `dep` only ties the requests to the arrival of the loads
         if (lane >= kEarly && lane < n_first && __float_as_uint(dep) != 0x7fedcba9u) {
             mbar_expect_tx(bars + lane * 8, p.unit_bytes);
@@ -343,11 +343,11 @@ __global__ void __launch_bounds__(kThreads, 1) qmatvec_kernel(const __grid_const
         // order - and writes the rows.  No global scratch, fence or counter is involved.
         __syncthreads();           // every warp gets here: its waits are bounded
         if (!*abortp) {
-            for (int tl = warp; tl < nci; tl += kWarps) {
+            for (int tl = warp; tl < nci; tl += NW) {
                 const int a0 = tl * p.upi, a1 = a0 + p.upi;
                 float acc0 = 0.f, acc1 = 0.f;   // elements lane and lane + 32 of the 16 * m results
-                for (int w = 0; w < kWarps; w++) {
-                    const int b0 = cta_units * w / kWarps, b1 = cta_units * (w + 1) / kWarps;
+                for (int w = 0; w < NW; w++) {
+                    const int b0 = cta_units * w / NW, b1 = cta_units * (w + 1) / NW;
                     if (b1 <= a0 || b0 >= a1 || b1 == b0) continue;
                     const float *sp = segbuf + ((size_t)w * p.max_seg + (tl - p.div_upi(b0))) * (16 * M);
                     if (lane < 16 * M) acc0 += sp[lane];
@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(kThreads, 1) qmatvec_kernel(const __grid_const
             }
             if (tpr) {
                 // the warp's tiles are on their way to every rank; now the other ranks' shares of them
-                for (int tl = warp; tl < nci; tl += kWarps) {
+                for (int tl = warp; tl < nci; tl += NW) {
                     ItemCursor cf;
                     cf.slice = 0;
                     cf.tile = ci0 + tl;
@@ -548,30 +548,40 @@ static int blocks_per_cta(int64_t n_items, int grid, int64_t tiles, int upi, int
 }
 
 // Relative cost (warp instructions on the critical path) of cutting K into upt / upi slices.
-static double slice_cost(int type, int m, int64_t tiles, int upt, int upi, int sm_count)
+static double slice_cost(int type, int m, int64_t tiles, int upt, int upi, int sm_count, int nw)
 {
     const int kb = upt / upi;
     const int64_t n_items = tiles * kb;
     const int grid = (int)std::min<int64_t>(sm_count, n_items);
-    const int64_t ipc = (n_items + grid - 1) / grid, ipw = (ipc + kWarps - 1) / kWarps;
+    const int64_t ipc = (n_items + grid - 1) / grid, ipw = (ipc + nw - 1) / nw;
     const int nb = blocks_per_cta(n_items, grid, tiles, upi, upt);
     const double unit = type == TLB_GGML_Q6_K ? 300.0 : type == TLB_GGML_Q8_0 ? 150.0 : 210.0;
     // one slice: the CTA's units are cut evenly over its warps whatever the tile borders
-    const double stream = kb == 1 ? (double)((ipc * upi + kWarps - 1) / kWarps) * unit + 60.0 * ((ipc + kWarps - 1) / kWarps + 1)
+    const double stream = kb == 1 ? (double)((ipc * upi + nw - 1) / nw) * unit + 60.0 * ((ipc + nw - 1) / nw + 1)
                                   : (double)ipw * (upi * unit + 60.0);
-    const double quant = 300.0 * ((m * nb + kThreads / 64 - 1) / (kThreads / 64));
+    const double quant = 300.0 * ((m * nb + nw / 2 - 1) / (nw / 2));
     // Measured on the Llama-3-8B shapes: the end of a sliced launch (fence, counts, reading the slices back)
     // costs ~3 us; assembling tiles in shared memory costs a block barrier, which shows (~2 us of waiting
     // for the slowest warp) only when warps have so few units that their skew matters.
-    const bool few = (ipc * upi + kWarps - 1) / kWarps < 4;
-    const double fold = kb > 1 ? 600.0 + 16.0 * kb : (few ? 600.0 : 100.0);
+    // Three or four rows in several items per warp pay far more (14336 x 4096 Q8_0, four rows: 43 us in four slices, 23 in one).
+    const bool few = (ipc * upi + nw - 1) / nw < 4;
+    const double fold = kb == 1 ? (few ? 600.0 : 100.0) : 600.0 + 16.0 * kb + (m >= 3 && ipw > 1 ? 3000.0 : 0.0);
     return stream + quant + fold;
 }
 
-int qmatvec_plan_slices(int type, int64_t k, int m, int64_t tiles, int max_slices)
+// Warps of a CTA.  With one unit or less for each of eight warps the other eight only issue the prologue again: four calls of
+// 2048 x 2048 with norms between them take 49.2 us with sixteen and 46 with eight.  From two units per warp on, a lone launch
+// is faster with sixteen (2048 x 5632: 9.8 against 12.5 us), but in a chain of nothing but short launches eight leave the next
+// launch room to become resident (MatvecJob::few; TinyLlama shapes, 32 steps: 24.3 against 23.5 ms).
+static int warps_for(const MatvecJob &job, int64_t tiles, int upt, int sm_count)
 {
-    Context *c = ctx();
-    const int sm = c ? c->sm_count : 148;
+    return job.m == 1 && (job.few || (!job.pdl && tiles * upt <= (int64_t)kFewWarps * sm_count)) ? kFewWarps : kWarps;
+}
+
+// K-slices of a launch of `tiles` 16-row tiles (all tensors) over inner dimension k: as many as the cost model likes, at
+// most max_slices.
+static int plan_slices(int type, int64_t k, int m, int64_t tiles, int max_slices, int sm, size_t smem_max, int nw)
+{
     const int upt = (int)(k / 256);
     if (upt < 1 || tiles < 1) return 1;
     max_slices = std::max(1, std::min(max_slices, kMaxSlices));
@@ -581,13 +591,17 @@ int qmatvec_plan_slices(int type, int64_t k, int m, int64_t tiles, int max_slice
         if (upt % upi) continue;
         const int kb = upt / upi;
         if (kb > max_slices) break;
-        const double cost = slice_cost(type, m, tiles, upt, upi, sm);
+        double cost = slice_cost(type, m, tiles, upt, upi, sm, nw);
+        if (kb == 1) {                       // the whole row, two stages per warp and the slots of partial results beside it
+            const size_t stages = (size_t)nw * 2 * (stage_bytes_of(qformat(type)) + 8), slots = (size_t)nw * 8 * 16 * m * sizeof(float);
+            if (plan_smem(type, m, m <= 2 ? 3 : 2, upt).fixed + stages + slots + 256 > smem_max) cost = 1e12;
+        }
         if (kb == 1 || cost < best_cost) { best = kb; best_cost = cost; }
     }
     return best;
 }
 
-template <int FMT, bool ONE>
+template <int FMT, int NW, bool ONE>
 static tlb_status launch_fmt_rows(const MvParams &p, int grid, size_t smem, bool pdl)
 {
     // Function attributes are set once, to their final values, before the first launch: a graph whose
@@ -596,13 +610,13 @@ static tlb_status launch_fmt_rows(const MvParams &p, int grid, size_t smem, bool
     // that SMs do not re-partition between launches.
     static bool prepared = false;
     if (!prepared) {
-        TLB_CUDA(cudaFuncSetAttribute((qmatvec_kernel<FMT, ONE>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx()->smem_optin));
-        TLB_CUDA(cudaFuncSetAttribute((qmatvec_kernel<FMT, ONE>), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        TLB_CUDA(cudaFuncSetAttribute((qmatvec_kernel<FMT, NW, ONE>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx()->smem_optin));
+        TLB_CUDA(cudaFuncSetAttribute((qmatvec_kernel<FMT, NW, ONE>), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         prepared = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(NW * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx()->stream;
     cudaLaunchAttribute at[1];
@@ -614,15 +628,16 @@ static tlb_status launch_fmt_rows(const MvParams &p, int grid, size_t smem, bool
     }
     cfg.attrs = at;
     cfg.numAttrs = na;
-    TLB_CUDA(cudaLaunchKernelEx(&cfg, (qmatvec_kernel<FMT, ONE>), p));
+    TLB_CUDA(cudaLaunchKernelEx(&cfg, (qmatvec_kernel<FMT, NW, ONE>), p));
     count_launch();
     return TLB_OK;
 }
 
 template <int FMT>
-static tlb_status launch_fmt(const MvParams &p, int grid, size_t smem, bool pdl)
+static tlb_status launch_fmt(const MvParams &p, int nw, int grid, size_t smem, bool pdl)
 {
-    return p.m == 1 ? launch_fmt_rows<FMT, true>(p, grid, smem, pdl) : launch_fmt_rows<FMT, false>(p, grid, smem, pdl);
+    if (p.m != 1) return launch_fmt_rows<FMT, kWarps, false>(p, grid, smem, pdl);
+    return nw == kFewWarps ? launch_fmt_rows<FMT, kFewWarps, true>(p, grid, smem, pdl) : launch_fmt_rows<FMT, kWarps, true>(p, grid, smem, pdl);
 }
 
 tlb_status launch_qmatvec(const MatvecJob &job)
@@ -656,11 +671,12 @@ tlb_status launch_qmatvec(const MatvecJob &job)
     p.m = job.m;
     p.nl = job.m <= 2 ? 3 : 2;
     if (tiles > INT32_MAX / (64 * kMaxSlices)) return fail(TLB_ERR_SHAPE, "too many tiles for one launch");
+    const int nw = warps_for(job, tiles, p.upt, c->sm_count);
     // K-slices: as many as the cost model likes and the slice scratch and tile counters hold
     int max_slices = kMaxSlices;
     if (tiles > (int64_t)c->mv_cnt_n) max_slices = 1;
     while (max_slices > 1 && (size_t)max_slices * tiles * 16 * job.m > c->mv_part_floats) max_slices--;
-    p.kb = job.slices > 0 ? std::min(job.slices, max_slices) : qmatvec_plan_slices(job.type, job.k, job.m, tiles, max_slices);
+    p.kb = job.slices > 0 ? std::min(job.slices, max_slices) : plan_slices(job.type, job.k, job.m, tiles, max_slices, c->sm_count, c->smem_optin, nw);
     if (p.kb < 1 || p.upt % p.kb) return fail(TLB_ERR_ARG, "%d slices do not divide the %d units of K", p.kb, p.upt);
     p.upi = p.upt / p.kb;
     p.fold_poll = (job.m == 1 && (size_t)p.kb * tiles * 16 <= c->mv_part1_floats) ? 1 : 0;
@@ -678,33 +694,33 @@ tlb_status launch_qmatvec(const MatvecJob &job)
     p.nb_max = blocks_per_cta(p.n_items, grid, tiles, p.upi, p.upt);
     const SmemPlan sp = plan_smem(job.type, job.m, p.nl, p.nb_max);
     const size_t budget = c->smem_optin;                  // one CTA per SM
-    const size_t per_stage = (size_t)kWarps * (p.stage_bytes + 8);
+    const size_t per_stage = (size_t)nw * (p.stage_bytes + 8);
     if (sp.fixed + 128 + 2 * per_stage > budget)
         return fail(TLB_ERR_SHAPE, "K = %lld with %d rows needs more shared memory than one SM has (max K %zu)",
                     (long long)job.k, job.m, qmatvec_max_k(job.m));
     // (room for the local-mode slots: at most ~6 per warp)
-    const size_t seg_room = (p.kb == 1 ? (size_t)kWarps * 8 * 16 * job.m * sizeof(float) + 128 : 0) +
+    const size_t seg_room = (p.kb == 1 ? (size_t)nw * 8 * 16 * job.m * sizeof(float) + 128 : 0) +
                             (job.prologue == PRO_ATTN_MERGE ? (size_t)p.nb_max * 4 * std::max(1, job.att_max_splits) * sizeof(float) + 128 : 0);
-    int spw = (int)((budget - sp.fixed - 128 - seg_room) / per_stage);
+    int spw = budget > sp.fixed + 128 + seg_room ? (int)((budget - sp.fixed - 128 - seg_room) / per_stage) : 0;
     // no more stages than the longest warp has units, and no more than keeps ~1.5 us of HBM latency covered
     const int64_t ipc = (p.n_items + grid - 1) / grid;
-    const int64_t upw = (ipc + kWarps - 1) / kWarps * p.upi;
-    spw = (int)std::min<int64_t>(std::min(spw, 8), std::max<int64_t>(2, upw));
+    const int64_t upw = (ipc + nw - 1) / nw * p.upi;
+    spw = (int)std::min<int64_t>(std::max(2, std::min(spw, 8)), std::max<int64_t>(2, upw));      // a trip of the unit loop takes two stages
     p.spw = spw;
-    const size_t ring = (size_t)kWarps * spw * p.stage_bytes;
+    const size_t ring = (size_t)nw * spw * p.stage_bytes;
     p.off_xq = (int)ring + sp.off_xq; p.off_alam = (int)ring + sp.off_alam; p.off_xsum = (int)ring + sp.off_xsum;
     p.off_sa = (int)ring + sp.off_sa; p.off_minv = (int)ring + sp.off_minv; p.off_misc = (int)ring + sp.off_misc;
     p.off_bars = (int)(ring + sp.fixed);
     p.col_stride = sp.col_stride;
-    size_t smem = ring + sp.fixed + (size_t)kWarps * spw * 8;
+    size_t smem = ring + sp.fixed + (size_t)nw * spw * 8;
     // local mode (one K-slice): per warp, one slot of 16 * m partial results per tile its unit range touches
     p.max_seg = 1;
     p.off_seg = 0;
     if (p.kb == 1) {
-        const int64_t n_max = (ipc * p.upi + kWarps - 1) / kWarps;           // most units a warp gets
+        const int64_t n_max = (ipc * p.upi + nw - 1) / nw;           // most units a warp gets
         p.max_seg = (int)((n_max + p.upi - 2) / p.upi + 1);
         p.off_seg = (int)((smem + 127) / 128 * 128);
-        smem = (size_t)p.off_seg + (size_t)kWarps * p.max_seg * 16 * job.m * sizeof(float);
+        smem = (size_t)p.off_seg + (size_t)nw * p.max_seg * 16 * job.m * sizeof(float);
         if (smem > c->smem_optin) return fail(TLB_ERR_SHAPE, "launch needs %zu bytes of shared memory", smem);
     }
     p.prologue = job.prologue;
@@ -738,10 +754,10 @@ tlb_status launch_qmatvec(const MatvecJob &job)
     if (p.prologue == PRO_SILU_MUL && !p.x2) return fail(TLB_ERR_NULL, "null activation");
     if (job.dry_run) return TLB_OK;   // the shape is launchable
     switch (job.type) {
-    case TLB_GGML_Q4_K: return launch_fmt<TLB_GGML_Q4_K>(p, grid, smem, job.pdl);
-    case TLB_GGML_Q6_K: return launch_fmt<TLB_GGML_Q6_K>(p, grid, smem, job.pdl);
-    case TLB_GGML_Q8_0: return launch_fmt<TLB_GGML_Q8_0>(p, grid, smem, job.pdl);
-    default: return launch_fmt<TLB_GGML_Q4_0>(p, grid, smem, job.pdl);
+    case TLB_GGML_Q4_K: return launch_fmt<TLB_GGML_Q4_K>(p, nw, grid, smem, job.pdl);
+    case TLB_GGML_Q6_K: return launch_fmt<TLB_GGML_Q6_K>(p, nw, grid, smem, job.pdl);
+    case TLB_GGML_Q8_0: return launch_fmt<TLB_GGML_Q8_0>(p, nw, grid, smem, job.pdl);
+    default: return launch_fmt<TLB_GGML_Q4_0>(p, nw, grid, smem, job.pdl);
     }
 }
 

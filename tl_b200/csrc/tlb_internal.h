@@ -190,7 +190,7 @@ struct MatvecJob {
     int64_t n_rows[3] = {0, 0, 0};                 // valid output rows (<= n_tiles*16)
     // Output of tensor i: [M, n_rows], every element written (no clearing needed).
     float *out[3] = {nullptr, nullptr, nullptr};
-    int slices = 0;                  // K-slices the launch is cut into; 0: chosen by qmatvec_plan_slices()
+    int slices = 0;                  // K-slices the launch is cut into; 0: chosen by the launch
     int type = 0;
     int64_t k = 0;
     int m = 1;
@@ -204,6 +204,7 @@ struct MatvecJob {
     const float *emb_table = nullptr; // ADD_NORM with token lookup: x = emb_table[*token * K ...]
     const int *token = nullptr;
     bool pdl = false;                // launch with programmatic stream serialization
+    bool few = false;                // m == 1: part of a chain of short launches (CTAs of eight warps)
     // ADD_NORM without the statistics pass: x already holds the whole residual and ssq_parts[0 .. n_parts)
     // are partial sums of its squares left by the launch that produced it (finish == FIN_RESID there)
     const float *ssq_parts = nullptr;
@@ -227,9 +228,6 @@ struct MatvecJob {
     bool dry_run = false;            // validate and plan only: tells whether the launch would be accepted
 };
 tlb_status launch_qmatvec(const MatvecJob &job);
-// K-slices the kernel wants for a launch of `tiles` 16-row tiles (all tensors) over inner dimension k,
-// at most max_slices; a pure function of its arguments, so producer and consumer agree without talking.
-int qmatvec_plan_slices(int type, int64_t k, int m, int64_t tiles, int max_slices);
 size_t qmatvec_max_k(int m);   // largest K the single-pass kernel supports for m activation rows
 
 // ops.cu
