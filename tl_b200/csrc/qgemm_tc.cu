@@ -5,7 +5,11 @@
 // and calls a one-thread-per-output matmul); here the weight is read once per tile of 256 activation
 // rows and never exists in f32.
 //
-// One CTA computes 128 weight rows x NT activation rows (NT <= 256) on the 5th-generation tensor cores:
+// One CTA computes 128 weight rows x NT activation rows (NT <= 256) on the 5th-generation tensor cores.  Above 128 rows two
+// CTAs share a tile (cta_group::2): each brings half of the activation rows and dequantises its own 128 weight rows, which
+// halves the L2 -> shared memory traffic per product, and NT goes up to 384 as two accumulators.  Q4_K 14336 x 4096 with 129,
+// 256, 333 and 512 rows, whole call: 68, 70, 77 and 79 us with single CTAs, 41, 43, 55 and 81 us now (512 rows are 224 tiles of
+// 256 on 148 SMs either way: two waves, where 36 us of products would fill one and a half):
 //   * the weight tile is the A operand (MMA M = 128) and lives in TENSOR MEMORY, never in shared memory: sixteen
 //     producer warps (two per 16 weight rows, each taking two of a unit's four 64-wide groups) read the quantized
 //     units with coalesced 16-byte loads, dequantise in registers (f16 pair arithmetic on exact integers, see

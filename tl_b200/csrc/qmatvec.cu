@@ -4,7 +4,8 @@
 // re-read once per activation row) and the dequantise-then-naive-matmul route the reference takes
 // for Q4_0 / Q8_0 (crates/tl_runtime/src/system.rs:236-264).
 //
-// Shape of the kernel (one persistent CTA of 16 warps per SM, the whole register file at 128 per thread;
+// Shape of the kernel (one persistent CTA of 16 warps per SM, the whole register file at 128 per thread, or of 8 where a
+// launch is short, see warps_for;
 // a variant of two 8-warp CTAs that leaves room for a CTA of the next kernel measured 35 % slower
 // per step: at 80 registers the unit loop no longer keeps its shared loads in flight):
 //   * work is cut into ITEMS: one tile of 16 output rows x one K-slice of `upi` consecutive units
@@ -33,7 +34,8 @@
 //     no global scratch, fence or counter at all;
 //   * finishing a tile can fuse what follows the matvec in the decode chain: the residual add with
 //     per-tile sums of squares for the next RMSNorm, or SiLU(gate) * up over interleaved gate|up rows;
-//   * a host-side cost model (slice_cost) picks the number of K-slices per launch shape.
+//   * a host-side cost model (slice_cost) picks the number of K-slices per launch shape;
+//   * one activation row is a form of its own (ONE), without the loops and divisions that several rows take.
 #include "qmv_prologue.cuh"
 #include "qmv_units.cuh"
 
