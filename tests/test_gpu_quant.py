@@ -105,6 +105,21 @@ def test_qmatvec_warps_and_slices(orc, t, n, k, rows):
             assert relerr(got[i], ref[i]) < 1e-4, (m, i)
 
 
+@pytest.mark.parametrize("t,n,k,rows", [(synth.Q8_0, 40, 256 * 41, (3, 4)), (synth.Q8_0, 300, 256 * 43, (3, 4)), (synth.Q8_0, 2048, 256 * 46, (4,)),
+                                        (synth.Q8_0, 40, 256 * 47, (3, 4)), (synth.Q8_0, 40, 256 * 53, (2, 3, 4)), (synth.Q6_K, 40, 256 * 53, (3, 4))])
+def test_qmatvec_rows_too_long_for_four(t, n, k, rows):
+    """Long rows that do not fit shared memory four (or three) at a time: fewer go together (tests/test_launch_plans_cpu.py)."""
+    rng = np.random.default_rng(5400 + t + k)
+    q = tl.QTensor.from_gguf_bytes(t, n, k, synth.random_quant(t, n, k, rng))
+    w = q.dequantize().numpy().astype(np.float64)
+    for m in rows:
+        x = rng.standard_normal((m, k), dtype=np.float32)
+        got = tl.Tensor.from_numpy(x).matmul_quantized(q).numpy()
+        ref = x.astype(np.float64) @ w.T
+        for i in range(m):
+            assert relerr(got[i], ref[i]) < MATVEC_TOL, (m, i)
+
+
 @pytest.mark.parametrize("t,n,k", [(synth.Q4_K, 4096, 4096), (synth.Q4_K, 4096, 14336), (synth.Q6_K, 8192, 4096),
                                    (synth.Q8_0, 2048, 2048), (synth.Q4_0, 5632, 2048)])
 def test_qmatvec_model_shapes(orc, t, n, k):

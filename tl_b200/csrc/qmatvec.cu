@@ -580,27 +580,76 @@ static int warps_for(const MatvecJob &job, int64_t tiles, int upt, int sm_count)
     return job.m == 1 && (job.few || (!job.pdl && tiles * upt <= (int64_t)kFewWarps * sm_count)) ? kFewWarps : kWarps;
 }
 
-// K-slices of a launch of `tiles` 16-row tiles (all tensors) over inner dimension k: as many as the cost model likes, at
-// most max_slices.
-static int plan_slices(int type, int64_t k, int m, int64_t tiles, int max_slices, int sm, size_t smem_max, int nw)
+// How a launch of `tiles` 16-row tiles (all tensors) over upt units of K is laid out with kb K-slices.
+struct MvGeometry {
+    int upi, n_items, grid, nb, spw, max_seg;
+    int ring, off_seg, off_wtab;        // bytes of the ring; where the partial results and ATTN_MERGE's weights begin
+    SmemPlan sp;
+    size_t smem;
+    bool roomy;                         // two stages fit beside eight slots of partial results per warp
+};
+
+// heads, splits: ATTN_MERGE's softmax weights per block of 256 activations (0: none)
+static MvGeometry geometry(int type, int m, int upt, int64_t tiles, int kb, int nw, int sm, size_t smem_max, int heads, int splits)
 {
-    const int upt = (int)(k / 256);
-    if (upt < 1 || tiles < 1) return 1;
+    MvGeometry g = {};
+    const int stage = stage_bytes_of(qformat(type));
+    g.upi = upt / kb;
+    g.n_items = (int)(tiles * kb);
+    g.grid = (int)std::min<int64_t>(sm, g.n_items);
+    g.nb = blocks_per_cta(g.n_items, g.grid, tiles, g.upi, upt);
+    g.sp = plan_smem(type, m, m <= 2 ? 3 : 2, g.nb);
+    const int64_t ipc = (g.n_items + g.grid - 1) / g.grid;
+    // local mode (one K-slice): per warp, one slot of 16 * m partial results per tile its unit range touches, rarely over six
+    const int64_t n_max = (ipc * g.upi + nw - 1) / nw;           // most units a warp gets
+    g.max_seg = kb == 1 ? (int)((n_max + g.upi - 2) / g.upi + 1) : 1;
+    const size_t slot = kb == 1 ? (size_t)nw * 16 * m * sizeof(float) : 0, per_stage = (size_t)nw * (stage + 8);
+    const size_t beside = g.sp.fixed + 128 + (kb == 1 ? std::max(8, g.max_seg) * slot + 128 : 0) + (heads ? (size_t)g.nb * 4 * splits * sizeof(float) + 128 : 0);
+    // no more stages than the longest warp has units, and no more than keeps ~1.5 us of HBM latency covered; two at least,
+    // which a trip of the unit loop takes
+    const int64_t upw = (ipc + nw - 1) / nw * g.upi;
+    const int fit = smem_max > beside ? (int)((smem_max - beside) / per_stage) : 0;
+    g.roomy = g.sp.fixed + 2 * per_stage + 8 * slot + 256 <= smem_max;
+    g.spw = (int)std::min<int64_t>(std::max(2, std::min(fit, 8)), std::max<int64_t>(2, upw));
+    g.ring = nw * g.spw * stage;
+    g.smem = (size_t)g.ring + g.sp.fixed + (size_t)nw * g.spw * 8;
+    if (kb == 1) {
+        g.off_seg = (int)((g.smem + 127) / 128 * 128);
+        g.smem = (size_t)g.off_seg + g.max_seg * slot;
+    }
+    if (heads) {
+        g.off_wtab = (int)((g.smem + 127) / 128 * 128);
+        g.smem = (size_t)g.off_wtab + (size_t)g.nb * heads * splits * sizeof(float);
+    }
+    return g;
+}
+
+// K-slices of a launch: as many as the cost model likes, at most max_slices, among the counts whose launch fits shared memory
+// (0: none does).
+static int plan_slices(int type, int upt, int m, int64_t tiles, int max_slices, int nw, int sm, size_t smem_max, int heads, int splits)
+{
     max_slices = std::max(1, std::min(max_slices, kMaxSlices));
-    int best = 1;
+    int best = 0;
     double best_cost = 0.0;
     for (int upi = upt; upi >= 1; upi--) {
         if (upt % upi) continue;
         const int kb = upt / upi;
         if (kb > max_slices) break;
-        double cost = slice_cost(type, m, tiles, upt, upi, sm, nw);
-        if (kb == 1) {                       // the whole row, two stages per warp and the slots of partial results beside it
-            const size_t stages = (size_t)nw * 2 * (stage_bytes_of(qformat(type)) + 8), slots = (size_t)nw * 8 * 16 * m * sizeof(float);
-            if (plan_smem(type, m, m <= 2 ? 3 : 2, upt).fixed + stages + slots + 256 > smem_max) cost = 1e12;
-        }
-        if (kb == 1 || cost < best_cost) { best = kb; best_cost = cost; }
+        const MvGeometry g = geometry(type, m, upt, tiles, kb, nw, sm, smem_max, heads, splits);
+        if (g.smem > smem_max) continue;
+        const double cost = kb == 1 && !g.roomy ? 1e12 : slice_cost(type, m, tiles, upt, upi, sm, nw);
+        if (best == 0 || cost < best_cost) { best = kb; best_cost = cost; }
     }
     return best;
+}
+
+// K-slices of one row group of tlb_qtensor_matmul over a weight of n rows; 0: no launch of this many rows fits.
+extern "C" int tlb_matvec_slices(int type, int64_t n, int64_t k, int m, int sm, size_t smem_max)
+{
+    const int64_t tiles = (n + 15) / 16;
+    const int upt = (int)(k / 256);
+    const int nw = m == 1 && tiles * upt <= (int64_t)kFewWarps * sm ? kFewWarps : kWarps;
+    return plan_slices(type, upt, m, tiles, kMaxSlices, nw, sm, smem_max, 0, 0);
 }
 
 template <int FMT, int NW, bool ONE>
@@ -678,53 +727,33 @@ tlb_status launch_qmatvec(const MatvecJob &job)
     int max_slices = kMaxSlices;
     if (tiles > (int64_t)c->mv_cnt_n) max_slices = 1;
     while (max_slices > 1 && (size_t)max_slices * tiles * 16 * job.m > c->mv_part_floats) max_slices--;
-    p.kb = job.slices > 0 ? std::min(job.slices, max_slices) : plan_slices(job.type, job.k, job.m, tiles, max_slices, c->sm_count, c->smem_optin, nw);
-    if (p.kb < 1 || p.upt % p.kb) return fail(TLB_ERR_ARG, "%d slices do not divide the %d units of K", p.kb, p.upt);
-    p.upi = p.upt / p.kb;
+    const int heads = job.prologue == PRO_ATTN_MERGE && job.att_dim > 0 ? 256 / job.att_dim : 0, splits = std::max(1, job.att_max_splits);
+    p.kb = job.slices > 0 ? std::min(job.slices, max_slices) : plan_slices(job.type, p.upt, job.m, tiles, max_slices, nw, c->sm_count, c->smem_optin, heads, splits);
+    if (p.kb < 1) return fail(TLB_ERR_SHAPE, "K = %lld with %d rows needs more shared memory than one SM has (max K %zu)", (long long)job.k, job.m, qmatvec_max_k(job.m));
+    if (p.upt % p.kb) return fail(TLB_ERR_ARG, "%d slices do not divide the %d units of K", p.kb, p.upt);
+    const MvGeometry g = geometry(job.type, job.m, p.upt, tiles, p.kb, nw, c->sm_count, c->smem_optin, heads, splits);
+    if (g.smem > c->smem_optin) return fail(TLB_ERR_SHAPE, "launch needs %zu bytes of shared memory", g.smem);
+    p.upi = g.upi;
     p.fold_poll = (job.m == 1 && (size_t)p.kb * tiles * 16 <= c->mv_part1_floats) ? 1 : 0;
     p.part = p.fold_poll ? c->mv_part1 : c->mv_part;
     p.tile_cnt = c->mv_cnt;
     p.tiles = (int)tiles;
-    p.n_items = (int)(tiles * p.kb);
+    p.n_items = g.n_items;
     p.div_tiles = Divider((uint32_t)p.tiles);
     p.div_upi = Divider((uint32_t)p.upi);
     p.unit_bytes = f->unit_bytes;
     p.stage_bytes = stage_bytes_of(f);
-    const int grid = (int)std::min<int64_t>(c->sm_count, p.n_items);
-    p.ipc_q = p.n_items / grid;
-    p.ipc_r = p.n_items % grid;
-    p.nb_max = blocks_per_cta(p.n_items, grid, tiles, p.upi, p.upt);
-    const SmemPlan sp = plan_smem(job.type, job.m, p.nl, p.nb_max);
-    const size_t budget = c->smem_optin;                  // one CTA per SM
-    const size_t per_stage = (size_t)nw * (p.stage_bytes + 8);
-    if (sp.fixed + 128 + 2 * per_stage > budget)
-        return fail(TLB_ERR_SHAPE, "K = %lld with %d rows needs more shared memory than one SM has (max K %zu)",
-                    (long long)job.k, job.m, qmatvec_max_k(job.m));
-    // (room for the local-mode slots: at most ~6 per warp)
-    const size_t seg_room = (p.kb == 1 ? (size_t)nw * 8 * 16 * job.m * sizeof(float) + 128 : 0) +
-                            (job.prologue == PRO_ATTN_MERGE ? (size_t)p.nb_max * 4 * std::max(1, job.att_max_splits) * sizeof(float) + 128 : 0);
-    int spw = budget > sp.fixed + 128 + seg_room ? (int)((budget - sp.fixed - 128 - seg_room) / per_stage) : 0;
-    // no more stages than the longest warp has units, and no more than keeps ~1.5 us of HBM latency covered
-    const int64_t ipc = (p.n_items + grid - 1) / grid;
-    const int64_t upw = (ipc + nw - 1) / nw * p.upi;
-    spw = (int)std::min<int64_t>(std::max(2, std::min(spw, 8)), std::max<int64_t>(2, upw));      // a trip of the unit loop takes two stages
-    p.spw = spw;
-    const size_t ring = (size_t)nw * spw * p.stage_bytes;
-    p.off_xq = (int)ring + sp.off_xq; p.off_alam = (int)ring + sp.off_alam; p.off_xsum = (int)ring + sp.off_xsum;
-    p.off_sa = (int)ring + sp.off_sa; p.off_minv = (int)ring + sp.off_minv; p.off_misc = (int)ring + sp.off_misc;
-    p.off_bars = (int)(ring + sp.fixed);
-    p.col_stride = sp.col_stride;
-    size_t smem = ring + sp.fixed + (size_t)nw * spw * 8;
-    // local mode (one K-slice): per warp, one slot of 16 * m partial results per tile its unit range touches
-    p.max_seg = 1;
-    p.off_seg = 0;
-    if (p.kb == 1) {
-        const int64_t n_max = (ipc * p.upi + nw - 1) / nw;           // most units a warp gets
-        p.max_seg = (int)((n_max + p.upi - 2) / p.upi + 1);
-        p.off_seg = (int)((smem + 127) / 128 * 128);
-        smem = (size_t)p.off_seg + (size_t)nw * p.max_seg * 16 * job.m * sizeof(float);
-        if (smem > c->smem_optin) return fail(TLB_ERR_SHAPE, "launch needs %zu bytes of shared memory", smem);
-    }
+    p.ipc_q = p.n_items / g.grid;
+    p.ipc_r = p.n_items % g.grid;
+    p.nb_max = g.nb;
+    p.spw = g.spw;
+    p.off_xq = g.ring + g.sp.off_xq; p.off_alam = g.ring + g.sp.off_alam; p.off_xsum = g.ring + g.sp.off_xsum;
+    p.off_sa = g.ring + g.sp.off_sa; p.off_minv = g.ring + g.sp.off_minv; p.off_misc = g.ring + g.sp.off_misc;
+    p.off_bars = g.ring + (int)g.sp.fixed;
+    p.col_stride = g.sp.col_stride;
+    p.max_seg = g.max_seg;
+    p.off_seg = g.off_seg;
+    p.off_wtab = g.off_wtab;
     p.prologue = job.prologue;
     p.x = job.x; p.x2 = job.x2; p.norm_w = job.norm_w; p.eps = job.eps; p.x_out = job.x_out;
     p.tp_reduce = job.tp_reduce ? 1 : 0;
@@ -741,10 +770,6 @@ tlb_status launch_qmatvec(const MatvecJob &job)
         if (!job.att_part || !job.att_pos || job.att_max_splits < 1 || job.att_rep < 1 || job.att_keys < 1 ||
             (job.att_dim != 64 && job.att_dim != 128) || job.k % job.att_dim)
             return fail(TLB_ERR_ARG, "attention-merge prologue: incomplete or unsupported description of the split results");
-        // softmax weights of the splits, one row per query head of the CTA's blocks, after everything else
-        p.off_wtab = (int)((smem + 127) / 128 * 128);
-        smem = (size_t)p.off_wtab + (size_t)p.nb_max * (256 / job.att_dim) * job.att_max_splits * sizeof(float);
-        if (smem > c->smem_optin) return fail(TLB_ERR_SHAPE, "launch needs %zu bytes of shared memory", smem);
     }
     p.finish = job.finish; p.resid = job.resid; p.ssq_out = job.ssq_out;
     if (job.finish != FIN_PLAIN && (job.m != 1 || job.n_w != 1)) return fail(TLB_ERR_ARG, "fused tile finishing takes one tensor and one activation row");
@@ -756,10 +781,10 @@ tlb_status launch_qmatvec(const MatvecJob &job)
     if (p.prologue == PRO_SILU_MUL && !p.x2) return fail(TLB_ERR_NULL, "null activation");
     if (job.dry_run) return TLB_OK;   // the shape is launchable
     switch (job.type) {
-    case TLB_GGML_Q4_K: return launch_fmt<TLB_GGML_Q4_K>(p, nw, grid, smem, job.pdl);
-    case TLB_GGML_Q6_K: return launch_fmt<TLB_GGML_Q6_K>(p, nw, grid, smem, job.pdl);
-    case TLB_GGML_Q8_0: return launch_fmt<TLB_GGML_Q8_0>(p, nw, grid, smem, job.pdl);
-    default: return launch_fmt<TLB_GGML_Q4_0>(p, nw, grid, smem, job.pdl);
+    case TLB_GGML_Q4_K: return launch_fmt<TLB_GGML_Q4_K>(p, nw, g.grid, g.smem, job.pdl);
+    case TLB_GGML_Q6_K: return launch_fmt<TLB_GGML_Q6_K>(p, nw, g.grid, g.smem, job.pdl);
+    case TLB_GGML_Q8_0: return launch_fmt<TLB_GGML_Q8_0>(p, nw, g.grid, g.smem, job.pdl);
+    default: return launch_fmt<TLB_GGML_Q4_0>(p, nw, g.grid, g.smem, job.pdl);
     }
 }
 
@@ -822,7 +847,10 @@ extern "C" tlb_status tlb_qtensor_matmul(tlb_tensor **out, const tlb_tensor *x, 
         // more than four rows (batched decoding, prompt processing): the weight is read once per 256 rows
         st = launch_qgemm(w, xa->f32(), m, (*out)->f32());
     } else {
-        for (int64_t m0 = 0; m0 < m && st == TLB_OK; m0 += 4) {   // the weight stream is repeated per group of 4 rows
+        // the weight stream is repeated per group of rows: four, or fewer where the levels of four long rows and a ring do not
+        // fit shared memory in any number of slices (Q8_0, K = 11008: four rows want 238 KB of 227)
+        int group = 4;
+        for (int64_t m0 = 0; m0 < m && st == TLB_OK;) {
             MatvecJob job;
             job.n_w = 1;
             job.w[0] = w->dev();
@@ -831,9 +859,11 @@ extern "C" tlb_status tlb_qtensor_matmul(tlb_tensor **out, const tlb_tensor *x, 
             job.out[0] = (*out)->f32() + m0 * w->n;
             job.type = w->type;
             job.k = k;
-            job.m = (int)std::min<int64_t>(4, m - m0);
+            job.m = (int)std::min<int64_t>(group, m - m0);
             job.x = xa->f32() + m0 * k;
             st = launch_qmatvec(job);
+            if (st == TLB_ERR_SHAPE && job.m > 1) { group = (job.m + 1) / 2; st = TLB_OK; }
+            else m0 += job.m;
         }
     }
     tlb_tensor_release(xcopy);   // stream-ordered pool: the storage outlives the kernels already enqueued
