@@ -5,6 +5,7 @@ import pytest
 
 import tl_b200 as tl
 from tl_b200 import synth
+from test_launch_plans_cpu import gemm_plan
 
 pytestmark = pytest.mark.gpu
 LOGIT_TOL = 2e-2
@@ -253,6 +254,25 @@ def test_prefill_tensor_core_attention_chunks_and_offsets():
     assert a == b
     assert relerr(la, dec2.logits()) < 2e-3
     assert dec.generate(a, 370, 8) == dec2.generate(b, 370, 8)
+
+
+def test_prefill_pair_of_ctas_straddles_weights():
+    """1100 tokens at once: q, k and v (32 + 1 + 1 row tiles) share a launch in tiles of 320 rows by pairs of CTAs, one of which
+    has k's tile in one CTA and v's in the other.  The same prompt 100 tokens at a time runs on single CTAs; both round
+    operands to f16."""
+    assert gemm_plan(1100, 4352, 512) == (320, 1) and gemm_plan(100, 4352, 512)[0] <= 256
+    cfg = dict(n_layers=1, d_model=512, n_heads=64, n_kv_heads=2, head_dim=64, ffn=512, vocab=300, eps=1e-5, rope_base=10000.0, attn_scale=0.125)
+    tens = synth.llama_tensors(cfg, 31, synth.Q8_0, synth.Q8_0)
+    toks = [int(v) for v in np.random.default_rng(32).integers(0, cfg["vocab"], 1100)]
+    want = [0, 319, 320, 500, 959, 1099]
+    whole = tl.Decoder(cfg, tl.map_from_tensors(tens), kv_f16=True, max_seq=1100).prefill_logits(toks, 0, want=want)
+    dec = tl.Decoder(cfg, tl.map_from_tensors(tens), kv_f16=True, max_seq=1100)
+    for off in range(0, 1100, 100):
+        here = [w - off for w in want if off <= w < off + 100]
+        got = dec.prefill_logits(toks[off:off + 100], off, want=here)
+        for w, lg in zip(here, got):
+            ref = whole[want.index(off + w)]
+            assert np.linalg.norm(lg - ref) < 2e-3 * np.linalg.norm(ref), off + w
 
 
 def test_prefill_f32_cache_head_dim_128():

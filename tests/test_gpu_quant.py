@@ -5,6 +5,7 @@ import pytest
 
 import tl_b200 as tl
 from tl_b200 import synth
+from test_launch_plans_cpu import gemm_plan
 
 pytestmark = pytest.mark.gpu
 
@@ -218,9 +219,31 @@ def test_qgemm_matches_oracle(orc, t, n, k, m):
 @pytest.mark.parametrize("t", TYPES)
 @pytest.mark.parametrize("n,k,m", [(128, 256, 129), (300, 512, 256), (257, 768, 257), (1000, 2304, 333), (640, 1024, 384), (129, 4096, 385), (2000, 512, 769)])
 def test_qgemm_pairs_of_ctas(orc, t, n, k, m):
-    """More than 128 rows run on pairs of CTAs: an odd number of row tiles, one and two accumulators, token tiles that end
-    inside either CTA's half or before it begins, K ranges of unequal length."""
+    """More than 128 rows on few row tiles run in token tiles of 128 to 256: one tile and several, the last one ragged, an odd
+    number of row tiles, several K ranges (129 x 4096)."""
     rng = np.random.default_rng(5100 + t + n + m)
+    w = synth.random_quant(t, n, k, rng)
+    x = rng.standard_normal((m, k), dtype=np.float32)
+    x[m // 2] *= 300.0
+    q = tl.QTensor.from_gguf_bytes(t, n, k, w)
+    got = tl.Tensor.from_numpy(x).matmul_quantized(q).numpy()
+    again = tl.Tensor.from_numpy(x).matmul_quantized(q).numpy()
+    np.testing.assert_array_equal(got.view(np.uint32), again.view(np.uint32))
+    ref = x.astype(np.float64) @ q.dequantize().numpy().astype(np.float64).T
+    assert got.shape == (m, n)
+    for i in range(m):
+        assert relerr(got[i], ref[i]) < GEMM_TOL, i
+
+
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("n,k,m,plan", [(9530, 2048, 257, (320, 1)), (9530, 2304, 333, (384, 1)), (11170, 2048, 384, (384, 1)), (6000, 2048, 777, (320, 1)),
+                                        (5000, 2304, 1100, (384, 1)), (5940, 8192, 257, (320, 3)), (5000, 8192, 333, (384, 3))])
+def test_qgemm_wide_tiles_by_pairs(orc, t, n, k, m, plan):
+    """Tiles of 320 and 384 rows by pairs of CTAs, two accumulators: K longer than the activation ring (8 or 9 steps of 64), an
+    odd number of row tiles (9530, 5940) and a ragged last one, token tiles that end inside either CTA's part of either
+    accumulator or leave it empty, and K ranges of unequal length."""
+    assert gemm_plan(m, n, k) == plan
+    rng = np.random.default_rng(5500 + t + n + m)
     w = synth.random_quant(t, n, k, rng)
     x = rng.standard_normal((m, k), dtype=np.float32)
     x[m // 2] *= 300.0
@@ -300,9 +323,8 @@ def test_few_rows_kernel_shapes(orc, t, n, k):
 @pytest.mark.parametrize("t", TYPES)
 @pytest.mark.parametrize("m", [777, 1100])
 def test_qgemm_two_accumulators_ragged_rows(orc, t, m):
-    """148 row tiles x more than 512 activation rows: the GEMM gives each CTA 512 rows as two accumulators.  777 rows leave
-    the last CTA 9 rows in its second accumulator, 1100 rows leave the last CTA no second accumulator at all.  Sampled
-    weight rows against the oracle, every activation row."""
+    """148 row tiles x more than 512 activation rows, in tiles of 320 (777 rows: the last has 137, its second accumulator none)
+    and 384 (1100: the last has 332).  Sampled weight rows against the oracle, every activation row."""
     n, k = 148 * 128, 512
     rng = np.random.default_rng(6000 + t + m)
     w = synth.random_quant(t, n, k, rng)

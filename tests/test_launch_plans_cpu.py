@@ -32,3 +32,44 @@ def test_matvec_rows_that_go_in_smaller_groups():
     """Lengths of tests/test_gpu_quant.py that fit two rows or one, but neither three nor four."""
     for t, units, n, most in [(synth.Q8_0, 41, 40, 3), (synth.Q8_0, 43, 300, 3), (synth.Q8_0, 46, 2048, 3), (synth.Q8_0, 53, 128256, 1), (synth.Q6_K, 53, 40, 3)]:
         assert [matvec_slices(t, n, 256 * units, m) > 0 for m in (1, 2, 3, 4)] == [m <= most for m in (1, 2, 3, 4)], (t, units, n)
+
+
+def gemm_plan(m, n, k):
+    f = _lib.lib().tlb_gemm_plan
+    f.restype, f.argtypes = None, [C.c_int64] * 4 + [C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]
+    nt, splits = C.c_int(), C.c_int()
+    f(m, (n + 127) // 128, k // 256, n, SMS, C.byref(nt), C.byref(splits))
+    return nt.value, splits.value
+
+
+def test_gemm_plans_are_launchable():
+    """Tiles that an MMA takes (columns in steps of 16, of 64 where two CTAs halve two accumulators), K ranges of four units or
+    more, scratch for the partial sums that stays small beside the outputs' own size or a wave of tiles, a grid within its limit."""
+    for n in (1, 128, 256, 1000, 2048, 4096, 5632, 14336, 28672, 128256):
+        for k in (256, 768, 1024, 2048, 2304, 4096, 8192, 14336, 28672):
+            for m in (17, 31, 64, 65, 100, 128, 129, 160, 255, 256, 257, 300, 333, 384, 385, 512, 513, 769, 1000, 1536, 2048, 2821, 4096, 10000, 9000000):
+                nt, splits = gemm_plan(m, n, k)
+                assert nt == (m + 15) // 16 * 16 if m <= 128 else nt in (128, 160, 192, 224, 256, 320, 384), (n, k, m)
+                assert splits == 1 or 4 * splits <= k // 256 and splits <= (16 if m <= 128 else 8), (n, k, m)
+                assert splits * m * n <= max(2 * m * n, 16 * SMS * 128 * 384), (n, k, m)
+                assert (m + nt - 1) // nt <= 65535, (n, k, m)
+
+
+@pytest.mark.parametrize("n,k,m,plans", [
+    # plans within 2 % of the fastest of all measured for Q4_K on a B200, and one that took the time given
+    (256, 2048, 4096, [(128, 1)]),                          # 34.0 us; 384 rows: 44.5
+    (2048, 2048, 768, [(128, 1)]),                          # 26.8 us; 256 rows: 28.8
+    (2048, 2048, 4096, [(256, 1)]),                         # 60.5 us; 320 rows: 73.9
+    (5632, 2048, 4096, [(256, 1)]),                         # 128 us; 384 rows: 137
+    (4096, 4096, 384, [(128, 1)]),                          # 39.2 us; 192 rows: 41.1
+    (4096, 4096, 1536, [(384, 1)]),                         # 60.2 us; 256 rows: 80.4
+    (14336, 4096, 333, [(384, 1)]),                         # 55.7 us; 192 rows: 74.1
+    (14336, 4096, 512, [(256, 1)]),                         # 79.9 us; 192 rows: 107
+    (14336, 4096, 1024, [(256, 1)]),                        # 149 us; 384 rows: 154
+    (14336, 4096, 4096, [(384, 1)]),                        # 461 us; 256 rows: 488
+    (4096, 14336, 256, [(256, 4)]),                         # 62 us; in one K range: 104
+    (4096, 14336, 512, [(256, 2)]),                         # 90.6 us; in one K range: 111
+    (4096, 14336, 4096, [(256, 1)]),                        # 512 us; 320 rows: 534
+])
+def test_gemm_plans_as_measured(n, k, m, plans):
+    assert gemm_plan(m, n, k) in plans
