@@ -10,10 +10,10 @@ SMS, SMEM = 148, 227 * 1024          # a B200
 TYPES = [synth.Q4_0, synth.Q8_0, synth.Q4_K, synth.Q6_K]
 
 
-def matvec_slices(t, n, k, m):
+def matvec_slices(t, n, k, m, few=0):
     f = _lib.lib().tlb_matvec_slices
-    f.restype, f.argtypes = C.c_int, [C.c_int, C.c_int64, C.c_int64, C.c_int, C.c_int, C.c_size_t]
-    return f(t, n, k, m, SMS, SMEM)
+    f.restype, f.argtypes = C.c_int, [C.c_int, C.c_int64, C.c_int64, C.c_int, C.c_int, C.c_int, C.c_size_t]
+    return f(t, n, k, m, few, SMS, SMEM)
 
 
 @pytest.mark.parametrize("t", TYPES)
@@ -32,6 +32,17 @@ def test_matvec_rows_that_go_in_smaller_groups():
     """Lengths of tests/test_gpu_quant.py that fit two rows or one, but neither three nor four."""
     for t, units, n, most in [(synth.Q8_0, 41, 40, 3), (synth.Q8_0, 43, 300, 3), (synth.Q8_0, 46, 2048, 3), (synth.Q8_0, 53, 128256, 1), (synth.Q6_K, 53, 40, 3)]:
         assert [matvec_slices(t, n, 256 * units, m) > 0 for m in (1, 2, 3, 4)] == [m <= most for m in (1, 2, 3, 4)], (t, units, n)
+
+
+def test_chains_of_short_launches_as_measured():
+    """Eight warps a CTA where a decode layer was faster with them: rows of 2048 or less, launches of up to 80 units per SM."""
+    f = _lib.lib().tlb_matvec_few
+    f.restype, f.argtypes = C.c_int, [C.c_int64, C.c_int64, C.c_int]
+    for d_model, units, few in [(1024, 14, 1), (1536, 21, 1), (2048, 38, 1), (2048, 76, 1), (2048, 194, 0), (2304, 35, 0), (2560, 35, 0), (3072, 83, 0), (4096, 28, 0), (4096, 38, 0)]:
+        assert f(d_model, units * SMS, SMS) == few, (d_model, units)
+    # gate|up of width 1536 (31.9 us a layer unsliced, 34.8 in two slices), down of width 2048 (sliced: 34.8, unsliced: 39)
+    assert matvec_slices(synth.Q4_K, 2 * 4096, 1536, 1, few=1) == 1
+    assert matvec_slices(synth.Q4_K, 2048, 5632, 1, few=1) > 1
 
 
 def gemm_plan(m, n, k):

@@ -397,16 +397,16 @@ tlb_status enqueue_step_tp(tlb_decoder *d)
     return enqueue_head(d, nullptr, d->xa, d->part, d->xb);   // xb = xa + sum: the residual before output_norm
 }
 
-// Whether every linear layer of a step has so few units (16 rows x 256 weights) per SM that its launch is made of fixed costs.
+// Whether a step's layers are a chain of short launches, which run with eight warps a CTA (matvec_few)
 bool short_launches(const tlb_decoder *d)
 {
-    const int64_t most = 48 * (int64_t)ctx()->sm_count;
     auto units = [](const tlb_qtensor *w) { return (int64_t)w->n_tiles * w->upt; };
+    int64_t most = 0;
     for (int l = 0; l < d->cfg.n_layers; l++) {
         const LayerW &w = d->layers[l];
-        if (units(w.q) + units(w.k) + units(w.v) > most || units(w.o) > most || units(w.gu) > most || units(w.down) > most) return false;
+        for (int64_t u : {units(w.q) + units(w.k) + units(w.v), units(w.o), units(w.gu), units(w.down)}) most = std::max(most, u);
     }
-    return true;
+    return matvec_few(d->cfg.d_model, most, ctx()->sm_count);
 }
 
 tlb_status enqueue_step(tlb_decoder *d)

@@ -565,20 +565,32 @@ static double slice_cost(int type, int m, int64_t tiles, int upt, int upi, int s
     // Measured on the Llama-3-8B shapes: the end of a sliced launch (fence, counts, reading the slices back)
     // costs ~3 us; assembling tiles in shared memory costs a block barrier, which shows (~2 us of waiting
     // for the slowest warp) only when warps have so few units that their skew matters.
-    // Three or four rows in several items per warp pay far more (14336 x 4096 Q8_0, four rows: 43 us in four slices, 23 in one).
+    // Three or four rows in several items per warp pay far more (14336 x 4096 Q8_0, four rows: 43 us in four slices, 23 in one),
+    // eight warps a little (a layer of width 1536 and 21 units per SM: 34.8 us with gate|up in two slices, 31.9 in one; 500 more
+    // instead of 200 costs what slices gain elsewhere, 38.1 instead of 34.8 for width 2048 and 38 units).
     const bool few = (ipc * upi + nw - 1) / nw < 4;
-    const double fold = kb == 1 ? (few ? 600.0 : 100.0) : 600.0 + 16.0 * kb + (m >= 3 && ipw > 1 ? 3000.0 : 0.0);
+    const double fold = kb == 1 ? (few ? 600.0 : 100.0) : 600.0 + 16.0 * kb + (m >= 3 && ipw > 1 ? 3000.0 : 0.0) + (nw == kFewWarps ? 200.0 : 0.0);
     return stream + quant + fold;
 }
 
-// Warps of a CTA.  With one unit or less for each of eight warps the other eight only issue the prologue again: four calls of
+// Warps of a CTA.  A short launch is bounded by the instructions a warp issues outside its units, and eight warps issue half
+// of them; with one unit or less for each of eight warps the other eight only issue the prologue again: four calls of
 // 2048 x 2048 with norms between them take 49.2 us with sixteen and 46 with eight.  From two units per warp on, a lone launch
-// is faster with sixteen (2048 x 5632: 9.8 against 12.5 us), but in a chain of nothing but short launches eight leave the next
-// launch room to become resident (MatvecJob::few; TinyLlama shapes, 32 steps: 24.3 against 23.5 ms).
+// is faster with sixteen (2048 x 5632: 9.8 against 12.5 us).
 static int warps_for(const MatvecJob &job, int64_t tiles, int upt, int sm_count)
 {
     return job.m == 1 && (job.few || (!job.pdl && tiles * upt <= (int64_t)kFewWarps * sm_count)) ? kFewWarps : kWarps;
 }
+
+// In a chain, where launches follow each other at once, eight warps gain up to larger launches, if all of them have eight and as
+// long as they prepare a row in one pass: kKeep blocks of 256 for each two warps, 2048.  Microseconds a layer (Q4_K / Q8_0, f16
+// cache of 200 rows) with sixteen, and with eight, by width and units per SM of the largest launch:
+//   2048, 38 units: 37.2 / 37.7, 35.3 / 35.0;  76: 40.6 / 42.6, 39.5 / 40.6;  111: 42.6 / 47.9, 42.7 / 45.3;  194: 50.5 / 60.3, 54.5 / 61.2
+//   1536, 21 units: 33.2 / 33.8, 31.9 / 31.6;  1024, 14: 30.2 / 29.5, 27.9 / 27.4
+//   2560, 35 units: 40.7 / 41.5, 42.6 / 41.1;  3072, 83: 43.6 / 48.0, 46.8 / 51.1;  4096, 38: 43.0 / 44.6, 48.0 / 50.2
+// Eight warps for some launches of a layer and sixteen for the others is slower than either (2048, 38 units: gate|up alone +1.1).
+bool matvec_few(int64_t d_model, int64_t units, int sm) { return d_model <= kFewWarps / 2 * kKeep * 256 && units <= (int64_t)80 * sm; }
+extern "C" int tlb_matvec_few(int64_t d_model, int64_t units, int sm) { return matvec_few(d_model, units, sm); }
 
 // How a launch of `tiles` 16-row tiles (all tensors) over upt units of K is laid out with kb K-slices.
 struct MvGeometry {
@@ -643,12 +655,15 @@ static int plan_slices(int type, int upt, int m, int64_t tiles, int max_slices, 
     return best;
 }
 
-// K-slices of one row group of tlb_qtensor_matmul over a weight of n rows; 0: no launch of this many rows fits.
-extern "C" int tlb_matvec_slices(int type, int64_t n, int64_t k, int m, int sm, size_t smem_max)
+// K-slices of a launch of m rows over a weight of n rows, on its own or in a chain of short ones; 0: no such launch fits.
+extern "C" int tlb_matvec_slices(int type, int64_t n, int64_t k, int m, int few, int sm, size_t smem_max)
 {
     const int64_t tiles = (n + 15) / 16;
     const int upt = (int)(k / 256);
-    const int nw = m == 1 && tiles * upt <= (int64_t)kFewWarps * sm ? kFewWarps : kWarps;
+    MatvecJob job;
+    job.m = m;
+    job.few = few != 0;
+    const int nw = warps_for(job, tiles, upt, sm);
     return plan_slices(type, upt, m, tiles, kMaxSlices, nw, sm, smem_max, 0, 0);
 }
 

@@ -204,7 +204,7 @@ struct MatvecJob {
     const float *emb_table = nullptr; // ADD_NORM with token lookup: x = emb_table[*token * K ...]
     const int *token = nullptr;
     bool pdl = false;                // launch with programmatic stream serialization
-    bool few = false;                // m == 1: part of a chain of short launches (CTAs of eight warps)
+    bool few = false;                // m == 1: part of a chain of short launches (matvec_few): CTAs of eight warps
     // ADD_NORM without the statistics pass: x already holds the whole residual and ssq_parts[0 .. n_parts)
     // are partial sums of its squares left by the launch that produced it (finish == FIN_RESID there)
     const float *ssq_parts = nullptr;
@@ -228,6 +228,8 @@ struct MatvecJob {
     bool dry_run = false;            // validate and plan only: tells whether the launch would be accepted
 };
 tlb_status launch_qmatvec(const MatvecJob &job);
+// whether a decode chain over rows of d_model, whose largest launch has `units` units, runs with eight warps a CTA
+bool matvec_few(int64_t d_model, int64_t units, int sm);
 size_t qmatvec_max_k(int m);   // largest K the single-pass kernel supports for m activation rows
 
 // ops.cu
