@@ -292,6 +292,30 @@ def test_prefill_f32_cache_head_dim_128():
     assert a_dec.generate(a, 150, 6) == b_dec.generate(b, 150, 6)
 
 
+def _matvec_kernels(call):
+    """Names of the matvec kernels that a call launches, without their arguments."""
+    import torch
+    call()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+        tl.sync()
+    names = {e.key.split("(")[0] for e in prof.key_averages()}
+    if not names:
+        pytest.skip("no kernel trace on this machine")
+    return {n for n in names if "qmatvec_kernel" in n}
+
+
+@pytest.mark.parametrize("d_model", [512, 4096])      # a chain of short launches, and one of ordinary ones
+def test_time_kernel_times_the_kernels_of_the_chain(d_model):
+    cfg = dict(n_layers=1, d_model=d_model, n_heads=d_model // 64, n_kv_heads=d_model // 64, head_dim=64, ffn=1024, vocab=300, eps=1e-5, rope_base=10000.0,
+               attn_scale=0.125)
+    dec = tl.Decoder(cfg, tl.map_from_tensors(synth.llama_tensors(cfg, 33, synth.Q4_K, synth.Q8_0)), kv_f16=True, max_seq=32)
+    chain = _matvec_kernels(lambda: dec.step(3, 0))
+    for which in ("qkv", "o", "gate_up", "down", "head"):
+        timed = _matvec_kernels(lambda: dec.time_kernel(which, 1, 2))
+        assert len(timed) == 1 and timed <= chain, (which, timed, chain)
+
+
 def test_decoder_sampling_on_device(orc):
     """tlb_decoder_sample_top_p on the session's logits = the tensor-level sampler on the same logits = the oracle."""
     ref, dec, wmap = build(orc, SMALL, 21, synth.Q4_K, synth.Q6_K, True, 32)

@@ -1152,7 +1152,8 @@ tlb_status tlb_decoder_time_kernel(tlb_decoder *d, const char *which, int copies
         } else {
             j.n_w = 1; set_w(j, 0, d->head, o); j.type = d->head->type; j.k = dm; bytes = d->head->nbytes();
         }
-        j.pdl = d->pdl;   // as in the decode chain: a launch's set-up overlaps its predecessor
+        j.pdl = d->pdl;   // as in the decode chain: a launch's set-up overlaps its predecessor, and the layers' have as many warps
+        j.few = w != "head" && short_launches(d);
         st = launch_qmatvec(j);
     }
     cudaEventRecord(e1, ctx()->stream);
