@@ -84,3 +84,20 @@ def test_gemm_plans_are_launchable():
 ])
 def test_gemm_plans_as_measured(n, k, m, plans):
     assert gemm_plan(m, n, k) in plans
+
+
+def dense_matvec_plan(n, k, slots=1):
+    """(chunks in flight, most chunks of a tile per warp, most tiles per CTA) of a bf16 layer of one row"""
+    f = _lib.lib().tlb_dense_matvec_plan
+    f.restype, f.argtypes = C.c_int, [C.c_int] * 4 + [C.c_size_t] + [C.POINTER(C.c_int)] * 3
+    warps, chunks, rounds = C.c_int(), C.c_int(), C.c_int()
+    depth = f(n, k, slots, SMS, SMEM, C.byref(warps), C.byref(chunks), C.byref(rounds))
+    return depth, chunks.value, rounds.value
+
+
+def test_dense_matvec_rings_fit():
+    for k in list(range(1, 49153, 997)) + [8192, 45056, 45312, 45568, 49152]:
+        for n in (1, 40, 1000, 2048, 4096, 8192, 32768):
+            depth = dense_matvec_plan(n, k)[0]
+            row = (k + 255) // 256 * 1024
+            assert depth in (1, 2, 3) and row + depth * 16384 + 4096 <= SMEM, (n, k)      # 4 KB: the kernel's static part at most

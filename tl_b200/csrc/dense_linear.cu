@@ -791,22 +791,43 @@ tlb_status launched(const char *what)
     return TLB_OK;
 }
 
+// CTAs that fit beside each other with a row of `row` bytes and so many weight chunks in flight, for each of `slots` experts
+int matvec_ctas(size_t row, int depth, int slots, int sm)
+{
+    return sm * std::max(1, std::min(4, (int)(((size_t)220 << 10) / (row + depth * kMvStage + 2048)))) / slots;
+}
+
+// Two chunks deep where that lets every tile have a CTA at once and three do not; one beside a row that fills shared memory
+// (kMvStatic: what the kernel has besides, 2.3 KB with the norm in groups).
+constexpr size_t kMvStatic = 4096;
+int matvec_depth(size_t row, int tiles, int slots, int sm, size_t smem_max)
+{
+    if (row + kMvDepth * kMvStage + kMvStatic > smem_max) return 1;
+    return tiles > matvec_ctas(row, kMvDepth, slots, sm) && tiles <= matvec_ctas(row, 2, slots, sm) ? 2 : kMvDepth;
+}
+
+// the fewest warps per row group that still give every SM two tiles
+int matvec_warps(int n, int nch, int slots, int sm)
+{
+    int wk = 1;
+    while (wk < 8 && (n + kMvWarps / wk * kMvRows - 1) / (kMvWarps / wk * kMvRows) * slots < 2 * sm && wk * 2 <= nch) wk *= 2;
+    return wk;
+}
+
 template <int PRO, int WK>
 tlb_status run_matvec(DenseMvParams p, bool pdl)
 {
     Context *c = ctx();
     const size_t row = ((size_t)p.nch * kMvChunk + (PRO == DPRO_EXPERT ? route_scratch_floats(p.route) : 0)) * sizeof(float);
     const int slots = PRO == DPRO_EXPERT ? p.route.top : 1;
-    auto ctas = [&](int depth) { return c->sm_count * std::max(1, std::min(4, (int)(((size_t)220 << 10) / (row + depth * kMvStage + 2048)))) / slots; };
-    // two chunks deep where that lets every tile have a CTA at once and three do not; one beside a row that fills shared memory
-    p.depth = row + kMvDepth * kMvStage + 2048 > c->smem_optin ? 1 : p.tiles > ctas(kMvDepth) && p.tiles <= ctas(2) ? 2 : kMvDepth;
+    p.depth = matvec_depth(row, p.tiles, slots, c->sm_count, c->smem_optin);
     const size_t smem = row + p.depth * kMvStage;
     static size_t allowed = 40 << 10;      // with the static part, under the 48 KB that need no asking
     if (smem > allowed) {
         TLB_CUDA(cudaFuncSetAttribute(dense_matvec_kernel<PRO, WK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         allowed = smem;
     }
-    const int grid = std::min(p.tiles, std::max(1, ctas(p.depth)));
+    const int grid = std::min(p.tiles, std::max(1, matvec_ctas(row, p.depth, slots, c->sm_count)));
     TLB_CUDA(launch_chained(dense_matvec_kernel<PRO, WK>, dim3(grid, slots), dim3(kMvThreads), smem, pdl, p));
     count_launch();
     return TLB_OK;
@@ -815,12 +836,8 @@ tlb_status run_matvec(DenseMvParams p, bool pdl)
 template <int PRO>
 tlb_status pick_matvec(DenseMvParams p, bool pdl)
 {
-    // the fewest warps per row group that still give every SM two tiles
-    int wk = 1;
-    auto tiles = [&](int w) { return (p.n + kMvWarps / w * kMvRows - 1) / (kMvWarps / w * kMvRows); };
-    const int slots = PRO == DPRO_EXPERT ? p.route.top : 1;
-    while (wk < 8 && tiles(wk) * slots < 2 * ctx()->sm_count && wk * 2 <= p.nch) wk *= 2;
-    p.tiles = tiles(wk);
+    const int wk = matvec_warps(p.n, p.nch, PRO == DPRO_EXPERT ? p.route.top : 1, ctx()->sm_count);
+    p.tiles = (p.n + kMvWarps / wk * kMvRows - 1) / (kMvWarps / wk * kMvRows);
     switch (wk) {
     case 1: return run_matvec<PRO, 1>(p, pdl);
     case 2: return run_matvec<PRO, 2>(p, pdl);
@@ -830,6 +847,19 @@ tlb_status pick_matvec(DenseMvParams p, bool pdl)
 }
 
 }  // namespace
+
+// How a layer of n outputs over k inputs (the chosen expert's of `slots`) runs: warps that share a row group's columns, weight
+// chunks in flight (returned), the most chunks one warp reads of a tile, the most tiles a CTA takes.
+extern "C" int tlb_dense_matvec_plan(int n, int k, int slots, int sm, size_t smem_max, int *warps, int *out_chunks, int *out_rounds)
+{
+    const int nch = (k + kMvChunk - 1) / kMvChunk, wk = matvec_warps(n, nch, slots, sm), rows = kMvWarps / wk * kMvRows, tiles = (n + rows - 1) / rows;
+    const size_t row = (size_t)nch * kMvChunk * sizeof(float);
+    const int depth = matvec_depth(row, tiles, slots, sm, smem_max), grid = std::min(tiles, std::max(1, matvec_ctas(row, depth, slots, sm)));
+    *warps = wk;
+    *out_chunks = (nch + wk - 1) / wk;
+    *out_rounds = (tiles + grid - 1) / grid;
+    return depth;
+}
 
 bool dense_matvec_supported(int k) { return k >= 1 && k <= 48 * 1024; }
 
