@@ -11,6 +11,7 @@ import layered_session as S
 import plain_layers as P
 import tl_b200 as tl
 from layered_session import decode, err, greedy, run_portions, toks
+from test_launch_plans_cpu import dense_matvec_plan
 from tl_b200 import synth
 
 pytestmark = pytest.mark.gpu
@@ -95,6 +96,20 @@ def test_norms_feed_forward_and_scales(width, ff, vocab, eps, f32):
     assert close(d.prefill_logits(t[:33]), want[:33], f32)
     assert close(decode(d, t[33:], 33), want[33:], f32)
     assert np.allclose(d.hidden(), m_hidden(m, t), atol=(1e-4 if f32 else 6e-2) * np.max(np.abs(m_hidden(m, t))))
+
+
+@pytest.mark.parametrize("width,ff,vocab", [(2048, 4096, 20000), (64, 47104, 131), (72, 8999, 131), (8450, 60, 131)])
+def test_weight_ring_of_the_decode_matvec(width, ff, vocab):
+    """One, two and three weight chunks in flight, with more chunks of a tile than that (a slot read is filled again) and tiles
+    that follow one another in a CTA; rows that are not whole float4 and rows longer than the registers hold (8192)."""
+    plans = {(2048, 4096, 20000): [(4096, 2048, 2, 2, 1), (2048, 4096, 2, 2, 1), (20000, 2048, 3, 8, 2)], (64, 47104, 131): [(64, 47104, 1, 23, 1)],
+             (72, 8999, 131): [(72, 8999, 3, 5, 1)], (8450, 60, 131): [(131, 8450, 3, 5, 1)]}
+    for n, k, *plan in plans[width, ff, vocab]:
+        assert dense_matvec_plan(n, k) == tuple(plan), (n, k)
+    m = Model(config([retention()], width=width, ff=ff, vocab=vocab), seed=6)
+    t = toks(5, vocab)
+    d = m.dec(True)
+    assert close(decode(d, t, 0), m.ref(t), True)
 
 
 def m_hidden(m, t):

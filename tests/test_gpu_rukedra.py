@@ -14,6 +14,7 @@ import layered_session as S
 import plain_rukedra as P
 import tl_b200 as tl
 from layered_session import decode, err, greedy, run_portions, toks
+from test_launch_plans_cpu import dense_matvec_plan
 from tl_b200 import synth
 
 pytestmark = pytest.mark.gpu
@@ -172,6 +173,19 @@ def test_a_width_beyond_the_registers_of_a_launch(f32):
     d = m.dec(f32)
     assert close(d.prefill_logits(t[:9]), want[:9], f32)
     assert close(decode(d, t[9:], 9), want[9:], f32)
+
+
+@pytest.mark.parametrize("width,ff,experts,top,shared,vocab", [(2500, 400, 12, 8, 100, 9500), (72, 1000, 16, 8, 700, 131)])
+def test_weight_ring_of_the_experts(width, ff, experts, top, shared, vocab):
+    """More weight chunks per warp than are in flight: the experts' first layers and the head after a norm in groups (2500), and the
+    chosen experts' and the shared one's activations side by side, 35 chunks over eight warps (72)."""
+    if width == 2500:
+        assert dense_matvec_plan(2 * ff, width, top) == (3, 5, 1) and dense_matvec_plan(vocab, width) == (3, 10, 1)
+    else:
+        assert dense_matvec_plan(width, 256 * (top * 4 + 3)) == (3, 5, 1)
+    m = Model(config([(direct(), moe(experts=experts, top=top, ff=ff, groups=None, shared=shared))], width=width, groups=5 if width == 2500 else 3, vocab=vocab), seed=9)
+    t = toks(5, vocab)
+    assert close(decode(m.dec(True), t, 0), m.ref(t), True)
 
 
 def test_the_gate_and_the_norms_matter():
