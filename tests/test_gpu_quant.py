@@ -1,10 +1,14 @@
 """GPU parity: dequantisation (bit-exact) and the dequant-fused matvec against the CPU oracle,
 through the C ABI."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 import tl_b200 as tl
-from tl_b200 import synth
+from tl_b200 import _lib, synth
 from test_launch_plans_cpu import gemm_plan
 
 pytestmark = pytest.mark.gpu
@@ -255,6 +259,56 @@ def test_qgemm_wide_tiles_by_pairs(orc, t, n, k, m, plan):
     assert got.shape == (m, n)
     for i in range(m):
         assert relerr(got[i], ref[i]) < GEMM_TOL, i
+
+
+# stands before the library's allocator and turns down requests of one size
+NO_ROOM = r"""
+#include <cstddef>
+#include <cstdlib>
+#include <dlfcn.h>
+extern "C" { size_t turned_down_bytes = 0; int turned_down = 0; }
+namespace tlb {
+struct Storage;
+Storage *storage_alloc(size_t bytes)
+{
+    using Fn = Storage *(*)(size_t);
+    static Fn real = (Fn)dlsym(dlopen(getenv("TLB_SO"), RTLD_NOW | RTLD_NOLOAD), "_ZN3tlb13storage_allocEm");
+    if (bytes == turned_down_bytes) { turned_down++; return nullptr; }
+    return real(bytes);
+}
+}
+"""
+NO_ROOM_RUN = r"""
+import ctypes, sys
+import numpy as np
+import tl_b200 as tl
+from tl_b200 import synth
+n, k, m, splits = [int(a) for a in sys.argv[2:6]]
+shim = ctypes.CDLL(sys.argv[1])
+rng = np.random.default_rng(91)
+q = tl.QTensor.from_gguf_bytes(synth.Q8_0, n, k, synth.random_quant(synth.Q8_0, n, k, rng))
+x = tl.Tensor.from_numpy(rng.standard_normal((m, k), dtype=np.float32))
+a = x.matmul_quantized(q).numpy()
+ctypes.c_size_t.in_dll(shim, "turned_down_bytes").value = 4 * splits * m * n
+b = x.matmul_quantized(q).numpy()
+c = x.matmul_quantized(q).numpy()
+assert ctypes.c_int.in_dll(shim, "turned_down").value == 2
+assert np.array_equal(b, c) and np.max(np.abs(a - b)) < 2e-5 * np.max(np.abs(a))
+print("whole")
+"""
+
+
+def test_qgemm_without_room_for_partial_sums(tmp_path):
+    """A product planned in several K ranges whose scratch cannot be had is computed in one."""
+    n, k, m = 1024, 8192, 256
+    splits = gemm_plan(m, n, k)[1]
+    assert splits > 1
+    (tmp_path / "shim.cpp").write_text(NO_ROOM)
+    shim = str(tmp_path / "shim.so")
+    subprocess.check_call(["g++", "-shared", "-fPIC", "-O1", "-o", shim, str(tmp_path / "shim.cpp"), "-ldl"])
+    env = dict(os.environ, LD_PRELOAD=shim, TLB_SO=_lib.SO_PATH, PYTHONPATH=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    r = subprocess.run([sys.executable, "-c", NO_ROOM_RUN, shim] + [str(v) for v in (n, k, m, splits)], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "whole" in r.stdout, r.stdout + r.stderr
 
 
 @pytest.mark.parametrize("t,n,k", [(synth.Q4_K, 4096, 4096), (synth.Q6_K, 16384, 4096), (synth.Q4_0, 2048, 5632), (synth.Q8_0, 2048, 2048)])
