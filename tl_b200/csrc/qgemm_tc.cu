@@ -74,7 +74,6 @@ struct GemmParams {
     int nt;                 // activation rows per CTA (MMA N)
     int nb;                 // depth of the activation ring (stages)
     int gs;                 // 64-wide K groups per stage: 1, or 4 (a whole 256-wide unit per barrier round) for tiles of up to 64 rows
-    int kt_total;           // K / 64
     int unit_bytes;
     const float *inv_scale; // [m]
     const float *resid;     // [m, n] added to the result, or null
@@ -176,25 +175,18 @@ struct Q4KRegs {
     uint4 q[2];
     uint4 h[2];
 };
-// 16 bytes / 2 bytes of a unit: from global memory through the read-only path (G), or from wherever the generic pointer
-// leads (a stage in shared memory)
-template <bool G> __device__ __forceinline__ uint4 ldq(const uint8_t *p)
-{
-    return G ? __ldg(reinterpret_cast<const uint4 *>(p)) : *reinterpret_cast<const uint4 *>(p);
-}
-template <bool G> __device__ __forceinline__ __half ldh(const uint8_t *p)
-{
-    return G ? __ldg(reinterpret_cast<const __half *>(p)) : *reinterpret_cast<const __half *>(p);
-}
+// 16 bytes / 2 bytes of a unit, through the read-only path
+__device__ __forceinline__ uint4 ldq(const uint8_t *p) { return __ldg(reinterpret_cast<const uint4 *>(p)); }
+__device__ __forceinline__ __half ldh(const uint8_t *p) { return __ldg(reinterpret_cast<const __half *>(p)); }
 
-template <int HALF, bool G = true>
+template <int HALF>
 __device__ __forceinline__ void unit_load(Q4KRegs &u, const uint8_t *unit, int lane)
 {
     const int r = lane >> 2;
 #pragma unroll
-    for (int gg = 0; gg < 2; gg++) u.q[gg] = ldq<G>(unit + (HALF * 2 + gg) * 512 + lane * 16);
-    u.h[0] = ldq<G>(unit + 2048 + r * 16);
-    u.h[1] = ldq<G>(unit + 2048 + (r + 8) * 16);
+    for (int gg = 0; gg < 2; gg++) u.q[gg] = ldq(unit + (HALF * 2 + gg) * 512 + lane * 16);
+    u.h[0] = ldq(unit + 2048 + r * 16);
+    u.h[1] = ldq(unit + 2048 + (r + 8) * 16);
 }
 // Dequantise 64-group g of the unit (rows r and r + 8 of the warp's sixteen): chunks 0, 1 are the low nibbles
 // (k = byte index), chunks 2, 3 the high ones (k = 32 + byte index).
@@ -226,16 +218,16 @@ struct Q6KRegs {
     uint4 sc[2];
     float d[2];
 };
-template <int HALF, bool G = true>
+template <int HALF>
 __device__ __forceinline__ void unit_load(Q6KRegs &u, const uint8_t *unit, int lane)
 {
     const int r = lane >> 2;
 #pragma unroll
     for (int hi = 0; hi < 2; hi++) {
-        u.ql[hi] = ldq<G>(unit + (hi * 2 + HALF) * 512 + lane * 16);
-        u.qh[hi] = ldq<G>(unit + 2048 + hi * 512 + lane * 16);
-        u.sc[hi] = ldq<G>(unit + 3072 + (r + 8 * hi) * 16);
-        u.d[hi] = __half2float(ldh<G>(unit + 3328 + (r + 8 * hi) * 2));
+        u.ql[hi] = ldq(unit + (hi * 2 + HALF) * 512 + lane * 16);
+        u.qh[hi] = ldq(unit + 2048 + hi * 512 + lane * 16);
+        u.sc[hi] = ldq(unit + 3072 + (r + 8 * hi) * 16);
+        u.d[hi] = __half2float(ldh(unit + 3328 + (r + 8 * hi) * 2));
     }
 }
 // 64-group g = (n, sub): k = 128 n + 64 sub + [0, 64).  sub 0 takes the low nibbles of ql and bits 0-3 of qh,
@@ -265,14 +257,14 @@ struct Q40Regs {
     uint4 q[2];
     uint4 d[2];   // eight f16 block scales of rows r and r + 8
 };
-template <int HALF, bool G = true>
+template <int HALF>
 __device__ __forceinline__ void unit_load(Q40Regs &u, const uint8_t *unit, int lane)
 {
     const int r = lane >> 2;
 #pragma unroll
-    for (int gg = 0; gg < 2; gg++) u.q[gg] = ldq<G>(unit + (HALF * 2 + gg) * 512 + lane * 16);
-    u.d[0] = ldq<G>(unit + 2048 + r * 16);
-    u.d[1] = ldq<G>(unit + 2048 + (r + 8) * 16);
+    for (int gg = 0; gg < 2; gg++) u.q[gg] = ldq(unit + (HALF * 2 + gg) * 512 + lane * 16);
+    u.d[0] = ldq(unit + 2048 + r * 16);
+    u.d[1] = ldq(unit + 2048 + (r + 8) * 16);
 }
 __device__ __forceinline__ uint32_t h2_pair(const uint4 &v, int i)   // i-th f16 of the 16 bytes, in both halves
 {
@@ -299,14 +291,14 @@ struct Q80Regs {
     uint4 q[4];
     uint4 d[2];
 };
-template <int HALF, bool G = true>
+template <int HALF>
 __device__ __forceinline__ void unit_load(Q80Regs &u, const uint8_t *unit, int lane)
 {
     const int r = lane >> 2;
 #pragma unroll
-    for (int i = 0; i < 4; i++) u.q[i] = ldq<G>(unit + (HALF * 4 + i) * 512 + lane * 16);
-    u.d[0] = ldq<G>(unit + 4096 + r * 16);
-    u.d[1] = ldq<G>(unit + 4096 + (r + 8) * 16);
+    for (int i = 0; i < 4; i++) u.q[i] = ldq(unit + (HALF * 4 + i) * 512 + lane * 16);
+    u.d[0] = ldq(unit + 4096 + r * 16);
+    u.d[1] = ldq(unit + 4096 + (r + 8) * 16);
 }
 __device__ __forceinline__ void unit_emit(const Q80Regs &u, int g, AFrag &f)
 {
@@ -626,44 +618,6 @@ template <> struct RawTraits<14> { static constexpr int kPair = 1; static conste
 template <> struct RawTraits<2> { static constexpr int kPair = 2; static constexpr bool kMins = false; };
 template <> struct RawTraits<8> { static constexpr int kPair = 2; static constexpr bool kMins = false; };
 
-// Q4_K: chunks 0, 1 = the low nibbles (sub-block 2 g), chunks 2, 3 = the high ones in place (sub-block 2 g + 1)
-__device__ __forceinline__ void unit_raw(const Q4KRegs &u, int g, AFrag &f, RawScales &sc)
-{
-#pragma unroll
-    for (int rs = 0; rs < 2; rs++) {
-        uint32_t scw, mw;
-        q4k_scales4(u.h[rs], g >= 2, scw, mw);
-        const float d = h2_to_f2(u.h[rs].x).x;
-        // (2^23 + sc) * d 2^24 - 2^23 d 2^24 = sc d 2^24, rounded once
-        const float d24 = d * kTwo24, d20 = d * kTwo20;
-        sc.s[rs][0] = fmaf(__uint_as_float(prmt(scw, 0x4B000000u, 0x7650u + ((2 * g) & 3))), d24, -8388608.f * d24);
-        sc.s[rs][1] = fmaf(__uint_as_float(prmt(scw, 0x4B000000u, 0x7650u + ((2 * g + 1) & 3))), d20, -8388608.f * d20);
-#pragma unroll
-        for (int jl = 0; jl < 2; jl++) {
-            const uint32_t wd = word_of(u.q[g & 1], rs * 2 + jl), w8 = wd >> 8;
-            f.v[4 * jl + 2 * rs] = wd & 0x000F000Fu;
-            f.v[4 * jl + 2 * rs + 1] = w8 & 0x000F000Fu;
-            f.v[4 * (2 + jl) + 2 * rs] = wd & 0x00F000F0u;
-            f.v[4 * (2 + jl) + 2 * rs + 1] = w8 & 0x00F000F0u;
-        }
-    }
-}
-// the minima of sub-blocks c and c + 4 of rows r, r + 8 as the A operand of the sums MMA, and dmin of both rows
-__device__ __forceinline__ void q4k_mins(const Q4KRegs &u, int c, uint32_t (&a)[4], float (&dmin)[2])
-{
-#pragma unroll
-    for (int rs = 0; rs < 2; rs++) {
-        uint32_t scw, mlo, mhi;
-        q4k_scales4(u.h[rs], false, scw, mlo);
-        q4k_scales4(u.h[rs], true, scw, mhi);
-        a[rs] = bf16_pair(byte_f(mlo, c));
-        a[2 + rs] = bf16_pair(byte_f(mhi, c));
-        dmin[rs] = h2_to_f2(u.h[rs].x).y;
-    }
-}
-
-template <class R> __device__ __forceinline__ void q4k_mins(const R &, int, uint32_t (&)[4], float (&)[2]) {}   // the other formats have no minima
-
 // Q6_K: every chunk has its own int8 scale; q - 32 in f16
 __device__ __forceinline__ void unit_raw(const Q6KRegs &u, int g, AFrag &f, RawScales &sc)
 {
@@ -743,7 +697,7 @@ constexpr int kRowsSumBytes = 16 * 8 * 4;                // their sums over the 
 struct RowsParams {
     const uint8_t *w[kGemmMaxW];
     float *out[kGemmMaxW];
-    int n[kGemmMaxW], n_tiles16[kGemmMaxW], tg_end[kGemmMaxW], tile0[kGemmMaxW];   // tile groups / first tile of weight i among all
+    int n[kGemmMaxW], n_tiles16[kGemmMaxW], tg_end[kGemmMaxW];   // tile groups up to and including weight i
     int n_w, upt, unit_bytes, stage_w, wstages, m;
     int tgroups, total, maxp;       // total = tgroups x upt unit steps, cut evenly over the CTAs; maxp: tile groups a CTA can touch
     int64_t k;
@@ -756,13 +710,6 @@ struct RowsParams {
 };
 
 // unit registers from a stage in shared memory (the layouts of unit_load above)
-template <int HALF> __device__ __forceinline__ void unit_load_s(Q4KRegs &u, uint32_t unit, int lane)
-{
-    const int r = lane >> 2;
-    for (int gg = 0; gg < 2; gg++) u.q[gg] = lds128(unit + (HALF * 2 + gg) * 512 + lane * 16);
-    u.h[0] = lds128(unit + 2048 + r * 16);
-    u.h[1] = lds128(unit + 2048 + (r + 8) * 16);
-}
 template <int HALF> __device__ __forceinline__ void unit_load_s(Q6KRegs &u, uint32_t unit, int lane)
 {
     const int r = lane >> 2;
@@ -1364,7 +1311,7 @@ tlb_status qrows_run(const tlb_qtensor *const *ws, int n_w, const GemmAct &a, fl
     if (!c) return TLB_ERR_DEVICE;
     const tlb_qtensor *w0 = ws[0];
     RowsParams p = {};
-    int tgroups = 0, tiles_all = 0;
+    int tgroups = 0;
     for (int i = 0; i < kGemmMaxW; i++) {
         const tlb_qtensor *w = i < n_w ? ws[i] : nullptr;
         if (w && (w->type != w0->type || w->k != a.k || w->n > INT32_MAX))
@@ -1373,8 +1320,7 @@ tlb_status qrows_run(const tlb_qtensor *const *ws, int n_w, const GemmAct &a, fl
         p.out[i] = w ? outs[i] : nullptr;
         p.n[i] = w ? (int)w->n : 0;
         p.n_tiles16[i] = w ? (int)w->n_tiles : 0;
-        p.tile0[i] = tiles_all;
-        if (w) { tgroups += (int)((w->n_tiles + kRowsWarps - 1) / kRowsWarps); tiles_all += (int)w->n_tiles; }
+        if (w) tgroups += (int)((w->n_tiles + kRowsWarps - 1) / kRowsWarps);
         p.tg_end[i] = tgroups;
     }
     if ((int64_t)tgroups * w0->upt > INT32_MAX / 256) return fail(TLB_ERR_SHAPE, "quantized matmul (few rows): weight too large");
@@ -1469,7 +1415,6 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
     p.gs = !pair && nt <= 64 ? 4 : 1;
     const int stage_b = (pair ? nt / 2 : nt) * 128 * p.gs;
     p.nb = std::max(p.gs == 4 ? 3 : 4, std::min(kGemmMaxSlots, kGemmBBytes / stage_b));
-    p.kt_total = (int)(a.k / kGemmBK);
     p.unit_bytes = qformat(w0->type)->unit_bytes;
     p.inv_scale = (const float *)a.inv->ptr;
     p.resid = resid;
