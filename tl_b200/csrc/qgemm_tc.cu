@@ -15,15 +15,17 @@
 //     producer warps (two per 16 weight rows, each taking two of a unit's four 64-wide groups) read the quantized
 //     units with coalesced 16-byte loads, dequantise in registers (f16 pair arithmetic on exact integers, see
 //     store4) and write their 16 rows x 64 K of a stage with one tcgen05.st (eight stages of 32 columns beside the
-//     accumulator's 256);
+//     accumulator's 256; four beside a pair's two accumulators of 192; three of 128 columns, a whole unit each, for tiles
+//     of up to 64 rows);
 //   * the activation tile is the B operand (MMA N = NT): f16 rows, brought into a shared-memory ring by TMA
 //     (cp.async.bulk.tensor.2d, 128-byte swizzle, rows past M filled with zeros).  The ring is as deep as shared
-//     memory allows (6 stages of 32 KB at NT = 256, 16 for narrow tiles): a TMA load takes ~1.5 us from request to
-//     arrival, so a K step can only be as short as that divided by the depth;
-//   * one thread issues tcgen05.mma (kind::f16, A from tensor memory, B from shared memory, f32 accumulate) for each
-//     64-wide K step as soon as its barrier has the eight producer warps' arrivals and the TMA bytes; one
-//     tcgen05.commit per K step reports its completion, which frees the weight stage for the producers (8 K steps
-//     later) and the activation stage for the TMA thread (ring depth later);
+//     memory allows (6 stages of 32 KB at NT = 256, 16 for narrow tiles, 8 of 24 KB in each CTA of a pair at 384): a TMA
+//     load takes ~1.5 us from request to arrival, so a K step can only be as short as that divided by the depth;
+//   * one thread (of a pair: the even CTA's) issues tcgen05.mma (kind::f16, A from tensor memory, B from shared memory, f32
+//     accumulate) for each 64-wide K step - 256-wide for tiles of up to 64 rows - as soon as its barrier has the arrivals
+//     of the step's producer warps (eight; sixteen of a pair or of a 256-wide step) and the TMA bytes; one tcgen05.commit
+//     per K step reports its completion, which frees the weight stage for the producers (as many K steps later as there
+//     are stages) and the activation stage for the TMA thread (ring depth later);
 //   * the accumulator lives in tensor memory (128 lanes x NT columns f32); after the last K step the
 //     producer warps read it back with tcgen05.ld, undo the per-row activation scaling and write
 //     Y[token][row] (32 consecutive floats per warp store).
@@ -56,7 +58,7 @@ constexpr int kTmemA0 = 256;
 constexpr int kStageACols = kGemmBK / 2;
 constexpr int kGemmAStages = 8;
 constexpr int kTmemWideA0 = 384, kGemmWideStages = 4;   // two accumulators of up to 192 columns side by side: four weight stages above them
-// Shared memory: the activation ring.  One barrier pair per K step in flight: slot kt % slots, slots = max(8, ring depth)
+// Shared memory: the activation ring.  One barrier pair per K step in flight: slot kt % slots, slots = the larger of both rings' depths
 constexpr int kGemmBBytes = 192 * 1024;
 constexpr int kGemmMaxSlots = 16;
 constexpr int kGemmSmemMax = kGemmBBytes + 1024 + 8 * (2 * kGemmMaxSlots + 1) + 64;   // ring + alignment slack + barriers
@@ -78,8 +80,8 @@ struct GemmParams {
     const float *inv_scale; // [m]
     const float *resid;     // [m, n] added to the result, or null
     int *err;
-    // K-splits (few activation rows on a narrow weight: too few 128-row tiles to fill the SMs): grid.z CTAs share a tile,
-    // each over kt_total / splits of the K steps, writing its partial product to part[split][m][n_all]; a second small
+    // K-splits (where tiles are too few to fill the SMs, or their last wave: plan_gemm): grid.z CTAs share a tile,
+    // each over 1 / splits of the units of K, writing its partial product to part[split][m][n_all]; a second small
     // launch adds the splits (and the residual).  splits == 1: the result goes straight to out.
     int splits;
     float *part;
@@ -397,8 +399,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
     const uint32_t group_b = box_rows * 128u;                      // bytes of one 64-wide piece of them (multiple of 1024)
     const uint32_t stage_b = group_b * (uint32_t)gs;
     const uint32_t bars = sB + (uint32_t)nb * stage_b;
-    // Slot kt % slots serves K step kt.  full: eight producer warps + the TMA thread's expect_tx; empty: the commit
-    // after the step's MMAs.  A waiter for K step kt - d (d = 8 for the weight stage, nb for the activation stage) asks
+    // Slot kt % slots serves K step kt.  full: the step's producer warps + the TMA thread's expect_tx; empty: the commit
+    // after the step's MMAs.  A waiter for K step kt - d (d = na for the weight stage, nb for the activation stage) asks
     // for phase (kt - d) / slots of that slot; the phase before it has always completed by then (K steps complete in
     // order and the waiter itself saw step kt - d - 1 ... complete earlier), so the parity test cannot alias.
     auto full_bar = [&](int i) { return bars + 8u * (uint32_t)i; };
@@ -1004,8 +1006,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qrows_kernel(const RowsParams
                     // entry 32 i + lane of the tile's 16 x 16: (row, activation row).  The eight entries of a piece, their
                     // residuals and scales are requested together, so a fold waits for L2 about once per kFold pieces and not once
                     // per entry and piece.  What bounds a narrow launch is this chain of latencies: 4096 x 4096 Q4_K with
-                    // 16 rows (up to ten pieces a tile) took 21 us with the loads one after another and takes 16.  More than
-                    // three pieces at a time spill at the 96 registers of 544 threads.
+                    // 16 rows (up to ten pieces a tile) took 21 us with the loads one after another and takes 16.  At the
+                    // 96 registers of 544 threads three pieces at a time spill 4 (Q4_K) and 12 bytes (Q6_K) in the forms for 16
+                    // rows; 128256 x 4096 with two, three and four at a time: 110.1, 109.1, 109.1 us (Q4_K), 139.8, 140.4, 142.2 (Q6_K).
                     constexpr int kFold = 3;
                     float sum[8], res[8];
                     const int tok = lane & 15;

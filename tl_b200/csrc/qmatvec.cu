@@ -5,9 +5,9 @@
 // for Q4_0 / Q8_0 (crates/tl_runtime/src/system.rs:236-264).
 //
 // Shape of the kernel (one persistent CTA of 16 warps per SM, the whole register file at 128 per thread, or of 8 where a
-// launch is short, see warps_for;
-// a variant of two 8-warp CTAs that leaves room for a CTA of the next kernel measured 35 % slower
-// per step: at 80 registers the unit loop no longer keeps its shared loads in flight):
+// launch is short, see warps_for - at 134 to 146 registers a thread, one of them fills an SM as well for the next launch's;
+// a variant of two 8-warp CTAs beside a third of the next kernel measured 35 % slower per step: at the 80 registers
+// that three of them may have the unit loop no longer keeps its shared loads in flight):
 //   * work is cut into ITEMS: one tile of 16 output rows x one K-slice of `upi` consecutive units
 //     (a unit = 16 rows x 256 weights, quant.cu).  Items are numbered slice-major and dealt out in
 //     contiguous ranges, first to CTAs and then to the warps of a CTA, so every warp gets the same
@@ -17,7 +17,7 @@
 //     a ring of stages that belongs to it alone: after consuming a stage the warp refills it with the
 //     unit `spw` positions ahead.  No other warp is ever waited for - there is no block-wide barrier,
 //     no shared-memory reduction and no atomic in the streaming phase;
-//   * the copies do not depend on the activations, so the first `spw` are issued before the kernel
+//   * the copies do not depend on the activations, so the first two are issued before the kernel
 //     waits for its predecessor (programmatic dependent launch);
 //   * the prologue quantises the activation to int8 levels in shared memory (qmv_prologue.cuh) -
 //     only the 256-blocks the CTA's K-slices cover - and can fuse what precedes the matvec in the
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
     };
     if (local) {
         // The pieces of every tile of this CTA are in shared memory.  Tile t (CTA-local) is finished by
-        // warp t % kWarps: it adds the pieces in the order of the warps that produced them - a fixed
+        // warp t % NW: it adds the pieces in the order of the warps that produced them - a fixed
         // order - and writes the rows.  No global scratch, fence or counter is involved.
         __syncthreads();           // every warp gets here: its waits are bounded
         if (!*abortp) {
