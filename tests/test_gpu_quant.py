@@ -9,7 +9,7 @@ import pytest
 
 import tl_b200 as tl
 from tl_b200 import _lib, synth
-from test_launch_plans_cpu import gemm_plan
+from test_launch_plans_cpu import gemm_form, gemm_plan
 
 pytestmark = pytest.mark.gpu
 
@@ -259,6 +259,25 @@ def test_qgemm_wide_tiles_by_pairs(orc, t, n, k, m, plan):
     assert got.shape == (m, n)
     for i in range(m):
         assert relerr(got[i], ref[i]) < GEMM_TOL, i
+
+
+@pytest.mark.parametrize("t,n,k,m,form", [(synth.Q4_K, 14200, 4096, 500, (256, 1, True)), (synth.Q8_0, 4000, 14336, 512, (256, 2, True)), (synth.Q6_K, 10100, 8192, 512, (192, 1, True)),
+                                          (synth.Q4_0, 15000, 4096, 512, (256, 1, True))])
+def test_qgemm_large_launches_by_pairs(t, n, k, m, form):
+    """Tiles of up to 256 rows by pairs: odd numbers of row tiles, ragged last ones and token tiles, two K ranges.  Sampled weight
+    rows, every activation row."""
+    assert gemm_form(m, n, k) == form
+    rng = np.random.default_rng(5600 + t)
+    q = tl.QTensor.from_gguf_bytes(t, n, k, synth.random_quant(t, n, k, rng))
+    x = rng.standard_normal((m, k), dtype=np.float32)
+    x[m // 2] *= 300.0
+    got = tl.Tensor.from_numpy(x).matmul_quantized(q).numpy()
+    again = tl.Tensor.from_numpy(x).matmul_quantized(q).numpy()
+    np.testing.assert_array_equal(got.view(np.uint32), again.view(np.uint32))
+    rows = np.unique(np.concatenate([np.arange(0, n, 61), np.arange(n - 130, n), np.arange(100, 160)]))
+    ref = x.astype(np.float64) @ q.dequantize().numpy()[rows].astype(np.float64).T
+    for i in range(m):
+        assert relerr(got[i][rows], ref[i]) < GEMM_TOL, i
 
 
 # stands before the library's allocator and turns down requests of one size

@@ -45,12 +45,17 @@ def test_chains_of_short_launches_as_measured():
     assert matvec_slices(synth.Q4_K, 2048, 5632, 1, few=1) > 1
 
 
-def gemm_plan(m, n, k):
+def gemm_form(m, n, k):
+    """(activation rows per tile, K ranges, whether two CTAs share a tile)"""
     f = _lib.lib().tlb_gemm_plan
-    f.restype, f.argtypes = None, [C.c_int64] * 4 + [C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]
-    nt, splits = C.c_int(), C.c_int()
-    f(m, (n + 127) // 128, k // 256, n, SMS, C.byref(nt), C.byref(splits))
-    return nt.value, splits.value
+    f.restype, f.argtypes = None, [C.c_int64] * 4 + [C.c_int] + [C.POINTER(C.c_int)] * 3
+    nt, splits, pair = C.c_int(), C.c_int(), C.c_int()
+    f(m, (n + 127) // 128, k // 256, n, SMS, C.byref(nt), C.byref(splits), C.byref(pair))
+    return nt.value, splits.value, bool(pair.value)
+
+
+def gemm_plan(m, n, k):
+    return gemm_form(m, n, k)[:2]
 
 
 def test_gemm_plans_are_launchable():
@@ -59,7 +64,8 @@ def test_gemm_plans_are_launchable():
     for n in (1, 128, 256, 1000, 2048, 4096, 5632, 14336, 28672, 128256):
         for k in (256, 768, 1024, 2048, 2304, 4096, 8192, 14336, 28672):
             for m in (17, 31, 64, 65, 100, 128, 129, 160, 255, 256, 257, 300, 333, 384, 385, 512, 513, 769, 1000, 1536, 2048, 2821, 4096, 10000, 9000000):
-                nt, splits = gemm_plan(m, n, k)
+                nt, splits, pair = gemm_form(m, n, k)
+                assert pair == (nt > 256 or m > 128 and k >= 4096 and 2 * m * n * (k // 256 * 256) >= 5e10) and (not pair or nt % 32 == 0), (n, k, m)
                 assert nt == (m + 15) // 16 * 16 if m <= 128 else nt in (128, 160, 192, 224, 256, 320, 384), (n, k, m)
                 assert splits == 1 or 4 * splits <= k // 256 and splits <= (16 if m <= 128 else 8), (n, k, m)
                 assert splits * m * n <= max(2 * m * n, 16 * SMS * 128 * 384), (n, k, m)

@@ -6,10 +6,10 @@
 // rows and never exists in f32.
 //
 // One CTA computes 128 weight rows x NT activation rows (NT <= 256) on the 5th-generation tensor cores.  A pair of CTAs
-// (cta_group::2) takes 256 weight rows x NT of 320 or 384: each brings half of the activation rows and dequantises its own 128
-// weight rows, and the products go to two accumulators.  Q4_K 14336 x 4096 with 333 rows, whole call: 74 us as two tiles of 192,
-// 56 us as one of 384.  Tiles of up to 256 rows by pairs were no faster than by single CTAs, for all that they halve the traffic
-// from L2 to shared memory: 256, 512 and 1024 rows took 44.9, 81.2 and 152.8 us by pairs, 43.4, 79.9 and 149.1 by single CTAs
+// (cta_group::2) takes 256 weight rows: each brings half of the activation rows and dequantises its own 128 weight rows.  NT of
+// 320 and 384 needs one, as two accumulators: Q4_K 14336 x 4096 with 333 rows, whole call, 74 us as two tiles of 192, 56 us as
+// one of 384.  Up to 256 rows a pair halves the traffic from L2 to shared memory and pays for it in large launches only
+// (kPairWork): 256, 512 and 1024 rows alone took 44.9, 81.2 and 152.8 us by pairs, 43.4, 79.9 and 149.1 by single CTAs
 // (512 rows are 224 tiles of 256 on 148 SMs either way: two waves, where 36 us of products would fill one and a half):
 //   * the weight tile is the A operand (MMA M = 128) and lives in TENSOR MEMORY, never in shared memory: sixteen
 //     producer warps (two per 16 weight rows, each taking two of a unit's four 64-wide groups) read the quantized
@@ -57,7 +57,7 @@ constexpr int kTmemCols = 512;
 constexpr int kTmemA0 = 256;
 constexpr int kStageACols = kGemmBK / 2;
 constexpr int kGemmAStages = 8;
-constexpr int kTmemWideA0 = 384, kGemmWideStages = 4;   // two accumulators of up to 192 columns side by side: four weight stages above them
+constexpr int kTmemWideA0 = 384, kGemmWideStages = 4;   // PAIR 2: two accumulators of up to 192 columns side by side: four weight stages above them
 // Shared memory: the activation ring.  One barrier pair per K step in flight: slot kt % slots, slots = the larger of both rings' depths
 constexpr int kGemmBBytes = 192 * 1024;
 constexpr int kGemmMaxSlots = 16;
@@ -76,6 +76,7 @@ struct GemmParams {
     int nt;                 // activation rows per CTA (MMA N)
     int nb;                 // depth of the activation ring (stages)
     int gs;                 // 64-wide K groups per stage: 1, or 4 (a whole 256-wide unit per barrier round) for tiles of up to 64 rows
+    int pair;               // two CTAs (adjacent row tiles) share a token tile: half of it each
     int unit_bytes;
     const float *inv_scale; // [m]
     const float *resid;     // [m, n] added to the result, or null
@@ -327,11 +328,11 @@ template <> struct UnitRegs<8> { using type = Q80Regs; };
 // (the warp's 16 lanes, first column) of weight stage 0.  A stage holds gs 64-wide groups (gs = 1: K step = group, the
 // warp fills every other pair of K steps; gs = 4: K step = unit, both warps of a row tile fill the same stage).
 // Barrier slot of K step kt: kt % slots; weight stage: kt % na.
-template <int FMT, int HALF, int GS, bool PAIR>
+template <int FMT, int HALF, int GS, int PAIR>
 __device__ __forceinline__ bool produce(const GemmParams &p, const uint8_t *ub, bool have, int lane, uint32_t dst, int slots,
                                         uint32_t full0, uint32_t empty0, volatile int *abort_flag, int u0, int units)
 {
-    constexpr int na = GS == 4 ? 3 : PAIR ? kGemmWideStages : kGemmAStages;
+    constexpr int na = GS == 4 ? 3 : PAIR == 2 ? kGemmWideStages : kGemmAStages;
     typename UnitRegs<FMT>::type cur, nxt;
     ub += (size_t)u0 * p.unit_bytes;          // this CTA's K range starts at unit u0
     // Registers hold one unit ahead; one lane of the pair's first warp asks L2 for the units kAhead further on, so
@@ -376,8 +377,8 @@ __device__ __forceinline__ bool produce(const GemmParams &p, const uint8_t *ub, 
 }
 
 // ---- the kernel
-// PAIR: two CTAs share a token tile of up to 384 rows, as two accumulators; else one CTA has a tile of up to 256
-template <int FMT, int GS, bool PAIR>
+// PAIR: 0 one CTA per tile; 1 two CTAs share a token tile of up to 256 rows; 2 ... of up to 384, as two accumulators
+template <int FMT, int GS, int PAIR>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
 {
@@ -391,9 +392,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
     // gs = 4 (token tiles of up to 64 rows): a stage is a whole 256-wide unit - four TMA boxes, sixteen MMAs, one barrier
     // round - because with so little tensor work per group the round itself (arrive, wait, commit, wait) sets the pace.
     // The accumulator then takes columns [0, 64) and three weight stages of 128 columns follow from column 128.
-    constexpr int gs = GS, na = GS == 4 ? 3 : PAIR ? kGemmWideStages : kGemmAStages;
-    constexpr int kAcc = PAIR ? 2 : 1;
-    constexpr uint32_t tmem_a0 = GS == 4 ? 128u : PAIR ? (uint32_t)kTmemWideA0 : (uint32_t)kTmemA0;
+    constexpr int gs = GS, na = GS == 4 ? 3 : PAIR == 2 ? kGemmWideStages : kGemmAStages;
+    constexpr int kAcc = PAIR == 2 ? 2 : 1;
+    constexpr uint32_t tmem_a0 = GS == 4 ? 128u : PAIR == 2 ? (uint32_t)kTmemWideA0 : (uint32_t)kTmemA0;
     const int nb = p.nb, slots = max(na, nb);
     const uint32_t box_rows = (uint32_t)p.nt / (PAIR ? 2u : 1u);   // activation rows this CTA brings
     const uint32_t group_b = box_rows * 128u;                      // bytes of one 64-wide piece of them (multiple of 1024)
@@ -540,7 +541,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
                     for (int k16 = 0; k16 < kGemmBK / 16; k16++)   // 16 f16: 8 columns of tensor memory, 32 bytes along the swizzle row
                         if (PAIR) {
                             umma_f16_ts_pair(tmem, ta + 8u * k16, bd + 2u * k16, idesc, (kt | j | k16) != 0);
-                            umma_f16_ts_pair(tmem + (uint32_t)(p.nt / 2), ta + 8u * k16, bd + (group_b >> 5) + 2u * k16, idesc, (kt | k16) != 0);
+                            if (kAcc == 2) umma_f16_ts_pair(tmem + (uint32_t)(p.nt / 2), ta + 8u * k16, bd + (group_b >> 5) + 2u * k16, idesc, (kt | k16) != 0);
                         } else {
                             umma_f16_ts(tmem, ta + 8u * k16, bd + 2u * k16, idesc, (kt | j | k16) != 0);
                         }
@@ -1157,8 +1158,16 @@ __global__ void __launch_bounds__(NT) x_to_f16_kernel(const float *__restrict__ 
     if (threadIdx.x == 0) inv_scale[blockIdx.x] = inv;
 }
 
-// How a GEMM is cut: tiles of nt activation rows (above 256: by pairs of CTAs) and `splits` ranges of K.
-struct GemmPlan { int nt, splits; };
+// How a GEMM is cut: tiles of nt activation rows, by one CTA or a pair (always above 256), and `splits` ranges of K.
+struct GemmPlan { int nt, splits; bool pair; };
+
+// Tiles of up to 256 rows go to pairs in launches of so many operations and so long sums.  Halving the traffic from L2 saves
+// power, which sets the pace of a large launch; a short one only pays for the hand-over between the CTAs.  Loops of a quarter
+// second, us by pairs / by single CTAs: 32000 x 4096, 512 rows 168 / 171; 14336 x 4096, 1024 rows 157 / 161, 512 rows 78.8 / 78.4
+// and on another board 83.9 / 84.8; 4096 x 14336, 2048 rows 291 / 297; a prompt of 2048 tokens, four layers of the 8B shapes
+// 5290 / 5380; on the other side of the line 2048 x 2048, 4096 rows 61.5 / 59.4, 4096 x 4096, 512 rows 40.6 / 39.2.
+constexpr int kPairUnits = 16;
+constexpr double kPairWork = 5e10;
 
 // Up to 128 rows: one tile.  Above: tiles of 128 to 256 rows, or of 320 or 384 by a pair of CTAs.  A tile's time is its K length:
 // the dequantising warps set the pace, 0.4 us for a 64-wide step of 128 rows and 0.46 of 256 on a full chip, and with two
@@ -1173,6 +1182,7 @@ GemmPlan plan_gemm(int64_t m, int64_t row_tiles, int64_t units, int64_t n_all, i
 {
     GemmPlan best = {};
     double best_us = 1e30;
+    const bool large = units >= kPairUnits && 512.0 * (double)units * (double)m * (double)n_all >= kPairWork;
     auto consider = [&](int nt, int s) {
         const bool pair = nt > 256;
         const int64_t ctas = (pair ? (row_tiles + 1) / 2 * 2 : row_tiles) * ((m + nt - 1) / nt) * s, waves = (ctas + sms - 1) / sms;
@@ -1180,7 +1190,7 @@ GemmPlan plan_gemm(int64_t m, int64_t row_tiles, int64_t units, int64_t n_all, i
         const double step = pair ? 0.485 + 0.00037 * nt : 0.365 + (0.00022 + 0.00015 * busy) * nt;
         double us = (double)waves * (steps * step + 2.25 + 0.012 * nt) + (pair ? 1.25 : 0.0);   // + fill and drain, the read-back
         if (s > 1) us += 5.0 + 3.3e-6 * (double)(s * m * n_all);          // the summing launch: its latency + partials written and read
-        if (us < best_us * 0.98) { best_us = us; best = {nt, s}; }
+        if (us < best_us * 0.98) { best_us = us; best = {nt, s, pair || (m > 128 && large)}; }
     };
     const int most = m <= 128 ? 16 : 8;
     for (int nt : {256, 384, 320, 224, 192, 160, 128}) {
@@ -1195,17 +1205,18 @@ GemmPlan plan_gemm(int64_t m, int64_t row_tiles, int64_t units, int64_t n_all, i
 }  // namespace
 
 // The plan of a launch over row_tiles tiles of 128 weight rows (n_all outputs in all) and units of 256 weights of K
-extern "C" void tlb_gemm_plan(int64_t m, int64_t row_tiles, int64_t units, int64_t n_all, int sms, int *nt, int *splits)
+extern "C" void tlb_gemm_plan(int64_t m, int64_t row_tiles, int64_t units, int64_t n_all, int sms, int *nt, int *splits, int *pair)
 {
     const GemmPlan p = plan_gemm(m, row_tiles, units, n_all, sms);
     *nt = p.nt;
     *splits = p.splits;
+    *pair = p.pair;
 }
 
 bool qgemm_supported(int type) { return type == 12 || type == 14 || type == 2 || type == 8; }
 
 namespace {
-template <int FMT, int GS, bool PAIR>
+template <int FMT, int GS, int PAIR>
 tlb_status launch_fmt_gemm_gs(dim3 grid, size_t smem, cudaStream_t stream, const CUtensorMap &map, const GemmParams &p)
 {
     static bool attr_set = false;
@@ -1230,8 +1241,9 @@ tlb_status launch_fmt_gemm_gs(dim3 grid, size_t smem, cudaStream_t stream, const
 template <int FMT>
 tlb_status launch_fmt_gemm(dim3 grid, size_t smem, cudaStream_t stream, const CUtensorMap &map, const GemmParams &p)
 {
-    if (p.gs == 4) return launch_fmt_gemm_gs<FMT, 4, false>(grid, smem, stream, map, p);
-    return p.nt > 256 ? launch_fmt_gemm_gs<FMT, 1, true>(grid, smem, stream, map, p) : launch_fmt_gemm_gs<FMT, 1, false>(grid, smem, stream, map, p);
+    if (p.gs == 4) return launch_fmt_gemm_gs<FMT, 4, 0>(grid, smem, stream, map, p);
+    if (!p.pair) return launch_fmt_gemm_gs<FMT, 1, 0>(grid, smem, stream, map, p);
+    return p.nt > 256 ? launch_fmt_gemm_gs<FMT, 1, 2>(grid, smem, stream, map, p) : launch_fmt_gemm_gs<FMT, 1, 1>(grid, smem, stream, map, p);
 }
 }  // namespace
 
@@ -1401,11 +1413,11 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
     const GemmPlan plan = plan_gemm(m, row_tiles, w0->upt, n_all, c->sm_count);
     const int nt = plan.nt;
     int splits = plan.splits;
-    const bool pair = nt > 256;
+    const bool pair = plan.pair;
     CUtensorMap map;
     const cuuint64_t dims[2] = {(cuuint64_t)a.k, (cuuint64_t)m};
     const cuuint64_t strides[1] = {(cuuint64_t)a.k * sizeof(__half)};
-    const cuuint32_t box[2] = {(cuuint32_t)kGemmBK, (cuuint32_t)(pair ? nt / 4 : nt)};
+    const cuuint32_t box[2] = {(cuuint32_t)kGemmBK, (cuuint32_t)(!pair ? nt : nt > 256 ? nt / 4 : nt / 2)};
     const cuuint32_t estr[2] = {1, 1};
     CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.xh->ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1415,6 +1427,7 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
     p.upt = w0->upt;
     p.m = (int)m;
     p.nt = nt;
+    p.pair = pair;
     p.gs = !pair && nt <= 64 ? 4 : 1;
     const int stage_b = (pair ? nt / 2 : nt) * 128 * p.gs;
     p.nb = std::max(p.gs == 4 ? 3 : 4, std::min(kGemmMaxSlots, kGemmBBytes / stage_b));
