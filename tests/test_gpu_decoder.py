@@ -95,6 +95,19 @@ def test_llama3_shaped_one_layer_long_context(orc):
     run_parity(orc, ref, dec, [12345], 8, ctx0=300)
 
 
+@pytest.mark.parametrize("head_dim,kv_f16,context", [(64, False, 127), (64, True, 128), (64, True, 1030), (64, False, 2047), (64, True, 2050), (128, True, 4100)])
+def test_contexts_of_many_key_ranges(orc, head_dim, kv_f16, context):
+    """o_proj merges the attention's key ranges (128 rows each), eight rows and 16 (heads of 64) or 32 (of 128) ranges at a time."""
+    cfg = dict(SMALL, n_layers=1, n_heads=4, n_kv_heads=2, head_dim=head_dim, d_model=256 * (head_dim // 64), attn_scale=head_dim ** -0.5)
+    ref, dec, wmap = build(orc, cfg, 6, synth.Q8_0, synth.Q8_0, kv_f16, context + 8, sigma=0.002)
+    rng = np.random.default_rng(context)
+    kv = rng.standard_normal((2, context, 2 * head_dim)).astype(np.float16).astype(np.float32)
+    dec.kv_write(0, 0, kv[0], kv[1])
+    for p in range(context):
+        ref.kv_write(0, p, kv[0, p], kv[1, p])
+    run_parity(orc, ref, dec, [7], 4, ctx0=context)
+
+
 def test_decoder_argument_errors(orc):
     ref, dec, wmap = build(orc, SMALL, 5, synth.Q4_K, synth.Q6_K, True, 32)
     with pytest.raises(tl.TlbError) as e:

@@ -25,8 +25,8 @@
 //   * per unit: conflict-free 128-bit shared loads, one AND per four weights, integer tensor-core
 //     MMAs (qmv_units.cuh);
 //   * the 16 * m partial results of item (slice, tile) are written - not added - to a scratch slot of
-//     their own; the warp that finishes the last slice of a tile (a per-tile counter tells) adds the
-//     slices in index order and writes the output rows.  Nothing is accumulated atomically and nothing
+//     their own; one warp per tile - with several rows the one that finishes its last slice (a per-tile counter tells) - adds
+//     the slices in index order and writes the output rows.  Nothing is accumulated atomically and nothing
 //     has to be cleared beforehand, so results do not depend on scheduling;
 //   * with a single K-slice ("local" mode, chosen for launches with many units per warp such as
 //     gate|up and the head) a CTA's units are cut evenly over its warps whatever the tile borders, and
@@ -225,6 +225,9 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
 
     float4 wgt_first[kKeep];       // static inputs of the prologue, fetched while the previous kernel finishes
     load_norm_weights(p, tid, NW * 32, blk0, nb, wgt_first);
+    // key ranges of an attention output that is still split; the position was written by the step before, and the launch ahead
+    // of this one let it start when all that came before was over
+    const int nsplit = ONE && p.prologue == PRO_ATTN_MERGE ? (__ldcg(p.att_pos) + p.att_keys) / p.att_keys : 0;   // ceil((pos + 1) / keys)
     if (p.use_pdl) {
         pdl_wait();                // everything below may read what the previous kernel wrote
         // Released only after our own wait: a dependent's early part then runs with every kernel
@@ -233,7 +236,7 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
     }
     const unsigned tp_seq = p.tp_reduce ? ld_volatile_u32(p.tp.seq) : 0u;   // the launch before has completed: its exchange is over
     __syncthreads();               // abort_flag initialised; also keeps the CTA together for the prologue
-    build_activation<FMT, ONE>(p, sh, smem, tid, NW * 32, blk0, nb, wgt_first, [&](float dep) {
+    build_activation<FMT, ONE>(p, sh, smem, tid, NW * 32, blk0, nb, nsplit, wgt_first, [&](float dep) {
         // the rest of the ring's first round; the test on `dep` only ties the requests to the arrival of the loads
         if (lane >= kEarly && lane < n_first && __float_as_uint(dep) != 0x7fedcba9u) {
             mbar_expect_tx(bars + lane * 8, p.unit_bytes);
@@ -329,13 +332,15 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
     const bool tpr = p.tp_reduce != 0;
     int tp_finished = 0;                               // tiles this warp has completed over the ranks
     bool tp_ok = true;
-    // what a finished tile's 16 sums (lane e < 16: row e) turn into
-    auto finish_rows = [&](const ItemRef &fr, float y) {
+    // what a finished tile's 16 sums (lane e < 16: row e) turn into; the residual of the row is asked for ahead of the sums
+    auto residual = [&](const ItemRef &fr) {
+        return (p.finish == FIN_RESID && lane < 16 && fr.row0 + lane < p.n_rows[0]) ? __ldcg(p.resid + fr.row0 + lane) : 0.f;
+    };
+    auto finish_rows = [&](const ItemRef &fr, float y, float res) {
         if (p.finish == FIN_PLAIN) {
             const int g = fr.row0 + lane;
             if (lane < 16 && g < p.n_rows[fr.wi]) p.out[fr.wi][g] = y;
         } else {
-            const float res = (p.finish == FIN_RESID && lane < 16 && fr.row0 + lane < p.n_rows[0]) ? __ldcg(p.resid + fr.row0 + lane) : 0.f;
             finish_tile_fused(p, fr, lane < 16 ? y : 0.f, res, lane);
         }
     };
@@ -368,7 +373,7 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
                     if (lane < 16 * M && g < nrows) out[(size_t)(lane >> 4) * nrows + g] = acc0;
                     if (lane + 32 < 16 * M && g < nrows) out[(size_t)((lane >> 4) + 2) * nrows + g] = acc1;
                 } else {
-                    finish_rows(fr, acc0);
+                    finish_rows(fr, acc0, residual(fr));
                 }
             }
             if (tpr) {
@@ -378,23 +383,27 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
                     cf.slice = 0;
                     cf.tile = ci0 + tl;
                     const ItemRef fr = item_ref(p, cf);
-                    finish_rows(fr, tp_sum_tile(p, tp_seq, fr.row0, p.n_rows[0], lane, &tp_ok));
+                    finish_rows(fr, tp_sum_tile(p, tp_seq, fr.row0, p.n_rows[0], lane, &tp_ok), residual(fr));
                     tp_finished++;
                 }
             }
         }
-    } else if (ONE && ok && wu1 > wu0 && p.fold_poll) {
+    } else if (ONE && ok && p.fold_poll) {
         // One activation row.  The slice scratch rests at kFoldEmpty between launches, so a value that is not kFoldEmpty is
-        // a slice that has arrived: the warp that owns slice 0 of a tile reads the tile's slices (all requested at once,
-        // re-read while some are missing; bounded), adds them in slice order, puts kFoldEmpty back and writes the rows.
-        // No fence, counter or atomic: a 4-byte store is indivisible, and the next launch starts after this one is over.
-        const int i0 = ci0 + it0, i1 = ci0 + p.div_upi(wu1);
+        // a slice that has arrived: one warp per tile reads the tile's slices (all requested at once, re-read while some are
+        // missing; bounded), adds them in slice order, puts kFoldEmpty back and writes the rows.  No fence, counter or atomic:
+        // a 4-byte store is indivisible, and the next launch starts after this one is over.
+        // Tiles are dealt to the CTAs one by one, whoever streamed them: their slice 0 lies in the first tenth of the CTAs, where
+        // a warp took over a microsecond for each of two tiles (TinyLlama's ffn_down: 3.1 us from the last unit to the end of the
+        // launch, 1.5 dealt out).  A CTA's last warp begins, since it is never without units: a warp that polls from the start
+        // slows the stores of the slices down (four calls of 2048 x 2048: 48.2 us, 44.1 by the last warp, 46.1 before).
         const size_t sstride = (size_t)p.tiles * 16;
-        for (int item = i0; item < i1 && item < p.tiles; item++) {     // items below `tiles` are slice 0
+        for (int tile = b + (NW - 1 - warp) * (int)gridDim.x; tile < p.tiles; tile += NW * (int)gridDim.x) {
             ItemCursor cf;
             cf.slice = 0;
-            cf.tile = item;
+            cf.tile = tile;
             const ItemRef fr = item_ref(p, cf);
+            const float res = residual(fr);
             float *src = p.part + (size_t)fr.tile * 16 + (lane & 15);
             unsigned sl[kMaxSlices];
             bool got = true;
@@ -430,10 +439,10 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
             }
             if (tpr) {
                 tp_push_tile(p, tp_seq, fr.row0, p.n_rows[0], a, lane);
-                finish_rows(fr, tp_sum_tile(p, tp_seq, fr.row0, p.n_rows[0], lane, &tp_ok));
+                finish_rows(fr, tp_sum_tile(p, tp_seq, fr.row0, p.n_rows[0], lane, &tp_ok), res);
                 tp_finished++;
             } else {
-                finish_rows(fr, a);
+                finish_rows(fr, a, res);
             }
         }
     } else if (ok && wu1 > wu0) {
@@ -476,7 +485,7 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
 #pragma unroll
                     for (int s = 1; s < kMaxSlices; s++) a += sl[s];
                     if (tpr) tp_push_tile(p, tp_seq, fr.row0, nrows, a, lane);
-                    else finish_rows(fr, a);
+                    else finish_rows(fr, a, residual(fr));
                 }
                 if (lane == 0) p.tile_cnt[fr.tile] = 0;
             }
@@ -486,7 +495,7 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
                     cf.slice = 0;
                     cf.tile = __shfl_sync(0xffffffffu, cj.tile, __ffs(rest) - 1);
                     const ItemRef fr = item_ref(p, cf);
-                    finish_rows(fr, tp_sum_tile(p, tp_seq, fr.row0, p.n_rows[0], lane, &tp_ok));
+                    finish_rows(fr, tp_sum_tile(p, tp_seq, fr.row0, p.n_rows[0], lane, &tp_ok), residual(fr));
                     tp_finished++;
                 }
             }
@@ -595,14 +604,13 @@ extern "C" int tlb_matvec_few(int64_t d_model, int64_t units, int sm) { return m
 // How a launch of `tiles` 16-row tiles (all tensors) over upt units of K is laid out with kb K-slices.
 struct MvGeometry {
     int upi, n_items, grid, nb, spw, max_seg;
-    int ring, off_seg, off_wtab;        // bytes of the ring; where the partial results and ATTN_MERGE's weights begin
+    int ring, off_seg;                  // bytes of the ring; where the partial results begin
     SmemPlan sp;
     size_t smem;
     bool roomy;                         // two stages fit beside eight slots of partial results per warp
 };
 
-// heads, splits: ATTN_MERGE's softmax weights per block of 256 activations (0: none)
-static MvGeometry geometry(int type, int m, int upt, int64_t tiles, int kb, int nw, int sm, size_t smem_max, int heads, int splits)
+static MvGeometry geometry(int type, int m, int upt, int64_t tiles, int kb, int nw, int sm, size_t smem_max)
 {
     MvGeometry g = {};
     const int stage = stage_bytes_of(qformat(type));
@@ -616,7 +624,7 @@ static MvGeometry geometry(int type, int m, int upt, int64_t tiles, int kb, int 
     const int64_t n_max = (ipc * g.upi + nw - 1) / nw;           // most units a warp gets
     g.max_seg = kb == 1 ? (int)((n_max + g.upi - 2) / g.upi + 1) : 1;
     const size_t slot = kb == 1 ? (size_t)nw * 16 * m * sizeof(float) : 0, per_stage = (size_t)nw * (stage + 8);
-    const size_t beside = g.sp.fixed + 128 + (kb == 1 ? std::max(8, g.max_seg) * slot + 128 : 0) + (heads ? (size_t)g.nb * 4 * splits * sizeof(float) + 128 : 0);
+    const size_t beside = g.sp.fixed + 128 + (kb == 1 ? std::max(8, g.max_seg) * slot + 128 : 0);
     // no more stages than the longest warp has units, and no more than keeps ~1.5 us of HBM latency covered; two at least,
     // which a trip of the unit loop takes
     const int64_t upw = (ipc + nw - 1) / nw * g.upi;
@@ -629,16 +637,12 @@ static MvGeometry geometry(int type, int m, int upt, int64_t tiles, int kb, int 
         g.off_seg = (int)((g.smem + 127) / 128 * 128);
         g.smem = (size_t)g.off_seg + g.max_seg * slot;
     }
-    if (heads) {
-        g.off_wtab = (int)((g.smem + 127) / 128 * 128);
-        g.smem = (size_t)g.off_wtab + (size_t)g.nb * heads * splits * sizeof(float);
-    }
     return g;
 }
 
 // K-slices of a launch: as many as the cost model likes, at most max_slices, among the counts whose launch fits shared memory
 // (0: none does).
-static int plan_slices(int type, int upt, int m, int64_t tiles, int max_slices, int nw, int sm, size_t smem_max, int heads, int splits)
+static int plan_slices(int type, int upt, int m, int64_t tiles, int max_slices, int nw, int sm, size_t smem_max)
 {
     max_slices = std::max(1, std::min(max_slices, kMaxSlices));
     int best = 0;
@@ -647,7 +651,7 @@ static int plan_slices(int type, int upt, int m, int64_t tiles, int max_slices, 
         if (upt % upi) continue;
         const int kb = upt / upi;
         if (kb > max_slices) break;
-        const MvGeometry g = geometry(type, m, upt, tiles, kb, nw, sm, smem_max, heads, splits);
+        const MvGeometry g = geometry(type, m, upt, tiles, kb, nw, sm, smem_max);
         if (g.smem > smem_max) continue;
         const double cost = kb == 1 && !g.roomy ? 1e12 : slice_cost(type, m, tiles, upt, upi, sm, nw);
         if (best == 0 || cost < best_cost) { best = kb; best_cost = cost; }
@@ -664,7 +668,7 @@ extern "C" int tlb_matvec_slices(int type, int64_t n, int64_t k, int m, int few,
     job.m = m;
     job.few = few != 0;
     const int nw = warps_for(job, tiles, upt, sm);
-    return plan_slices(type, upt, m, tiles, kMaxSlices, nw, sm, smem_max, 0, 0);
+    return plan_slices(type, upt, m, tiles, kMaxSlices, nw, sm, smem_max);
 }
 
 template <int FMT, int NW, bool ONE>
@@ -742,11 +746,10 @@ tlb_status launch_qmatvec(const MatvecJob &job)
     int max_slices = kMaxSlices;
     if (tiles > (int64_t)c->mv_cnt_n) max_slices = 1;
     while (max_slices > 1 && (size_t)max_slices * tiles * 16 * job.m > c->mv_part_floats) max_slices--;
-    const int heads = job.prologue == PRO_ATTN_MERGE && job.att_dim > 0 ? 256 / job.att_dim : 0, splits = std::max(1, job.att_max_splits);
-    p.kb = job.slices > 0 ? std::min(job.slices, max_slices) : plan_slices(job.type, p.upt, job.m, tiles, max_slices, nw, c->sm_count, c->smem_optin, heads, splits);
+    p.kb = job.slices > 0 ? std::min(job.slices, max_slices) : plan_slices(job.type, p.upt, job.m, tiles, max_slices, nw, c->sm_count, c->smem_optin);
     if (p.kb < 1) return fail(TLB_ERR_SHAPE, "K = %lld with %d rows needs more shared memory than one SM has (max K %zu)", (long long)job.k, job.m, qmatvec_max_k(job.m));
     if (p.upt % p.kb) return fail(TLB_ERR_ARG, "%d slices do not divide the %d units of K", p.kb, p.upt);
-    const MvGeometry g = geometry(job.type, job.m, p.upt, tiles, p.kb, nw, c->sm_count, c->smem_optin, heads, splits);
+    const MvGeometry g = geometry(job.type, job.m, p.upt, tiles, p.kb, nw, c->sm_count, c->smem_optin);
     if (g.smem > c->smem_optin) return fail(TLB_ERR_SHAPE, "launch needs %zu bytes of shared memory", g.smem);
     p.upi = g.upi;
     p.fold_poll = (job.m == 1 && (size_t)p.kb * tiles * 16 <= c->mv_part1_floats) ? 1 : 0;
@@ -768,7 +771,6 @@ tlb_status launch_qmatvec(const MatvecJob &job)
     p.col_stride = g.sp.col_stride;
     p.max_seg = g.max_seg;
     p.off_seg = g.off_seg;
-    p.off_wtab = g.off_wtab;
     p.prologue = job.prologue;
     p.x = job.x; p.x2 = job.x2; p.norm_w = job.norm_w; p.eps = job.eps; p.x_out = job.x_out;
     p.tp_reduce = job.tp_reduce ? 1 : 0;

@@ -174,8 +174,8 @@ struct MvParams {
     float *out[3];            // [m][n_rows] per tensor
     float *part;              // slice scratch [kb][tiles][m][16] (kb > 1): the partial result of every item
     int *tile_cnt;            // [tiles] slices of a tile finished so far; zero between launches (m > 1)
-    int fold_poll;            // m == 1: `part` rests at kFoldEmpty between launches; the warp that owns slice 0 of a tile
-                              // waits for the other slices' values to replace it, adds them and puts it back
+    int fold_poll;            // m == 1: `part` rests at kFoldEmpty between launches; one warp per tile
+                              // waits for the slices' values to replace it, adds them and puts it back
     int tiles_end[3];         // cumulative tile counts
     int n_rows[3];            // valid output rows per tensor
     int n_w;
@@ -207,7 +207,6 @@ struct MvParams {
     const float *att_part;    // ATTN_MERGE: per-split attention results [kv head][att_max_splits][att_rep][att_dim + 4]
     const int *att_pos;
     int att_max_splits, att_rep, att_dim, att_keys;
-    int off_wtab;             // ATTN_MERGE: softmax weights of the splits per query head of this CTA
     int finish;               // FIN_*: what the warp completing a tile does with its results
     const float *resid;       // FIN_RESID: added to the result
     float *ssq_out;           // FIN_RESID: [tiles] sum of squares of each finished tile

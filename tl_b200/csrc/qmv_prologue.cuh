@@ -152,90 +152,91 @@ __device__ __forceinline__ void load_norm_weights(const MvParams &p, int tid, in
     }
 }
 
-// ONE: one activation row (three levels); its blocks are the items, no division tells them apart.
+// Elements 4j .. 4j+3 of local block lb of an attention output that is still split over the keys (D-element weighted sums, maximum
+// and sum of exponentials per split and query head): sum_s exp(m_s - M) v_s / sum_s exp(m_s - M) l_s.  A warp's 128 elements are one
+// head of 128 or two of 64, so lane s of a head's W lanes turns split s's pair into a weight and the others take it by shuffle; the
+// first rows are under way meanwhile, and more than W splits are taken W at a time.
+__device__ __forceinline__ float4 attn_value(const MvParams &p, int nsplit, int e, int lane)
+{
+    constexpr int kRows = 8;                 // rows asked for at once
+    const int W = p.att_dim >> 2, hl = lane & (W - 1);
+    const int head = e / p.att_dim, d = e - head * p.att_dim;
+    const int kvh = head / p.att_rep, hr = head - kvh * p.att_rep;
+    const size_t sstride = (size_t)p.att_rep * (p.att_dim + 4);
+    const float *row = p.att_part + ((size_t)kvh * p.att_max_splits * p.att_rep + hr) * (p.att_dim + 4);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float M = -INFINITY, sum = 0.f;
+    for (int s0 = 0; s0 < nsplit; s0 += W, row += W * sstride) {
+        const int n = min(W, nsplit - s0);
+        float2 ml = make_float2(-INFINITY, 0.f);
+        if (hl < n) ml = __ldcg(reinterpret_cast<const float2 *>(row + hl * sstride + p.att_dim));
+        float4 v[kRows];
+        auto load = [&](int sp) {
+#pragma unroll
+            for (int u = 0; u < kRows; u++)
+                if (sp + u < n) v[u] = __ldcg(reinterpret_cast<const float4 *>(row + (sp + u) * sstride + d));
+        };
+        load(0);
+        float mx = ml.x;
+        for (int o = W >> 1; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        mx = fmaxf(mx, M);
+        const float w = hl < n ? expf(ml.x - mx) : 0.f;
+        float l = ml.y * w;
+        for (int o = W >> 1; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        if (s0) {
+            const float c = expf(M - mx);
+            sum *= c; acc.x *= c; acc.y *= c; acc.z *= c; acc.w *= c;
+        }
+        sum += l;
+        M = mx;
+        for (int sp = 0;;) {
+#pragma unroll
+            for (int u = 0; u < kRows; u++)
+                if (sp + u < n) {
+                    const float ws = __shfl_sync(0xffffffffu, w, sp + u, W);
+                    acc.x = fmaf(ws, v[u].x, acc.x); acc.y = fmaf(ws, v[u].y, acc.y); acc.z = fmaf(ws, v[u].z, acc.z); acc.w = fmaf(ws, v[u].w, acc.w);
+                }
+            sp += kRows;
+            if (sp >= n) break;
+            load(sp);
+        }
+    }
+    const float inv = 1.f / sum;
+    return make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+}
+
+// ONE: one activation row (three levels); its blocks are the items, no division tells them apart.  Only it has fused prologues.
 template <int FMT, bool ONE, typename AfterLoads>
-__device__ void build_activation(const MvParams &p, MvShared *sh, uint8_t *smem, int tid, int nthreads, int blk0, int nb,
+__device__ void build_activation(const MvParams &p, MvShared *sh, uint8_t *smem, int tid, int nthreads, int blk0, int nb, int nsplit,
                                  const float4 (&wgt_first)[kKeep], AfterLoads after_loads)
 {
     const int lane = tid & 31, warp = tid >> 5, nwarps = nthreads >> 5;
     const int ngroups = nthreads >> 6, grp = tid >> 6, j = tid & 63;
     const int nblk = p.k / 256, n_mine = (ONE ? 1 : p.m) * nb;
-    const bool norm = p.prologue == PRO_ADD_NORM;
+    const bool norm = ONE && p.prologue == PRO_ADD_NORM, attn = ONE && p.prologue == PRO_ATTN_MERGE;
     const float *emb = nullptr;
     if (norm && p.token) emb = p.emb_table + (size_t)__ldg(p.token) * p.k;
-
-    // Attention output still split over the keys: first the softmax weight of every split for each query
-    // head this CTA needs - w[head][s] = exp(m_s - M) / sum_t l_t exp(m_t - M), one warp per head - then the
-    // values are the weighted sums of the splits' rows (attn_value below).
-    const bool attn = p.prologue == PRO_ATTN_MERGE;
-    int nsplit = 1;
-    float *wtab = reinterpret_cast<float *>(smem + p.off_wtab);   // [heads of this CTA][att_max_splits]
-    if (attn) {
-        const int hpb = 256 / p.att_dim;     // query heads per block of 256
-        nsplit = (__ldcg(p.att_pos) + p.att_keys) / p.att_keys;   // ceil((pos + 1) / keys per split)
-        const size_t sstride = (size_t)p.att_rep * (p.att_dim + 4);
-        for (int hl = warp; hl < nb * hpb; hl += nwarps) {
-            const int head = blk0 * hpb + hl, kvh = head / p.att_rep, hr = head - kvh * p.att_rep;
-            const float *row0 = p.att_part + ((size_t)kvh * p.att_max_splits * p.att_rep + hr) * (p.att_dim + 4) + p.att_dim;
-            // lane s holds split s (and s + 32, ... for very long contexts, re-read in the later passes)
-            const float m0 = lane < nsplit ? __ldcg(row0 + lane * sstride) : -INFINITY;
-            const float l0 = lane < nsplit ? __ldcg(row0 + lane * sstride + 1) : 0.f;
-            float mx = m0;
-            for (int sp = lane + 32; sp < nsplit; sp += 32) mx = fmaxf(mx, __ldcg(row0 + sp * sstride));
-            for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            const float w0 = lane < nsplit ? expf(m0 - mx) : 0.f;
-            float lsum = l0 * w0;
-            for (int sp = lane + 32; sp < nsplit; sp += 32) lsum += __ldcg(row0 + sp * sstride + 1) * expf(__ldcg(row0 + sp * sstride) - mx);
-            for (int o = 16; o; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-            const float inv_l = 1.f / lsum;
-            if (lane < nsplit) wtab[hl * p.att_max_splits + lane] = w0 * inv_l;
-            for (int sp = lane + 32; sp < nsplit; sp += 32) wtab[hl * p.att_max_splits + sp] = expf(__ldcg(row0 + sp * sstride) - mx) * inv_l;
-        }
-        __syncthreads();
-    }
-    auto attn_value = [&](int lb) {   // elements 4j .. 4j+3 of local block lb
-        const int e = ((blk0 + lb) * 64 + j) * 4;
-        const int head = e / p.att_dim, d = e - head * p.att_dim;
-        const int kvh = head / p.att_rep, hr = head - kvh * p.att_rep, hl = head - blk0 * (256 / p.att_dim);
-        const float *row = p.att_part + ((size_t)kvh * p.att_max_splits * p.att_rep + hr) * (p.att_dim + 4) + d;
-        const size_t sstride = (size_t)p.att_rep * (p.att_dim + 4);
-        const float *wr = wtab + hl * p.att_max_splits;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-        for (int sp = 0; sp < nsplit; sp++) {
-            const float4 v = __ldcg(reinterpret_cast<const float4 *>(row + sp * sstride));
-            const float w = wr[sp];
-            acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
-        }
-        return acc;
-    };
 
     float inv_rms = 0.f;
     for (int first = 0; first < n_mine || (norm && first == 0); first += ngroups * kKeep) {
         float4 keep[kKeep], wgt[kKeep];
-        float ssq = 0.f;
 #pragma unroll
         for (int i = 0; i < kKeep; i++) {
             const int item = first + grp + i * ngroups;
             if (item < n_mine) {
                 const int mrow = ONE ? 0 : item / nb, lb = item - mrow * nb, k4 = (blk0 + lb) * 64 + j;
-                keep[i] = attn ? attn_value(lb) : prologue_value(p, emb, mrow, k4, 0.f);
+                keep[i] = attn ? attn_value(p, nsplit, k4 * 4, lane) : prologue_value(p, emb, mrow, k4, 0.f);
                 if (norm) wgt[i] = first == 0 ? wgt_first[i] : __ldg(reinterpret_cast<const float4 *>(p.norm_w) + k4);
             }
         }
+        float ssq = 0.f;
         if (norm && first == 0 && p.ssq_parts) {
-            // The producer of x left partial sums of squares: every warp adds them itself, in one fixed
-            // order, so no block-wide exchange is needed and nothing of the row is re-read.
-            for (int i = lane; i < p.n_parts; i += 32) ssq += __ldcg(p.ssq_parts + i);
-            float dep = ssq;
-#pragma unroll
-            for (int i = 0; i < kKeep; i++)
-                if (grp + i * ngroups < n_mine) dep += keep[i].x;
-            after_loads(dep);
-            for (int o = 16; o; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
-            inv_rms = 1.f / sqrtf(ssq / (float)p.k + p.eps);
+            // The producer of x left partial sums of squares.  Each is read once per CTA and the sums meet at the barrier below:
+            // the warps of all CTAs reading all of them met on a handful of L2 lines.  With tiles' slices dealt to all CTAs
+            // (qmatvec.cu), a 32-token answer of the TinyLlama shapes 23.4 -> 22.5 ms, 16 of eight Llama-3-8B layers 8.18 -> 8.05.
+            for (int i = tid; i < p.n_parts; i += nthreads) ssq += __ldcg(p.ssq_parts + i);
         } else if (norm && first == 0) {
-            // the blocks outside [blk0, blk0 + nb): only their squares are needed (m == 1 with this prologue)
+            // the blocks outside [blk0, blk0 + nb): only their squares are needed
             for (int o = grp; o < nblk - nb; o += ngroups) {
                 const int k4 = (o < blk0 ? o : o + nb) * 64 + j;
                 const float4 v = prologue_value(p, emb, 0, k4, 0.f);
@@ -258,45 +259,50 @@ __device__ void build_activation(const MvParams &p, MvShared *sh, uint8_t *smem,
                     if (p.x_out && blockIdx.x == 0) reinterpret_cast<float4 *>(p.x_out)[(blk0 + item) * 64 + j] = v;
                 }
             }
-            after_loads(ssq);
-            for (int o = 16; o; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
-            if (lane == 0) sh->red_sum[warp] = ssq;
-            __syncthreads();
-            ssq = 0.f;
-            for (int w = 0; w < nwarps; w++) ssq += sh->red_sum[w];
-            inv_rms = 1.f / sqrtf(ssq / (float)p.k + p.eps);
         }
-        if (!norm && first == 0) {
-            float dep = 0.f;
+        if (first == 0) {
+            float dep = ssq;
 #pragma unroll
             for (int i = 0; i < kKeep; i++)
                 if (grp + i * ngroups < n_mine) dep += keep[i].x;
             after_loads(dep);
         }
-        // step 1 of this pass's blocks: final values and each warp's maximum
+        // step 1 of this pass's blocks: the values, of a norm without their common factor 1 / rms, and each warp's maximum
         float *pair_max = &sh->red_max[grp * 2 * kKeep];
 #pragma unroll
         for (int i = 0; i < kKeep; i++) {
             const int item = first + grp + i * ngroups;
             if (item < n_mine) {
                 float4 v = keep[i];
-                if (norm) {   // (x / rms) * weight (crates/tl_cpu/src/ffi.rs:2444-2486), the division as a multiply by 1/rms
-                    v.x = (v.x * inv_rms) * wgt[i].x; v.y = (v.y * inv_rms) * wgt[i].y;
-                    v.z = (v.z * inv_rms) * wgt[i].z; v.w = (v.w * inv_rms) * wgt[i].w;
-                }
+                if (norm) { v.x *= wgt[i].x; v.y *= wgt[i].y; v.z *= wgt[i].z; v.w *= wgt[i].w; }
                 keep[i] = v;
                 const float mx = warp_absmax(v);
                 if (lane == 0) pair_max[2 * i + (j >> 5)] = mx;
             }
         }
-        if (first + grp < n_mine) named_bar(2 + grp, 64);
-        // step 2: the blocks are independent from here on, their instruction streams interleave
+        if (norm && first == 0) {
+            // the squares meet at the barrier that the maxima take anyway
+            for (int o = 16; o; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
+            if (lane == 0) sh->red_sum[warp] = ssq;
+            __syncthreads();
+            ssq = 0.f;
+            for (int w = 0; w < nwarps; w++) ssq += sh->red_sum[w];
+            inv_rms = 1.f / sqrtf(ssq / (float)p.k + p.eps);
+        } else if (first + grp < n_mine) {
+            named_bar(2 + grp, 64);
+        }
+        // step 2: the blocks are independent from here on, their instruction streams interleave.  x * weight / rms
+        // (crates/tl_cpu/src/ffi.rs:2444-2486), the division as a multiply by 1 / rms; rounding keeps order, so the largest
+        // product is the product of the largest
 #pragma unroll
         for (int i = 0; i < kKeep; i++) {
             const int item = first + grp + i * ngroups;
             if (item < n_mine) {
                 const int mrow = ONE ? 0 : item / nb, lb = item - mrow * nb;
-                quantise_block<FMT, ONE>(p, smem, fmaxf(pair_max[2 * i], pair_max[2 * i + 1]), keep[i], mrow, lb, j, lane);
+                float4 v = keep[i];
+                float mx = fmaxf(pair_max[2 * i], pair_max[2 * i + 1]);
+                if (norm) { v.x *= inv_rms; v.y *= inv_rms; v.z *= inv_rms; v.w *= inv_rms; mx *= inv_rms; }
+                quantise_block<FMT, ONE>(p, smem, mx, v, mrow, lb, j, lane);
             }
         }
         if (first + grp < n_mine && first + ngroups * kKeep < n_mine) named_bar(2 + grp, 64);   // pair_max is reused by the next pass
