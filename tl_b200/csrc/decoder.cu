@@ -529,9 +529,10 @@ __global__ void add_rows_kernel(const float *__restrict__ a, const float *__rest
 // Block b: argmax of logits row b (n entries; tie rule as tlb_argmax).  pairs == null: the token goes straight to the
 // sequence's state (rows [row0, row0 + gridDim.x)).  Otherwise (vocabulary split over ranks) the (value, global index)
 // pair of this shard goes to pairs[b] for the exchange.
-__global__ void __launch_bounds__(1024) argmax_rows_kernel(const float *__restrict__ logits, int n, int tie_first, int offset, float *pairs,
+__global__ void __launch_bounds__(1024) argmax_rows_kernel(const float *logits, int n, int tie_first, int offset, float *pairs,
                                                             int *tok, int *pos, int *rope, const int *idx, int *tokens_out, int B, int cap, int row0)
 {
+    pdl_enter();
     __shared__ float sv[32];
     __shared__ int si[32];
     const float *x = logits + (size_t)blockIdx.x * n;
@@ -600,7 +601,11 @@ __global__ void argmax_rows_pick_kernel(const float *__restrict__ pairs, int tp,
     tok[b] = bi; pos[b] += 1; rope[b] += 1;
 }
 
-__global__ void bump_index_kernel(int *idx) { *idx += 1; }
+__global__ void bump_index_kernel(int *idx)
+{
+    pdl_enter();
+    *idx += 1;
+}
 
 tlb_status add_rows(const float *a, const float *b, float *out, int64_t n)
 {
@@ -643,8 +648,7 @@ tlb_status batch_head(tlb_decoder *d, const float *x, int rows, int row0, bool h
         TLB_CUDA(cudaGetLastError());
         count_launch(2);
     } else {
-        argmax_rows_kernel<<<rows, 1024, 0, ctx()->stream>>>(lg, d->V, tie_first, 0, nullptr, d->btok, d->bpos, d->brope, d->bidx, d->btokens_out, d->B, d->tokens_cap, row0);
-        TLB_CUDA(cudaGetLastError());
+        TLB_CUDA(launch_chained(argmax_rows_kernel, dim3(rows), dim3(1024), 0, d->pdl, lg, d->V, tie_first, 0, nullptr, d->btok, d->bpos, d->brope, d->bidx, d->btokens_out, d->B, d->tokens_cap, row0));
         count_launch();
     }
     return TLB_OK;
@@ -660,8 +664,7 @@ tlb_status enqueue_step_batch(tlb_decoder *d)
     if (d->lay) {
         TLB_TRY(layered_step_batch(d->lay, d->btok, d->bpos, d->brope, B, d->bx, d->blogits));
         TLB_TRY(batch_head(d, d->bx, B, 0, true));
-        bump_index_kernel<<<1, 1, 0, ctx()->stream>>>(d->bidx);
-        TLB_CUDA(cudaGetLastError());
+        TLB_CUDA(launch_chained(bump_index_kernel, dim3(1), dim3(1), 0, d->pdl, d->bidx));
         count_launch();
         return TLB_OK;
     }
@@ -696,7 +699,7 @@ tlb_status enqueue_step_batch(tlb_decoder *d)
             j.vcache = (char *)d->vcache + (size_t)l * d->kv_layer_elems * esz;
             j.kv_f16 = c.kv_f16; j.H = d->H; j.KVH = d->KVH; j.D = c.head_dim; j.max_seq = c.max_seq;
             j.pos = d->bpos; j.rope_pos = d->brope; j.cos_t = d->cos_t; j.sin_t = d->sin_t; j.scale = c.attn_scale;
-            j.partial = d->bpartial; j.counters = d->bcounters; j.splits = d->max_splits; j.out = d->battn; j.pdl = false;
+            j.partial = d->bpartial; j.counters = d->bcounters; j.splits = d->max_splits; j.out = d->battn; j.pdl = d->pdl;
             j.defer_merge = false;
             TLB_TRY(launch_decode_attention(j));
         }
@@ -718,8 +721,7 @@ tlb_status enqueue_step_batch(tlb_decoder *d)
         TLB_TRY(st);
     }
     TLB_TRY(batch_head(d, x, B, 0));
-    bump_index_kernel<<<1, 1, 0, ctx()->stream>>>(d->bidx);
-    TLB_CUDA(cudaGetLastError());
+    TLB_CUDA(launch_chained(bump_index_kernel, dim3(1), dim3(1), 0, d->pdl, d->bidx));
     count_launch();
     return TLB_OK;
 }

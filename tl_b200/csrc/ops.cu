@@ -21,9 +21,10 @@ enum { UN_SILU = 0, UN_SCALE = 1 };
 
 // add_kernel / mul_kernel (autograd.cu:185-201) with numpy broadcasting done by index arithmetic
 // instead of materialising both operands (crates/tl_cuda/src/ops/binary.rs:136-155)
-__global__ void binary_kernel(int op, const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ out,
+__global__ void binary_kernel(int op, const float *a, const float *b, float *out,
                               Strides s, int64_t n)
 {
+    pdl_enter();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         int64_t rem = i, ia = 0, ib = 0;
         for (int d = s.rank - 1; d >= 0; d--) {
@@ -37,25 +38,28 @@ __global__ void binary_kernel(int op, const float *__restrict__ a, const float *
     }
 }
 
-__global__ void same_shape_binary_kernel(int op, const float *__restrict__ a, const float *__restrict__ b,
-                                         float *__restrict__ out, int64_t n)
+__global__ void same_shape_binary_kernel(int op, const float *a, const float *b,
+                                         float *out, int64_t n)
 {
+    pdl_enter();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = op == OP_ADD ? a[i] + b[i] : a[i] * b[i];
 }
 
 // silu_kernel (autograd.cu:317-321) in the CPU formulation x * (1 / (1 + exp(-x))) (crates/tl_cpu/src/ffi.rs:2102);
 // mul_scalar_kernel (autograd.cu:151-155)
-__global__ void unary_kernel(int op, const float *__restrict__ a, float *__restrict__ out, int64_t n, float s)
+__global__ void unary_kernel(int op, const float *a, float *out, int64_t n, float s)
 {
+    pdl_enter();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         float x = a[i];
         out[i] = op == UN_SILU ? x * (1.0f / (1.0f + expf(-x))) : x * s;
     }
 }
 
-__global__ void silu_mul_kernel(const float *__restrict__ g, const float *__restrict__ u, float *__restrict__ out, int64_t n)
+__global__ void silu_mul_kernel(const float *g, const float *u, float *out, int64_t n)
 {
+    pdl_enter();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         float x = g[i];
         out[i] = (x * (1.0f / (1.0f + expf(-x)))) * u[i];
@@ -64,6 +68,7 @@ __global__ void silu_mul_kernel(const float *__restrict__ g, const float *__rest
 // the same on four elements per thread (16-byte aligned operands, n a multiple of 4); out may be g
 __global__ void silu_mul4_kernel(const float4 *g, const float4 *u, float4 *out, int64_t n4)
 {
+    pdl_enter();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
         const float4 a = g[i], b = u[i];
         float4 o;
@@ -109,8 +114,9 @@ __device__ float block_max(float v, float *sh)
 }
 
 // softmax_kernel (autograd.cu:457-486: one thread per row, three passes) -> one block per row
-__global__ void softmax_kernel(const float *__restrict__ a, float *__restrict__ out, int64_t axis, int64_t inner)
+__global__ void softmax_kernel(const float *a, float *out, int64_t axis, int64_t inner)
 {
+    pdl_enter();
     __shared__ float sh[32];
     int64_t row = blockIdx.x;
     int64_t o = row / inner, k = row % inner;
@@ -131,9 +137,10 @@ __global__ void softmax_kernel(const float *__restrict__ a, float *__restrict__ 
 
 // matmul_naive_kernel (autograd.cu:430-450: one thread per output) -> 64x64 shared-memory tiles,
 // 4x4 outputs per thread, f32 FMA.  Used by the per-op attention route (matmul_4d) only.
-__global__ void __launch_bounds__(256) matmul_kernel(const float *__restrict__ A, const float *__restrict__ B,
-                                                     float *__restrict__ C, int64_t m, int64_t k, int64_t n, int b_batched)
+__global__ void __launch_bounds__(256) matmul_kernel(const float *A, const float *B,
+                                                     float *C, int64_t m, int64_t k, int64_t n, int b_batched)
 {
+    pdl_enter();
     __shared__ float As[16][64 + 4], Bs[16][64 + 4];
     const float *a = A + (int64_t)blockIdx.z * m * k;
     const float *b = B + (b_batched ? (int64_t)blockIdx.z * k * n : 0);
@@ -172,8 +179,9 @@ __global__ void __launch_bounds__(256) matmul_kernel(const float *__restrict__ A
 
 // narrow_kernel / cat_kernel / transpose_nd_kernel / repeat_interleave_kernel / broadcast_to_kernel
 // (autograd.cu:743-776,1253-1299,781-799): one strided gather serves them all
-__global__ void copy_strided_kernel(const float *__restrict__ a, float *__restrict__ out, Strides s, int64_t n, int64_t a_off)
+__global__ void copy_strided_kernel(const float *a, float *out, Strides s, int64_t n, int64_t a_off)
 {
+    pdl_enter();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         int64_t rem = i, ia = a_off;
         for (int d = s.rank - 1; d >= 0; d--) {
@@ -188,8 +196,9 @@ __global__ void copy_strided_kernel(const float *__restrict__ a, float *__restri
 // The same gather when the innermost output dimension is contiguous in the source as well (narrow, cat, repeat_interleave,
 // transposes of outer dimensions): rows of `inner4` float4, the row's source offset from 32-bit index arithmetic.
 struct RowStrides { unsigned o[kMaxRank]; long long a[kMaxRank]; int rank; };   // outer dimensions only
-__global__ void copy_rows4_kernel(const float4 *__restrict__ a, float4 *__restrict__ out, RowStrides s, unsigned rows, unsigned inner4, long long a_off4)
+__global__ void copy_rows4_kernel(const float4 *a, float4 *out, RowStrides s, unsigned rows, unsigned inner4, long long a_off4)
 {
+    pdl_enter();
     const unsigned long long total = (unsigned long long)rows * inner4;
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < total; i += (unsigned long long)gridDim.x * blockDim.x) {
         const unsigned row = (unsigned)(i / inner4), col = (unsigned)(i - (unsigned long long)row * inner4);
@@ -206,8 +215,9 @@ __global__ void copy_rows4_kernel(const float4 *__restrict__ a, float4 *__restri
 
 // out[b][j][i] = a[b][i][j]: the last two dimensions exchanged, through a 32 x 33 shared-memory tile so that both the
 // reads and the writes are coalesced.
-__global__ void __launch_bounds__(256) transpose_last2_kernel(const float *__restrict__ a, float *__restrict__ out, int rows, int cols)
+__global__ void __launch_bounds__(256) transpose_last2_kernel(const float *a, float *out, int rows, int cols)
 {
+    pdl_enter();
     __shared__ float tile[32][33];
     const float *src = a + (size_t)blockIdx.z * rows * cols;
     float *dst = out + (size_t)blockIdx.z * rows * cols;
@@ -225,9 +235,10 @@ __global__ void __launch_bounds__(256) transpose_last2_kernel(const float *__res
 // Wide results take 64 columns per CTA; narrow ones (P.V: 128 columns, thousands of k) take 16, so that there are enough
 // CTAs and each thread's share of k stays short.
 template <int COLS>
-__global__ void __launch_bounds__(512) matmul_rows_kernel(const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ C,
+__global__ void __launch_bounds__(512) matmul_rows_kernel(const float *A, const float *B, float *C,
                                                           int m, int k, int n, int b_batched)
 {
+    pdl_enter();
     constexpr int SL = 512 / COLS;
     __shared__ float red[SL][4][COLS];
     const float *a = A + (size_t)blockIdx.y * m * k;
@@ -240,7 +251,7 @@ __global__ void __launch_bounds__(512) matmul_rows_kernel(const float *__restric
             const float bv = b[(size_t)kk * n + col];
 #pragma unroll
             for (int r = 0; r < 4; r++)
-                if (r < m) acc[r] = fmaf(__ldg(a + (size_t)r * k + kk), bv, acc[r]);
+                if (r < m) acc[r] = fmaf(a[(size_t)r * k + kk], bv, acc[r]);
         }
     }
 #pragma unroll
@@ -253,9 +264,10 @@ __global__ void __launch_bounds__(512) matmul_rows_kernel(const float *__restric
     }
 }
 
-__global__ void copy_into_kernel(const float *__restrict__ a, float *__restrict__ out, int64_t outer, int64_t a_inner,
+__global__ void copy_into_kernel(const float *a, float *out, int64_t outer, int64_t a_inner,
                                  int64_t o_inner, int64_t o_off)
 {
+    pdl_enter();
     int64_t n = outer * a_inner;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[(i / a_inner) * o_inner + o_off + i % a_inner] = a[i];
@@ -264,9 +276,10 @@ __global__ void copy_into_kernel(const float *__restrict__ a, float *__restrict_
 // rms_norm_kernel + mul_kernel (autograd.cu:612-627, two launches, one thread per row) and
 // fused_add_rms_norm_kernel (autograd.cu:2508-2525) -> one block per row, weight and residual fused.
 // x / sqrt(mean(x^2) + eps) then * w, in the CPU back end's operation order.
-__global__ void rms_norm_kernel(const float *__restrict__ x, const float *__restrict__ res, const float *__restrict__ w,
-                                float eps, float *__restrict__ out, int64_t d)
+__global__ void rms_norm_kernel(const float *x, const float *res, const float *w,
+                                float eps, float *out, int64_t d)
 {
+    pdl_enter();
     __shared__ float sh[32];
     const float *xr = x + (int64_t)blockIdx.x * d;
     const float *rr = res ? res + (int64_t)blockIdx.x * d : nullptr;
@@ -286,9 +299,10 @@ __global__ void rms_norm_kernel(const float *__restrict__ x, const float *__rest
 }
 
 // crates/tl_cpu/src/ffi.rs:2629-2685: adjacent pairs, table row 0 for every vector
-__global__ void rope_cpu_kernel(const float *__restrict__ x, const float *__restrict__ cos_t, const float *__restrict__ sin_t,
-                                int64_t tab_len, float *__restrict__ out, int64_t npairs, int64_t d)
+__global__ void rope_cpu_kernel(const float *x, const float *cos_t, const float *sin_t,
+                                int64_t tab_len, float *out, int64_t npairs, int64_t d)
 {
+    pdl_enter();
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npairs; p += (int64_t)gridDim.x * blockDim.x) {
         int64_t v = p / (d / 2), i = (p % (d / 2)) * 2;
         float c = i < tab_len ? cos_t[i] : 1.0f, s = i < tab_len ? sin_t[i] : 0.0f;
@@ -299,9 +313,10 @@ __global__ void rope_cpu_kernel(const float *__restrict__ x, const float *__rest
 }
 
 // apply_rope_kernel (autograd.cu:1196-1227): rotate-half, one table row per token
-__global__ void rope_half_kernel(const float *__restrict__ x, const float *__restrict__ cos_t, const float *__restrict__ sin_t,
-                                 float *__restrict__ out, int64_t tokens, int64_t heads, int64_t d)
+__global__ void rope_half_kernel(const float *x, const float *cos_t, const float *sin_t,
+                                 float *out, int64_t tokens, int64_t heads, int64_t d)
 {
+    pdl_enter();
     int64_t half = d / 2, n = tokens * heads * half;
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
         int64_t i = p % half, vh = p / half, t = vh / heads;
@@ -314,9 +329,10 @@ __global__ void rope_half_kernel(const float *__restrict__ x, const float *__res
 
 // embedding_f32_kernel (autograd.cu:66-81); an out-of-range id raises a flag (the CPU back end
 // errors, crates/tl_cpu/src/tensor.rs:1094-1112; the CUDA one silently writes zeros)
-__global__ void embedding_kernel(const float *__restrict__ table, const float *__restrict__ idx, float *__restrict__ out,
+__global__ void embedding_kernel(const float *table, const float *idx, float *out,
                                  int64_t n, int64_t vocab, int64_t dim, int *oob)
 {
+    pdl_enter();
     int64_t total = n * dim;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         int64_t r = i / dim, id = (int64_t)idx[r];
@@ -340,8 +356,9 @@ __device__ __forceinline__ bool better(float v, int64_t i, float bv, int64_t bi,
     return tie_first ? i < bi : i > bi;
 }
 
-__global__ void argmax_partial_kernel(const float *__restrict__ x, int64_t n, int tie_first, float *pv, long long *pi)
+__global__ void argmax_partial_kernel(const float *x, int64_t n, int tie_first, float *pv, long long *pi)
 {
+    pdl_enter();
     __shared__ float sv[32];
     __shared__ long long si[32];
     float bv = 0.f;
@@ -368,6 +385,7 @@ __global__ void argmax_partial_kernel(const float *__restrict__ x, int64_t n, in
 
 __global__ void argmax_final_kernel(const float *pv, const long long *pi, int nparts, int tie_first, float *out_f32, int *out_i32)
 {
+    pdl_enter();
     if (threadIdx.x == 0) {
         float bv = 0.f;
         int64_t bi = -1;
@@ -381,6 +399,7 @@ __global__ void argmax_final_kernel(const float *pv, const long long *pi, int np
 
 __global__ void causal_mask_kernel(float *out, int64_t size)
 {
+    pdl_enter();
     int64_t n = size * size;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = (i % size > i / size) ? -INFINITY : 0.f;
@@ -390,6 +409,7 @@ __global__ void causal_mask_kernel(float *out, int64_t size)
 // (crates/tl_cpu/src/device_impl.rs:967-1000 dedups the token list)
 __global__ void rep_penalty_kernel(float *logits, const float *tokens, int64_t rows, int64_t vocab, int64_t nt, float p)
 {
+    pdl_enter();
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nt; t += (int64_t)gridDim.x * blockDim.x) {
         float tf = tokens[t];
         int64_t id = tf < 0.f ? 0 : (int64_t)tf;
@@ -410,6 +430,7 @@ __global__ void rep_penalty_kernel(float *logits, const float *tokens, int64_t r
 
 __global__ void f32_to_f16_kernel(const float *a, __half *out, int64_t n)
 {
+    pdl_enter();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = __float2half_rn(a[i]);
 }
@@ -423,7 +444,7 @@ __global__ void f32_to_f16_kernel(const float *a, __half *out, int64_t n)
 tlb_status launch_unary(int op, const float *a, float *out, int64_t n, float s)
 {
     if (n == 0) return TLB_OK;
-    unary_kernel<<<grid_for(n, 256), 256, 0, ctx()->stream>>>(op, a, out, n, s);
+    TLB_CUDA(launch_chained(unary_kernel, dim3(grid_for(n, 256)), dim3(256), 0, true, op, a, out, n, s));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -432,9 +453,9 @@ tlb_status launch_silu_mul(const float *g, const float *u, float *out, int64_t n
 {
     if (n == 0) return TLB_OK;
     if (n % 4 == 0 && (((uintptr_t)g | (uintptr_t)u | (uintptr_t)out) & 15) == 0)
-        silu_mul4_kernel<<<grid_for(n / 4, 256), 256, 0, ctx()->stream>>>((const float4 *)g, (const float4 *)u, (float4 *)out, n / 4);
+        TLB_CUDA(launch_chained(silu_mul4_kernel, dim3(grid_for(n / 4, 256)), dim3(256), 0, true, (const float4 *)g, (const float4 *)u, (float4 *)out, n / 4));
     else
-        silu_mul_kernel<<<grid_for(n, 256), 256, 0, ctx()->stream>>>(g, u, out, n);
+        TLB_CUDA(launch_chained(silu_mul_kernel, dim3(grid_for(n, 256)), dim3(256), 0, true, g, u, out, n));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -443,7 +464,7 @@ tlb_status launch_softmax(const float *a, float *out, int64_t outer, int64_t axi
 {
     if (outer * axis * inner == 0) return TLB_OK;
     int threads = axis >= 1024 ? 256 : (axis >= 128 ? 128 : 32);
-    softmax_kernel<<<(unsigned)(outer * inner), threads, 0, ctx()->stream>>>(a, out, axis, inner);
+    TLB_CUDA(launch_chained(softmax_kernel, dim3((unsigned)(outer * inner)), dim3(threads), 0, true, a, out, axis, inner));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -454,16 +475,16 @@ tlb_status launch_matmul(const float *a, const float *b, float *out, int64_t bat
     if (m <= 4 && k <= INT32_MAX && n <= INT32_MAX && batch <= 65535) {
         if (n <= 256) {
             dim3 grid((unsigned)((n + 15) / 16), (unsigned)batch);
-            matmul_rows_kernel<16><<<grid, 512, 0, ctx()->stream>>>(a, b, out, (int)m, (int)k, (int)n, b_batched ? 1 : 0);
+            TLB_CUDA(launch_chained(matmul_rows_kernel<16>, grid, dim3(512), 0, true, a, b, out, (int)m, (int)k, (int)n, b_batched ? 1 : 0));
         } else {
             dim3 grid((unsigned)((n + 63) / 64), (unsigned)batch);
-            matmul_rows_kernel<64><<<grid, 512, 0, ctx()->stream>>>(a, b, out, (int)m, (int)k, (int)n, b_batched ? 1 : 0);
+            TLB_CUDA(launch_chained(matmul_rows_kernel<64>, grid, dim3(512), 0, true, a, b, out, (int)m, (int)k, (int)n, b_batched ? 1 : 0));
         }
         LAUNCH_CHECK();
         return TLB_OK;
     }
     dim3 grid((unsigned)((n + 63) / 64), (unsigned)((m + 63) / 64), (unsigned)batch);
-    matmul_kernel<<<grid, 256, 0, ctx()->stream>>>(a, b, out, m, k, n, b_batched ? 1 : 0);
+    TLB_CUDA(launch_chained(matmul_kernel, grid, dim3(256), 0, true, a, b, out, m, k, n, b_batched ? 1 : 0));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -479,7 +500,7 @@ tlb_status launch_copy_strided(const float *a, float *out, const int64_t *oshape
         const int rows = (int)oshape[rank - 1], cols = (int)oshape[rank - 2];   // of the source: [rows][cols] -> [cols][rows]
         if (outer_plain && batch <= 65535 && (rows + 31) / 32 <= 65535) {
             dim3 grid((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32), (unsigned)batch);
-            transpose_last2_kernel<<<grid, 256, 0, ctx()->stream>>>(a, out, rows, cols);
+            TLB_CUDA(launch_chained(transpose_last2_kernel, grid, dim3(256), 0, true, a, out, rows, cols));
             LAUNCH_CHECK();
             return TLB_OK;
         }
@@ -497,8 +518,8 @@ tlb_status launch_copy_strided(const float *a, float *out, const int64_t *oshape
         }
         if (ok) {
             const unsigned rows = (unsigned)(n / oshape[rank - 1]), inner4 = (unsigned)(oshape[rank - 1] / 4);
-            copy_rows4_kernel<<<grid_for(n / 4, 256), 256, 0, ctx()->stream>>>(reinterpret_cast<const float4 *>(a), reinterpret_cast<float4 *>(out), r, rows,
-                                                                               inner4, a_off / 4);
+            TLB_CUDA(launch_chained(copy_rows4_kernel, dim3(grid_for(n / 4, 256)), dim3(256), 0, true, reinterpret_cast<const float4 *>(a), reinterpret_cast<float4 *>(out), r, rows,
+                                                                               inner4, a_off / 4));
             LAUNCH_CHECK();
             return TLB_OK;
         }
@@ -506,7 +527,7 @@ tlb_status launch_copy_strided(const float *a, float *out, const int64_t *oshape
     Strides s;
     s.rank = rank;
     for (int i = 0; i < rank; i++) { s.o[i] = oshape[i]; s.a[i] = astr[i]; s.b[i] = 0; }
-    copy_strided_kernel<<<grid_for(n, 256), 256, 0, ctx()->stream>>>(a, out, s, n, a_off);
+    TLB_CUDA(launch_chained(copy_strided_kernel, dim3(grid_for(n, 256)), dim3(256), 0, true, a, out, s, n, a_off));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -515,7 +536,7 @@ tlb_status launch_rms_norm(const float *x, const float *res, const float *w, flo
 {
     if (rows * d == 0) return TLB_OK;
     int threads = d >= 2048 ? 512 : (d >= 256 ? 128 : 32);
-    rms_norm_kernel<<<(unsigned)rows, threads, 0, ctx()->stream>>>(x, res, w, eps, out, d);
+    TLB_CUDA(launch_chained(rms_norm_kernel, dim3((unsigned)rows), dim3(threads), 0, true, x, res, w, eps, out, d));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -524,7 +545,7 @@ tlb_status launch_rope_cpu(const float *x, const float *cos_t, const float *sin_
 {
     int64_t np = nvec * (d / 2);
     if (np == 0) return TLB_OK;
-    rope_cpu_kernel<<<grid_for(np, 256), 256, 0, ctx()->stream>>>(x, cos_t, sin_t, tab_len, out, np, d);
+    TLB_CUDA(launch_chained(rope_cpu_kernel, dim3(grid_for(np, 256)), dim3(256), 0, true, x, cos_t, sin_t, tab_len, out, np, d));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -533,7 +554,7 @@ tlb_status launch_rope_half(const float *x, const float *cos_t, const float *sin
 {
     int64_t np = tokens * heads * (d / 2);
     if (np == 0) return TLB_OK;
-    rope_half_kernel<<<grid_for(np, 256), 256, 0, ctx()->stream>>>(x, cos_t, sin_t, out, tokens, heads, d);
+    TLB_CUDA(launch_chained(rope_half_kernel, dim3(grid_for(np, 256)), dim3(256), 0, true, x, cos_t, sin_t, out, tokens, heads, d));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -541,7 +562,7 @@ tlb_status launch_rope_half(const float *x, const float *cos_t, const float *sin
 tlb_status launch_embedding(const float *table, const float *idx, float *out, int64_t n, int64_t vocab, int64_t dim, int *oob)
 {
     if (n * dim == 0) return TLB_OK;
-    embedding_kernel<<<grid_for(n * dim, 256), 256, 0, ctx()->stream>>>(table, idx, out, n, vocab, dim, oob);
+    TLB_CUDA(launch_chained(embedding_kernel, dim3(grid_for(n * dim, 256)), dim3(256), 0, true, table, idx, out, n, vocab, dim, oob));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -556,9 +577,9 @@ tlb_status launch_argmax(const float *x, int64_t n, int tie_first, float *out_f3
         TLB_CUDA(cudaMalloc(&pi, parts * sizeof(long long)));
     }
     int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(parts, (n + 1023) / 1024));
-    argmax_partial_kernel<<<blocks, 256, 0, ctx()->stream>>>(x, n, tie_first, pv, pi);
+    TLB_CUDA(launch_chained(argmax_partial_kernel, dim3(blocks), dim3(256), 0, true, x, n, tie_first, pv, pi));
     LAUNCH_CHECK();
-    argmax_final_kernel<<<1, 32, 0, ctx()->stream>>>(pv, pi, blocks, tie_first, out_f32, out_i32);
+    TLB_CUDA(launch_chained(argmax_final_kernel, dim3(1), dim3(32), 0, true, pv, pi, blocks, tie_first, out_f32, out_i32));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -566,7 +587,7 @@ tlb_status launch_argmax(const float *x, int64_t n, int tie_first, float *out_f3
 tlb_status launch_causal_mask(float *out, int64_t size)
 {
     if (size == 0) return TLB_OK;
-    causal_mask_kernel<<<grid_for(size * size, 256), 256, 0, ctx()->stream>>>(out, size);
+    TLB_CUDA(launch_chained(causal_mask_kernel, dim3(grid_for(size * size, 256)), dim3(256), 0, true, out, size));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -574,7 +595,7 @@ tlb_status launch_causal_mask(float *out, int64_t size)
 tlb_status launch_rep_penalty(float *logits, const float *tokens, int64_t rows, int64_t vocab, int64_t nt, float p)
 {
     if (nt == 0 || rows * vocab == 0) return TLB_OK;
-    rep_penalty_kernel<<<grid_for(nt, 128), 128, 0, ctx()->stream>>>(logits, tokens, rows, vocab, nt, p);
+    TLB_CUDA(launch_chained(rep_penalty_kernel, dim3(grid_for(nt, 128)), dim3(128), 0, true, logits, tokens, rows, vocab, nt, p));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -582,7 +603,7 @@ tlb_status launch_rep_penalty(float *logits, const float *tokens, int64_t rows, 
 tlb_status launch_f32_to_f16(const float *a, __half *out, int64_t n)
 {
     if (n == 0) return TLB_OK;
-    f32_to_f16_kernel<<<grid_for(n, 256), 256, 0, ctx()->stream>>>(a, out, n);
+    TLB_CUDA(launch_chained(f32_to_f16_kernel, dim3(grid_for(n, 256)), dim3(256), 0, true, a, out, n));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -612,9 +633,9 @@ tlb_status launch_binary_bcast(int op, const tlb_tensor *a, const tlb_tensor *b,
     int64_t n = (*out)->numel();
     if (n == 0) return TLB_OK;
     if (a->numel() == n && b->numel() == n)
-        same_shape_binary_kernel<<<grid_for(n, 256), 256, 0, ctx()->stream>>>(op, a->f32(), b->f32(), (*out)->f32(), n);
+        TLB_CUDA(launch_chained(same_shape_binary_kernel, dim3(grid_for(n, 256)), dim3(256), 0, true, op, a->f32(), b->f32(), (*out)->f32(), n));
     else
-        binary_kernel<<<grid_for(n, 256), 256, 0, ctx()->stream>>>(op, a->f32(), b->f32(), (*out)->f32(), s, n);
+        TLB_CUDA(launch_chained(binary_kernel, dim3(grid_for(n, 256)), dim3(256), 0, true, op, a->f32(), b->f32(), (*out)->f32(), s, n));
     LAUNCH_CHECK();
     return TLB_OK;
 }
@@ -623,7 +644,7 @@ tlb_status launch_copy_into(const float *a, float *out, int64_t outer, int64_t a
 {
     int64_t n = outer * a_inner;
     if (n == 0) return TLB_OK;
-    copy_into_kernel<<<grid_for(n, 256), 256, 0, ctx()->stream>>>(a, out, outer, a_inner, o_inner, o_off);
+    TLB_CUDA(launch_chained(copy_into_kernel, dim3(grid_for(n, 256)), dim3(256), 0, true, a, out, outer, a_inner, o_inner, o_off));
     LAUNCH_CHECK();
     return TLB_OK;
 }

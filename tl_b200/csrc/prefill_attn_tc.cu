@@ -107,6 +107,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __gr
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    pdl_enter();
 
     if (warp < 4) {
         // ------------------------------------------------ softmax: thread = query row
@@ -349,8 +350,9 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __gr
 }
 
 // q f32 [T, cols] -> f16, and V rows [kvh][key][128] of the cache -> V^T [kvh][128][keys_ld] for keys < n_keys
-__global__ void q_to_f16_kernel(const float *__restrict__ q, __half *__restrict__ qh, size_t n4)
+__global__ void q_to_f16_kernel(const float *q, __half *qh, size_t n4)
 {
+    pdl_enter();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
         const float4 v = reinterpret_cast<const float4 *>(q)[i];
         __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
@@ -360,8 +362,9 @@ __global__ void q_to_f16_kernel(const float *__restrict__ q, __half *__restrict_
         reinterpret_cast<uint2 *>(qh)[i] = o;
     }
 }
-__global__ void __launch_bounds__(256) v_transpose_kernel(const __half *__restrict__ vcache, __half *__restrict__ vt, int max_seq, int n_keys, int keys_ld)
+__global__ void __launch_bounds__(256) v_transpose_kernel(const __half *vcache, __half *vt, int max_seq, int n_keys, int keys_ld)
 {
+    pdl_enter();
     __shared__ __half tile[32][34];
     const __half *src = vcache + (size_t)blockIdx.z * max_seq * kAtD;
     __half *dst = vt + (size_t)blockIdx.z * kAtD * keys_ld;
@@ -481,9 +484,9 @@ tlb_status launch_prefill_attention_tc(const float *q, const void *kcache, const
     if (!qh || !vt) { if (qh) storage_release(qh); if (vt) storage_release(vt); return TLB_ERR_ALLOC; }
     auto done = [&](tlb_status st) { storage_release(qh); storage_release(vt); return st; };   // stream-ordered: freed after the launches below
     const size_t n4 = (size_t)T * H * kAtD / 4;
-    q_to_f16_kernel<<<(unsigned)std::min<size_t>(148 * 8, (n4 + 255) / 256), 256, 0, c->stream>>>(q, (__half *)qh->ptr, n4);
+    TLB_CUDA(launch_chained(q_to_f16_kernel, dim3((unsigned)std::min<size_t>(148 * 8, (n4 + 255) / 256)), dim3(256), 0, true, q, (__half *)qh->ptr, n4));
     dim3 tg(kAtD / 32, (unsigned)(keys_ld / 32), (unsigned)KVH);
-    v_transpose_kernel<<<tg, 256, 0, c->stream>>>((const __half *)vcache, (__half *)vt->ptr, max_seq, n_keys, keys_ld);
+    TLB_CUDA(launch_chained(v_transpose_kernel, tg, dim3(256), 0, true, (const __half *)vcache, (__half *)vt->ptr, max_seq, n_keys, keys_ld));
     count_launch(2);
     CUtensorMap qmap, kmap, vtmap;
     if (!encode_f16_map(&qmap, qh->ptr, (uint64_t)H * kAtD, (uint64_t)T, (uint64_t)H * kAtD * 2, 64, 128) ||
@@ -502,9 +505,8 @@ tlb_status launch_prefill_attention_tc(const float *q, const void *kcache, const
         attr_set = true;
     }
     dim3 grid((unsigned)((T + kAtQ - 1) / kAtQ), (unsigned)H);
-    prefill_attention_tc_kernel<false, 2><<<grid, kAtThreads, smem, c->stream>>>(qmap, kmap, vtmap, p);
+    cudaError_t e = launch_chained(prefill_attention_tc_kernel<false, 2>, grid, dim3(kAtThreads), smem, true, qmap, kmap, vtmap, p);
     count_launch();
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return done(cuda_fail(e, "prompt attention launch"));
     return done(TLB_OK);
 }

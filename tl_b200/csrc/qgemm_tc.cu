@@ -457,6 +457,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
         const bool ok = warp < 8 ? produce<FMT, 0, GS, PAIR>(p, ub, have, lane, dst, slots, full_lead, empty_bar(0), abort_flag, u0, u1 - u0)
                                  : produce<FMT, 1, GS, PAIR>(p, ub, have, lane, dst, slots, full_lead, empty_bar(0), abort_flag, u0, u1 - u0);
         // ------------------------------------------------ epilogue: tensor memory -> Y[token][row]
+        pdl_wait();                      // row scales, residual and outputs belong to the launches before; the weights above do not
         if (ok && mbar_wait(accum_bar, 0, abort_flag, p.err, 22)) {
             tc_fence_after();
             const int quad = warp & 3, part = warp >> 2;    // tensor-memory lanes 32 quad .., a quarter of the columns
@@ -473,8 +474,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
                 for (int j = 0; j < 8; j++) {
                     const int tok = tok0 + c0 + j;
                     const bool live = tok < p.m && row < n_rows;
-                    sc[j] = tok < p.m ? __ldg(p.inv_scale + tok) : 0.f;
-                    rs[j] = (live && p.resid && !partial) ? __ldg(p.resid + (size_t)tok * n_rows + row) : 0.f;
+                    sc[j] = tok < p.m ? p.inv_scale[tok] : 0.f;
+                    rs[j] = (live && p.resid && !partial) ? p.resid[(size_t)tok * n_rows + row] : 0.f;
                 }
                 uint32_t v[8];
                 tmem_ld8(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
@@ -491,6 +492,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
     } else if (warp == kGemmProducers) {
         // ------------------------------------------------ TMA: activation tile of each K step, nb steps ahead of the MMAs
         if (lane == 0) {
+            pdl_enter();                                       // the activations are the launch before's
             int issued = 0;
             int st = 0, slot = 0, bslot = 0, bround = 0;       // kt % nb, kt % slots, (kt - nb) % slots, (kt - nb) / slots
             for (int kt = 0; kt < KT; kt++) {
@@ -575,6 +577,7 @@ struct SplitSum {
 };
 __global__ void __launch_bounds__(256) qgemm_split_sum_kernel(const SplitSum a)
 {
+    pdl_enter();
     const size_t total = (size_t)a.m * a.n_all, stride = total;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const int tok = (int)(i / a.n_all), col = (int)(i - (size_t)tok * a.n_all);
@@ -583,7 +586,7 @@ __global__ void __launch_bounds__(256) qgemm_split_sum_kernel(const SplitSum a)
         const int row = col - a.col0[w];
         float acc = __ldcg(a.part + i);
         for (int s = 1; s < a.splits; s++) acc += __ldcg(a.part + s * stride + i);
-        if (a.resid) acc += __ldg(a.resid + (size_t)tok * a.n[w] + row);
+        if (a.resid) acc += __ldcg(a.resid + (size_t)tok * a.n[w] + row);
         a.out[w][(size_t)tok * a.n[w] + row] = acc;
     }
 }
@@ -896,6 +899,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qrows_kernel(const RowsParams
     };
     for (int i = 0; i < wstages && pf_pos < end; i++) issue(i);
     pdl_wait();                                // from here on: activations, scales, residual, outputs, scratch and counters
+    pdl_launch_dependents();
 
     int g = 0, ws = 0;                         // units consumed, their weight stage
     uint32_t wph = 0;
@@ -1059,14 +1063,13 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qrows_kernel(const RowsParams
 // NC > 0: the row (k <= 4 NT NC) stays in registers, NC float4 per thread, between the pass that finds its scale and
 // the pass that writes; NC = 0 reads (and recomputes) it twice.
 template <int NT, int NC>
-__global__ void __launch_bounds__(NT) x_to_f16_kernel(const float *__restrict__ x, const float *__restrict__ x2, const float *__restrict__ norm_w,
-                                                        float eps, __half *__restrict__ xh, float *__restrict__ inv_scale, int64_t k,
-                                                        uint32_t *__restrict__ sums)
+__global__ void __launch_bounds__(NT) x_to_f16_kernel(const float *x, const float *x2, const float *__restrict__ norm_w,
+                                                        float eps, __half *xh, float *inv_scale, int64_t k, uint32_t *sums)
 {
     constexpr bool CACHED = NC > 0;
     constexpr int kActCache = NC;
     __shared__ float red[2][NT / 32];
-    pdl_launch_dependents();     // a dependent launch (the few-rows kernel) may start its prologue; it waits for this grid's end before it reads
+    pdl_enter();                 // the products behind it may start their prologues; they wait for this grid's end before they read
     const float *row = x + (size_t)blockIdx.x * k;
     const float *row2 = x2 ? x2 + (size_t)blockIdx.x * k : nullptr;
     __half *orow = xh + (size_t)blockIdx.x * k;
@@ -1097,6 +1100,7 @@ __global__ void __launch_bounds__(NT) x_to_f16_kernel(const float *__restrict__ 
             if (i < k) pass1(i, it);
         }
     } else {
+#pragma unroll 4
         for (int64_t i = threadIdx.x * 4; i < k; i += NT * 4) pass1(i, 0);
     }
     for (int o = 16; o; o >>= 1) {
@@ -1229,12 +1233,14 @@ tlb_status launch_fmt_gemm_gs(dim3 grid, size_t smem, cudaStream_t stream, const
     cfg.blockDim = dim3(kGemmThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = 2;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = PAIR ? 1 : 0;
+    cfg.numAttrs = PAIR ? 2 : 1;
     TLB_CUDA(cudaLaunchKernelEx(&cfg, qgemm_kernel<FMT, GS, PAIR>, map, p));
     return TLB_OK;
 }
@@ -1270,9 +1276,11 @@ tlb_status qgemm_prepare(GemmAct *a, const float *x, const float *x2, int64_t m,
         sums = (uint32_t *)a->sums->ptr;
     }
     // few rows are few CTAs: each takes its row with 1024 threads and keeps it in registers
-    if (m <= 16 && k > 4096 && k <= 32768) x_to_f16_kernel<1024, 8><<<(unsigned)m, 1024, 0, c->stream>>>(x, x2, norm_w, eps, xh, inv, k, sums);
-    else if (k <= 4096) x_to_f16_kernel<256, 4><<<(unsigned)m, 256, 0, c->stream>>>(x, x2, norm_w, eps, xh, inv, k, sums);
-    else x_to_f16_kernel<256, 0><<<(unsigned)m, 256, 0, c->stream>>>(x, x2, norm_w, eps, xh, inv, k, sums);
+    cudaError_t e;
+    if (m <= 16 && k > 4096 && k <= 32768) e = launch_chained(x_to_f16_kernel<1024, 8>, dim3((unsigned)m), dim3(1024), 0, true, x, x2, norm_w, eps, xh, inv, k, sums);
+    else if (k <= 4096) e = launch_chained(x_to_f16_kernel<256, 4>, dim3((unsigned)m), dim3(256), 0, true, x, x2, norm_w, eps, xh, inv, k, sums);
+    else e = launch_chained(x_to_f16_kernel<256, 0>, dim3((unsigned)m), dim3(256), 0, true, x, x2, norm_w, eps, xh, inv, k, sums);
+    if (e != cudaSuccess) { qgemm_release(a); return cuda_fail(e, "f16 conversion launch"); }
     count_launch();
     return TLB_OK;
 }
@@ -1287,32 +1295,21 @@ void qgemm_release(GemmAct *a)
 
 namespace {
 template <int FMT, int NT>
-tlb_status launch_fmt_rows(int grid, size_t smem, cudaStream_t stream, const RowsParams &p)
+tlb_status launch_fmt_rows(int grid, size_t smem, const RowsParams &p)
 {
     static bool attr_set = false;
     if (!attr_set) {
         TLB_CUDA(cudaFuncSetAttribute(qrows_kernel<FMT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024));
         attr_set = true;
     }
-    // programmatic dependent launch: the CTAs start - barriers, the first weight copies - while x_to_f16_kernel, which
-    // releases its dependents at once, still converts the activations; griddepcontrol.wait stands before their first use
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kRowsThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    TLB_CUDA(cudaLaunchKernelEx(&cfg, qrows_kernel<FMT, NT>, p));
+    // the CTAs start - barriers, the first weight copies - while x_to_f16_kernel still converts the activations
+    TLB_CUDA(launch_chained(qrows_kernel<FMT, NT>, dim3((unsigned)grid), dim3(kRowsThreads), smem, true, p));
     return TLB_OK;
 }
 template <int FMT>
-tlb_status launch_fmt_rows_nt(int grid, size_t smem, cudaStream_t stream, const RowsParams &p)
+tlb_status launch_fmt_rows_nt(int grid, size_t smem, const RowsParams &p)
 {
-    return p.m <= 8 ? launch_fmt_rows<FMT, 1>(grid, smem, stream, p) : launch_fmt_rows<FMT, 2>(grid, smem, stream, p);
+    return p.m <= 8 ? launch_fmt_rows<FMT, 1>(grid, smem, p) : launch_fmt_rows<FMT, 2>(grid, smem, p);
 }
 }  // namespace
 
@@ -1371,10 +1368,10 @@ tlb_status qrows_run(const tlb_qtensor *const *ws, int n_w, const GemmAct &a, fl
     const size_t smem = (size_t)kRowsAStages * (kRowsABytes + kRowsSumBytes) + (size_t)kRowsWarps * p.wstages * p.stage_w + 8 * (2 * kRowsAStages + kRowsWarps * p.wstages) + 128 + 64;
     tlb_status ls;
     switch (w0->type) {
-        case 12: ls = launch_fmt_rows_nt<12>(grid, smem, c->stream, p); break;
-        case 14: ls = launch_fmt_rows_nt<14>(grid, smem, c->stream, p); break;
-        case 2: ls = launch_fmt_rows_nt<2>(grid, smem, c->stream, p); break;
-        default: ls = launch_fmt_rows_nt<8>(grid, smem, c->stream, p); break;
+        case 12: ls = launch_fmt_rows_nt<12>(grid, smem, p); break;
+        case 14: ls = launch_fmt_rows_nt<14>(grid, smem, p); break;
+        case 2: ls = launch_fmt_rows_nt<2>(grid, smem, p); break;
+        default: ls = launch_fmt_rows_nt<8>(grid, smem, p); break;
     }
     if (ls != TLB_OK) { if (part) storage_release(part); return ls; }
     count_launch();
@@ -1462,9 +1459,8 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
         for (int i = 0; i < kGemmMaxW; i++) { a.out[i] = p.out[i]; a.n[i] = p.n[i]; a.col0[i] = p.col0[i]; }
         a.n_w = n_w; a.n_all = (int)n_all; a.m = (int)m; a.splits = splits; a.part = p.part; a.resid = resid;
         const unsigned blocks = (unsigned)std::min<int64_t>(4 * c->sm_count, (m * n_all + 255) / 256);
-        qgemm_split_sum_kernel<<<blocks, 256, 0, c->stream>>>(a);
+        e = launch_chained(qgemm_split_sum_kernel, dim3(blocks), dim3(256), 0, true, a);
         count_launch();
-        e = cudaGetLastError();
     }
     if (part) storage_release(part);     // stream-ordered: freed after the launches above have run
     if (e != cudaSuccess) return cuda_fail(e, "qgemm launch");

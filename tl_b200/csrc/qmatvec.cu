@@ -588,7 +588,7 @@ static double slice_cost(int type, int m, int64_t tiles, int upt, int upi, int s
 // is faster with sixteen (2048 x 5632: 9.8 against 12.5 us).
 static int warps_for(const MatvecJob &job, int64_t tiles, int upt, int sm_count)
 {
-    return job.m == 1 && (job.few || (!job.pdl && tiles * upt <= (int64_t)kFewWarps * sm_count)) ? kFewWarps : kWarps;
+    return job.m == 1 && (job.few || ((job.lone || !job.pdl) && tiles * upt <= (int64_t)kFewWarps * sm_count)) ? kFewWarps : kWarps;
 }
 
 // In a chain, where launches follow each other at once, eight warps gain up to larger launches, if all of them have eight and as
@@ -878,6 +878,7 @@ extern "C" tlb_status tlb_qtensor_matmul(tlb_tensor **out, const tlb_tensor *x, 
             job.k = k;
             job.m = (int)std::min<int64_t>(group, m - m0);
             job.x = xa->f32() + m0 * k;
+            job.pdl = job.lone = true;
             st = launch_qmatvec(job);
             if (st == TLB_ERR_SHAPE && job.m > 1) { group = (job.m + 1) / 2; st = TLB_OK; }
             else m0 += job.m;

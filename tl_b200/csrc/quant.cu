@@ -51,6 +51,17 @@ __global__ void repack_kernel(int type, const uint8_t *__restrict__ raw, uint8_t
     }
 }
 
+// Products read weights ahead of their wait for the launch before them (tlb_internal.h): a launch behind the one that writes a
+// weight, which ends before any product can be started early, makes that sound for a product that follows at once.
+__global__ void settle_kernel() {}
+static tlb_status settle()
+{
+    settle_kernel<<<1, 32, 0, ctx()->stream>>>();
+    count_launch();
+    TLB_CUDA(cudaGetLastError());
+    return TLB_OK;
+}
+
 tlb_status launch_repack(int type, const uint8_t *raw, uint8_t *tiled, int64_t n, int64_t k)
 {
     const QFormat *f = qformat(type);
@@ -62,7 +73,7 @@ tlb_status launch_repack(int type, const uint8_t *raw, uint8_t *tiled, int64_t n
     repack_kernel<<<blocks, 256, 0, ctx()->stream>>>(type, raw, tiled, n, k, seg, f->unit_bytes);
     count_launch();
     TLB_CUDA(cudaGetLastError());
-    return TLB_OK;
+    return settle();
 }
 
 // Builds, from two tiled tensors a and b of equal shape [n, k], the tiled tensor of 2n rows whose
@@ -100,7 +111,7 @@ tlb_status launch_interleave8(int type, const uint8_t *a, const uint8_t *b, uint
     interleave8_kernel<<<blocks, 256, 0, ctx()->stream>>>(type, a, b, dst, n, k, seg, f->unit_bytes);
     count_launch();
     TLB_CUDA(cudaGetLastError());
-    return TLB_OK;
+    return settle();
 }
 
 // ---- bit-exact dequantisation ------------------------------------------------------------

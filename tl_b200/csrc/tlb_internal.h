@@ -204,6 +204,7 @@ struct MatvecJob {
     const float *emb_table = nullptr; // ADD_NORM with token lookup: x = emb_table[*token * K ...]
     const int *token = nullptr;
     bool pdl = false;                // launch with programmatic stream serialization
+    bool lone = false;               // a call of its own, not a launch of a decode chain (also where pdl is not set)
     bool few = false;                // m == 1: part of a chain of short launches (matvec_few): CTAs of eight warps
     // ADD_NORM without the statistics pass: x already holds the whole residual and ssq_parts[0 .. n_parts)
     // are partial sums of its squares left by the launch that produced it (finish == FIN_RESID there)
@@ -291,5 +292,34 @@ struct DecodeAttnJob {
 tlb_status launch_decode_attention(const DecodeAttnJob &j);
 tlb_status launch_sdpa(const float *q, const float *k, const float *v, const float *mask, int mask_mode,
                        float *out, int64_t bh, int64_t sq, int64_t sk, int64_t d, int64_t mask_bh);
+
+// ---- launches that overlap with the one before (programmatic dependent launch).  A kernel is started while its predecessor on
+// the stream still runs and calls pdl_wait() before it touches anything that a launch before it may have written or may still
+// read; only then it lets its own dependent start, so that whatever a kernel reads ahead of its wait, the launch before its
+// predecessor has written at the latest.  Data of earlier launches is not read through const __restrict__ or __ldg: such loads
+// may be moved ahead of the wait.  What bounds small launches is the 1 to 2 us between the end of one and the start of the next:
+// 333 tokens through eight TinyLlama layers 1.41 -> 1.17 ms, four op-by-op steps of four such layers 3.41 -> 2.39, four rows
+// through 14336 x 4096 in Q8_0 26.4 -> 20.9 us, 2048 tokens of four Llama-3-8B layers 5.30 -> 5.22 ms.
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_enter() { pdl_wait(); pdl_launch_dependents(); }
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, bool pdl, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx()->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+#endif
 
 }  // namespace tlb
