@@ -9,7 +9,7 @@ import pytest
 
 import tl_b200 as tl
 from tl_b200 import _lib, synth
-from test_launch_plans_cpu import gemm_form, gemm_plan
+from test_launch_plans_cpu import gemm_form, gemm_plan, gemm_ranges
 
 pytestmark = pytest.mark.gpu
 
@@ -276,6 +276,28 @@ def test_qgemm_large_launches_by_pairs(t, n, k, m, form):
     np.testing.assert_array_equal(got.view(np.uint32), again.view(np.uint32))
     rows = np.unique(np.concatenate([np.arange(0, n, 61), np.arange(n - 130, n), np.arange(100, 160)]))
     ref = x.astype(np.float64) @ q.dequantize().numpy()[rows].astype(np.float64).T
+    for i in range(m):
+        assert relerr(got[i][rows], ref[i]) < GEMM_TOL, i
+
+
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("n,k,m,form", [(300, 1024, 17, (32, 2, False)), (2050, 2304, 63, (64, 3, False)), (1500, 5632, 31, (32, 6, False)), (1000, 1024, 100, (112, 2, False)),
+                                        (1500, 5632, 128, (128, 6, False)), (2500, 2304, 300, (160, 3, False)), (1900, 3328, 200, (128, 4, False)),
+                                        (3000, 4096, 700, (256, 2, False)), (5940, 8192, 333, (384, 2, True)), (4900, 8192, 380, (384, 3, True))])
+def test_qgemm_ranges_in_a_cluster(t, n, k, m, form):
+    """K ranges that add their sums through each other's shared memory: two to six, of unequal length, 64- and 256-wide steps,
+    columns that do not divide by the ranges, ragged last tiles, pairs with an odd number of row tiles.  Sampled weight rows."""
+    assert gemm_ranges(m, n, k) == form
+    rng = np.random.default_rng(5700 + t + n + m)
+    q = tl.QTensor.from_gguf_bytes(t, n, k, synth.random_quant(t, n, k, rng))
+    x = rng.standard_normal((m, k), dtype=np.float32)
+    x[m // 2] *= 300.0
+    got = tl.Tensor.from_numpy(x).matmul_quantized(q).numpy()
+    again = tl.Tensor.from_numpy(x).matmul_quantized(q).numpy()
+    np.testing.assert_array_equal(got.view(np.uint32), again.view(np.uint32))
+    rows = np.unique(np.concatenate([np.arange(0, n, 17), np.arange(max(0, n - 130), n)]))
+    ref = x.astype(np.float64) @ q.dequantize().numpy()[rows].astype(np.float64).T
+    assert got.shape == (m, n)
     for i in range(m):
         assert relerr(got[i][rows], ref[i]) < GEMM_TOL, i
 

@@ -58,6 +58,32 @@ def gemm_plan(m, n, k):
     return gemm_form(m, n, k)[:2]
 
 
+def gemm_ranges(m, n, k):
+    """(rows of a tile, K ranges in one cluster, by pairs) where a product takes that form, or None"""
+    f = _lib.lib().tlb_gemm_ranges
+    f.restype, f.argtypes = C.c_int, [C.c_int64] * 4 + [C.c_int] + [C.POINTER(C.c_int)] * 3
+    nt, splits, pair = C.c_int(), C.c_int(), C.c_int()
+    found = f(m, (n + 127) // 128, k // 256, n, SMS, C.byref(nt), C.byref(splits), C.byref(pair))
+    return (nt.value, splits.value, bool(pair.value)) if found else None
+
+
+def test_gemm_ranges_are_launchable():
+    """Clusters of two to six CTAs, two units or more a range, and the other ranges' sums of a CTA's columns fit the activation ring."""
+    for n in (1, 128, 256, 1000, 2048, 4096, 5632, 14336, 28672, 128256):
+        for k in (256, 768, 1024, 2048, 2304, 4096, 8192, 14336, 28672):
+            for m in (17, 31, 64, 65, 100, 128, 129, 160, 255, 256, 257, 300, 333, 384, 385, 512, 513, 769, 1000, 1536, 2048, 2821, 4096, 10000, 9000000):
+                form = gemm_ranges(m, n, k)
+                if form is None:
+                    continue
+                nt, splits, pair = form
+                assert nt == (m + 15) // 16 * 16 if m <= 128 else nt in ((320, 384) if pair else (128, 160, 192, 224, 256)), (n, k, m)
+                assert splits in (2, 3, 4, 6) and splits * (1 + pair) <= 6 and 2 * splits <= k // 256, (n, k, m)
+                stage = (nt // 2 if pair else nt) * 128 * (4 if not pair and nt <= 64 else 1)
+                ring = max(3 if nt <= 64 else 4, min(16, 192 * 1024 // stage)) * stage
+                assert (splits - 1) * -(-(nt // 8) // splits) * 4096 <= ring, (n, k, m)
+                assert (m + nt - 1) // nt <= 65535, (n, k, m)
+
+
 def test_gemm_plans_are_launchable():
     """Tiles that an MMA takes (columns in steps of 16, of 64 where two CTAs halve two accumulators), K ranges of four units or
     more, scratch for the partial sums that stays small beside the outputs' own size or a wave of tiles, a grid within its limit."""

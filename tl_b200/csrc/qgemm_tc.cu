@@ -81,9 +81,10 @@ struct GemmParams {
     const float *inv_scale; // [m]
     const float *resid;     // [m, n] added to the result, or null
     int *err;
-    // K-splits (where tiles are too few to fill the SMs, or their last wave: plan_gemm): grid.z CTAs share a tile,
-    // each over 1 / splits of the units of K, writing its partial product to part[split][m][n_all]; a second small
-    // launch adds the splits (and the residual).  splits == 1: the result goes straight to out.
+    // K-splits (where tiles are too few to fill the SMs, or their last wave: plan_gemm, plan_ranges): grid.z CTAs share a tile,
+    // each over 1 / splits of the units of K.  Without `part` they (or the pairs) are one cluster and add their sums through
+    // each other's shared memory; with it each writes its partial product to part[split][m][n_all], and a second small launch
+    // adds the splits (and the residual).
     int splits;
     float *part;
     int n_all;              // columns of one partial row: the sum of the weights' rows
@@ -378,7 +379,9 @@ __device__ __forceinline__ bool produce(const GemmParams &p, const uint8_t *ub, 
 
 // ---- the kernel
 // PAIR: 0 one CTA per tile; 1 two CTAs share a token tile of up to 256 rows; 2 ... of up to 384, as two accumulators
-template <int FMT, int GS, int PAIR>
+// RANGES: the cluster takes all K ranges of its tiles (a form of its own: with a run-time flag the plain one lost 2 %, 512 rows
+// of 14336 x 4096 82.6 instead of 80.5 us)
+template <int FMT, int GS, int PAIR, bool RANGES>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
 {
@@ -418,7 +421,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
     const int rt = (int)blockIdx.x - (wi ? p.rt_end[wi - 1] : 0);   // 128-row tile inside weight wi
     const int n_rows = p.n[wi];
 
-    const uint32_t rank = PAIR ? cluster_rank() : 0u;             // 0: the CTA that issues the MMAs and owns the full barriers
+    // of a pair, 0 is the CTA that issues the MMAs and owns the full barriers, cluster rank `lead`
+    const uint32_t crank = PAIR || RANGES ? cluster_rank() : 0u, rank = PAIR ? crank & 1u : 0u, lead = crank - rank;
     if (tid == 0) {
         abort_word = 0;
         for (int i = 0; i < slots; i++) {
@@ -443,8 +447,37 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
     if (PAIR) cluster_sync();               // the other CTA's barriers are there
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    const uint32_t full_lead = PAIR ? cluster_addr(full_bar(0), 0) : full_bar(0);
+    const uint32_t full_lead = PAIR ? cluster_addr(full_bar(0), lead) : full_bar(0);
 
+    // What the dequantising warps do at the end: tensor memory -> Y[token][row]
+    // (chunks of 8 columns; add(chunk, sums): what else belongs to it).  A warp reaches tensor-memory lanes 32 (warp % 4) ..
+    auto finish = [&](int ch0, int ch1, auto add) {
+        const int row = rt * kGemmRows + (warp & 3) * 32 + lane;
+        const uint32_t tacc = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        // without RANGES, partial products may go to part[split][token][col0 + row], residual-free
+        const bool partial = !RANGES && p.splits > 1;
+        float *out = partial ? p.part + (size_t)split * p.m * p.n_all + p.col0[wi] : p.out[wi];
+        const int ld = partial ? p.n_all : n_rows;
+        for (int c0 = 8 * ch0; c0 < 8 * ch1; c0 += 8) {
+            // the residual and the row scales first (independent loads in flight together), then the accumulator
+            float rs[8], sc[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int tok = tok0 + c0 + j;
+                sc[j] = tok < p.m ? p.inv_scale[tok] : 0.f;
+                rs[j] = tok < p.m && row < n_rows && p.resid && !partial ? p.resid[(size_t)tok * n_rows + row] : 0.f;
+            }
+            uint32_t v[8];
+            tmem_ld8(tacc + (uint32_t)c0, v);
+            add(c0 >> 3, v);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int tok = tok0 + c0 + j;
+                if (tok < p.m && row < n_rows) out[(size_t)tok * ld + row] = rs[j] + __uint_as_float(v[j]) * sc[j];
+            }
+        }
+    };
+    bool live = false;                       // a producer warp whose accumulator is complete
     if (warp < kGemmProducers) {
         // ------------------------------------------------ dequantise the weight tile, stage by stage
         // 16 rows per warp.  A warp reaches only the tensor-memory lanes of its quarter (warp % 4), so warps w and
@@ -456,38 +489,12 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
         const uint32_t dst = tmem + ((uint32_t)(sub * 16) << 16) + tmem_a0;
         const bool ok = warp < 8 ? produce<FMT, 0, GS, PAIR>(p, ub, have, lane, dst, slots, full_lead, empty_bar(0), abort_flag, u0, u1 - u0)
                                  : produce<FMT, 1, GS, PAIR>(p, ub, have, lane, dst, slots, full_lead, empty_bar(0), abort_flag, u0, u1 - u0);
-        // ------------------------------------------------ epilogue: tensor memory -> Y[token][row]
         pdl_wait();                      // row scales, residual and outputs belong to the launches before; the weights above do not
-        if (ok && mbar_wait(accum_bar, 0, abort_flag, p.err, 22)) {
+        live = ok && mbar_wait(accum_bar, 0, abort_flag, p.err, 22);
+        if (!RANGES && live) {
             tc_fence_after();
-            const int quad = warp & 3, part = warp >> 2;    // tensor-memory lanes 32 quad .., a quarter of the columns
-            const int row = rt * kGemmRows + quad * 32 + lane;
-            float *out = p.out[wi];
-            const bool partial = p.splits > 1;   // partial products go to part[split][token][col0 + row], unscaled residual-free
-            float *pout = partial ? p.part + (size_t)split * p.m * p.n_all + p.col0[wi] : nullptr;
-            const int chunks = p.nt >> 3;
-            const int c_begin = 8 * (part * chunks / 4), c_end = 8 * ((part + 1) * chunks / 4);
-            for (int c0 = c_begin; c0 < c_end; c0 += 8) {
-                // the residual and the row scales first (independent loads in flight together), then the accumulator
-                float rs[8], sc[8];
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const int tok = tok0 + c0 + j;
-                    const bool live = tok < p.m && row < n_rows;
-                    sc[j] = tok < p.m ? p.inv_scale[tok] : 0.f;
-                    rs[j] = (live && p.resid && !partial) ? p.resid[(size_t)tok * n_rows + row] : 0.f;
-                }
-                uint32_t v[8];
-                tmem_ld8(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const int tok = tok0 + c0 + j;
-                    if (tok < p.m && row < n_rows) {
-                        if (partial) pout[(size_t)tok * p.n_all + row] = __uint_as_float(v[j]) * sc[j];
-                        else out[(size_t)tok * n_rows + row] = rs[j] + __uint_as_float(v[j]) * sc[j];
-                    }
-                }
-            }
+            const int part = warp >> 2, chunks = p.nt >> 3;         // a quarter of the columns
+            finish(part * chunks / 4, (part + 1) * chunks / 4, [](int, uint32_t (&)[8]) {});
         }
     } else if (warp == kGemmProducers) {
         // ------------------------------------------------ TMA: activation tile of each K step, nb steps ahead of the MMAs
@@ -548,15 +555,62 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
                             umma_f16_ts(tmem, ta + 8u * k16, bd + 2u * k16, idesc, (kt | j | k16) != 0);
                         }
                 }
-                if (PAIR) umma_commit_pair(empty_bar(slot));
+                if (PAIR) umma_commit_pair(empty_bar(slot), lead);
                 else umma_commit(empty_bar(slot));   // arrives when the MMAs above have read both stages
                 if (++st == nb) st = 0;
                 if (++slot == slots) { slot = 0; round++; }
             }
-            if (PAIR) umma_commit_pair(accum_bar);
+            if (PAIR) umma_commit_pair(accum_bar, lead);
             else umma_commit(accum_bar);
             if (!ok) mbar_wait_drain(accum_bar, 0);   // MMAs already issued finish before the tensor memory is freed
         }
+    }
+    if constexpr (RANGES) {
+        // The K ranges' sums meet in shared memory: of each CTA's columns, range o's CTA finishes chunks [chunks o / splits ..)
+        // and gets the other ranges' values of them, [range][column / 4][row][4], where its activation ring was.
+        constexpr uint32_t kPiece = kGemmRows * 16;     // 4 columns of a tile: 128 rows of 16 bytes
+        const int spl = p.splits, chunks = min(p.nt, (p.m - tok0 + 7) / 8 * 8) >> 3;      // pieces of 8 columns that hold a token
+        const int quad = warp & 3, part = warp >> 2;
+        const uint32_t at = (uint32_t)(quad * 32 + lane) * 16u, tacc = tmem + ((uint32_t)(quad * 32) << 16);
+        __syncwarp();
+        tc_fence_after();
+        cluster_sync();                             // nobody's ring is in use any more
+        if (live) {
+            for (int o = 0; o < spl; o++) {
+                if (o == split) continue;
+                const int b0 = chunks * o / spl, b1 = chunks * (o + 1) / spl, slot = split - (split > o);
+                const uint32_t dst = cluster_addr(sB, PAIR ? 2u * (uint32_t)o + rank : (uint32_t)o) + (uint32_t)(slot * (b1 - b0) * 2) * kPiece + at;
+                for (int ch = b0 + part; ch < b1; ch += 4) {
+                    uint32_t v[8];
+                    tmem_ld8(tacc + (uint32_t)(ch * 8), v);
+                    st_cluster_v4(dst + (uint32_t)((ch - b0) * 2) * kPiece, v, 0);
+                    st_cluster_v4(dst + (uint32_t)((ch - b0) * 2 + 1) * kPiece, v, 4);
+                }
+            }
+        }
+        __syncwarp();
+        cluster_sync();
+        const int own0 = chunks * split / spl, own = chunks * (split + 1) / spl - own0;
+        if (live)
+            finish(own0 + part * own / 4, own0 + (part + 1) * own / 4, [&](int ch, uint32_t (&v)[8]) {
+                // in the order of the ranges
+                const uint32_t src = sB + (uint32_t)((ch - own0) * 2) * kPiece + at, stride = (uint32_t)(own * 2) * kPiece;
+                float acc[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) acc[j] = 0.f;
+                for (int o = 0; o < spl; o++) {
+                    if (o == split) {
+#pragma unroll
+                        for (int j = 0; j < 8; j++) acc[j] += __uint_as_float(v[j]);
+                    } else {
+                        const uint4 a = lds128(src + (uint32_t)(o - (o > split)) * stride), b = lds128(src + (uint32_t)(o - (o > split)) * stride + kPiece);
+                        acc[0] += __uint_as_float(a.x); acc[1] += __uint_as_float(a.y); acc[2] += __uint_as_float(a.z); acc[3] += __uint_as_float(a.w);
+                        acc[4] += __uint_as_float(b.x); acc[5] += __uint_as_float(b.y); acc[6] += __uint_as_float(b.z); acc[7] += __uint_as_float(b.w);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++) v[j] = __float_as_uint(acc[j]);
+            });
     }
     tc_fence_before();
     __syncthreads();
@@ -1206,7 +1260,66 @@ GemmPlan plan_gemm(int64_t m, int64_t row_tiles, int64_t units, int64_t n_all, i
     return best;
 }
 
+// K ranges whose CTAs are one cluster and add their sums through shared memory: no scratch, no second launch, and 1 to 2 us
+// instead of 5 to 12 for them, so that small products gain by more and shorter ranges.  Q4_K, whole calls, us so / in one range or
+// with a summing launch:
+//   2048 x 2048: 17 rows 9.3 / 11.0, 128 rows 12.3 / 20.0, 333 rows 15.5 / 20.7, 1024 rows 21.6 / 23.7
+//   4096 x 4096: 333 rows 25.8 / 35.1, 512 rows 28.8 / 36.2;  6144 x 4096: 64 rows 16.5 / 22.6;  2048 x 5632: 512 rows 28.6 / 45.7
+// The cheapest by a model of the same form as plan_gemm's, fitted to 2300 calls with this form (5 %; chosen forms 0.2 % from the
+// fastest on average).  Clusters of up to six: the GPU holds 74 of two CTAs at a time, 45 of three, 33 of four and 22 of
+// six, but 15 of eight (120 of 148 SMs), so where plan_gemm wants more than six ranges it keeps the scratch.
+constexpr int kMostRanges = 6;
+bool plan_ranges(int64_t m, int64_t row_tiles, int64_t units, int64_t n_all, int sms, GemmPlan *plan)
+{
+    if (plan->splits > kMostRanges || units < 4) return false;
+    constexpr int kHeld[kMostRanges + 1] = {0, 148, 74, 45, 33, 0, 22};        // clusters of so many CTAs that 148 SMs hold
+    auto step_us = [](int nt, double busy) {                                   // a 64-wide K step of a tile of nt rows
+        return nt > 256 ? 0.431 + 0.00029 * nt : nt <= 64 ? 0.259 + (0.00043 * busy - 0.00032) * nt : 0.381 + (0.00033 * busy - 0.00011) * nt;
+    };
+    auto model = [&](int nt, int s, bool pair) {
+        const int64_t clusters = (pair ? (row_tiles + 1) / 2 : row_tiles) * ((m + nt - 1) / nt);
+        const int size = s * (pair ? 2 : 1), held = std::max(1, kHeld[size] * sms / 148);
+        const int64_t waves = (clusters + held - 1) / held;
+        const double steps = 4.0 * (double)((units + s - 1) / s), busy = (double)(clusters * size) / (double)(waves * sms);
+        return (double)waves * (steps * step_us(nt, busy) + 3.6 + 0.018 * nt) + (pair ? 0.8 : 0.0) + (s > 1 ? 0.5 + 0.3 * s : 0.0);
+    };
+    // the plan as it stands
+    const int64_t most = plan->splits;
+    double best_us;
+    {
+        const int64_t ctas = (plan->pair ? (row_tiles + 1) / 2 * 2 : row_tiles) * ((m + plan->nt - 1) / plan->nt) * most, waves = (ctas + sms - 1) / sms;
+        if (most == 1) best_us = model(plan->nt, 1, plan->pair);
+        else {
+            const double busy = (double)ctas / (double)(waves * sms), steps = 4.0 * (double)((units + most - 1) / most);
+            best_us = (double)waves * (steps * step_us(plan->nt, busy) + 3.6 + 0.018 * plan->nt) + 4.0 + 3.3e-6 * (double)(most * m * n_all);
+        }
+    }
+    bool found = false;
+    auto consider = [&](int nt, int s, bool pair) {
+        if (2 * s > units || s * (pair ? 2 : 1) > kMostRanges || (m + nt - 1) / nt > 65535) return;
+        const double us = model(nt, s, pair);
+        if (us < best_us * 0.98) { best_us = us; *plan = {nt, s, pair}; found = true; }
+    };
+    for (int s : {2, 3, 4, 6}) {
+        if (m <= 128) { consider((int)((m + 15) / 16 * 16), s, false); continue; }
+        for (int nt : {256, 224, 192, 160, 128}) consider(nt, s, false);
+        for (int nt : {384, 320}) consider(nt, s, true);
+    }
+    return found;
+}
+
 }  // namespace
+
+// K ranges in one cluster, where plan_ranges takes them: 1 and their form, or 0
+extern "C" int tlb_gemm_ranges(int64_t m, int64_t row_tiles, int64_t units, int64_t n_all, int sms, int *nt, int *splits, int *pair)
+{
+    GemmPlan p = plan_gemm(m, row_tiles, units, n_all, sms);
+    const bool found = plan_ranges(m, row_tiles, units, n_all, sms, &p);
+    *nt = p.nt;
+    *splits = p.splits;
+    *pair = p.pair;
+    return found;
+}
 
 // The plan of a launch over row_tiles tiles of 128 weight rows (n_all outputs in all) and units of 256 weights of K
 extern "C" void tlb_gemm_plan(int64_t m, int64_t row_tiles, int64_t units, int64_t n_all, int sms, int *nt, int *splits, int *pair)
@@ -1220,12 +1333,12 @@ extern "C" void tlb_gemm_plan(int64_t m, int64_t row_tiles, int64_t units, int64
 bool qgemm_supported(int type) { return type == 12 || type == 14 || type == 2 || type == 8; }
 
 namespace {
-template <int FMT, int GS, int PAIR>
+template <int FMT, int GS, int PAIR, bool RANGES>
 tlb_status launch_fmt_gemm_gs(dim3 grid, size_t smem, cudaStream_t stream, const CUtensorMap &map, const GemmParams &p)
 {
     static bool attr_set = false;
     if (!attr_set) {
-        TLB_CUDA(cudaFuncSetAttribute(qgemm_kernel<FMT, GS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemMax));
+        TLB_CUDA(cudaFuncSetAttribute(qgemm_kernel<FMT, GS, PAIR, RANGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemMax));
         attr_set = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -1237,19 +1350,25 @@ tlb_status launch_fmt_gemm_gs(dim3 grid, size_t smem, cudaStream_t stream, const
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = 2;
-    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    at[1].val.clusterDim.x = PAIR ? 2 : 1;
+    at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = RANGES ? (unsigned)p.splits : 1;
     cfg.attrs = at;
-    cfg.numAttrs = PAIR ? 2 : 1;
-    TLB_CUDA(cudaLaunchKernelEx(&cfg, qgemm_kernel<FMT, GS, PAIR>, map, p));
+    cfg.numAttrs = PAIR || RANGES ? 2 : 1;
+    TLB_CUDA(cudaLaunchKernelEx(&cfg, qgemm_kernel<FMT, GS, PAIR, RANGES>, map, p));
     return TLB_OK;
 }
 template <int FMT>
 tlb_status launch_fmt_gemm(dim3 grid, size_t smem, cudaStream_t stream, const CUtensorMap &map, const GemmParams &p)
 {
-    if (p.gs == 4) return launch_fmt_gemm_gs<FMT, 4, 0>(grid, smem, stream, map, p);
-    if (!p.pair) return launch_fmt_gemm_gs<FMT, 1, 0>(grid, smem, stream, map, p);
-    return p.nt > 256 ? launch_fmt_gemm_gs<FMT, 1, 2>(grid, smem, stream, map, p) : launch_fmt_gemm_gs<FMT, 1, 1>(grid, smem, stream, map, p);
+    if (p.splits > 1 && !p.part) {           // plan_ranges: pairs for wide tiles only
+        if (p.gs == 4) return launch_fmt_gemm_gs<FMT, 4, 0, true>(grid, smem, stream, map, p);
+        if (!p.pair) return launch_fmt_gemm_gs<FMT, 1, 0, true>(grid, smem, stream, map, p);
+        return launch_fmt_gemm_gs<FMT, 1, 2, true>(grid, smem, stream, map, p);
+    }
+    if (p.gs == 4) return launch_fmt_gemm_gs<FMT, 4, 0, false>(grid, smem, stream, map, p);
+    if (!p.pair) return launch_fmt_gemm_gs<FMT, 1, 0, false>(grid, smem, stream, map, p);
+    return p.nt > 256 ? launch_fmt_gemm_gs<FMT, 1, 2, false>(grid, smem, stream, map, p) : launch_fmt_gemm_gs<FMT, 1, 1, false>(grid, smem, stream, map, p);
 }
 }  // namespace
 
@@ -1407,9 +1526,9 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
     const int64_t m = a.m;
     int64_t n_all = 0;
     for (int i = 0; i < kGemmMaxW; i++) { p.col0[i] = (int)n_all; n_all += p.n[i]; }
-    const GemmPlan plan = plan_gemm(m, row_tiles, w0->upt, n_all, c->sm_count);
+    GemmPlan plan = plan_gemm(m, row_tiles, w0->upt, n_all, c->sm_count);
+    const bool ranges = plan_ranges(m, row_tiles, w0->upt, n_all, c->sm_count, &plan);
     const int nt = plan.nt;
-    int splits = plan.splits;
     const bool pair = plan.pair;
     CUtensorMap map;
     const cuuint64_t dims[2] = {(cuuint64_t)a.k, (cuuint64_t)m};
@@ -1436,14 +1555,14 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
     const size_t smem = (size_t)p.nb * stage_b + (kGemmSmemMax - kGemmBBytes);
     const int64_t tok_tiles = (m + nt - 1) / nt;
     Storage *part = nullptr;
-    if (splits > 1) {
-        part = storage_alloc((size_t)splits * m * n_all * sizeof(float));
-        if (!part) { cudaGetLastError(); splits = 1; }      // no room for the partial sums: one K range takes none
+    p.splits = plan.splits;
+    if (p.splits > 1 && !ranges) {
+        part = storage_alloc((size_t)p.splits * m * n_all * sizeof(float));
+        if (!part) { cudaGetLastError(); p.splits = 1; }    // no room for the partial sums: one K range takes none
     }
-    p.splits = splits;
     p.part = part ? (float *)part->ptr : nullptr;
     p.n_all = (int)n_all;
-    dim3 grid((unsigned)(pair ? (row_tiles + 1) / 2 * 2 : row_tiles), (unsigned)tok_tiles, (unsigned)splits);
+    dim3 grid((unsigned)(pair ? (row_tiles + 1) / 2 * 2 : row_tiles), (unsigned)tok_tiles, (unsigned)p.splits);
     tlb_status ls;
     switch (w0->type) {
         case 12: ls = launch_fmt_gemm<12>(grid, smem, c->stream, map, p); break;
@@ -1454,10 +1573,10 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
     if (ls != TLB_OK) { if (part) storage_release(part); return ls; }
     count_launch();
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess && splits > 1) {
+    if (e == cudaSuccess && part) {
         SplitSum a;
         for (int i = 0; i < kGemmMaxW; i++) { a.out[i] = p.out[i]; a.n[i] = p.n[i]; a.col0[i] = p.col0[i]; }
-        a.n_w = n_w; a.n_all = (int)n_all; a.m = (int)m; a.splits = splits; a.part = p.part; a.resid = resid;
+        a.n_w = n_w; a.n_all = (int)n_all; a.m = (int)m; a.splits = p.splits; a.part = p.part; a.resid = resid;
         const unsigned blocks = (unsigned)std::min<int64_t>(4 * c->sm_count, (m * n_all + 255) / 256);
         e = launch_chained(qgemm_split_sum_kernel, dim3(blocks), dim3(256), 0, true, a);
         count_launch();

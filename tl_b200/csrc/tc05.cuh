@@ -35,7 +35,7 @@ __device__ __forceinline__ void umma_commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// ---- a pair of CTAs (cluster of two) on one 256-row tile: each CTA's tensor memory holds its own 128 rows of A and of the
+// ---- a pair of CTAs (neighbours in a cluster, `lead` the even one's rank) on one 256-row tile: each CTA's tensor memory holds its own 128 rows of A and of the
 // accumulator, its shared memory half of B's columns.  One thread of the even CTA issues; the commit reports to both CTAs.
 __device__ __forceinline__ void umma_f16_ts_pair(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
 {
@@ -45,9 +45,9 @@ __device__ __forceinline__ void umma_f16_ts_pair(uint32_t tmem_d, uint32_t tmem_
         "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar)
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint32_t lead)
 {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)(3u << lead)) : "memory");
 }
 // the address of this CTA's `addr` in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank)
@@ -65,6 +65,10 @@ __device__ __forceinline__ uint32_t cluster_rank()
 __device__ __forceinline__ void cluster_sync()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t (&v)[8], int first)
+{
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[first]), "r"(v[first + 1]), "r"(v[first + 2]), "r"(v[first + 3]) : "memory");
 }
 // What a thread hands over with this arrival lies in tensor memory, which the tcgen05 fences order; a release at cluster
 // scope would flush the caches on every K step (14336 x 4096, 512 rows: 111 us with it, 83 us without).
