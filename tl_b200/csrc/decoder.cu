@@ -475,6 +475,7 @@ tlb_status enqueue_step(tlb_decoder *d)
             j.att_part = d->partial; j.att_pos = d->state + 1; j.att_max_splits = d->max_splits;
             j.att_rep = c.n_heads / c.n_kv_heads; j.att_dim = c.head_dim; j.att_keys = kAttnKeysPerSplit;
             j.finish = FIN_RESID; j.resid = d->xb; j.ssq_out = d->ssq_o;   // xa = xb + o_proj(attn)
+            j.ahead = w.ffn_norm->f32(); j.ahead_n = dm;
             j.tp_reduce = tpr;
             j.few = few; j.pdl = d->pdl;
             j.dry_run = d->dry;
@@ -499,6 +500,7 @@ tlb_status enqueue_step(tlb_decoder *d)
             j.type = w.down->type; j.k = F; j.m = 1;
             j.prologue = PRO_PLAIN; j.x = d->hbuf;
             j.finish = FIN_RESID; j.resid = d->xa; j.ssq_out = d->ssq_d;   // xb = xa + down(h)
+            j.ahead = (l + 1 < L ? d->layers[l + 1].attn_norm : d->out_norm)->f32(); j.ahead_n = dm;
             j.tp_reduce = tpr;
             j.few = few; j.pdl = d->pdl;
             j.dry_run = d->dry;

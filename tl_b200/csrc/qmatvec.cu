@@ -234,6 +234,11 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
         // before our predecessor complete, so it may read state those kernels wrote.
         pdl_launch_dependents();
     }
+    // Norm weights are read once per token and miss L2, and the launch that needs them starts too shortly before its wait (about
+    // 0.7 us) to have them from memory in time, so the one before asks for them.  A 32-token answer of the TinyLlama shapes
+    // 22.40 -> 21.71 ms, 16 tokens of eight Llama-3-8B layers 8.01 -> 7.93.
+    if (p.ahead_n && b == (int)gridDim.x - 1)
+        for (int i = tid * 32; i < p.ahead_n; i += NW * 32 * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.ahead + i));
     const unsigned tp_seq = p.tp_reduce ? ld_volatile_u32(p.tp.seq) : 0u;   // the launch before has completed: its exchange is over
     __syncthreads();               // abort_flag initialised; also keeps the CTA together for the prologue
     build_activation<FMT, ONE>(p, sh, smem, tid, NW * 32, blk0, nb, nsplit, wgt_first, [&](float dep) {
@@ -794,6 +799,7 @@ tlb_status launch_qmatvec(const MatvecJob &job)
     if (job.ssq_parts && (job.prologue != PRO_ADD_NORM || job.n_parts < 1)) return fail(TLB_ERR_ARG, "partial sums of squares go with the fused RMSNorm prologue");
     p.err = c->err_flag;
     p.use_pdl = job.pdl ? 1 : 0;
+    p.ahead = job.ahead; p.ahead_n = job.ahead ? job.ahead_n : 0;
     if (!p.x && !(p.prologue == PRO_ADD_NORM && p.token) && p.prologue != PRO_ATTN_MERGE) return fail(TLB_ERR_NULL, "null activation");
     if (p.prologue == PRO_SILU_MUL && !p.x2) return fail(TLB_ERR_NULL, "null activation");
     if (job.dry_run) return TLB_OK;   // the shape is launchable

@@ -213,6 +213,8 @@ struct MvParams {
     const float *emb_table;
     const int *token;
     int *err;
+    const float *ahead;       // asked into L2 for a later launch
+    int ahead_n;
     int use_pdl;
     int tp_reduce;            // the tile results are partial sums over tensor-parallel ranks: summed inside the launch (TpFuse)
     TpFuse tp;

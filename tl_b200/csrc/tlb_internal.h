@@ -204,6 +204,8 @@ struct MatvecJob {
     const float *emb_table = nullptr; // ADD_NORM with token lookup: x = emb_table[*token * K ...]
     const int *token = nullptr;
     bool pdl = false;                // launch with programmatic stream serialization
+    const float *ahead = nullptr;    // ahead_n floats that a later launch reads (norm weights, once a token): asked into L2
+    int ahead_n = 0;
     bool lone = false;               // a call of its own, not a launch of a decode chain (also where pdl is not set)
     bool few = false;                // m == 1: part of a chain of short launches (matvec_few): CTAs of eight warps
     // ADD_NORM without the statistics pass: x already holds the whole residual and ssq_parts[0 .. n_parts)
