@@ -40,6 +40,7 @@
 #include "qmv_units.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace tlb {
 
@@ -200,6 +201,7 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
         }
     }
     if (tid == 0) sh->abort_flag = 0;
+    if (ONE && tid < 64) *reinterpret_cast<uint32_t *>(smem + p.off_xq + 3 * p.col_stride + tid * 4) = 0u;   // the column of zeros
     __syncwarp();
 
     // Copy cursor (used by lane 0 only): the next unit to request and how many remain.
@@ -251,9 +253,24 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
     volatile int *abortp = &sh->abort_flag;
 
     const int ncols = M * NL;
-    LaneCtx L;
+    typename std::conditional<ONE, LaneOne, LaneCtx>::type L;
     L.lane = lane; L.r = lane >> 2; L.c = lane & 3;
-    {
+    if constexpr (ONE) {
+        const int r = L.r, c = L.c;
+        const uint32_t xq = smem_u32(smem + p.off_xq), zero = xq + 3 * p.col_stride;
+        const bool first = r < 3, second = r >= 4 && r < 7;
+        L.xa = (first ? xq + r * p.col_stride : zero) + c * 8;
+        L.xb = (second ? xq + (r - 4) * p.col_stride : zero) + c * 8;
+        L.xa_step = first ? 256 : 0;
+        L.xb_step = second ? 256 : 0;
+        L.alam_b = smem_u32(smem + p.off_alam) + 2 * c * 4;
+        L.xsum_b = smem_u32(smem + p.off_xsum) + (r & 1) * (p.nb_max * 8) * 2;
+        L.minv_b = smem_u32(smem + p.off_minv);
+        L.sa_b = smem_u32(smem + p.off_sa) + (FMT == TLB_GGML_Q4_0 ? c * 8 : (first ? r : 3) * 32);
+        L.half_sh = (c >> 1) * 16;
+        L.sel_u = 0x4440u + (c >> 1);
+        L.sel_s = 0x8880u + (c >> 1) * 0x1111u;
+    } else {
         const int r = L.r, c = L.c;
         const int colr = r < ncols ? r : 0, c0 = 2 * c < ncols ? 2 * c : 0, c1 = 2 * c + 1 < ncols ? 2 * c + 1 : 0;
         L.xq_b = smem_u32(smem + p.off_xq) + colr * p.col_stride;
@@ -318,7 +335,7 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
                             : p.part + ((size_t)ir.slice * p.tiles + ir.tile) * (16 * M);
         for (int mi = 0; mi < M; mi++) {
             const int lo = mi * NL, hi = lo + NL, cA = 2 * L.c, cB = 2 * L.c + 1;
-            const bool inA = cA >= lo && cA < hi, inB = cB >= lo && cB < hi;
+            const bool inA = ONE || (cA >= lo && cA < hi), inB = ONE || (cB >= lo && cB < hi);      // one row: all columns are its own
             float v0 = (inA ? master[0] : 0.f) + (inB ? master[1] : 0.f);   // row r
             float v1 = (inA ? master[2] : 0.f) + (inB ? master[3] : 0.f);   // row r + 8
             v0 += __shfl_xor_sync(0xffffffffu, v0, 1); v0 += __shfl_xor_sync(0xffffffffu, v0, 2);
@@ -531,11 +548,13 @@ static SmemPlan plan_smem(int type, int m, int nl, int nb)
     SmemPlan s;
     size_t o = 0;
     auto take = [&](size_t bytes) { size_t at = o; o += (bytes + 127) / 128 * 128; return (int)at; };
-    s.col_stride = nb * 256 + 64;   // == 64 mod 128: two neighbouring columns never share a bank group
-    s.off_xq = take((size_t)m * nl * s.col_stride);
+    // two neighbouring columns never share a bank group (16-byte reads); one row: four neighbouring columns, the last of them a
+    // block of zeros, never share one (8-byte reads)
+    s.col_stride = nb * 256 + (m == 1 ? 32 : 64);
+    s.off_xq = take((size_t)m * nl * s.col_stride + (m == 1 ? 256 : 0));
     s.off_alam = take((size_t)nb * kMaxCols * 4);
     s.off_xsum = take(type == TLB_GGML_Q4_K ? (size_t)2 * m * (nb * 8) * 2 : 0);
-    s.off_sa = take(type == TLB_GGML_Q6_K ? (size_t)nb * kMaxCols * 32 : type == TLB_GGML_Q4_0 ? (size_t)(nb * 8) * kMaxCols * 4 : 0);
+    s.off_sa = take(type == TLB_GGML_Q6_K ? (size_t)nb * kMaxCols * 32 : type == TLB_GGML_Q4_0 ? (size_t)(nb * (m == 1 ? 4 : 8)) * kMaxCols * 4 : 0);
     s.off_minv = take(type == TLB_GGML_Q4_K ? (size_t)nb * 4 * 4 : 0);
     s.off_misc = take(sizeof(MvShared));
     s.fixed = o;

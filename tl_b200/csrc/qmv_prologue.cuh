@@ -64,11 +64,20 @@ __device__ __forceinline__ void quantise_block(const MvParams &p, uint8_t *smem,
     }
     // k = 256*blk + 4*j + byte  ->  G = j >> 4, t = j & 15: sub = t >> 3, h = (t >> 2) & 1, c = t & 3
     const int G = j >> 4, t = j & 15;
-    const int off = lb * 256 + G * 64 + (t & 3) * 16 + (t >> 3) * 8 + ((t >> 2) & 1) * 4;
+    // one row: a sub-block's 32 bytes together, for 8-byte reads
+    const int off = lb * 256 + G * 64 + (ONE ? (t >> 3) * 32 + (t & 3) * 8 : (t & 3) * 16 + (t >> 3) * 8) + ((t >> 2) & 1) * 4;
 #pragma unroll
     for (int l = 0; l < 3; l++)
         if (l < NL) *reinterpret_cast<uint32_t *>(smem + p.off_xq + (size_t)(mrow * NL + l) * p.col_stride + off) = words[l];
-    if (j < kMaxCols) {   // alam[lb][0..7]: this row's levels; other rows' columns are written by their own groups
+    if (ONE) {
+        // columns 0 .. 2 and 4 .. 6: the levels for either sub-block (Q4_K's second one enters as q << 4), 3 and 7 unused
+        if (j < kMaxCols) {
+            const int l = j & 3;
+            float a = l < 3 ? alpha : 0.f;
+            for (int i = 0; i < l; i++) a *= (1.f / 254.f);
+            reinterpret_cast<float *>(smem + p.off_alam)[lb * kMaxCols + j] = FMT == TLB_GGML_Q4_K && j >= 4 ? a * 0.0625f : a;
+        }
+    } else if (j < kMaxCols) {   // alam[lb][0..7]: this row's levels; other rows' columns are written by their own groups
         const int col = j, l = col - mrow * NL;
         float *alam = reinterpret_cast<float *>(smem + p.off_alam);
         if (l >= 0 && l < NL) {
@@ -110,6 +119,7 @@ __device__ __forceinline__ void quantise_block(const MvParams &p, uint8_t *smem,
                 s += __shfl_xor_sync(0xffffffffu, s, 2);
                 if ((lane & 3) == 0) sa[((size_t)lb * kMaxCols + mrow * NL + l) * 16 + (j >> 2)] = __float2half_rn(s);
             }
+        if (ONE && (lane & 3) == 1) sa[((size_t)lb * kMaxCols + 3) * 16 + (j >> 2)] = __ushort_as_half(0);
     }
     if (FMT == TLB_GGML_Q4_0) {   // level sums over blocks of 32 = 8 consecutive lanes, int32; [lb*8 + j/8][8 cols]
         int *sa = reinterpret_cast<int *>(smem + p.off_sa);
@@ -120,8 +130,13 @@ __device__ __forceinline__ void quantise_block(const MvParams &p, uint8_t *smem,
                 s += __shfl_xor_sync(0xffffffffu, s, 1);
                 s += __shfl_xor_sync(0xffffffffu, s, 2);
                 s += __shfl_xor_sync(0xffffffffu, s, 4);
-                if ((lane & 7) == 0) sa[(size_t)(lb * 8 + (j >> 3)) * kMaxCols + mrow * NL + l] = __float2int_rn(s);
+                // one row: [lb*4 + j/16][8 cols], -8 times the sums of the even block in columns 0 .. 2, of the odd one in 4 .. 6
+                if ((lane & 7) == 0) {
+                    if (ONE) sa[(lb * 4 + (j >> 4)) * kMaxCols + ((j >> 3) & 1) * 4 + l] = -8 * __float2int_rn(s);
+                    else sa[(size_t)(lb * 8 + (j >> 3)) * kMaxCols + mrow * NL + l] = __float2int_rn(s);
+                }
             }
+        if (ONE && (lane & 7) == 1) sa[(lb * 4 + (j >> 4)) * kMaxCols + ((j >> 3) & 1) * 4 + 3] = 0;
     }
 }
 
