@@ -458,6 +458,7 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_cons
     const int n0 = blockIdx.y * kTcRows;
     int t0 = blockIdx.x * p.nt, t_end = p.T, wrow0 = n0;
     if (p.tiles) {                         // rows of one of several stacked weights
+        pdl_wait();
         const int4 tile = p.tiles[blockIdx.x];
         if (tile.z <= 0) return;
         t0 = tile.y; t_end = tile.y + tile.z; wrow0 = tile.x * p.n + n0;
@@ -480,6 +481,7 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_cons
     const uint32_t tmem = tmem_slot;
 
     if (warp < 4) {
+        pdl_wait();                        // residual and outputs belong to the launches before
         if (mbar_wait(done, 0, abort_flag, p.err, 61)) {
             tc_fence_after();
             const int row = n0 + warp * 32 + lane;
@@ -550,9 +552,21 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_cons
     } else if (warp == 4) {
         if (lane == 0) {
             int issued = 0;
-            for (int k = 0; k < p.kt; k++) {
+            // the weights do not depend on the launch before.  Dependents may start from here on, where this CTA has its tensor
+            // memory: one that took theirs first would wait for it and be waited for
+            const int early = min(p.kt, p.stages);
+            for (int k = 0; k < early; k++) {
+                mbar_expect_tx(full + 8 * k, stage);
+                tma_load_2d(base + (uint32_t)k * stage, &wmap, k * kTcK, wrow0, full + 8 * k);
+            }
+            pdl_enter();
+            for (int k = 0; k < early; k++) {
+                tma_load_2d(base + (uint32_t)k * stage + kTcWBytes, &xmap, k * kTcK, t0, full + 8 * k);
+                issued = k + 1;
+            }
+            for (int k = early; k < p.kt; k++) {
                 const int s = k % p.stages;
-                if (k >= p.stages && !mbar_wait(empty + 8 * s, (uint32_t)(k / p.stages - 1) & 1u, abort_flag, p.err, 62)) break;
+                if (!mbar_wait(empty + 8 * s, (uint32_t)(k / p.stages - 1) & 1u, abort_flag, p.err, 62)) break;
                 mbar_expect_tx(full + 8 * s, stage);
                 tma_load_2d(base + (uint32_t)s * stage, &wmap, k * kTcK, wrow0, full + 8 * s);
                 tma_load_2d(base + (uint32_t)s * stage + kTcWBytes, &xmap, k * kTcK, t0, full + 8 * s);
@@ -604,6 +618,7 @@ constexpr int kSgT = kF32GemmRows, kSgN = 64, kSgK = 16;
 
 __global__ void __launch_bounds__(256) dense_gemm_f32_kernel(const DenseF32Params p)
 {
+    pdl_enter();
     __shared__ float sx[kSgK][kSgT + 4], sw[kSgK][kSgN + 4];
     const int tid = threadIdx.x, n0 = blockIdx.y * kSgN;
     const int tn = tid & 15, tt = tid >> 4;
@@ -672,9 +687,10 @@ __device__ __forceinline__ void store_act4(__nv_bfloat16 *p, float a, float b, f
 }
 
 template <typename TA>
-__global__ void __launch_bounds__(256) norm_rows_kernel(const float *__restrict__ x, int width, int ldx, const float *__restrict__ w, float offset, float eps,
-                                                        TA *__restrict__ out, int ld)
+__global__ void __launch_bounds__(256) norm_rows_kernel(const float *x, int width, int ldx, const float *__restrict__ w, float offset, float eps,
+                                                        TA *out, int ld)
 {
+    pdl_enter();
     __shared__ float red[8];
     const float *row = x + (size_t)blockIdx.x * ldx;
     TA *o = out + (size_t)blockIdx.x * ld;
@@ -707,9 +723,10 @@ __global__ void __launch_bounds__(256) norm_rows_kernel(const float *__restrict_
 }
 
 template <typename TA>
-__global__ void __launch_bounds__(512) poly_rows_kernel(const float *__restrict__ z, int ff, int ldz, const float *__restrict__ coef, float eps,
-                                                        TA *__restrict__ out, int ld)
+__global__ void __launch_bounds__(512) poly_rows_kernel(const float *z, int ff, int ldz, const float *__restrict__ coef, float eps,
+                                                        TA *out, int ld)
 {
+    pdl_enter();
     __shared__ float red[16 * 3];
     const float *row = z + (size_t)blockIdx.x * ldz;
     TA *o = out + (size_t)blockIdx.x * ld;
@@ -745,8 +762,9 @@ __global__ void __launch_bounds__(512) poly_rows_kernel(const float *__restrict_
     for (int i = threadIdx.x; i < ff; i += 512) store_act(o + i, row[i] * (a + row[i] * (b + row[i] * c)) + d);
 }
 
-__global__ void embed_bf16_kernel(const int *__restrict__ tokens, const __nv_bfloat16 *__restrict__ table, int width, int ld, float *__restrict__ x)
+__global__ void embed_bf16_kernel(const int *tokens, const __nv_bfloat16 *__restrict__ table, int width, int ld, float *x)
 {
+    pdl_enter();
     const __nv_bfloat16 *src = table + (size_t)tokens[blockIdx.x] * ld;
     if (width % 8 == 0) {
         float4 *dst = reinterpret_cast<float4 *>(x + (size_t)blockIdx.x * width);
@@ -760,8 +778,9 @@ __global__ void embed_bf16_kernel(const int *__restrict__ tokens, const __nv_bfl
     for (int i = threadIdx.x; i < width; i += blockDim.x) x[(size_t)blockIdx.x * width + i] = __bfloat162float(src[i]);
 }
 
-__global__ void gather_rows_kernel(const float *__restrict__ x, int width, const int *__restrict__ idx, float *__restrict__ out)
+__global__ void gather_rows_kernel(const float *x, int width, const int *idx, float *out)
 {
+    pdl_enter();
     const float *src = x + (size_t)idx[blockIdx.x] * width;
     for (int i = threadIdx.x; i < width; i += blockDim.x) out[(size_t)blockIdx.x * width + i] = src[i];
 }
@@ -905,7 +924,7 @@ tlb_status launch_dense_gemm(const DenseGemmJob &j, bool f32)
         p.glu = j.w.glu; p.act = glu_const(j.w.glu_act); p.ld_act = j.ld_act; p.act_out = (float *)j.act_out;
         p.w = j.w.w; p.n = j.w.n; p.k = j.w.k; p.ld = j.w.ld; p.bias = j.w.bias; p.x = (const float *)j.x; p.resid_scale = j.resid_scale;
         p.ldx = j.ldx; p.T = j.T; p.ldo = j.ldo; p.out = j.out;
-        dense_gemm_f32_kernel<<<dim3(j.tiles ? j.n_tiles : (j.T + kSgT - 1) / kSgT, (j.w.n + kSgN - 1) / kSgN), 256, 0, c->stream>>>(p);
+        TLB_CUDA(launch_chained(dense_gemm_f32_kernel, dim3(j.tiles ? j.n_tiles : (j.T + kSgT - 1) / kSgT, (j.w.n + kSgN - 1) / kSgN), dim3(256), 0, true, p));
         return launched("f32 GEMM launch");
     }
     DenseTcParams p;
@@ -933,33 +952,33 @@ tlb_status launch_dense_gemm(const DenseGemmJob &j, bool f32)
         TLB_CUDA(cudaFuncSetAttribute(dense_gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         allowed = smem;
     }
-    dense_gemm_tc_kernel<<<dim3(j.tiles ? j.n_tiles : (j.T + p.nt - 1) / p.nt, (j.w.n + kTcRows - 1) / kTcRows), kTcThreads, smem, c->stream>>>(wmap, xmap, p);
+    TLB_CUDA(launch_chained(dense_gemm_tc_kernel, dim3(j.tiles ? j.n_tiles : (j.T + p.nt - 1) / p.nt, (j.w.n + kTcRows - 1) / kTcRows), dim3(kTcThreads), smem, true, wmap, xmap, p));
     return launched("GEMM launch");
 }
 
 tlb_status launch_norm_rows(const float *x, int T, int width, int ldx, const float *w, float offset, float eps, void *out, int ld, bool f32)
 {
-    if (f32) norm_rows_kernel<<<T, 256, 0, ctx()->stream>>>(x, width, ldx, w, offset, eps, (float *)out, ld);
-    else norm_rows_kernel<<<T, 256, 0, ctx()->stream>>>(x, width, ldx, w, offset, eps, (__nv_bfloat16 *)out, ld);
+    if (f32) TLB_CUDA(launch_chained(norm_rows_kernel<float>, dim3(T), dim3(256), 0, true, x, width, ldx, w, offset, eps, (float *)out, ld));
+    else TLB_CUDA(launch_chained(norm_rows_kernel<__nv_bfloat16>, dim3(T), dim3(256), 0, true, x, width, ldx, w, offset, eps, (__nv_bfloat16 *)out, ld));
     return launched("norm launch");
 }
 
 tlb_status launch_poly_rows(const float *z, int T, int ff, int ldz, const float *coef, float eps, void *out, int ld, bool f32)
 {
-    if (f32) poly_rows_kernel<<<T, 512, 0, ctx()->stream>>>(z, ff, ldz, coef, eps, (float *)out, ld);
-    else poly_rows_kernel<<<T, 512, 0, ctx()->stream>>>(z, ff, ldz, coef, eps, (__nv_bfloat16 *)out, ld);
+    if (f32) TLB_CUDA(launch_chained(poly_rows_kernel<float>, dim3(T), dim3(512), 0, true, z, ff, ldz, coef, eps, (float *)out, ld));
+    else TLB_CUDA(launch_chained(poly_rows_kernel<__nv_bfloat16>, dim3(T), dim3(512), 0, true, z, ff, ldz, coef, eps, (__nv_bfloat16 *)out, ld));
     return launched("PolyNorm launch");
 }
 
 tlb_status launch_embed_bf16(const int *tokens, const __nv_bfloat16 *table, int width, int ld, float *x, int T)
 {
-    embed_bf16_kernel<<<T, 256, 0, ctx()->stream>>>(tokens, table, width, ld, x);
+    TLB_CUDA(launch_chained(embed_bf16_kernel, dim3(T), dim3(256), 0, true, tokens, table, width, ld, x));
     return launched("embedding launch");
 }
 
 tlb_status launch_gather_rows(const float *x, int width, const int *idx, int n, float *out)
 {
-    gather_rows_kernel<<<n, 256, 0, ctx()->stream>>>(x, width, idx, out);
+    TLB_CUDA(launch_chained(gather_rows_kernel, dim3(n), dim3(256), 0, true, x, width, idx, out));
     return launched("gather launch");
 }
 

@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(kDecThreads) mix_attn_decode_kernel(const MixA
 template <typename CT>
 __global__ void mix_attn_append_kernel(const MixAttn a, int seq, int pos0)
 {
+    pdl_enter();
     const int t = blockIdx.x;
     const float *row = a.proj + (size_t)t * a.ldp + (size_t)a.H * a.D;
     CT *kc = reinterpret_cast<CT *>(a.kcache) + (size_t)seq * a.seq_stride_k, *vc = reinterpret_cast<CT *>(a.vcache) + (size_t)seq * a.seq_stride_v;
@@ -288,8 +289,9 @@ __global__ void mix_attn_append_kernel(const MixAttn a, int seq, int pos0)
 constexpr int kRowWarps = 4;
 
 template <typename CT, typename TO>
-__global__ void __launch_bounds__(kRowWarps * 32) mix_attn_rows_kernel(const MixAttn a, int seq, int T, int pos0, TO *__restrict__ out, int ldo)
+__global__ void __launch_bounds__(kRowWarps * 32) mix_attn_rows_kernel(const MixAttn a, int seq, int T, int pos0, TO *out, int ldo)
 {
+    pdl_enter();
     constexpr int VE = Vec<CT>::N;
     __shared__ __align__(16) float sq[kRowWarps][kMaxHeadDim];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.x * kRowWarps + warp, h = blockIdx.y, g = h / (a.H / a.KVH);
@@ -380,8 +382,8 @@ tlb_status launch_mix_attn_prefill(const MixAttn &a, int seq, int T, int pos0, v
 {
     Context *c = ctx();
     if (!c) return TLB_ERR_DEVICE;
-    if (f32) mix_attn_append_kernel<float><<<T, 256, 0, c->stream>>>(a, seq, pos0);
-    else mix_attn_append_kernel<__half><<<T, 256, 0, c->stream>>>(a, seq, pos0);
+    if (f32) TLB_CUDA(launch_chained(mix_attn_append_kernel<float>, dim3(T), dim3(256), 0, true, a, seq, pos0));
+    else TLB_CUDA(launch_chained(mix_attn_append_kernel<__half>, dim3(T), dim3(256), 0, true, a, seq, pos0));
     count_launch();
     TLB_CUDA(cudaGetLastError());
     return launch_mix_attn_prompt(a, seq, T, pos0, out, ldo, f32);
@@ -393,8 +395,8 @@ tlb_status launch_mix_attn_prompt(const MixAttn &a, int seq, int T, int pos0, vo
     if (!f32 && mix_attn_prefill_tc5_supported(a.D, a.DV, T)) return launch_mix_attn_prefill_tc5(a, seq, T, pos0, out, ldo);
     if (!f32 && mix_attn_prefill_tc_supported(a.D, a.DV)) return launch_mix_attn_prefill_tc(a, seq, T, pos0, out, ldo);
     const dim3 grid((T + kRowWarps - 1) / kRowWarps, a.H);
-    if (f32) mix_attn_rows_kernel<float, float><<<grid, kRowWarps * 32, 0, c->stream>>>(a, seq, T, pos0, (float *)out, ldo);
-    else mix_attn_rows_kernel<__half, __nv_bfloat16><<<grid, kRowWarps * 32, 0, c->stream>>>(a, seq, T, pos0, (__nv_bfloat16 *)out, ldo);
+    if (f32) TLB_CUDA(launch_chained(mix_attn_rows_kernel<float, float>, grid, dim3(kRowWarps * 32), 0, true, a, seq, T, pos0, (float *)out, ldo));
+    else TLB_CUDA(launch_chained(mix_attn_rows_kernel<__half, __nv_bfloat16>, grid, dim3(kRowWarps * 32), 0, true, a, seq, T, pos0, (__nv_bfloat16 *)out, ldo));
     count_launch();
     TLB_CUDA(cudaGetLastError());
     return TLB_OK;

@@ -49,8 +49,9 @@ template <int P> constexpr size_t attn_smem() { return (size_t)(4 * kK + kQ) * (
 
 template <int P>     // head sizes padded to P
 __global__ void __launch_bounds__(kThreads, P <= 128 ? 2 : 1)
-mix_attn_tc_kernel(const MixAttn a, int seq, int T, int pos0, __nv_bfloat16 *__restrict__ out, int ldo)
+mix_attn_tc_kernel(const MixAttn a, int seq, int T, int pos0, __nv_bfloat16 *out, int ldo)
 {
+    pdl_enter();
     constexpr int RS = P + 8;
     extern __shared__ __align__(16) __half at_smem[];
     __half *sQ = at_smem + 4 * kK * RS;
@@ -235,7 +236,7 @@ tlb_status run(const MixAttn &a, int seq, int T, int pos0, void *out, int ldo)
         TLB_CUDA(cudaFuncSetAttribute(mix_attn_tc_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_smem<P>()));
         set = true;
     }
-    mix_attn_tc_kernel<P><<<dim3((T + kQ - 1) / kQ, a.H), kThreads, attn_smem<P>(), ctx()->stream>>>(a, seq, T, pos0, (__nv_bfloat16 *)out, ldo);
+    TLB_CUDA(launch_chained(mix_attn_tc_kernel<P>, dim3((T + kQ - 1) / kQ, a.H), dim3(kThreads), attn_smem<P>(), true, a, seq, T, pos0, (__nv_bfloat16 *)out, ldo));
     TLB_CUDA(cudaGetLastError());
     count_launch();
     return TLB_OK;

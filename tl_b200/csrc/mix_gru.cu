@@ -13,8 +13,9 @@ namespace {
 constexpr int kGruWarps = 16, kGruRun = 8, kGruTile = kGruWarps * kGruRun;
 
 template <typename TO>
-__global__ void __launch_bounds__(kGruWarps * 32) gru_scan_kernel(const MixGru m, int seq, int T, int pos0, TO *__restrict__ out, int ldo)
+__global__ void __launch_bounds__(kGruWarps * 32) gru_scan_kernel(const MixGru m, int seq, int T, int pos0, TO *out, int ldo)
 {
+    pdl_enter();
     __shared__ float s_a[2][kGruWarps][32], s_b[2][kGruWarps][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
     const bool live = c < m.width;
@@ -102,8 +103,8 @@ tlb_status launch_gru_rows(const MixGru &m, int batch, const int *pos, void *out
 tlb_status launch_gru_prefill(const MixGru &m, int seq, int T, int pos0, void *out, int ldo, bool f32)
 {
     const int grid = (m.width + 31) / 32;
-    if (f32) gru_scan_kernel<<<grid, kGruWarps * 32, 0, ctx()->stream>>>(m, seq, T, pos0, (float *)out, ldo);
-    else gru_scan_kernel<<<grid, kGruWarps * 32, 0, ctx()->stream>>>(m, seq, T, pos0, (__nv_bfloat16 *)out, ldo);
+    if (f32) TLB_CUDA(launch_chained(gru_scan_kernel<float>, grid, dim3(kGruWarps * 32), 0, false, m, seq, T, pos0, (float *)out, ldo));
+    else TLB_CUDA(launch_chained(gru_scan_kernel<__nv_bfloat16>, grid, dim3(kGruWarps * 32), 0, false, m, seq, T, pos0, (__nv_bfloat16 *)out, ldo));
     return launched("gated recurrence scan launch");
 }
 

@@ -470,8 +470,9 @@ __global__ void __launch_bounds__(kThreads) latent_value_kernel(const MixLatentR
 // ================================================================ long portions
 // rotates the queries of a token in place (or, with QD, into f16 rows whose heads are padded to QD) and appends its cache row
 template <typename CT, int QD>
-__global__ void __launch_bounds__(kThreads) latent_prep_kernel(const MixLatent m, int seq, int pos0, int rope0, int rope_step, __half *__restrict__ q16)
+__global__ void __launch_bounds__(kThreads) latent_prep_kernel(const MixLatent m, int seq, int pos0, int rope0, int rope_step, __half *q16)
 {
+    pdl_enter();
     constexpr int kPairs = QD ? QD / 2 : 1;
     __shared__ float part[kWarps], inv[1];
     const int t = blockIdx.x, rope = rope0 + t * rope_step, half = m.rot / 2, hd = m.D + m.RD;
@@ -513,8 +514,9 @@ __global__ void __launch_bounds__(kThreads) latent_prep_kernel(const MixLatent m
 
 // the rotated part of every key beside each head's expanded one, and zeros up to the pitch
 template <typename CT>
-__global__ void __launch_bounds__(kThreads) latent_rot_kernel(const MixLatent m, const CT *__restrict__ cache, CT *__restrict__ keys, int n_keys, int ldk)
+__global__ void __launch_bounds__(kThreads) latent_rot_kernel(const MixLatent m, const CT *cache, CT *keys, int n_keys, int ldk)
 {
+    pdl_enter();
     const int key = blockIdx.x, tail = ldk - m.D;
     const CT *src = cache + (size_t)key * m.ld + m.R;
     constexpr int VE = 16 / sizeof(CT);
@@ -651,10 +653,10 @@ tlb_status launch_latent_prompt(const MixLatent &m, int seq, int T, int pos0, in
     void *keys = get((size_t)m.H * n_keys * ldk * es), *vals = get((size_t)m.H * (tc5 ? (size_t)128 * vt_ld : (size_t)n_keys * ldv) * es);
     __half *q16 = tc5 ? (__half *)get((size_t)T * m.H * qd * 2) : nullptr;
     if (!keys || !vals || (tc5 && !q16)) return done(TLB_ERR_ALLOC);
-    if (f32) latent_prep_kernel<float, 0><<<T, kThreads, 0, c->stream>>>(m, seq, pos0, rope0, rope_step, nullptr);
-    else if (!tc5) latent_prep_kernel<__half, 0><<<T, kThreads, 0, c->stream>>>(m, seq, pos0, rope0, rope_step, nullptr);
-    else if (qd == 128) latent_prep_kernel<__half, 128><<<T, kThreads, 0, c->stream>>>(m, seq, pos0, rope0, rope_step, q16);
-    else latent_prep_kernel<__half, 192><<<T, kThreads, 0, c->stream>>>(m, seq, pos0, rope0, rope_step, q16);
+    if (f32) TLB_CUDA(launch_chained(latent_prep_kernel<float, 0>, dim3(T), dim3(kThreads), 0, true, m, seq, pos0, rope0, rope_step, nullptr));
+    else if (!tc5) TLB_CUDA(launch_chained(latent_prep_kernel<__half, 0>, dim3(T), dim3(kThreads), 0, true, m, seq, pos0, rope0, rope_step, nullptr));
+    else if (qd == 128) TLB_CUDA(launch_chained(latent_prep_kernel<__half, 128>, dim3(T), dim3(kThreads), 0, true, m, seq, pos0, rope0, rope_step, q16));
+    else TLB_CUDA(launch_chained(latent_prep_kernel<__half, 192>, dim3(T), dim3(kThreads), 0, true, m, seq, pos0, rope0, rope_step, q16));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return done(cuda_fail(e, "latent preparation launch"));
     const char *cache = (const char *)m.cache + ((size_t)seq * m.seq_stride + (size_t)key_first * m.ld) * es;
@@ -670,8 +672,8 @@ tlb_status launch_latent_prompt(const MixLatent &m, int seq, int T, int pos0, in
     else { (f32 ? (void *&)j.out : (void *&)j.out_h) = vals; j.ldo = ldv; j.block_stride = (size_t)n_keys * ldv; }
     st = launch_dense_gemm(j, f32);
     if (st != TLB_OK) return done(st);
-    if (f32) latent_rot_kernel<float><<<n_keys, kThreads, 0, c->stream>>>(m, (const float *)cache, (float *)keys, n_keys, ldk);
-    else latent_rot_kernel<__half><<<n_keys, kThreads, 0, c->stream>>>(m, (const __half *)cache, (__half *)keys, n_keys, ldk);
+    if (f32) TLB_CUDA(launch_chained(latent_rot_kernel<float>, dim3(n_keys), dim3(kThreads), 0, true, m, (const float *)cache, (float *)keys, n_keys, ldk));
+    else TLB_CUDA(launch_chained(latent_rot_kernel<__half>, dim3(n_keys), dim3(kThreads), 0, true, m, (const __half *)cache, (__half *)keys, n_keys, ldk));
     e = cudaGetLastError();
     if (e != cudaSuccess) return done(cuda_fail(e, "latent expansion launch"));
     count_launch(2);

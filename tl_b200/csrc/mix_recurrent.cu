@@ -186,6 +186,7 @@ __device__ __forceinline__ void all_sum(float (&y)[N], int lane)
 template <int NC, bool DELTA>
 __global__ void __launch_bounds__(kScanThreads + 32) scan_kernel(const ScanParams p)
 {
+    pdl_enter();
     using S = ScanShape<NC>;
     constexpr int DP = S::DP, L = S::L, N4 = S::N4, CB = S::CB, TB = S::TB, COLS = S::COLS, NP = 2 * N4;
     constexpr int NV = DELTA ? 4 : 2, ROW = NV * DP + COLS, BUF = kScanTok * ROW + DP + 2 * kScanTok;     // k has one row more than the chunk
@@ -375,6 +376,7 @@ __global__ void __launch_bounds__(kScanThreads + 32) scan_kernel(const ScanParam
 // q and k of one token: rotate the leading dims (rotate-half pairs), scale k
 __global__ void retention_prep_kernel(const MixRecur m, int rope0, int rope_step, float kscale)
 {
+    pdl_enter();
     const int half = m.rot / 2;
     float *row = m.proj + (size_t)blockIdx.x * m.ldp;
     const size_t tab = (size_t)(rope0 + (int)blockIdx.x * rope_step) * half;
@@ -396,8 +398,9 @@ __global__ void retention_prep_kernel(const MixRecur m, int rope0, int rope_step
 
 // one warp per (token, head): decay <- exp(-exp(-1/2) sigmoid(decay + w0)), a <- sigmoid(a) k / (k . k + eps), and the two products
 // with the next token's key that the scan looks ahead with.  The bias of a is in already.
-__global__ void __launch_bounds__(256) delta_prep_kernel(const MixRecur m, int T, float *__restrict__ decay, float2 *__restrict__ look, int look_ld)
+__global__ void __launch_bounds__(256) delta_prep_kernel(const MixRecur m, int T, float *decay, float2 *look, int look_ld)
 {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int64_t u = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (u >= (int64_t)T * m.H) return;
@@ -442,8 +445,9 @@ __device__ __forceinline__ float gate_value(bool delta, float y, float g, float 
 
 // ---- what leaves it: one warp per (token, head)
 template <typename TO>
-__global__ void __launch_bounds__(256) recur_post_kernel(const MixRecur m, int T, const float *__restrict__ o, int g_col, TO *__restrict__ out, int ldo)
+__global__ void __launch_bounds__(256) recur_post_kernel(const MixRecur m, int T, const float *o, int g_col, TO *out, int ldo)
 {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int64_t u = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (u >= (int64_t)T * m.H) return;
@@ -479,8 +483,9 @@ __global__ void __launch_bounds__(256) recur_post_kernel(const MixRecur m, int T
 }
 
 template <typename TA>
-__global__ void tanh_split_kernel(const float *__restrict__ x, int rank, int ldx, TA *__restrict__ out, int ldh)
+__global__ void tanh_split_kernel(const float *x, int rank, int ldx, TA *out, int ldh)
 {
+    pdl_enter();
     const float *row = x + (size_t)blockIdx.x * ldx;
     TA *o = out + (size_t)blockIdx.x * 2 * ldh;
     for (int i = threadIdx.x; i < ldh; i += blockDim.x) {
@@ -621,7 +626,7 @@ tlb_status scan_nc(const ScanParams &p)
         TLB_CUDA(cudaFuncSetAttribute(scan_kernel<NC, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         set = true;
     }
-    scan_kernel<NC, DELTA><<<dim3((p.DV + COLS - 1) / COLS, p.H), kScanThreads + 32, smem, ctx()->stream>>>(p);
+    TLB_CUDA(launch_chained(scan_kernel<NC, DELTA>, dim3((p.DV + COLS - 1) / COLS, p.H), dim3(kScanThreads + 32), smem, false, p));
     TLB_CUDA(cudaGetLastError());
     count_launch();
     return TLB_OK;
@@ -674,8 +679,8 @@ tlb_status run_step(const MixRecurDecode &j)
 tlb_status post(const MixRecur &m, int T, const float *o, int g_col, void *out, int ldo, bool f32)
 {
     const unsigned grid = (unsigned)(((int64_t)T * m.H + 7) / 8);
-    if (f32) recur_post_kernel<<<grid, 256, 0, ctx()->stream>>>(m, T, o, g_col, (float *)out, ldo);
-    else recur_post_kernel<<<grid, 256, 0, ctx()->stream>>>(m, T, o, g_col, (__nv_bfloat16 *)out, ldo);
+    if (f32) TLB_CUDA(launch_chained(recur_post_kernel<float>, grid, dim3(256), 0, true, m, T, o, g_col, (float *)out, ldo));
+    else TLB_CUDA(launch_chained(recur_post_kernel<__nv_bfloat16>, grid, dim3(256), 0, true, m, T, o, g_col, (__nv_bfloat16 *)out, ldo));
     TLB_CUDA(cudaGetLastError());
     count_launch();
     return TLB_OK;
@@ -693,7 +698,7 @@ tlb_status launch_delta_decode(const MixRecurDecode &j) { return run_step<true>(
 tlb_status launch_retention_prefill(const MixRecur &m, int seq, int T, int pos0, int rope0, int rope_step, float *o, void *out, int ldo, bool f32)
 {
     const int HD = m.H * m.D;
-    retention_prep_kernel<<<T, 256, 0, ctx()->stream>>>(m, rope0, rope_step, 1.f / sqrtf((float)m.D));
+    TLB_CUDA(launch_chained(retention_prep_kernel, dim3(T), dim3(256), 0, true, m, rope0, rope_step, 1.f / sqrtf((float)m.D)));
     TLB_CUDA(cudaGetLastError());
     count_launch();
     ScanParams p = {};
@@ -712,7 +717,7 @@ tlb_status launch_retention_prefill(const MixRecur &m, int seq, int T, int pos0,
 tlb_status launch_delta_prefill(const MixRecur &m, int seq, int T, int pos0, float *decay, float2 *look, float *o, void *out, int ldo, bool f32)
 {
     const int HD = m.H * m.D;
-    delta_prep_kernel<<<(unsigned)(((int64_t)T * m.H + 7) / 8), 256, 0, ctx()->stream>>>(m, T, decay, look, scan_look_ld(T));
+    TLB_CUDA(launch_chained(delta_prep_kernel, dim3((unsigned)(((int64_t)T * m.H + 7) / 8)), dim3(256), 0, true, m, T, decay, look, scan_look_ld(T)));
     TLB_CUDA(cudaGetLastError());
     count_launch();
     ScanParams p = {};
@@ -731,8 +736,8 @@ tlb_status launch_delta_prefill(const MixRecur &m, int seq, int T, int pos0, flo
 
 tlb_status launch_tanh_split(const float *x, int T, int rank, int ldx, void *out, int ldh, bool f32)
 {
-    if (f32) tanh_split_kernel<<<T, 128, 0, ctx()->stream>>>(x, rank, ldx, (float *)out, ldh);
-    else tanh_split_kernel<<<T, 128, 0, ctx()->stream>>>(x, rank, ldx, (__nv_bfloat16 *)out, ldh);
+    if (f32) TLB_CUDA(launch_chained(tanh_split_kernel<float>, dim3(T), dim3(128), 0, true, x, rank, ldx, (float *)out, ldh));
+    else TLB_CUDA(launch_chained(tanh_split_kernel<__nv_bfloat16>, dim3(T), dim3(128), 0, true, x, rank, ldx, (__nv_bfloat16 *)out, ldh));
     TLB_CUDA(cudaGetLastError());
     count_launch();
     return TLB_OK;

@@ -9,9 +9,10 @@ namespace tlb {
 
 namespace {
 
-__global__ void __launch_bounds__(128) route_rows_kernel(const RouteDesc r, const float *__restrict__ logits, int ldl, int *__restrict__ sel, float *__restrict__ weight,
-                                                         int *__restrict__ place, int *__restrict__ count)
+__global__ void __launch_bounds__(128) route_rows_kernel(const RouteDesc r, const float *logits, int ldl, int *sel, float *weight,
+                                                         int *place, int *count)
 {
+    pdl_enter();
     extern __shared__ float scratch[];
     __shared__ int s_sel[kMaxTop];
     __shared__ float s_w[kMaxTop];
@@ -25,8 +26,9 @@ __global__ void __launch_bounds__(128) route_rows_kernel(const RouteDesc r, cons
 }
 
 // first row of every expert and the tiles; one CTA
-__global__ void __launch_bounds__(256) moe_tiles_kernel(int experts, int *__restrict__ count, int tile_rows, int4 *__restrict__ tiles, int max_tiles)
+__global__ void __launch_bounds__(256) moe_tiles_kernel(int experts, int *count, int tile_rows, int4 *tiles, int max_tiles)
 {
+    pdl_enter();
     extern __shared__ int s_first[];                       // [experts + 1] counts, then first rows; [experts + 1] tiles
     int *s_tile = s_first + experts + 1;
     for (int e = threadIdx.x; e < experts; e += 256) s_first[e] = count[e];
@@ -52,9 +54,10 @@ __global__ void __launch_bounds__(256) moe_tiles_kernel(int experts, int *__rest
 }
 
 // one CTA per (token, choice): the row moves to its place, which becomes an index over all experts' rows
-__global__ void __launch_bounds__(128) moe_gather_kernel(int top, const int *__restrict__ sel, int *__restrict__ place, const int *__restrict__ first,
-                                                         const char *__restrict__ act, size_t row_bytes, char *__restrict__ out)
+__global__ void __launch_bounds__(128) moe_gather_kernel(int top, const int *sel, int *place, const int *first,
+                                                         const char *act, size_t row_bytes, char *out)
 {
+    pdl_enter();
     const int i = blockIdx.x, t = i / top;
     const int dst = first[sel[i]] + place[i];
     const uint4 *s = reinterpret_cast<const uint4 *>(act + (size_t)t * row_bytes);
@@ -90,15 +93,15 @@ int moe_max_tiles(const RouteDesc &r, int T, bool f32)
 tlb_status launch_moe_plan(const RouteDesc &r, const float *logits, int ldl, int T, const MoePlan &p, bool f32)
 {
     TLB_CUDA(cudaMemsetAsync(p.count, 0, (size_t)r.experts * sizeof(int), ctx()->stream));
-    route_rows_kernel<<<T, 128, route_scratch_floats(r) * sizeof(float), ctx()->stream>>>(r, logits, ldl, p.sel, p.weight, p.place, p.count);
+    TLB_CUDA(launch_chained(route_rows_kernel, dim3(T), dim3(128), route_scratch_floats(r) * sizeof(float), true, r, logits, ldl, p.sel, p.weight, p.place, p.count));
     TLB_TRY(launched("router launch"));
-    moe_tiles_kernel<<<1, 256, (size_t)2 * (r.experts + 1) * sizeof(int), ctx()->stream>>>(r.experts, p.count, moe_tile_rows(r, T, f32), p.tiles, moe_max_tiles(r, T, f32));
+    TLB_CUDA(launch_chained(moe_tiles_kernel, dim3(1), dim3(256), (size_t)2 * (r.experts + 1) * sizeof(int), true, r.experts, p.count, moe_tile_rows(r, T, f32), p.tiles, moe_max_tiles(r, T, f32)));
     return launched("expert tiles launch");
 }
 
 tlb_status launch_moe_gather(const RouteDesc &r, const MoePlan &p, const void *act, int T, int ld, void *out, bool f32)
 {
-    moe_gather_kernel<<<T * r.top, 128, 0, ctx()->stream>>>(r.top, p.sel, p.place, p.count + r.experts, (const char *)act, (size_t)ld * (f32 ? 4 : 2), (char *)out);
+    TLB_CUDA(launch_chained(moe_gather_kernel, dim3(T * r.top), dim3(128), 0, true, r.top, p.sel, p.place, p.count + r.experts, (const char *)act, (size_t)ld * (f32 ? 4 : 2), (char *)out));
     return launched("expert gather launch");
 }
 

@@ -379,8 +379,9 @@ __global__ void __launch_bounds__(256) v_transpose_kernel(const __half *vcache, 
 
 // queries of the projection rows as f16, every head padded to QD columns
 template <int QD>
-__global__ void __launch_bounds__(256) mix_q_to_f16_kernel(const float *__restrict__ proj, int ldp, int H, int D, __half *__restrict__ qh)
+__global__ void __launch_bounds__(256) mix_q_to_f16_kernel(const float *proj, int ldp, int H, int D, __half *qh)
 {
+    pdl_enter();
     const float *row = proj + (size_t)blockIdx.x * ldp;
     for (int i = threadIdx.x; i < H * QD / 2; i += blockDim.x) {
         const int h = i / (QD / 2), d = (i % (QD / 2)) * 2;
@@ -390,8 +391,9 @@ __global__ void __launch_bounds__(256) mix_q_to_f16_kernel(const float *__restri
     }
 }
 // cache rows key_first .. of V as V^T [KV head][128][keys_ld] (columns counted from key_first, rows past DV zero)
-__global__ void __launch_bounds__(256) mix_v_transpose_kernel(const __half *__restrict__ vcache, __half *__restrict__ vt, int max_seq, int ldv, int key_first, int n_keys, int keys_ld)
+__global__ void __launch_bounds__(256) mix_v_transpose_kernel(const __half *vcache, __half *vt, int max_seq, int ldv, int key_first, int n_keys, int keys_ld)
 {
+    pdl_enter();
     __shared__ __half tile[32][34];
     const __half *src = vcache + (size_t)blockIdx.z * max_seq * ldv;
     __half *dst = vt + (size_t)blockIdx.z * kAtD * keys_ld;
@@ -419,20 +421,23 @@ tlb_status run_mix_tc5(const MixAttn &a, int seq, int T, int pos0, void *out, in
     // cache rows some query sees, from a tile border on; V^T that is given starts with row 0
     const int key_first = a.vt ? 0 : std::max(0, pos0 - a.window + 1) / kAtK * kAtK, n_keys = pos0 + T - key_first, keys_ld = a.vt ? a.vt_ld : (n_keys + 127) / 128 * 128;
     Storage *qh = nullptr, *vt = nullptr;
+    cudaError_t e;
     auto done = [&](tlb_status st) { if (qh) storage_release(qh); if (vt) storage_release(vt); return st; };
     const __half *kc = (const __half *)a.kcache + (size_t)seq * a.seq_stride_k, *vc = (const __half *)a.vcache + (size_t)seq * a.seq_stride_v;
     const void *q16 = a.q16, *v16 = a.vt;
     if (!q16) {
         qh = storage_alloc((size_t)T * a.H * QD * sizeof(__half));
         if (!qh) return done(TLB_ERR_ALLOC);
-        mix_q_to_f16_kernel<QD><<<T, 256, 0, c->stream>>>(a.proj, a.ldp, a.H, a.D, (__half *)qh->ptr);
+        e = launch_chained(mix_q_to_f16_kernel<QD>, dim3(T), dim3(256), 0, true, a.proj, a.ldp, a.H, a.D, (__half *)qh->ptr);
+        if (e != cudaSuccess) return done(cuda_fail(e, "prompt attention operands"));
         count_launch();
         q16 = qh->ptr;
     }
     if (!v16) {
         vt = storage_alloc((size_t)a.KVH * kAtD * keys_ld * sizeof(__half));
         if (!vt) return done(TLB_ERR_ALLOC);
-        mix_v_transpose_kernel<<<dim3(kAtD / 32, (unsigned)(keys_ld / 32), (unsigned)a.KVH), 256, 0, c->stream>>>(vc, (__half *)vt->ptr, a.max_seq, a.ldv, key_first, n_keys, keys_ld);
+        e = launch_chained(mix_v_transpose_kernel, dim3(kAtD / 32, (unsigned)(keys_ld / 32), (unsigned)a.KVH), dim3(256), 0, true, vc, (__half *)vt->ptr, a.max_seq, a.ldv, key_first, n_keys, keys_ld);
+        if (e != cudaSuccess) return done(cuda_fail(e, "prompt attention operands"));
         count_launch();
         v16 = vt->ptr;
     }
@@ -451,13 +456,12 @@ tlb_status run_mix_tc5(const MixAttn &a, int seq, int T, int pos0, void *out, in
     constexpr size_t smem = at_smem_bytes(KB);
     static bool attr_set = false;
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_attention_tc_kernel<true, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(prefill_attention_tc_kernel<true, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return done(cuda_fail(e, "prompt attention attribute"));
         attr_set = true;
     }
-    prefill_attention_tc_kernel<true, KB><<<dim3((unsigned)((T + kAtQ - 1) / kAtQ), (unsigned)a.H), kAtThreads, smem, c->stream>>>(qmap, kmap, vtmap, p);
+    e = launch_chained(prefill_attention_tc_kernel<true, KB>, dim3((unsigned)((T + kAtQ - 1) / kAtQ), (unsigned)a.H), dim3(kAtThreads), smem, true, qmap, kmap, vtmap, p);
     count_launch();
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return done(cuda_fail(e, "prompt attention launch"));
     return done(TLB_OK);
 }

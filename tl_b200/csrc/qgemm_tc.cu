@@ -86,6 +86,7 @@ struct GemmParams {
     // each other's shared memory; with it each writes its partial product to part[split][m][n_all], and a second small launch
     // adds the splits (and the residual).
     int splits;
+    int glu;                // the rows are gate and up of 8 hidden units by turns: out [m, n / 2] is silu(gate) * up
     float *part;
     int n_all;              // columns of one partial row: the sum of the weights' rows
     int col0[kGemmMaxW];    // first column of weight i inside a partial row
@@ -470,6 +471,19 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
             uint32_t v[8];
             tmem_ld8(tacc + (uint32_t)c0, v);
             add(c0 >> 3, v);
+            if (p.glu) {
+                // lanes l and l + 8 of sixteen hold gate and up of a hidden unit: the former takes tokens 0 .. 3, the latter 4 .. 7
+                const bool hi = lane & 8;
+                float *o = p.out[0] + (size_t)(tok0 + c0 + (hi ? 4 : 0)) * (n_rows / 2) + (row >> 4) * 8 + (lane & 7);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float own = __uint_as_float(hi ? v[j + 4] : v[j]) * (hi ? sc[j + 4] : sc[j]);
+                    const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(hi ? v[j] : v[j + 4]) * (hi ? sc[j] : sc[j + 4]), 8);
+                    const float gate = hi ? other : own, up = hi ? own : other;
+                    if (row < n_rows && tok0 + c0 + j + (hi ? 4 : 0) < p.m) o[(size_t)j * (n_rows / 2)] = __fdividef(gate, 1.f + expf(-gate)) * up;
+                }
+                continue;
+            }
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 const int tok = tok0 + c0 + j;
@@ -1500,14 +1514,30 @@ tlb_status qrows_run(const tlb_qtensor *const *ws, int n_w, const GemmAct &a, fl
     return TLB_OK;
 }
 
+static tlb_status run_gemm(const tlb_qtensor *const *ws, int n_w, const GemmAct &a, float *const *outs, const float *resid, bool glu, bool *taken);
+
 tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct &a, float *const *outs, const float *resid)
 {
+    bool taken;
+    return run_gemm(ws, n_w, a, outs, resid, false, &taken);
+}
+
+// silu(gate) * up of a weight whose rows are interleaved by eights (launch_interleave8); *taken is false, and nothing ran, where
+// the rows are few or the product's K ranges would go through scratch
+tlb_status qgemm_run_glu(const tlb_qtensor *w, const GemmAct &a, float *out, bool *taken) { return run_gemm(&w, 1, a, &out, nullptr, true, taken); }
+
+static tlb_status run_gemm(const tlb_qtensor *const *ws, int n_w, const GemmAct &a, float *const *outs, const float *resid, bool glu, bool *taken)
+{
+    *taken = true;
     Context *c = ctx();
     if (!c) return TLB_ERR_DEVICE;
     if (n_w < 1 || n_w > kGemmMaxW || (resid && n_w != 1)) return fail(TLB_ERR_ARG, "tensor-core GEMM: %d weights in one launch", n_w);
     const tlb_qtensor *w0 = ws[0];
     if (!qgemm_supported(w0->type)) return fail(TLB_ERR_TYPE, "tensor-core GEMM: GGML type %d is not supported", w0->type);
-    if (qrows_rows(a.m)) return qrows_run(ws, n_w, a, outs, resid);
+    if (qrows_rows(a.m)) {
+        if (glu) { *taken = false; return TLB_OK; }
+        return qrows_run(ws, n_w, a, outs, resid);
+    }
     GemmParams p;
     int64_t row_tiles = 0;
     for (int i = 0; i < kGemmMaxW; i++) {
@@ -1528,6 +1558,7 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
     for (int i = 0; i < kGemmMaxW; i++) { p.col0[i] = (int)n_all; n_all += p.n[i]; }
     GemmPlan plan = plan_gemm(m, row_tiles, w0->upt, n_all, c->sm_count);
     const bool ranges = plan_ranges(m, row_tiles, w0->upt, n_all, c->sm_count, &plan);
+    if (glu && plan.splits > 1 && !ranges) { *taken = false; return TLB_OK; }
     const int nt = plan.nt;
     const bool pair = plan.pair;
     CUtensorMap map;
@@ -1556,6 +1587,7 @@ tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct 
     const int64_t tok_tiles = (m + nt - 1) / nt;
     Storage *part = nullptr;
     p.splits = plan.splits;
+    p.glu = glu;
     if (p.splits > 1 && !ranges) {
         part = storage_alloc((size_t)p.splits * m * n_all * sizeof(float));
         if (!part) { cudaGetLastError(); p.splits = 1; }    // no room for the partial sums: one K range takes none

@@ -21,8 +21,9 @@ struct ResidNormParams {
 };
 
 template <typename TA>
-__global__ void __launch_bounds__(256) resid_norm_rows_kernel(const ResidNormParams p, TA *__restrict__ out)
+__global__ void __launch_bounds__(256) resid_norm_rows_kernel(const ResidNormParams p, TA *out)
 {
+    pdl_enter();
     extern __shared__ __align__(16) float row[];
     __shared__ float part[kMaxNormGroups], inv[kMaxNormGroups];
     __shared__ int s_slot[kMaxTop];
@@ -120,7 +121,7 @@ tlb_status run_resid(const ResidNormParams &p, int T, void *out)
         TLB_CUDA(cudaFuncSetAttribute(resid_norm_rows_kernel<TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         allowed = smem;
     }
-    resid_norm_rows_kernel<TA><<<T, 256, smem, ctx()->stream>>>(p, (TA *)out);
+    TLB_CUDA(launch_chained(resid_norm_rows_kernel<TA>, dim3(T), dim3(256), smem, true, p, (TA *)out));
     return launched("residual norm launch");
 }
 

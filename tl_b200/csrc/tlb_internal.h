@@ -133,6 +133,7 @@ struct GemmAct { Storage *xh = nullptr, *inv = nullptr, *sums = nullptr; int64_t
 tlb_status qgemm_prepare(GemmAct *a, const float *x, const float *x2, int64_t m, int64_t k, const float *norm_w, float eps);
 tlb_status qgemm_run(const tlb_qtensor *w, const GemmAct &a, float *out, const float *resid);
 // up to three weights of one type and K (q | k | v, gate | up) in one launch: outs[i] = act . ws[i]^T
+tlb_status qgemm_run_glu(const tlb_qtensor *w, const GemmAct &a, float *out, bool *taken);
 tlb_status qgemm_run_multi(const tlb_qtensor *const *ws, int n_w, const GemmAct &a, float *const *outs, const float *resid);
 void qgemm_release(GemmAct *a);
 // sampling.cu: temperature / top-p sampling of n logits with the draw u in [0, 1); the token id as f32 into out[0]
@@ -302,6 +303,8 @@ tlb_status launch_sdpa(const float *q, const float *k, const float *v, const flo
 // may be moved ahead of the wait.  What bounds small launches is the 1 to 2 us between the end of one and the start of the next:
 // 333 tokens through eight TinyLlama layers 1.41 -> 1.17 ms, four op-by-op steps of four such layers 3.41 -> 2.39, four rows
 // through 14336 x 4096 in Q8_0 26.4 -> 20.9 us, 2048 tokens of four Llama-3-8B layers 5.30 -> 5.22 ms.
+// Not so for the scans: an SM holds several of their CTAs, each a chain of steps, and started early they gather on the SMs that
+// are free by then (a delta-rule scan of 512 tokens 236 instead of 143 us).
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
