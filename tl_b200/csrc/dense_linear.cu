@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(kMvThreads, 4) dense_matvec_kernel(const Dense
     extern __shared__ __align__(16) float mv_smem[];
     float *xs = mv_smem + p.depth * (kMvStage / sizeof(float));
     __shared__ float red[GNORM ? 2 * kMaxNormGroups : kMvWarps * 3];
+    constexpr int kSeg = 128;                         // elements a warp takes at a time in the fast form of GNORM
     __shared__ float fold[2][GROUPS][WK][kMvRows];
     __shared__ int s_sel[EXPERT ? kMaxTop : 1];
     __shared__ float s_weight[EXPERT || EXPERTS ? kMaxTop + 1 : 1];
@@ -161,6 +162,19 @@ __global__ void __launch_bounds__(kMvThreads, 4) dense_matvec_kernel(const Dense
         for (int e = tid * 32; e < p.k; e += kMvThreads * 32) {
             asm volatile("prefetch.global.L2 [%0];" ::"l"(p.norm_w + e));
             if (p.post_w) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.post_w + e));
+        }
+    }
+    // GNORM, rows of up to 2048 whose parts are whole runs of 128 elements: see below; its static weights are loaded here
+    const bool by_runs = GNORM && !p.emb && p.k <= 2 * 4 * kMvThreads && p.k % (p.groups * kSeg) == 0 && (reinterpret_cast<uintptr_t>(p.y_gate) & 15) == 0;
+    float4 wpost[GNORM ? 2 : 1], wnorm[GNORM ? 2 : 1];
+    if (GNORM && by_runs) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int e = (tid + i * kMvThreads) * 4;
+            if (e < p.k) {
+                if (p.y) wpost[i] = *reinterpret_cast<const float4 *>(p.post_w + e);
+                wnorm[i] = *reinterpret_cast<const float4 *>(p.norm_w + e);
+            }
         }
     }
     pdl_wait();
@@ -237,7 +251,68 @@ __global__ void __launch_bounds__(kMvThreads, 4) dense_matvec_kernel(const Dense
                                v.z * inv[group_of(e + 2, inv_len)] * (w.z + p.norm_offset), v.w * inv[group_of(e + 3, inv_len)] * (w.w + p.norm_offset));
         };
         constexpr int NV = 4;
-        if (!er && p.k % 4 == 0 && p.k <= NV * 4 * kMvThreads && (reinterpret_cast<uintptr_t>(p.y_gate) & 15) == 0) {
+        if (by_runs) {
+            // Every warp's 128 elements lie in one part, so sums of squares come from registers, one per run, and a part is the sum of
+            // its runs.  (By parts, through shared memory, as below, the values stood 5 to 8 us after the wait, most of the launch.)
+            // With the experts' activations below, 16 tokens behind a prompt of 509 of a three-layer Rukedra model 4.78 -> 4.46 ms.
+            float4 v[2], x[2];
+            const int len = p.k / p.groups, per = len / kSeg;
+            auto ld4 = [&](const float *src, int e) { return e < p.k ? __ldcg(reinterpret_cast<const float4 *>(src + e)) : make_float4(0.f, 0.f, 0.f, 0.f); };
+            auto runs = [&](const float4 (&u)[2], float *sums) {
+                float ss[2];
+#pragma unroll
+                for (int i = 0; i < 2; i++) ss[i] = (u[i].x * u[i].x + u[i].y * u[i].y) + (u[i].z * u[i].z + u[i].w * u[i].w);
+#pragma unroll
+                for (int o = 16; o; o >>= 1) { ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o); ss[1] += __shfl_xor_sync(0xffffffffu, ss[1], o); }
+                if (lane == 0) { sums[warp] = ss[0]; sums[kMvWarps + warp] = ss[1]; }
+                __syncthreads();
+            };
+            auto inv_rms = [&](const float *sums, int run) {       // of the part that holds the run
+                const int first = run / per * per;
+                float ss = 0.f;
+                for (int r = 0; r < per; r++) ss += sums[first + r];
+                return 1.f / sqrtf(ss / (float)len + p.eps);
+            };
+            if (p.y) {
+                float4 g[2];
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const int e = (tid + i * kMvThreads) * 4;
+                    v[i] = ld4(p.y, e);
+                    g[i] = p.y_gate ? ld4(p.y_gate, e) : make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
+                    x[i] = ld4(p.x, e);
+                }
+#pragma unroll
+                for (int i = 0; i < 2; i++) { v[i].x *= sigmoidf(g[i].x); v[i].y *= sigmoidf(g[i].y); v[i].z *= sigmoidf(g[i].z); v[i].w *= sigmoidf(g[i].w); }
+                runs(v, red);
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const int e = (tid + i * kMvThreads) * 4;
+                    if (e >= p.k) continue;
+                    const float f = inv_rms(red, i * kMvWarps + warp);
+                    x[i].x += v[i].x * f * (wpost[i].x + p.norm_offset); x[i].y += v[i].y * f * (wpost[i].y + p.norm_offset);
+                    x[i].z += v[i].z * f * (wpost[i].z + p.norm_offset); x[i].w += v[i].w * f * (wpost[i].w + p.norm_offset);
+                    if (blockIdx.x == 0) *reinterpret_cast<float4 *>(p.x_out + e) = x[i];
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 2; i++) x[i] = ld4(p.x, (tid + i * kMvThreads) * 4);
+            }
+            runs(x, red + 2 * kMvWarps);
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int e = (tid + i * kMvThreads) * 4;
+                if (e >= kp) continue;
+                float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (e < p.k) {
+                    const float f = inv_rms(red + 2 * kMvWarps, i * kMvWarps + warp);
+                    a = make_float4(x[i].x * f * (wnorm[i].x + p.norm_offset), x[i].y * f * (wnorm[i].y + p.norm_offset),
+                                    x[i].z * f * (wnorm[i].z + p.norm_offset), x[i].w * f * (wnorm[i].w + p.norm_offset));
+                    if (p.h_out && blockIdx.x == 0) *reinterpret_cast<float4 *>(p.h_out + e) = a;
+                }
+                *reinterpret_cast<float4 *>(xs + xs_at(e)) = a;
+            }
+        } else if (!er && p.k % 4 == 0 && p.k <= NV * 4 * kMvThreads && (reinterpret_cast<uintptr_t>(p.y_gate) & 15) == 0) {
             // 16 elements per thread: every load of the rows is on its way before the first is used
             float4 v[NV], x[NV];
             auto ld4 = [&](const float *src, int e) { return e < p.k ? __ldcg(reinterpret_cast<const float4 *>(src + e)) : make_float4(0.f, 0.f, 0.f, 0.f); };
@@ -316,21 +391,56 @@ __global__ void __launch_bounds__(kMvThreads, 4) dense_matvec_kernel(const Dense
         }
     } else if (EXPERTS) {
         const int top = p.route.top, seg = p.seg_nch * kMvChunk, first = top * seg;
+        // The activations of the chosen experts and the shared one, scaled by their weights.  In whole float4 they are requested
+        // kIn at a time, the first before the weights are known: one after another, expert by expert, they took 15 us.
+        constexpr int kIn = 6;
+        const bool vec4 = p.k % 4 == 0 && p.ldx % 4 == 0 && p.shared_k % 4 == 0 && ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.shared_x)) & 15) == 0;
+        const float inv_seg = 1.f / (float)seg;
+        auto where = [&](int e, int &s, int &o) {                  // segment of element e, and its place there
+            s = e < first ? (int)(((float)e + 0.5f) * inv_seg) : top;
+            o = e - s * seg;
+        };
+        float4 in[kIn];
+        auto request = [&](int e0) {
+#pragma unroll
+            for (int i = 0; i < kIn; i++) {
+                const int e = e0 + i * 4 * kMvThreads;
+                int s, o;
+                where(e, s, o);
+                in[i] = e < kp && o < (s < top ? p.k : p.shared_k) ? __ldcg(reinterpret_cast<const float4 *>((s < top ? p.x + (size_t)s * p.ldx : p.shared_x) + o)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        };
+        if (vec4) request(tid * 4);
         for (int s = tid; s <= top; s += kMvThreads) {
             s_weight[s] = s < top ? __ldcg(p.weight + s) : (p.shared_gate ? sigmoidf(__ldcg(p.shared_gate)) : 1.f);
             s_base[s] = s < top ? p.w + (size_t)__ldcg(p.sel + s) * p.n * p.ld : p.shared_w;
         }
         __syncthreads();
         fill();
-        for (int s = 0; s < top; s++) {
-            const float w = s_weight[s];
-            const float *x = p.x + (size_t)s * p.ldx;
+        if (vec4) {
+            for (int e0 = tid * 4; e0 < kp; e0 += kIn * 4 * kMvThreads) {
+                if (e0 >= kIn * 4 * kMvThreads) request(e0);
+#pragma unroll
+                for (int i = 0; i < kIn; i++) {
+                    const int e = e0 + i * 4 * kMvThreads;
+                    if (e >= kp) continue;
+                    int s, o;
+                    where(e, s, o);
+                    const float w = s_weight[s];
+                    *reinterpret_cast<float4 *>(xs + xs_at(e)) = make_float4(w * in[i].x, w * in[i].y, w * in[i].z, w * in[i].w);
+                }
+            }
+        } else {
+            for (int s = 0; s < top; s++) {
+                const float w = s_weight[s];
+                const float *x = p.x + (size_t)s * p.ldx;
 #pragma unroll 8
-            for (int e = tid; e < seg; e += kMvThreads) xs[s * seg + xs_at(e)] = e < p.k ? w * __ldcg(x + e) : 0.f;
+                for (int e = tid; e < seg; e += kMvThreads) xs[s * seg + xs_at(e)] = e < p.k ? w * __ldcg(x + e) : 0.f;
+            }
+            const float w = s_weight[top];
+#pragma unroll 8
+            for (int e = tid; e < kp - first; e += kMvThreads) xs[first + xs_at(e)] = e < p.shared_k ? w * __ldcg(p.shared_x + e) : 0.f;
         }
-        const float w = s_weight[top];
-#pragma unroll 8
-        for (int e = tid; e < kp - first; e += kMvThreads) xs[first + xs_at(e)] = e < p.shared_k ? w * __ldcg(p.shared_x + e) : 0.f;
     } else {
         float ss[3] = {0.f, 0.f, 0.f};
         auto add = [&](float v) { const float v2 = v * v; ss[0] += v2; ss[1] += v2 * v2; ss[2] += v2 * v2 * v2; };
@@ -810,10 +920,12 @@ tlb_status launched(const char *what)
     return TLB_OK;
 }
 
-// CTAs that fit beside each other with a row of `row` bytes and so many weight chunks in flight, for each of `slots` experts
+// CTAs that fit beside each other with a row of `row` bytes and so many weight chunks in flight, for each of `slots` experts.
+// An SM has 228 KB; a CTA takes 1 KB more than it asks for, and 0.5 KB (2.3 with the norm in groups) are static.  It matters
+// where the fourth just fits: 2048 x 5632 is 512 tiles, which at three CTAs an SM left 68 for a second round (9 us instead of 6).
 int matvec_ctas(size_t row, int depth, int slots, int sm)
 {
-    return sm * std::max(1, std::min(4, (int)(((size_t)220 << 10) / (row + depth * kMvStage + 2048)))) / slots;
+    return sm * std::max(1, std::min(4, (int)(((size_t)228 << 10) / (row + depth * kMvStage + 3072)))) / slots;
 }
 
 // Two chunks deep where that lets every tile have a CTA at once and three do not; one beside a row that fills shared memory
