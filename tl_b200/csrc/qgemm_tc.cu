@@ -773,13 +773,13 @@ struct RowsParams {
     float *out[kGemmMaxW];
     int n[kGemmMaxW], n_tiles16[kGemmMaxW], tg_end[kGemmMaxW];   // tile groups up to and including weight i
     int n_w, upt, unit_bytes, stage_w, wstages, m;
-    int tgroups, total, maxp;       // total = tgroups x upt unit steps, cut evenly over the CTAs; maxp: tile groups a CTA can touch
+    int total;                      // tile groups x upt unit steps, cut evenly over the CTAs
     int64_t k;
     const __half *xh;               // [m][k], rows in the order described above
     const float *inv_scale, *resid;
     const uint8_t *sums;            // [K / 256][16][8] sub-block sums of the activation rows (x_to_f16_kernel)
-    float *part;                    // [CTA][tile group of the CTA][16 tiles][16 rows][16 activation rows]: pieces of split tile groups
-    int *cnt;                       // [tile group][16 tiles]: pieces of the tile that are written; zero between launches
+    float *part;                    // [CTA][2][16 tiles][16 activation rows][16 rows]: pieces of a CTA's first and last tile group where they
+                                    // are split; rests at kFoldEmpty between launches
     int *err;
 };
 
@@ -1043,74 +1043,116 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qrows_kernel(const RowsParams
         }
         if (!ok) break;
         // results: lane (r, c) holds weight rows r and r + 8 x activation rows 8 t + 2 c, + 1.  A tile group that lies
-        // in one CTA goes to the output.  The pieces of a split one go to this CTA's scratch slot of the group; the warp that
-        // writes a tile's last piece (a count per tile tells) adds them, CTAs in index order, and writes the output rows.
+        // in one CTA goes to the output, the pieces of a split one to this CTA's scratch slot of the group.
         if (have) {
             const bool whole = len == upt;
-            float *slot = p.part + (((size_t)blockIdx.x * p.maxp + (tg - tg_first)) * kRowsWarps + warp) * 256;
+            float *slot = p.part + (((size_t)blockIdx.x * 2 + (tg != tg_first)) * kRowsWarps + warp) * 256;
 #pragma unroll
             for (int t = 0; t < NT; t++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
                     const int rt = r + (e >> 1) * 8, row = tile16 * 16 + rt, tok = 8 * t + 2 * c + (e & 1);
                     if (tok >= p.m) continue;
-                    if (!whole) slot[rt * 16 + tok] = acc[t][e];
+                    if (!whole) slot[tok * 16 + rt] = acc[t][e];
                     else if (row < p.n[wi]) {
-                        const float res = p.resid ? __ldg(p.resid + (size_t)tok * p.n[wi] + row) : 0.f;
-                        p.out[wi][(size_t)tok * p.n[wi] + row] = res + acc[t][e] * __ldg(p.inv_scale + tok);
+                        const float res = p.resid ? __ldcg(p.resid + (size_t)tok * p.n[wi] + row) : 0.f;
+                        p.out[wi][(size_t)tok * p.n[wi] + row] = res + acc[t][e] * p.inv_scale[tok];
                     }
                 }
-            if (!whole) {
-                // the CTA of unit step x is the last one whose range starts at or before x
-                const int64_t x0 = (int64_t)tg * upt, x1 = x0 + upt - 1;
-                const int b_lo = (int)(((x0 + 1) * gridDim.x - 1) / p.total), b_hi = (int)(((x1 + 1) * gridDim.x - 1) / p.total);
-                __threadfence();
-                __syncwarp();
-                int before = 0;
-                if (lane == 0) before = atomicAdd(p.cnt + tg * kRowsWarps + warp, 1);
-                before = __shfl_sync(0xffffffffu, before, 0);
-                if (before == b_hi - b_lo) {
-                    __threadfence();
-                    if (lane == 0) p.cnt[tg * kRowsWarps + warp] = 0;
-                    const size_t cta_stride = (size_t)p.maxp * kRowsWarps * 256;
-                    const int tgf_lo = (int)((int64_t)p.total * b_lo / gridDim.x) / upt;
-                    const float *src = p.part + (size_t)warp * 256 + lane;
-                    const float *first = src + b_lo * cta_stride + (size_t)(tg - tgf_lo) * kRowsWarps * 256;
-                    // entry 32 i + lane of the tile's 16 x 16: (row, activation row).  The eight entries of a piece, their
-                    // residuals and scales are requested together, so a fold waits for L2 about once per kFold pieces and not once
-                    // per entry and piece.  What bounds a narrow launch is this chain of latencies: 4096 x 4096 Q4_K with
-                    // 16 rows (up to ten pieces a tile) took 21 us with the loads one after another and takes 16.  At the
-                    // 96 registers of 544 threads three pieces at a time spill 4 (Q4_K) and 12 bytes (Q6_K) in the forms for 16
-                    // rows; 128256 x 4096 with two, three and four at a time: 110.1, 109.1, 109.1 us (Q4_K), 139.8, 140.4, 142.2 (Q6_K).
-                    constexpr int kFold = 3;
-                    float sum[8], res[8];
-                    const int tok = lane & 15;
-                    const float inv = tok < p.m ? __ldg(p.inv_scale + tok) : 0.f;
-                    const bool live = tok < p.m;
+        }
+    }
+    // Split tiles, once the warp is through its own units: the CTAs that hold pieces of a tile group share its sixteen tiles out.
+    // The scratch rests at kFoldEmpty, so a value that is not kFoldEmpty is a piece that has arrived (a 4-byte store is
+    // indivisible): the warp reads a tile's pieces, kFold at a time, again while some are missing (bounded), adds them in CTA
+    // order, puts kFoldEmpty back and writes the rows.  What bounds a narrow launch is this tail of latencies: with a fence, a count
+    // and another fence per piece, the last arriver adding, 4096 x 4096 with 16 rows took 19.2 us in Q4_K (now 18.5), 14336 x 4096
+    // 26.1 (24.0), 5120 x 5120 with 5 rows in Q8_0 16.9 (13.9), eight steps of 16 sequences 5.17 ms (4.62).
+    for (int part = 0; part < 2 && ok; part++) {
+        const int tgs = part == 0 ? tg_first : (end - 1) / upt;
+        if (part == 1 && tgs == tg_first) break;
+        // the CTA of unit step x is the last one whose range starts at or before x
+        const int64_t x0 = (int64_t)tgs * upt, x1 = x0 + upt - 1;
+        const int b_lo = (int)(((x0 + 1) * gridDim.x - 1) / p.total), np = (int)(((x1 + 1) * gridDim.x - 1) / p.total) - b_lo + 1;
+        int wi, tile16;
+        bool have;
+        tile_of(tgs, wi, tile16, have);
+        if (np == 1 || !have || (int)blockIdx.x != b_lo + warp % np) continue;
+        // in the first CTA of several the group is its last one, unless that is also its first; in the others it is their first
+        const bool lo_first = (int)((int64_t)p.total * b_lo / gridDim.x) / upt == tgs;
+        const size_t cta_stride = (size_t)2 * kRowsWarps * 256;
+        float *const src0 = p.part + (size_t)b_lo * cta_stride + (size_t)warp * 256 + lane * 4;
+        auto piece = [&](int q, int i) { return src0 + q * cta_stride + (q == 0 && !lo_first ? (size_t)kRowsWarps * 256 : 0) + 128 * i; };
+        // item lane + 32 i: four weight rows of one activation row
+        constexpr int kFold = 3;
+        const int n = p.n[wi], row = tile16 * 16 + 4 * (lane & 3);
+        float4 sum[NT], res[NT];
+        float inv[NT];
 #pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const int row = tile16 * 16 + 2 * i + (lane >> 4);
-                        sum[i] = __ldcg(first + 32 * i);
-                        res[i] = p.resid && live && row < p.n[wi] ? __ldg(p.resid + (size_t)tok * p.n[wi] + row) : 0.f;
-                    }
-                    for (int cta = b_lo + 1; cta <= b_hi; cta += kFold) {
-                        float v[kFold][8];
+        for (int i = 0; i < NT; i++) {
+            const int tok = (lane >> 2) + 8 * i;
+            sum[i] = res[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            inv[i] = tok < p.m ? __ldcg(p.inv_scale + tok) : 0.f;
+            if (p.resid && tok < p.m) {
+                const float *rp = p.resid + (size_t)tok * n + row;
+                if (row < n) res[i].x = __ldcg(rp);
+                if (row + 1 < n) res[i].y = __ldcg(rp + 1);
+                if (row + 2 < n) res[i].z = __ldcg(rp + 2);
+                if (row + 3 < n) res[i].w = __ldcg(rp + 3);
+            }
+        }
+        for (int q0 = 0; q0 < np && ok; q0 += kFold) {
+            uint4 v[kFold][NT];
+            auto wanted = [&](int q, int i) { return q0 + q < np && (lane >> 2) + 8 * i < p.m; };
 #pragma unroll
-                        for (int q = 0; q < kFold; q++)
+            for (int q = 0; q < kFold; q++)
 #pragma unroll
-                            for (int i = 0; i < 8; i++) v[q][i] = cta + q <= b_hi ? __ldcg(src + (cta + q) * cta_stride + 32 * i) : 0.f;
+                for (int i = 0; i < NT; i++) v[q][i] = wanted(q, i) ? ld_volatile_u4(piece(q0 + q, i)) : make_uint4(0u, 0u, 0u, 0u);
+            bool got = true;
+            unsigned long long t0 = 0;
+            for (unsigned it = 0;; it++) {
+                bool all = true;
 #pragma unroll
-                        for (int q = 0; q < kFold; q++)
+                for (int q = 0; q < kFold; q++)
 #pragma unroll
-                            for (int i = 0; i < 8; i++) sum[i] += v[q][i];
-                    }
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const int row = tile16 * 16 + 2 * i + (lane >> 4);
-                        if (live && row < p.n[wi]) p.out[wi][(size_t)tok * p.n[wi] + row] = res[i] + sum[i] * inv;
-                    }
+                    for (int i = 0; i < NT; i++)
+                        if (v[q][i].x == kFoldEmpty || v[q][i].y == kFoldEmpty || v[q][i].z == kFoldEmpty || v[q][i].w == kFoldEmpty) {
+                            v[q][i] = ld_volatile_u4(piece(q0 + q, i));
+                            all = false;
+                        }
+                if (all) break;
+                if ((it & 255) == 255) {
+                    const unsigned long long t = global_ns();
+                    if (!t0) t0 = t;
+                    if (t - t0 > 1000000000ull) { got = false; break; }
                 }
             }
+            if (!__all_sync(0xffffffffu, got)) {
+                if (lane == 0) atomicExch(p.err, 54);
+                ok = false;
+                break;
+            }
+#pragma unroll
+            for (int q = 0; q < kFold; q++)
+#pragma unroll
+                for (int i = 0; i < NT; i++) {
+                    if (!wanted(q, i)) continue;
+                    sum[i].x += __uint_as_float(v[q][i].x); sum[i].y += __uint_as_float(v[q][i].y);
+                    sum[i].z += __uint_as_float(v[q][i].z); sum[i].w += __uint_as_float(v[q][i].w);
+                    *reinterpret_cast<uint4 *>(piece(q0 + q, i)) = make_uint4(kFoldEmpty, kFoldEmpty, kFoldEmpty, kFoldEmpty);
+                }
+        }
+        if (!ok) break;
+#pragma unroll
+        for (int i = 0; i < NT; i++) {
+            const int tok = (lane >> 2) + 8 * i;
+            if (tok >= p.m) continue;
+            const float4 y = make_float4(res[i].x + sum[i].x * inv[i], res[i].y + sum[i].y * inv[i], res[i].z + sum[i].z * inv[i], res[i].w + sum[i].w * inv[i]);
+            float *o = p.out[wi] + (size_t)tok * n + row;
+            if (row + 3 < n && (reinterpret_cast<uintptr_t>(o) & 15) == 0) { *reinterpret_cast<float4 *>(o) = y; continue; }
+            if (row < n) o[0] = y.x;
+            if (row + 1 < n) o[1] = y.y;
+            if (row + 2 < n) o[2] = y.z;
+            if (row + 3 < n) o[3] = y.w;
         }
     }
     if (!ok && lane == 0) {
@@ -1475,29 +1517,18 @@ tlb_status qrows_run(const tlb_qtensor *const *ws, int n_w, const GemmAct &a, fl
     p.stage_w = (p.unit_bytes + 127) / 128 * 128;
     p.wstages = std::max(2, std::min(4, kRowsWBytes / kRowsWarps / p.stage_w));
     p.m = (int)a.m;
-    p.tgroups = tgroups;
     p.total = tgroups * p.upt;
     // the unit steps (tile group x unit) are cut evenly over the CTAs, whatever the borders of the tile groups
     const int grid = std::min(p.total, c->sm_count);
-    const int per = (p.total + grid - 1) / grid;
-    p.maxp = (per + p.upt - 2) / p.upt + 1;
-    bool split = false;
-    for (int b = 1; b < grid && !split; b++) split = ((int64_t)p.total * b / grid) % p.upt != 0;
     p.inv_scale = (const float *)a.inv->ptr;
     p.resid = resid;
     p.sums = a.sums ? (const uint8_t *)a.sums->ptr : nullptr;
     if (!p.sums) return fail(TLB_ERR_ARG, "quantized matmul (few rows): activations prepared without their block sums");
     p.err = c->err_flag;
-    p.cnt = c->mv_cnt;
-    if ((size_t)tgroups * kRowsWarps > c->mv_cnt_n) return fail(TLB_ERR_SHAPE, "quantized matmul (few rows): more tiles than the context's counters");
+    if ((size_t)tgroups * kRowsWarps > c->mv_cnt_n || (size_t)grid * 2 * kRowsWarps * 256 > c->mv_part1_floats) return fail(TLB_ERR_SHAPE, "quantized matmul (few rows): more tiles than the context's scratch");
+    p.part = c->mv_part1;           // at rest at kFoldEmpty, as the one-row matvec's slices
     p.k = a.k;
     p.xh = (const __half *)a.xh->ptr;
-    Storage *part = nullptr;
-    if (split) {
-        part = storage_alloc((size_t)grid * p.maxp * kRowsWarps * 256 * sizeof(float));
-        if (!part) return TLB_ERR_ALLOC;
-        p.part = (float *)part->ptr;
-    }
     const size_t smem = (size_t)kRowsAStages * (kRowsABytes + kRowsSumBytes) + (size_t)kRowsWarps * p.wstages * p.stage_w + 8 * (2 * kRowsAStages + kRowsWarps * p.wstages) + 128 + 64;
     tlb_status ls;
     switch (w0->type) {
@@ -1506,10 +1537,9 @@ tlb_status qrows_run(const tlb_qtensor *const *ws, int n_w, const GemmAct &a, fl
         case 2: ls = launch_fmt_rows_nt<2>(grid, smem, p); break;
         default: ls = launch_fmt_rows_nt<8>(grid, smem, p); break;
     }
-    if (ls != TLB_OK) { if (part) storage_release(part); return ls; }
+    if (ls != TLB_OK) return ls;
     count_launch();
     cudaError_t e = cudaGetLastError();
-    if (part) storage_release(part);
     if (e != cudaSuccess) return cuda_fail(e, "quantized matmul (few rows) launch");
     return TLB_OK;
 }

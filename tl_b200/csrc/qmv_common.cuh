@@ -261,6 +261,13 @@ __device__ __forceinline__ unsigned ld_volatile_u32(const unsigned *p)
     return v;
 }
 
+__device__ __forceinline__ uint4 ld_volatile_u4(const float *p)
+{
+    uint4 v;
+    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ float silu_f(float g) { return g * (1.0f / (1.0f + expf(-g))); }
 
 // Elements 4*i4 .. 4*i4+3 of an activation written by an earlier kernel of the stream, hence the
