@@ -1179,6 +1179,16 @@ __global__ void __launch_bounds__(NT) x_to_f16_kernel(const float *x, const floa
     constexpr bool CACHED = NC > 0;
     constexpr int kActCache = NC;
     __shared__ float red[2][NT / 32];
+    // the norm's weights, read once per pass over the layers, come from memory: requested ahead of the wait
+    constexpr bool KEEPW = CACHED && NC <= 4;
+    float4 wkeep[KEEPW ? kActCache : 1];
+    if (KEEPW && norm_w) {
+#pragma unroll
+        for (int it = 0; it < (KEEPW ? kActCache : 1); it++) {
+            const int64_t i = threadIdx.x * 4 + it * (NT * 4);
+            if (i < k) wkeep[it] = __ldg(reinterpret_cast<const float4 *>(norm_w + i));
+        }
+    }
     pdl_enter();                 // the products behind it may start their prologues; they wait for this grid's end before they read
     const float *row = x + (size_t)blockIdx.x * k;
     const float *row2 = x2 ? x2 + (size_t)blockIdx.x * k : nullptr;
@@ -1198,7 +1208,7 @@ __global__ void __launch_bounds__(NT) x_to_f16_kernel(const float *x, const floa
         if (CACHED) cache[slot] = v;
         if (norm_w) {
             ssq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            const float4 w = __ldg(reinterpret_cast<const float4 *>(norm_w + i));
+            const float4 w = KEEPW ? wkeep[slot] : __ldg(reinterpret_cast<const float4 *>(norm_w + i));
             v.x *= w.x; v.y *= w.y; v.z *= w.z; v.w *= w.w;
         }
         amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
@@ -1235,7 +1245,7 @@ __global__ void __launch_bounds__(NT) x_to_f16_kernel(const float *x, const floa
     auto pass2 = [&](int64_t i, int slot) {
         float4 v = CACHED ? cache[slot] : value(i);
         if (norm_w) {
-            const float4 w = __ldg(reinterpret_cast<const float4 *>(norm_w + i));
+            const float4 w = KEEPW ? wkeep[slot] : __ldg(reinterpret_cast<const float4 *>(norm_w + i));
             v.x = v.x * inv_rms * w.x; v.y = v.y * inv_rms * w.y; v.z = v.z * inv_rms * w.z; v.w = v.w * inv_rms * w.w;
         }
         // inside every group of four the middle two are exchanged, as store4 lays the weights out
