@@ -11,7 +11,7 @@ import layered_session as S
 import plain_layers as P
 import tl_b200 as tl
 from layered_session import decode, err, greedy, run_portions, toks
-from test_launch_plans_cpu import dense_matvec_plan
+from test_launch_plans_cpu import dense_gemm_ranges, dense_matvec_plan
 from tl_b200 import synth
 
 pytestmark = pytest.mark.gpu
@@ -96,6 +96,15 @@ def test_norms_feed_forward_and_scales(width, ff, vocab, eps, f32):
     assert close(d.prefill_logits(t[:33]), want[:33], f32)
     assert close(decode(d, t[33:], 33), want[33:], f32)
     assert np.allclose(d.hidden(), m_hidden(m, t), atol=(1e-4 if f32 else 6e-2) * np.max(np.abs(m_hidden(m, t))))
+
+
+@pytest.mark.parametrize("width,ff,tokens,ranges", [(1100, 2304, 40, (2, 4)), (1600, 2304, 300, (3, 4)), (1536, 2050, 140, (3, 4)), (1100, 3000, 33, (2, 4))])
+def test_prompt_products_in_ranges(width, ff, tokens, ranges):
+    """K ranges of one cluster, two to four and of unequal length, in tiles of one to eight pieces of 32 tokens, the last of them ragged."""
+    assert (dense_gemm_ranges(tokens, ff, width), dense_gemm_ranges(tokens, width, ff)) == ranges
+    m = Model(config([retention()], width=width, ff=ff), seed=12)
+    t = toks(tokens)
+    assert close(m.dec(False, max_seq=tokens).prefill_logits(t), m.ref(t), False)
 
 
 @pytest.mark.parametrize("width,ff,vocab", [(2048, 4096, 20000), (64, 47104, 131), (72, 8999, 131), (8450, 60, 131)])

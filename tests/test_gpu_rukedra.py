@@ -188,6 +188,16 @@ def test_weight_ring_of_the_experts(width, ff, experts, top, shared, vocab):
     assert close(decode(m.dec(True), t, 0), m.ref(t), True)
 
 
+@BOTH
+@pytest.mark.parametrize("width,groups,ff,shared", [(256, 2, 402, 102), (384, 1, 28, 36), (640, 5, 60, 30), (1024, 8, 20, 300), (2048, 2, 28, 36), (2048, 16, 36, 0), (2176, 17, 28, 36)])
+def test_decoding_with_norms_of_whole_runs(width, groups, ff, shared, f32):
+    """Parts of whole runs of 128 elements, one run and several, up to 2048 elements and beyond, the last elements of a row in either
+    half of a thread's; experts of whole float4 and others, with a shared one and without."""
+    m = Model(config([(direct(), moe(8, 3, ff, None, 1.3, shared)), (gru(), dense())], width=width, groups=groups), seed=31)
+    t, want = m.sure(6)
+    assert close(decode(m.dec(f32), t, 0), want, f32)
+
+
 def test_the_gate_and_the_norms_matter():
     """Dropping a mechanism moves the plain logits far beyond the tolerances above."""
     m = Model(config([(latent(), moe())]), seed=5)

@@ -127,6 +127,27 @@ def dense_matvec_plan(n, k, slots=1):
     return depth, chunks.value, rounds.value
 
 
+def dense_gemm_ranges(T, n, k):
+    """K ranges of a bf16 product without gates or experts, as launch_dense_gemm asks for them"""
+    kt = (k + 63) // 64
+    two = kt <= 16                                       # CTAs share an SM
+    nt = min(128 if two else 256, (T + 31) // 32 * 32)
+    stages = min(8, (104 if two else 216) * 1024 // (16384 + nt * 128))
+    f = _lib.lib().tlb_dense_gemm_ranges
+    f.restype, f.argtypes = C.c_int, [C.c_int] * 7
+    s = f(T, n, kt, nt, two, stages, SMS)
+    assert s == 1 or (s - 1) * -(-(-(-nt // 32)) // s) * 16384 <= stages * (16384 + nt * 128), (T, n, k)      # the exchange fits the ring
+    return s
+
+
+def test_dense_gemm_ranges_are_launchable():
+    for k in (64, 512, 1024, 1100, 2048, 5632, 14336):
+        for n in (128, 1000, 2048, 3072, 5632, 10368, 32768):
+            for T in (1, 17, 32, 33, 64, 100, 128, 250, 256, 512, 800, 2048):
+                s = dense_gemm_ranges(T, n, k)
+                assert s in (1, 2, 3, 4) and (s == 1 or (k + 63) // 64 >= 8 * s), (T, n, k)
+
+
 def test_dense_matvec_rings_fit():
     for k in list(range(1, 49153, 997)) + [8192, 45056, 45312, 45568, 49152]:
         for n in (1, 40, 1000, 2048, 4096, 8192, 32768):

@@ -549,10 +549,13 @@ struct DenseTcParams {
     GluConst act;
     __nv_bfloat16 *act_out;
     uint32_t type_bits;                    // operand types in the instruction descriptor
+    int splits;                            // RANGES: CTAs of a cluster, each over 1 / splits of the K steps
 };
 
 // One CTA: 128 weight rows (lanes of the accumulator) x nt tokens (its columns).  Warps 0-3 write out (a warp's 32 lanes are 32
 // consecutive output features of one token: coalesced), warp 4 lane 0 issues TMA, warp 5 lane 0 the MMAs.  Every wait is bounded.
+// RANGES: the CTAs of a cluster take the K ranges of one tile and add their sums through each other's shared memory (as qgemm_kernel does).
+template <bool RANGES>
 __global__ void __launch_bounds__(kTcThreads, 2)
 dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const DenseTcParams p)
 {
@@ -590,20 +593,73 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_cons
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
 
+    // K steps of this CTA
+    const int split = RANGES ? (int)blockIdx.z : 0, ka = RANGES ? p.kt * split / p.splits : 0, kt = (RANGES ? p.kt * (split + 1) / p.splits : p.kt) - ka;
+    // pieces of 32 columns that are written out (rows past T come as zeros; a transposed output wants them up to 128)
+    const int t_last = p.out_t ? (t_end + 127) / 128 * 128 : t_end, chunks = (min(p.nt, t_last - t0) + 31) / 32;
+    int own0 = 0, own1 = chunks;
+    constexpr uint32_t kPiece = kTcRows * 16;      // four columns of a tile: 128 rows of 16 bytes
+    auto exchange = [&](bool live) {
+        // range o's CTA finishes chunks [chunks o / splits ..) and gets the other ranges' values of them, [range][column / 4][row][4]
+        __syncwarp();
+        cluster_sync();                            // nobody's ring is in use any more
+        if (live) {
+            for (int o = 0; o < p.splits; o++) {
+                if (o == split) continue;
+                const int b0 = chunks * o / p.splits, b1 = chunks * (o + 1) / p.splits, slot = split - (split > o);
+                const uint32_t dst = cluster_addr(base, (uint32_t)o) + (uint32_t)(slot * (b1 - b0) * 8) * kPiece + (uint32_t)(warp * 32 + lane) * 16u;
+                for (int ch = b0; ch < b1; ch++) {
+                    uint32_t v[32];
+                    tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(ch * 32), v);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int q = 0; q < 8; q++) st_cluster_v4(dst + (uint32_t)((ch - b0) * 8 + q) * kPiece, v, 4 * q);
+                }
+            }
+        }
+        __syncwarp();
+        cluster_sync();
+        own0 = chunks * split / p.splits;
+        own1 = chunks * (split + 1) / p.splits;
+    };
+
     if (warp < 4) {
         pdl_wait();                        // residual and outputs belong to the launches before
-        if (mbar_wait(done, 0, abort_flag, p.err, 61)) {
-            tc_fence_after();
+        const bool live = mbar_wait(done, 0, abort_flag, p.err, 61);
+        tc_fence_after();
+        if (RANGES) exchange(live);
+        if (live) {
             const int row = n0 + warp * 32 + lane;
             const bool in = row < p.n;
             const float bias = in && p.bias ? p.bias[row] : 0.f, rs = in && p.resid_scale ? p.resid_scale[row] : 0.f;
             const int col = row - p.glu;
             const size_t place = (size_t)(col / p.per) * p.block_stride + col % p.per;
-            if (p.out_t) t_end = (t_end + 127) / 128 * 128;        // rows past T came as zeros
-            for (int c0 = 0; c0 < p.nt && t0 + c0 < t_end; c0 += 32) {
+            t_end = t_last;
+            for (int c0 = 32 * own0; c0 < 32 * own1; c0 += 32) {
                 uint32_t v[32];
                 tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
                 tmem_wait_ld();
+                if (RANGES) {              // in the order of the ranges
+                    const uint32_t src = base + (uint32_t)((c0 / 32 - own0) * 8) * kPiece + (uint32_t)(warp * 32 + lane) * 16u, stride = (uint32_t)((own1 - own0) * 8) * kPiece;
+                    float acc[32];
+#pragma unroll
+                    for (int i = 0; i < 32; i++) acc[i] = 0.f;
+                    for (int o = 0; o < p.splits; o++) {
+                        if (o == split) {
+#pragma unroll
+                            for (int i = 0; i < 32; i++) acc[i] += __uint_as_float(v[i]);
+                        } else {
+                            const uint32_t at = src + (uint32_t)(o - (o > split)) * stride;
+#pragma unroll
+                            for (int q = 0; q < 8; q++) {
+                                const uint4 a = lds128(at + (uint32_t)q * kPiece);
+                                acc[4 * q] += __uint_as_float(a.x); acc[4 * q + 1] += __uint_as_float(a.y); acc[4 * q + 2] += __uint_as_float(a.z); acc[4 * q + 3] += __uint_as_float(a.w);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 32; i++) v[i] = __float_as_uint(acc[i]);
+                }
                 if (n0 + warp * 32 < p.glu) {
                     // lanes (0, 1), (2, 3) of four hold gates and ups of two units: the former take tokens 0 .. 15, the latter 16 .. 31
                     const bool hi = lane & 2;
@@ -664,22 +720,22 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_cons
             int issued = 0;
             // the weights do not depend on the launch before.  Dependents may start from here on, where this CTA has its tensor
             // memory: one that took theirs first would wait for it and be waited for
-            const int early = min(p.kt, p.stages);
+            const int early = min(kt, p.stages);
             for (int k = 0; k < early; k++) {
                 mbar_expect_tx(full + 8 * k, stage);
-                tma_load_2d(base + (uint32_t)k * stage, &wmap, k * kTcK, wrow0, full + 8 * k);
+                tma_load_2d(base + (uint32_t)k * stage, &wmap, (ka + k) * kTcK, wrow0, full + 8 * k);
             }
             pdl_enter();
             for (int k = 0; k < early; k++) {
-                tma_load_2d(base + (uint32_t)k * stage + kTcWBytes, &xmap, k * kTcK, t0, full + 8 * k);
+                tma_load_2d(base + (uint32_t)k * stage + kTcWBytes, &xmap, (ka + k) * kTcK, t0, full + 8 * k);
                 issued = k + 1;
             }
-            for (int k = early; k < p.kt; k++) {
+            for (int k = early; k < kt; k++) {
                 const int s = k % p.stages;
                 if (!mbar_wait(empty + 8 * s, (uint32_t)(k / p.stages - 1) & 1u, abort_flag, p.err, 62)) break;
                 mbar_expect_tx(full + 8 * s, stage);
-                tma_load_2d(base + (uint32_t)s * stage, &wmap, k * kTcK, wrow0, full + 8 * s);
-                tma_load_2d(base + (uint32_t)s * stage + kTcWBytes, &xmap, k * kTcK, t0, full + 8 * s);
+                tma_load_2d(base + (uint32_t)s * stage, &wmap, (ka + k) * kTcK, wrow0, full + 8 * s);
+                tma_load_2d(base + (uint32_t)s * stage + kTcWBytes, &xmap, (ka + k) * kTcK, t0, full + 8 * s);
                 issued = k + 1;
             }
             if (*abort_flag)
@@ -689,7 +745,7 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_cons
         // f32 accumulator, operands of one 16-bit type, both K-major, M 128, N nt
         const int cols = p.tiles ? (t_end - t0 + 15) / 16 * 16 : p.nt;       // a tile that is not full multiplies fewer columns
         const uint32_t idesc = (1u << 4) | p.type_bits | ((uint32_t)(cols >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24);
-        for (int k = 0; k < p.kt; k++) {
+        for (int k = 0; k < kt; k++) {
             const int s = k % p.stages;
             if (!mbar_wait(full + 8 * s, (uint32_t)(k / p.stages) & 1u, abort_flag, p.err, 63)) break;
             tc_fence_after();
@@ -701,6 +757,7 @@ dense_gemm_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_cons
         umma_commit(done);                       // also after an abort: MMAs in flight end before the tensor memory is freed
         if (*abort_flag) mbar_wait_drain(done, 0);
     }
+    if (RANGES && warp >= 4) exchange(false);
     tc_fence_before();
     __syncthreads();
     if (warp == 5) {
@@ -1024,6 +1081,24 @@ tlb_status launch_dense_matvec(const DenseMatvecJob &j)
     return pick_matvec<DPRO_PLAIN>(p, j.pdl);
 }
 
+// K ranges of a product of T rows and n outputs over kt steps of 64 in tiles of nt rows, one CTA an SM or (pair) two: as many as
+// the SMs hold at once (74 clusters of two CTAs, 45 of three, 33 of four) with eight steps or more each.  A tile's time is its
+// number of steps, and a second wave takes back more than a range gives.  Microseconds of a product in one to four ranges:
+//   512 rows: 2048 x 2048 25.3, 20.4, 18.5, 17.2; 2048 x 5632 47.4, 30.8, 26.7, 23.6; 3072 x 2048 17.8, 16.0, 27.2; 5632 x 2048 19.7, 31.4
+//   100 rows: 2048 x 5632 37.6, 23.8, 19.7, 15.8; 5632 x 2048 15.3, 13.4, 12.7, 20.2; 3072 x 2048 14.9, 12.0, 11.5, 10.7
+int dense_gemm_ranges(int T, int n, int kt, int nt, bool pair, int stages, int sm)
+{
+    constexpr int kHeld[5] = {0, 148, 74, 45, 33};
+    const int64_t tiles = (int64_t)((T + nt - 1) / nt) * ((n + kTcRows - 1) / kTcRows);
+    const size_t ring = (size_t)stages * (kTcWBytes + (size_t)nt * kTcK * 2);
+    for (int s = 4; s > 1; s--) {
+        const size_t sums = (size_t)(s - 1) * (((nt + 31) / 32 + s - 1) / s) * 32 * kTcRows * sizeof(float);     // the other ranges', in the ring
+        if (kt >= 8 * s && tiles <= (int64_t)kHeld[s] * sm / 148 * (pair ? 2 : 1) && sums <= ring) return s;
+    }
+    return 1;
+}
+extern "C" int tlb_dense_gemm_ranges(int T, int n, int kt, int nt, int pair, int stages, int sm) { return dense_gemm_ranges(T, n, kt, nt, pair != 0, stages, sm); }
+
 tlb_status launch_dense_gemm(const DenseGemmJob &j, bool f32)
 {
     Context *c = ctx();
@@ -1059,12 +1134,32 @@ tlb_status launch_dense_gemm(const DenseGemmJob &j, bool f32)
         !encode_f16_map(&xmap, j.x, (uint64_t)j.w.k, (uint64_t)j.T, (uint64_t)j.ldx * 2, kTcK, (uint32_t)p.nt, type))
         return fail(TLB_ERR_DEVICE, "GEMM: cuTensorMapEncodeTiled failed or is not available");
     const size_t smem = (size_t)p.stages * stage + 16 * p.stages + 8 + 1024;
+    p.splits = j.tiles ? 1 : dense_gemm_ranges(j.T, j.w.n, p.kt, p.nt, pair, p.stages, c->sm_count);
     static size_t allowed = 0;
     if (smem > allowed) {
-        TLB_CUDA(cudaFuncSetAttribute(dense_gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        TLB_CUDA(cudaFuncSetAttribute(dense_gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        TLB_CUDA(cudaFuncSetAttribute(dense_gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         allowed = smem;
     }
-    TLB_CUDA(launch_chained(dense_gemm_tc_kernel, dim3(j.tiles ? j.n_tiles : (j.T + p.nt - 1) / p.nt, (j.w.n + kTcRows - 1) / kTcRows), dim3(kTcThreads), smem, true, wmap, xmap, p));
+    const dim3 grid(j.tiles ? j.n_tiles : (j.T + p.nt - 1) / p.nt, (j.w.n + kTcRows - 1) / kTcRows, p.splits);
+    if (p.splits == 1) {
+        TLB_CUDA(launch_chained(dense_gemm_tc_kernel<false>, grid, dim3(kTcThreads), smem, true, wmap, xmap, p));
+        return launched("GEMM launch");
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = (unsigned)p.splits;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    TLB_CUDA(cudaLaunchKernelEx(&cfg, dense_gemm_tc_kernel<true>, wmap, xmap, p));
     return launched("GEMM launch");
 }
 

@@ -66,7 +66,7 @@ __device__ __forceinline__ void cluster_sync()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t (&v)[8], int first)
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t *v, int first)
 {
     asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[first]), "r"(v[first + 1]), "r"(v[first + 2]), "r"(v[first + 3]) : "memory");
 }
