@@ -595,8 +595,8 @@ static double slice_cost(int type, int m, int64_t tiles, int upt, int upi, int s
     const double stream = kb == 1 ? (double)((ipc * upi + nw - 1) / nw) * unit + 60.0 * ((ipc + nw - 1) / nw + 1)
                                   : (double)ipw * (upi * unit + 60.0);
     const double quant = 300.0 * ((m * nb + nw / 2 - 1) / (nw / 2));
-    // Measured on the Llama-3-8B shapes: the end of a sliced launch (fence, counts, reading the slices back)
-    // costs ~3 us; assembling tiles in shared memory costs a block barrier, which shows (~2 us of waiting
+    // The end of a sliced launch (stores, reading the slices back) costs 1.5 us with one row, ~3 with several (fence, counts);
+    // with 300 for it the plans of the TinyLlama and Llama-3-8B chains are the same, with 1000 they are 3 and 10 % slower; assembling tiles in shared memory costs a block barrier, which shows (~2 us of waiting
     // for the slowest warp) only when warps have so few units that their skew matters.
     // Three or four rows in several items per warp pay far more (14336 x 4096 Q8_0, four rows: 43 us in four slices, 23 in one),
     // eight warps a little (a layer of width 1536 and 21 units per SM: 34.8 us with gate|up in two slices, 31.9 in one; 500 more
@@ -618,11 +618,11 @@ static int warps_for(const MatvecJob &job, int64_t tiles, int upt, int sm_count)
 // In a chain, where launches follow each other at once, eight warps gain up to larger launches, if all of them have eight and as
 // long as they prepare a row in one pass: kKeep blocks of 256 for each two warps, 2048.  Microseconds a layer (Q4_K / Q8_0, f16
 // cache of 200 rows) with sixteen, and with eight, by width and units per SM of the largest launch:
-//   2048, 38 units: 37.2 / 37.7, 35.3 / 35.0;  76: 40.6 / 42.6, 39.5 / 40.6;  111: 42.6 / 47.9, 42.7 / 45.3;  194: 50.5 / 60.3, 54.5 / 61.2
-//   1536, 21 units: 33.2 / 33.8, 31.9 / 31.6;  1024, 14: 30.2 / 29.5, 27.9 / 27.4
-//   2560, 35 units: 40.7 / 41.5, 42.6 / 41.1;  3072, 83: 43.6 / 48.0, 46.8 / 51.1;  4096, 38: 43.0 / 44.6, 48.0 / 50.2
-// Eight warps for some launches of a layer and sixteen for the others is slower than either (2048, 38 units: gate|up alone +1.1).
-bool matvec_few(int64_t d_model, int64_t units, int sm) { return d_model <= kFewWarps / 2 * kKeep * 256 && units <= (int64_t)80 * sm; }
+//   2048, 38 units: 30.1 / 30.1, 27.9 / 26.6;  76: 32.9 / 34.8, 31.6 / 31.5;  111: 35.0 / 40.0, 33.9 / 35.8;  138: 38.3 / 44.5, 38.0 / 41.2;
+//   194: 42.2 / 52.3, 44.3 / 50.1;  1536, 21 units: 26.4 / 26.0, 25.0 / 24.0;  1024, 14: 23.4 / 22.9, 21.3 / 20.3
+// Wider rows take a second pass: 4096, 111 units: 38.2 / 44.0, 38.9 / 44.6;  138: 40.0 / 48.3, 42.6 / 50.4.  Their short launches gain
+// all the same (2560, 35 units: 30.7 / 31.3, 29.5 / 28.4;  4096, 38: 32.7 / 34.4, 31.6 / 33.8), which this line by width leaves out.
+bool matvec_few(int64_t d_model, int64_t units, int sm) { return d_model <= kFewWarps / 2 * kKeep * 256 && units <= (int64_t)140 * sm; }
 extern "C" int tlb_matvec_few(int64_t d_model, int64_t units, int sm) { return matvec_few(d_model, units, sm); }
 
 // How a launch of `tiles` 16-row tiles (all tensors) over upt units of K is laid out with kb K-slices.
