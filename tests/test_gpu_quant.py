@@ -174,6 +174,28 @@ def test_qmatvec_wide_dynamic_range(orc):
     assert np.isfinite(got).all()
 
 
+# Root mean square error of the draws below against 64 bits, relative to the result, with every sum of a unit in one accumulator
+# per level (a build in which one row went through unit_q40 .. unit_q6k, as two to four rows do): what the three levels leave, 1.0e-7,
+# and the f32 roundings of sixteen units.  Other orders of the same sums move these figures by 2 %.
+ONE_ROW_ERR = {(synth.Q4_0, False): 1.513e-7, (synth.Q4_0, True): 0.706e-7, (synth.Q8_0, False): 1.487e-7, (synth.Q8_0, True): 1.475e-7,
+               (synth.Q4_K, False): 1.445e-7, (synth.Q4_K, True): 0.673e-7, (synth.Q6_K, False): 1.420e-7, (synth.Q6_K, True): 1.442e-7}
+
+
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("positive", [False, True])
+def test_one_row_error_against_64_bits(t, positive):
+    n, k, e = 2048, 4096, []
+    for seed in range(6):
+        rng = np.random.default_rng(1000 * seed + k)
+        q = tl.QTensor.from_gguf_bytes(t, n, k, synth.random_quant(t, n, k, rng))
+        x = rng.standard_normal((1, k)).astype(np.float32)
+        if positive:
+            x = np.abs(x)
+        ref = x.astype(np.float64) @ q.dequantize().numpy().astype(np.float64).T
+        e.append(np.linalg.norm(tl.Tensor.from_numpy(x).matmul_quantized(q).numpy() - ref) / np.linalg.norm(ref))
+    assert np.sqrt(np.mean(np.square(e))) < 1.03 * ONE_ROW_ERR[t, positive]
+
+
 def test_qmatvec_shape_errors():
     q = tl.QTensor.from_gguf_bytes(synth.Q4_K, 16, 256, np.zeros(16 * 144, dtype=np.uint8))
     with pytest.raises(tl.TlbError) as e:

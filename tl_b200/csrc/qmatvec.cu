@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
         L.alam_b = smem_u32(smem + p.off_alam) + 2 * c * 4;
         L.xsum_b = smem_u32(smem + p.off_xsum) + (r & 1) * (p.nb_max * 8) * 2;
         L.minv_b = smem_u32(smem + p.off_minv);
-        L.sa_b = smem_u32(smem + p.off_sa) + (FMT == TLB_GGML_Q4_0 ? c * 8 : (first ? r : 3) * 32);
+        L.sa_b = smem_u32(smem + p.off_sa) + (FMT == TLB_GGML_Q4_0 ? c * 8 : (first || second ? r : 3) * 32);
         L.half_sh = (c >> 1) * 16;
         L.sel_u = 0x4440u + (c >> 1);
         L.sel_s = 0x8880u + (c >> 1) * 0x1111u;

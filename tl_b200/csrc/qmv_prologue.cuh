@@ -117,9 +117,15 @@ __device__ __forceinline__ void quantise_block(const MvParams &p, uint8_t *smem,
                 float s = lsum[l];
                 s += __shfl_xor_sync(0xffffffffu, s, 1);
                 s += __shfl_xor_sync(0xffffffffu, s, 2);
-                if ((lane & 3) == 0) sa[((size_t)lb * kMaxCols + mrow * NL + l) * 16 + (j >> 2)] = __float2half_rn(s);
+                // one row: columns 0 .. 2 have the sums of the even groups and zeros for the odd ones, 4 .. 6 the other way round
+                if (ONE) {
+                    const int col = ((j >> 2) & 1) * 4 + l;
+                    if ((lane & 3) < 2) sa[((size_t)lb * kMaxCols + ((lane & 3) ? col ^ 4 : col)) * 16 + (j >> 2)] = __float2half_rn((lane & 3) ? 0.f : s);
+                } else if ((lane & 3) == 0) {
+                    sa[((size_t)lb * kMaxCols + mrow * NL + l) * 16 + (j >> 2)] = __float2half_rn(s);
+                }
             }
-        if (ONE && (lane & 3) == 1) sa[((size_t)lb * kMaxCols + 3) * 16 + (j >> 2)] = __ushort_as_half(0);
+        if (ONE && (lane & 3) == 2) sa[((size_t)lb * kMaxCols + 3) * 16 + (j >> 2)] = __ushort_as_half(0);
     }
     if (FMT == TLB_GGML_Q4_0) {   // level sums over blocks of 32 = 8 consecutive lanes, int32; [lb*8 + j/8][8 cols]
         int *sa = reinterpret_cast<int *>(smem + p.off_sa);
