@@ -653,11 +653,11 @@ tlb_status launch_latent_prompt(const MixLatent &m, int seq, int T, int pos0, in
     void *keys = get((size_t)m.H * n_keys * ldk * es), *vals = get((size_t)m.H * (tc5 ? (size_t)128 * vt_ld : (size_t)n_keys * ldv) * es);
     __half *q16 = tc5 ? (__half *)get((size_t)T * m.H * qd * 2) : nullptr;
     if (!keys || !vals || (tc5 && !q16)) return done(TLB_ERR_ALLOC);
-    if (f32) TLB_CUDA(launch_chained(latent_prep_kernel<float, 0>, dim3(T), dim3(kThreads), 0, true, m, seq, pos0, rope0, rope_step, nullptr));
-    else if (!tc5) TLB_CUDA(launch_chained(latent_prep_kernel<__half, 0>, dim3(T), dim3(kThreads), 0, true, m, seq, pos0, rope0, rope_step, nullptr));
-    else if (qd == 128) TLB_CUDA(launch_chained(latent_prep_kernel<__half, 128>, dim3(T), dim3(kThreads), 0, true, m, seq, pos0, rope0, rope_step, q16));
-    else TLB_CUDA(launch_chained(latent_prep_kernel<__half, 192>, dim3(T), dim3(kThreads), 0, true, m, seq, pos0, rope0, rope_step, q16));
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e;
+    if (f32) e = launch_chained(latent_prep_kernel<float, 0>, dim3(T), dim3(kThreads), 0, true, m, seq, pos0, rope0, rope_step, nullptr);
+    else if (!tc5) e = launch_chained(latent_prep_kernel<__half, 0>, dim3(T), dim3(kThreads), 0, true, m, seq, pos0, rope0, rope_step, nullptr);
+    else if (qd == 128) e = launch_chained(latent_prep_kernel<__half, 128>, dim3(T), dim3(kThreads), 0, true, m, seq, pos0, rope0, rope_step, q16);
+    else e = launch_chained(latent_prep_kernel<__half, 192>, dim3(T), dim3(kThreads), 0, true, m, seq, pos0, rope0, rope_step, q16);
     if (e != cudaSuccess) return done(cuda_fail(e, "latent preparation launch"));
     const char *cache = (const char *)m.cache + ((size_t)seq * m.seq_stride + (size_t)key_first * m.ld) * es;
     DenseGemmJob j;
@@ -672,9 +672,8 @@ tlb_status launch_latent_prompt(const MixLatent &m, int seq, int T, int pos0, in
     else { (f32 ? (void *&)j.out : (void *&)j.out_h) = vals; j.ldo = ldv; j.block_stride = (size_t)n_keys * ldv; }
     st = launch_dense_gemm(j, f32);
     if (st != TLB_OK) return done(st);
-    if (f32) TLB_CUDA(launch_chained(latent_rot_kernel<float>, dim3(n_keys), dim3(kThreads), 0, true, m, (const float *)cache, (float *)keys, n_keys, ldk));
-    else TLB_CUDA(launch_chained(latent_rot_kernel<__half>, dim3(n_keys), dim3(kThreads), 0, true, m, (const __half *)cache, (__half *)keys, n_keys, ldk));
-    e = cudaGetLastError();
+    if (f32) e = launch_chained(latent_rot_kernel<float>, dim3(n_keys), dim3(kThreads), 0, true, m, (const float *)cache, (float *)keys, n_keys, ldk);
+    else e = launch_chained(latent_rot_kernel<__half>, dim3(n_keys), dim3(kThreads), 0, true, m, (const __half *)cache, (__half *)keys, n_keys, ldk);
     if (e != cudaSuccess) return done(cuda_fail(e, "latent expansion launch"));
     count_launch(2);
     MixAttn a = {};

@@ -488,9 +488,10 @@ tlb_status launch_prefill_attention_tc(const float *q, const void *kcache, const
     if (!qh || !vt) { if (qh) storage_release(qh); if (vt) storage_release(vt); return TLB_ERR_ALLOC; }
     auto done = [&](tlb_status st) { storage_release(qh); storage_release(vt); return st; };   // stream-ordered: freed after the launches below
     const size_t n4 = (size_t)T * H * kAtD / 4;
-    TLB_CUDA(launch_chained(q_to_f16_kernel, dim3((unsigned)std::min<size_t>(148 * 8, (n4 + 255) / 256)), dim3(256), 0, true, q, (__half *)qh->ptr, n4));
+    cudaError_t e = launch_chained(q_to_f16_kernel, dim3((unsigned)std::min<size_t>(148 * 8, (n4 + 255) / 256)), dim3(256), 0, true, q, (__half *)qh->ptr, n4);
     dim3 tg(kAtD / 32, (unsigned)(keys_ld / 32), (unsigned)KVH);
-    TLB_CUDA(launch_chained(v_transpose_kernel, tg, dim3(256), 0, true, (const __half *)vcache, (__half *)vt->ptr, max_seq, n_keys, keys_ld));
+    if (e == cudaSuccess) e = launch_chained(v_transpose_kernel, tg, dim3(256), 0, true, (const __half *)vcache, (__half *)vt->ptr, max_seq, n_keys, keys_ld);
+    if (e != cudaSuccess) return done(cuda_fail(e, "prompt attention operands"));
     count_launch(2);
     CUtensorMap qmap, kmap, vtmap;
     if (!encode_f16_map(&qmap, qh->ptr, (uint64_t)H * kAtD, (uint64_t)T, (uint64_t)H * kAtD * 2, 64, 128) ||
@@ -504,12 +505,12 @@ tlb_status launch_prefill_attention_tc(const float *q, const void *kcache, const
     constexpr size_t smem = at_smem_bytes(2);
     static bool attr_set = false;
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(prefill_attention_tc_kernel<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(prefill_attention_tc_kernel<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return done(cuda_fail(e, "prompt attention attribute"));
         attr_set = true;
     }
     dim3 grid((unsigned)((T + kAtQ - 1) / kAtQ), (unsigned)H);
-    cudaError_t e = launch_chained(prefill_attention_tc_kernel<false, 2>, grid, dim3(kAtThreads), smem, true, qmap, kmap, vtmap, p);
+    e = launch_chained(prefill_attention_tc_kernel<false, 2>, grid, dim3(kAtThreads), smem, true, qmap, kmap, vtmap, p);
     count_launch();
     if (e != cudaSuccess) return done(cuda_fail(e, "prompt attention launch"));
     return done(TLB_OK);
