@@ -202,3 +202,13 @@ def test_sample_top_p_matches_oracle(orc, n, temp, top_p):
     with pytest.raises(tl.TlbError) as e:
         t.sample_top_p(1.0, top_p, 1.0)
     assert e.value.code == 8
+
+
+def test_a_refused_launch_does_not_fail_the_next_call():
+    """70,000 matrices are more than a grid has layers: the runtime refuses the launch, and the calls after it run."""
+    a, b = T(np.ones((70000, 8, 4), dtype=np.float32)), T(np.ones((4, 3), dtype=np.float32))
+    x = T(np.arange(8, dtype=np.float32))
+    with pytest.raises(tl.TlbError):
+        a.matmul(b)
+    np.testing.assert_array_equal(x.add(x).numpy(), 2 * np.arange(8, dtype=np.float32))
+    np.testing.assert_array_equal(T(np.ones((3, 8, 4), dtype=np.float32)).matmul(b).numpy(), np.full((3, 8, 3), 4, dtype=np.float32))

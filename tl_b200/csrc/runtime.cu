@@ -24,6 +24,7 @@ tlb_status fail(tlb_status code, const char *fmt, ...)
 
 tlb_status cuda_fail(cudaError_t e, const char *what)
 {
+    cudaGetLastError();      // reported here: the runtime would hand it to the next call that looks for an error of its own launch
     return fail(e == cudaErrorMemoryAllocation ? TLB_ERR_ALLOC : TLB_ERR_DEVICE, "CUDA error %d (%s) in %s",
                 (int)e, cudaGetErrorString(e), what);
 }
