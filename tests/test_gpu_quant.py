@@ -176,7 +176,7 @@ def test_qmatvec_wide_dynamic_range(orc):
 
 # Root mean square error of the draws below against 64 bits, relative to the result, with every sum of a unit in one accumulator
 # per level (a build in which one row went through unit_q40 .. unit_q6k, as two to four rows do): what the three levels leave, 1.0e-7,
-# and the f32 roundings of sixteen units.  Other orders of the same sums move these figures by 2 %.
+# and the f32 roundings of sixteen units.  The draws are fixed; 1 % is for their rounding here.
 ONE_ROW_ERR = {(synth.Q4_0, False): 1.513e-7, (synth.Q4_0, True): 0.706e-7, (synth.Q8_0, False): 1.487e-7, (synth.Q8_0, True): 1.475e-7,
                (synth.Q4_K, False): 1.445e-7, (synth.Q4_K, True): 0.673e-7, (synth.Q6_K, False): 1.420e-7, (synth.Q6_K, True): 1.442e-7}
 
@@ -193,7 +193,7 @@ def test_one_row_error_against_64_bits(t, positive):
             x = np.abs(x)
         ref = x.astype(np.float64) @ q.dequantize().numpy().astype(np.float64).T
         e.append(np.linalg.norm(tl.Tensor.from_numpy(x).matmul_quantized(q).numpy() - ref) / np.linalg.norm(ref))
-    assert np.sqrt(np.mean(np.square(e))) < 1.03 * ONE_ROW_ERR[t, positive]
+    assert np.sqrt(np.mean(np.square(e))) < 1.01 * ONE_ROW_ERR[t, positive]
 
 
 def test_qmatvec_shape_errors():
