@@ -1,0 +1,59 @@
+"""After a kernel gave up a wait: the error is reported once, and whatever it may have left in the library's scratch is gone before the
+next launch reads it.  The error word and the leftovers are put there from the host; no kernel gives anything up here."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import tl_b200 as tl
+from tl_b200 import _lib, synth
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PEEK = r"""
+#include "tlb_internal.h"
+extern "C" int *error_word() { return tlb::ctx()->err_flag; }
+extern "C" unsigned long long slices(unsigned long long *bytes) { *bytes = tlb::ctx()->mv_part1_floats * 4; return (unsigned long long)tlb::ctx()->mv_part1; }
+extern "C" unsigned long long counts(unsigned long long *bytes) { *bytes = tlb::ctx()->mv_cnt_n * 4; return (unsigned long long)tlb::ctx()->mv_cnt; }
+"""
+
+
+@pytest.fixture(scope="module")
+def peek(tmp_path_factory):
+    tl.init()
+    d = tmp_path_factory.mktemp("peek")
+    (d / "peek.cpp").write_text(PEEK)
+    so = str(d / "peek.so")
+    cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    subprocess.check_call(["g++", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(ROOT, "tl_b200", "csrc"), "-I", cuda, "-o", so, str(d / "peek.cpp"), _lib.SO_PATH])
+    L = C.CDLL(so)
+    L.error_word.restype = C.POINTER(C.c_int)
+    L.slices.restype = L.counts.restype = C.c_uint64
+    return L
+
+
+@pytest.mark.parametrize("m", [1, 3, 8, 40])
+def test_leftovers_of_an_abandoned_launch(peek, m):
+    """2048 x 4096 Q8_0: one row folds slices that rest at a sentinel, three rows and eight count theirs, forty take the tensor cores."""
+    drv = C.CDLL("libcuda.so.1")
+    rng = np.random.default_rng(40 + m)
+    q = tl.QTensor.from_gguf_bytes(synth.Q8_0, 2048, 4096, synth.random_quant(synth.Q8_0, 2048, 4096, rng))
+    x = tl.Tensor.from_numpy(rng.standard_normal((m, 4096), dtype=np.float32))
+    want = x.matmul_quantized(q).numpy()
+    for _ in range(3):
+        tl.sync()
+        for area, value in ((peek.slices, 0x3F800000), (peek.counts, 1)):
+            size = C.c_uint64()
+            at = area(C.byref(size))
+            assert drv.cuMemsetD32_v2(C.c_uint64(at), C.c_uint(value), C.c_size_t(size.value // 4)) == 0
+        assert drv.cuCtxSynchronize() == 0
+        peek.error_word()[0] = 2
+        with pytest.raises(tl.TlbError, match="code 2"):
+            tl.sync()
+        got = [x.matmul_quantized(q) for _ in range(4)]
+        tl.sync()
+        for g in got:
+            np.testing.assert_array_equal(g.numpy().view(np.uint32), want.view(np.uint32))

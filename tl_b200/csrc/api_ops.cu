@@ -247,7 +247,7 @@ tlb_status tlb_embedding(tlb_tensor **out, const tlb_tensor *table, const tlb_te
     REQ(!tlb_stream_is_capturing(), TLB_ERR_ARG, "embedding reads its out-of-range flag back from the device: not allowed during a stream capture");
     TLB_TRY(new_tensor(out, TLB_F32, oshape, idx->rank + 1));
     static int *oob = nullptr;
-    if (!oob) { TLB_CUDA(cudaMalloc(&oob, sizeof(int))); TLB_CUDA(cudaMemset(oob, 0, sizeof(int))); }
+    if (!oob) { TLB_CUDA(cudaMalloc(&oob, sizeof(int))); TLB_CUDA(cudaMemsetAsync(oob, 0, sizeof(int), ctx()->stream)); }
     tlb_status st = launch_embedding(table->f32(), idx->f32(), (*out)->f32(), idx->numel(), table->shape[0], table->shape[1], oob);
     if (st == TLB_OK) {
         int flag = 0;

@@ -29,6 +29,15 @@ tlb_status cuda_fail(cudaError_t e, const char *what)
                 (int)e, cudaGetErrorString(e), what);
 }
 
+// The scratch as every launch finds and leaves it.  On the library's stream: a fill on the default stream is not ordered before the
+// launches behind it, which does not wait for that one.
+static tlb_status reset_scratch()
+{
+    TLB_CUDA(cudaMemsetAsync(g_ctx.mv_cnt, 0, g_ctx.mv_cnt_n * sizeof(int), g_ctx.stream));
+    TLB_CUDA(cudaMemsetAsync(g_ctx.mv_part1, 0xFF, g_ctx.mv_part1_floats * sizeof(float), g_ctx.stream));
+    return TLB_OK;
+}
+
 static tlb_status do_init(int device)
 {
     int count = 0;
@@ -62,10 +71,9 @@ static tlb_status do_init(int device)
     TLB_CUDA(cudaMalloc(&g_ctx.mv_part, g_ctx.mv_part_floats * sizeof(float)));
     g_ctx.mv_part1_floats = (size_t)4 << 20;  // 16 MB: 16 slices of a 128k-row head with one activation row, twice over
     TLB_CUDA(cudaMalloc(&g_ctx.mv_part1, g_ctx.mv_part1_floats * sizeof(float)));
-    TLB_CUDA(cudaMemset(g_ctx.mv_part1, 0xFF, g_ctx.mv_part1_floats * sizeof(float)));
     g_ctx.mv_cnt_n = (size_t)1 << 20;
     TLB_CUDA(cudaMalloc(&g_ctx.mv_cnt, g_ctx.mv_cnt_n * sizeof(int)));
-    TLB_CUDA(cudaMemset(g_ctx.mv_cnt, 0, g_ctx.mv_cnt_n * sizeof(int)));
+    TLB_TRY(reset_scratch());
     g_inited = true;
     return TLB_OK;
 }
@@ -193,8 +201,7 @@ tlb_status tlb_sync(void)
     const int flag = *(volatile int *)g_ctx.err_flag;
     if (flag) {
         *(volatile int *)g_ctx.err_flag = 0;
-        cudaMemset(g_ctx.mv_cnt, 0, g_ctx.mv_cnt_n * sizeof(int));   // an abandoned launch may have left counts behind
-        cudaMemset(g_ctx.mv_part1, 0xFF, g_ctx.mv_part1_floats * sizeof(float));   // ... or slices nobody collected
+        TLB_TRY(reset_scratch());        // an abandoned launch may have left counts behind, or slices nobody collected
         return fail(TLB_ERR_DEVICE, "a kernel gave up a bounded wait (code %d)", flag);
     }
     return TLB_OK;

@@ -418,12 +418,12 @@ tlb_status tlb_tp_p2p_export(void *handle_out, size_t handle_bytes)
     std::lock_guard<std::mutex> lk(g_tp_mu);
     if (!g_tp.mine) {
         TLB_CUDA(cudaMalloc((void **)&g_tp.mine, sizeof(P2pRegion)));
-        TLB_CUDA(cudaMemset(g_tp.mine, 0, sizeof(P2pRegion)));
+        TLB_CUDA(cudaMemsetAsync(g_tp.mine, 0, sizeof(P2pRegion), ctx()->stream));
         TLB_CUDA(cudaMalloc((void **)&g_tp.seq, sizeof(unsigned)));
         TLB_CUDA(cudaMalloc((void **)&g_tp.arrive, 4 * sizeof(int)));   // [0] all-reduce kernel, [1] tiles finished by an in-launch exchange
         const unsigned one = 1;       // flags start at 0: the first all-reduce waits for 1
         TLB_CUDA(cudaMemcpy(g_tp.seq, &one, sizeof one, cudaMemcpyHostToDevice));
-        TLB_CUDA(cudaMemset(g_tp.arrive, 0, 4 * sizeof(int)));
+        TLB_CUDA(cudaMemsetAsync(g_tp.arrive, 0, 4 * sizeof(int), ctx()->stream));
         TLB_CUDA(cudaDeviceSynchronize());
     }
     cudaIpcMemHandle_t h;
