@@ -16,6 +16,11 @@ def lines(pattern):
     return found
 
 
+def test_quantised_models_divide_exactly():
+    """__fdividef (two units in the last place) is for the sigmoids of layered models, whose sessions state it."""
+    assert {f for f, _ in lines(r"\b__(fdividef|expf)\(")} <= {"act.cuh"}
+
+
 def test_device_memory_is_filled_in_stream_order():
     """cudaMemset fills on the default stream, which the library's stream does not wait for."""
     assert lines(r"\bcudaMemset(2D|3D)?\(") == []

@@ -480,7 +480,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap xmap, const GemmParams p)
                     const float own = __uint_as_float(hi ? v[j + 4] : v[j]) * (hi ? sc[j + 4] : sc[j]);
                     const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(hi ? v[j] : v[j + 4]) * (hi ? sc[j] : sc[j + 4]), 8);
                     const float gate = hi ? other : own, up = hi ? own : other;
-                    if (row < n_rows && tok0 + c0 + j + (hi ? 4 : 0) < p.m) o[(size_t)j * (n_rows / 2)] = __fdividef(gate, 1.f + expf(-gate)) * up;
+                    if (row < n_rows && tok0 + c0 + j + (hi ? 4 : 0) < p.m) o[(size_t)j * (n_rows / 2)] = silu_f(gate) * up;
                 }
                 continue;
             }
