@@ -21,6 +21,12 @@ def test_quantised_models_divide_exactly():
     assert {f for f, _ in lines(r"\b__(fdividef|expf)\(")} <= {"act.cuh"}
 
 
+def test_non_coherent_loads_read_weights_and_tables():
+    """Kernels start while the one before them ends, and such a load may be moved ahead of the wait for it."""
+    table = r"__ldg\((cs|sn|src) \+|__ldg\(reinterpret_cast<const (uint4|__half|float4) \*>\((p|norm_w|p\.norm_w|emb)\b"
+    assert [s for s in lines(r"\b__ldg\(") if len(re.findall(r"\b__ldg\(", s[1])) != len(re.findall(table, s[1]))] == []
+
+
 def test_device_memory_is_filled_in_stream_order():
     """cudaMemset fills on the default stream, which the library's stream does not wait for."""
     assert lines(r"\bcudaMemset(2D|3D)?\(") == []

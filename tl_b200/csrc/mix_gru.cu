@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kGruWarps * 32) gru_scan_kernel(const MixGru m
 }
 
 template <typename TO>
-__global__ void __launch_bounds__(128) gru_rows_kernel(const MixGru m, const int *__restrict__ pos, TO *__restrict__ out, int ldo)
+__global__ void __launch_bounds__(128) gru_rows_kernel(const MixGru m, const int *pos, TO *out, int ldo)
 {
     const int c = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;
     const bool live = c < m.width;

@@ -236,7 +236,7 @@ __device__ void build_activation(const MvParams &p, MvShared *sh, uint8_t *smem,
     const int nblk = p.k / 256, n_mine = (ONE ? 1 : p.m) * nb;
     const bool norm = ONE && p.prologue == PRO_ADD_NORM, attn = ONE && p.prologue == PRO_ATTN_MERGE;
     const float *emb = nullptr;
-    if (norm && p.token) emb = p.emb_table + (size_t)__ldg(p.token) * p.k;
+    if (norm && p.token) emb = p.emb_table + (size_t)__ldcg(p.token) * p.k;
 
     float inv_rms = 0.f;
     for (int first = 0; first < n_mine || (norm && first == 0); first += ngroups * kKeep) {
