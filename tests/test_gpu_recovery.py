@@ -1,14 +1,16 @@
 """After a kernel gave up a wait: the error is reported once, and whatever it may have left in the library's scratch is gone before the
-next launch reads it.  The error word and the leftovers are put there from the host; no kernel gives anything up here."""
+next launch reads it.  The error word and the leftovers are put there from the host; no kernel gives anything up here.  And a launch
+whose CTAs do not all start at once needs no such end."""
 import ctypes as C
 import os
 import subprocess
+import time
 
 import numpy as np
 import pytest
 
 import tl_b200 as tl
-from tl_b200 import _lib, synth
+from tl_b200 import _lib, build, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -19,6 +21,55 @@ extern "C" int *error_word() { return tlb::ctx()->err_flag; }
 extern "C" unsigned long long slices(unsigned long long *bytes) { *bytes = tlb::ctx()->mv_part1_floats * 4; return (unsigned long long)tlb::ctx()->mv_part1; }
 extern "C" unsigned long long counts(unsigned long long *bytes) { *bytes = tlb::ctx()->mv_cnt_n * 4; return (unsigned long long)tlb::ctx()->mv_cnt; }
 """
+
+HOLD = r"""
+__global__ void hold(unsigned long long ns)
+{
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    do { __nanosleep(10000); asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t)); } while (t - t0 < ns);
+}
+static cudaStream_t stream;
+extern "C" int hold_all_but(int free_sms, int ms)      // one CTA an SM, by its shared memory
+{
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
+    if (!stream) cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+    cudaFuncSetAttribute(hold, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 << 10);
+    hold<<<sms - free_sms, 32, 200 << 10, stream>>>(1000000ull * ms);
+    return (int)cudaGetLastError();
+}
+extern "C" int let_go() { return (int)cudaStreamSynchronize(stream); }
+"""
+
+
+@pytest.fixture(scope="module")
+def hold(tmp_path_factory):
+    tl.init()
+    d = tmp_path_factory.mktemp("hold")
+    (d / "hold.cu").write_text(HOLD)
+    subprocess.check_call([build.NVCC, *build.FLAGS, "-shared", "-o", str(d / "hold.so"), str(d / "hold.cu")])
+    return C.CDLL(str(d / "hold.so"))
+
+
+@pytest.mark.parametrize("t,k,m", [(synth.Q4_K, 2560, 16), (synth.Q8_0, 2560, 5), (synth.Q6_K, 4096, 11), (synth.Q4_0, 8192, 8)])
+def test_few_rows_beside_a_kernel_that_holds_the_sms(hold, t, k, m):
+    """One group of tiles in 10 to 32 pieces, on six SMs: the CTAs that are there cannot wait for the others, which start when they
+    have ended.  The kernel beside them holds the other SMs for longer than any wait of the library."""
+    rng = np.random.default_rng(60 + t)
+    q = tl.QTensor.from_gguf_bytes(t, 250, k, synth.random_quant(t, 250, k, rng))
+    x = tl.Tensor.from_numpy(rng.standard_normal((m, k), dtype=np.float32))
+    want = x.matmul_quantized(q).numpy()
+    assert hold.hold_all_but(6, 1500) == 0
+    time.sleep(0.02)
+    began = time.monotonic()
+    got = [x.matmul_quantized(q) for _ in range(3)]
+    tl.sync()
+    took = time.monotonic() - began
+    assert hold.let_go() == 0
+    for g in got:
+        np.testing.assert_array_equal(g.numpy().view(np.uint32), want.view(np.uint32))
+    assert took < 1.0
 
 
 @pytest.fixture(scope="module")

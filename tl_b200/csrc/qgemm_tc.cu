@@ -758,14 +758,15 @@ __device__ __forceinline__ void unit_raw(const Q80Regs &u, int g, AFrag &f, RawS
 // The activation piece of a unit is 512 bytes per row, copied row by row to a pitch of 528 bytes; x_to_f16_kernel writes
 // these rows with the chunk index and the lane's index c exchanged inside every 64-group (order [c][j][4]), so that a lane's
 // B operands of four chunks are 32 consecutive bytes: two conflict-free 128-bit loads per 64-group and activation half.
-// A CTA works through items = 16 consecutive tiles x a range of K units; with several ranges per tile group (narrow
-// weights) the partial products go to scratch and a second launch adds them in range order.
+// The unit steps (16 consecutive tiles x one K unit) are cut evenly over the CTAs; a tile whose K range is split goes to scratch
+// in pieces, which one of its CTAs adds.
 constexpr int kRowsWarps = 16;
 constexpr int kRowsThreads = (kRowsWarps + 1) * 32;     // + the copy warp of the activations
 constexpr int kRowsWBytes = 168 * 1024;                  // weight rings of all warps: 2 to 4 stages each, by the unit's size
 constexpr int kRowsAStages = 4;                          // activation ring per CTA
 constexpr int kRowsAPitch = 528;                         // bytes between activation rows of a stage
 constexpr int kRowsABytes = 16 * kRowsAPitch;
+constexpr unsigned long long kPatience = 50000;          // ns that a fold waits for pieces before it leaves them to the late CTA
 constexpr int kRowsSumBytes = 16 * 8 * 4;                // their sums over the unit's eight 32-blocks, (high, remainder) bf16 pairs
 
 struct RowsParams {
@@ -780,6 +781,7 @@ struct RowsParams {
     const uint8_t *sums;            // [K / 256][16][8] sub-block sums of the activation rows (x_to_f16_kernel)
     float *part;                    // [CTA][2][16 tiles][16 activation rows][16 rows]: pieces of a CTA's first and last tile group where they
                                     // are split; rests at kFoldEmpty between launches
+    unsigned *left;                 // [tile group][16 tiles]: set where the fold of a split tile is left to a late CTA; rests at zero
     int *err;
 };
 
@@ -966,7 +968,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qrows_kernel(const RowsParams
         }
     };
     for (int i = 0; i < wstages && pf_pos < end; i++) issue(i);
-    pdl_wait();                                // from here on: activations, scales, residual, outputs, scratch and counters
+    pdl_wait();                                // from here on: activations, scales, residual, outputs, the scratch and its words
     pdl_launch_dependents();
 
     int g = 0, ws = 0;                         // units consumed, their weight stage
@@ -1063,27 +1065,67 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qrows_kernel(const RowsParams
     }
     // Split tiles, once the warp is through its own units: the CTAs that hold pieces of a tile group share its sixteen tiles out.
     // The scratch rests at kFoldEmpty, so a value that is not kFoldEmpty is a piece that has arrived (a 4-byte store is
-    // indivisible): the warp reads a tile's pieces, kFold at a time, again while some are missing (bounded), adds them in CTA
-    // order, puts kFoldEmpty back and writes the rows.  What bounds a narrow launch is this tail of latencies: with a fence, a count
-    // and another fence per piece, the last arriver adding, 4096 x 4096 with 16 rows took 19.2 us in Q4_K (now 18.5), 14336 x 4096
-    // 26.1 (24.0), 5120 x 5120 with 5 rows in Q8_0 16.9 (13.9), eight steps of 16 sequences 5.17 ms (4.62).
-    for (int part = 0; part < 2 && ok; part++) {
-        const int tgs = part == 0 ? tg_first : (end - 1) / upt;
-        if (part == 1 && tgs == tg_first) break;
-        // the CTA of unit step x is the last one whose range starts at or before x
-        const int64_t x0 = (int64_t)tgs * upt, x1 = x0 + upt - 1;
-        const int b_lo = (int)(((x0 + 1) * gridDim.x - 1) / p.total), np = (int)(((x1 + 1) * gridDim.x - 1) / p.total) - b_lo + 1;
+    // indivisible): the warp reads a tile's pieces, kFold at a time, again while some are missing, adds them in CTA
+    // order, puts kFoldEmpty back and writes the rows.
+    // It waits kPatience at most, since a CTA may start late: a kernel of another stream can hold its SM for as long as it likes.
+    // Then it leaves the tile to whoever is late: what it has added becomes the piece before the first missing one, and the tile's
+    // word, zero otherwise, that one's number plus one.  Whoever has written a piece looks at the word, and whoever has set it at the
+    // pieces, with a fence between both steps: the last of them finds the word set and the pieces there, takes the word and goes on.
+    // What bounds a narrow launch is this tail of latencies.  Calls in microseconds - 4096 x 4096 and 14336 x 4096 with 16 rows in Q4_K,
+    // 5120 x 5120 with 5 in Q8_0 - and eight steps of 16 sequences in ms: 13.8, 24.0, 15.3, 4.61; without the way out for late CTAs
+    // 13.1, 23.7, 14.8, 4.57; all pieces counted at the end, the last arriver adding 14.9, 23.3, 15.9, 4.77.
+    const int tg_last = (end - 1) / upt, tg_mine = lane ? tg_last : tg_first;
+    // lanes 0 and 1: the warp's tile of the first and the last tile group; the CTA of unit step x is the last one whose range starts at or before x
+    int b_lo = 0, np = 1;
+    if (ok && (lane == 0 || (lane == 1 && tg_last != tg_first))) {
+        int wi, tile16;
+        bool have;
+        tile_of(tg_mine, wi, tile16, have);
+        const int64_t x0 = (int64_t)tg_mine * upt, x1 = x0 + upt - 1;
+        b_lo = (int)(((x0 + 1) * gridDim.x - 1) / p.total);
+        if (have) np = (int)(((x1 + 1) * gridDim.x - 1) / p.total) - b_lo + 1;
+    }
+    const unsigned split = __ballot_sync(0xffffffffu, np > 1), owned = __ballot_sync(0xffffffffu, np > 1 && (int)blockIdx.x == b_lo + warp % np);
+    unsigned word = 0u, watched = split & ~owned;
+    if (watched) {
+        __threadfence();                   // this warp's pieces before the look at their tiles' words
+        __syncwarp();
+        if ((watched >> lane) & 1u) word = ld_volatile_u32(p.left + tg_mine * kRowsWarps + warp);
+    }
+    for (int step = 0; step < 4; step++) {
+        const int part = step & 1;
+        if (step == 2) {
+            watched = __ballot_sync(0xffffffffu, word != 0u);
+            if (!watched) break;
+        }
+        if (!(((step < 2 ? owned : watched) >> part) & 1u)) continue;
+        const int tgs = part ? tg_last : tg_first, blo = __shfl_sync(0xffffffffu, b_lo, part), pieces = __shfl_sync(0xffffffffu, np, part);
+        unsigned *const left = p.left + tgs * kRowsWarps + warp;
         int wi, tile16;
         bool have;
         tile_of(tgs, wi, tile16, have);
-        if (np == 1 || !have || (int)blockIdx.x != b_lo + warp % np) continue;
         // in the first CTA of several the group is its last one, unless that is also its first; in the others it is their first
-        const bool lo_first = (int)((int64_t)p.total * b_lo / gridDim.x) / upt == tgs;
+        const bool lo_first = (int)((int64_t)p.total * blo / gridDim.x) / upt == tgs;
         const size_t cta_stride = (size_t)2 * kRowsWarps * 256;
-        float *const src0 = p.part + (size_t)b_lo * cta_stride + (size_t)warp * 256 + lane * 4;
+        float *const src0 = p.part + (size_t)blo * cta_stride + (size_t)warp * 256 + lane * 4;
         auto piece = [&](int q, int i) { return src0 + q * cta_stride + (q == 0 && !lo_first ? (size_t)kRowsWarps * 256 : 0) + 128 * i; };
+        auto mine = [&](int i) { return (lane >> 2) + 8 * i < p.m; };
+        auto missing = [&](const uint4 &v) { return v.x == kFoldEmpty || v.y == kFoldEmpty || v.z == kFoldEmpty || v.w == kFoldEmpty; };
+        int from = 0;
+        if (step >= 2) {                   // left by its owner: taken, if all is there
+            from = (int)__shfl_sync(0xffffffffu, word, part) - 1;
+            bool all = true;
+            for (int q = from; q < pieces; q++)
+#pragma unroll
+                for (int i = 0; i < NT; i++) all = all && !(mine(i) && missing(ld_volatile_u4(piece(q, i))));
+            if (!__all_sync(0xffffffffu, all)) continue;
+            unsigned took = 0u;
+            if (lane == 0) took = atomicExch(left, 0u);
+            if (!__shfl_sync(0xffffffffu, took, 0)) continue;
+            __threadfence();
+        }
         // item lane + 32 i: four weight rows of one activation row
-        constexpr int kFold = 3;
+        constexpr int kFold = FMT == 14 && NT == 2 ? 2 : 3;      // three at a time spill 28 bytes there: 4096 x 14336 29.4 us, with two 28.7
         const int n = p.n[wi], row = tile16 * 16 + 4 * (lane & 3);
         float4 sum[NT], res[NT];
         float inv[NT];
@@ -1091,6 +1133,10 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qrows_kernel(const RowsParams
         for (int i = 0; i < NT; i++) {
             const int tok = (lane >> 2) + 8 * i;
             sum[i] = res[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (from && mine(i)) {
+                sum[i] = __ldcg(reinterpret_cast<const float4 *>(piece(from - 1, i)));
+                *reinterpret_cast<uint4 *>(piece(from - 1, i)) = make_uint4(kFoldEmpty, kFoldEmpty, kFoldEmpty, kFoldEmpty);
+            }
             inv[i] = tok < p.m ? __ldcg(p.inv_scale + tok) : 0.f;
             if (p.resid && tok < p.m) {
                 const float *rp = p.resid + (size_t)tok * n + row;
@@ -1100,9 +1146,10 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qrows_kernel(const RowsParams
                 if (row + 3 < n) res[i].w = __ldcg(rp + 3);
             }
         }
-        for (int q0 = 0; q0 < np && ok; q0 += kFold) {
+        int q0 = from;
+        for (; q0 < pieces; q0 += kFold) {
             uint4 v[kFold][NT];
-            auto wanted = [&](int q, int i) { return q0 + q < np && (lane >> 2) + 8 * i < p.m; };
+            auto wanted = [&](int q, int i) { return q0 + q < pieces && mine(i); };
 #pragma unroll
             for (int q = 0; q < kFold; q++)
 #pragma unroll
@@ -1115,22 +1162,18 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qrows_kernel(const RowsParams
                 for (int q = 0; q < kFold; q++)
 #pragma unroll
                     for (int i = 0; i < NT; i++)
-                        if (v[q][i].x == kFoldEmpty || v[q][i].y == kFoldEmpty || v[q][i].z == kFoldEmpty || v[q][i].w == kFoldEmpty) {
+                        if (missing(v[q][i])) {
                             v[q][i] = ld_volatile_u4(piece(q0 + q, i));
                             all = false;
                         }
                 if (all) break;
-                if ((it & 255) == 255) {
+                if ((it & 31) == 31) {
                     const unsigned long long t = global_ns();
                     if (!t0) t0 = t;
-                    if (t - t0 > 1000000000ull) { got = false; break; }
+                    if (t - t0 > kPatience) { got = false; break; }
                 }
             }
-            if (!__all_sync(0xffffffffu, got)) {
-                if (lane == 0) atomicExch(p.err, 54);
-                ok = false;
-                break;
-            }
+            if (!__all_sync(0xffffffffu, got)) break;
 #pragma unroll
             for (int q = 0; q < kFold; q++)
 #pragma unroll
@@ -1141,7 +1184,20 @@ __global__ void __launch_bounds__(kRowsThreads, 1) qrows_kernel(const RowsParams
                     *reinterpret_cast<uint4 *>(piece(q0 + q, i)) = make_uint4(kFoldEmpty, kFoldEmpty, kFoldEmpty, kFoldEmpty);
                 }
         }
-        if (!ok) break;
+        if (q0 < pieces) {                 // left to whoever is late, this warp among them
+#pragma unroll
+            for (int i = 0; i < NT; i++)
+                if (q0 && mine(i)) __stcg(reinterpret_cast<float4 *>(piece(q0 - 1, i)), sum[i]);
+            __threadfence();
+            __syncwarp();
+            if (lane == part) {
+                word = (unsigned)q0 + 1u;
+                atomicExch(left, word);
+            }
+            __threadfence();
+            __syncwarp();
+            continue;
+        }
 #pragma unroll
         for (int i = 0; i < NT; i++) {
             const int tok = (lane >> 2) + 8 * i;
@@ -1537,6 +1593,7 @@ tlb_status qrows_run(const tlb_qtensor *const *ws, int n_w, const GemmAct &a, fl
     p.err = c->err_flag;
     if ((size_t)tgroups * kRowsWarps > c->mv_cnt_n || (size_t)grid * 2 * kRowsWarps * 256 > c->mv_part1_floats) return fail(TLB_ERR_SHAPE, "quantized matmul (few rows): more tiles than the context's scratch");
     p.part = c->mv_part1;           // at rest at kFoldEmpty, as the one-row matvec's slices
+    p.left = (unsigned *)c->mv_cnt;
     p.k = a.k;
     p.xh = (const __half *)a.xh->ptr;
     const size_t smem = (size_t)kRowsAStages * (kRowsABytes + kRowsSumBytes) + (size_t)kRowsWarps * p.wstages * p.stage_w + 8 * (2 * kRowsAStages + kRowsWarps * p.wstages) + 128 + 64;
