@@ -63,6 +63,35 @@ def test_batch_decode_matches_per_sequence_oracles(orc, linear, head, kv_f16, ba
     assert len(hist) == 12
 
 
+def test_the_largest_batch():
+    """64 sequences, as many as a session holds, at positions of their own: each against a session of its own, and the same tokens step
+    by step as in one call."""
+    tens = synth.llama_tensors(SMALL, 44, synth.Q4_K, synth.Q6_K)
+    wmap = tl.map_from_tensors(tens)
+    rng = np.random.default_rng(45)
+    prompts = [[int(t) for t in rng.integers(0, SMALL["vocab"], n)] for n in rng.integers(2, 40, 64)]
+    runs = []
+    for _ in range(2):
+        dec = tl.Decoder(SMALL, wmap, kv_f16=True, max_seq=64, batch=64)
+        runs.append((dec, [dec.prefill_seq(b, p) for b, p in enumerate(prompts)]))
+    (dec, first), (whole, again) = runs
+    assert first == again
+    toks, pos, hist = list(first), [len(p) for p in prompts], []
+    for step in range(5):
+        nxt = dec.step_batch(toks, pos)
+        lg = dec.logits_batch()
+        assert list(nxt) == [int(np.flatnonzero(row == row.max())[-1]) for row in lg]
+        if step == 0:
+            for b in range(64):
+                one = tl.Decoder(SMALL, wmap, kv_f16=True, max_seq=64)
+                one.prefill(prompts[b])
+                one.step(toks[b], pos[b])
+                assert relerr(lg[b], one.logits()) < LOGIT_TOL, b
+        toks, pos = list(nxt), [p + 1 for p in pos]
+        hist.append(list(nxt))
+    assert np.array_equal(np.array(hist), np.array(whole.generate_batch(first, [len(p) for p in prompts], 5)).reshape(5, 64))
+
+
 WIDE = dict(n_layers=1, d_model=1024, n_heads=8, n_kv_heads=2, head_dim=128, ffn=1024, vocab=512,
             eps=1e-5, rope_base=500000.0, attn_scale=0.08839)
 

@@ -288,6 +288,20 @@ def test_prefill_pair_of_ctas_straddles_weights():
             assert np.linalg.norm(lg - ref) < 2e-3 * np.linalg.norm(ref), off + w
 
 
+def test_logits_of_many_prompt_tokens_in_any_order():
+    """150 of 170 tokens, more than one list of rows holds, shuffled and some twice: each row where it was asked for.  Rows that share
+    a product in other company round their operands alike; few of them at once take the kernel for few rows."""
+    tens = synth.llama_tensors(SMALL, 33, synth.Q8_0, synth.Q8_0, scale_sigma=0.002)
+    rng = np.random.default_rng(34)
+    toks = [int(v) for v in rng.permutation(SMALL["vocab"])[:170]]
+    dec = tl.Decoder(SMALL, tl.map_from_tensors(tens), kv_f16=True, max_seq=256)
+    whole = dec.prefill_logits(toks, 0)
+    for want in (rng.permutation(170)[:150], np.concatenate([rng.permutation(170)[:80], [5, 5, 169]]), np.arange(169, -1, -1), [3, 4, 5, 2, 1, 0, 7]):
+        got = dec.prefill_logits(toks, 0, want=[int(w) for w in want])
+        assert np.max(np.linalg.norm(got - whole[want], axis=1) / np.linalg.norm(whole[want], axis=1)) < 2e-3
+    assert np.min(np.linalg.norm(whole[1:] - whole[:-1], axis=1) / np.linalg.norm(whole[1:], axis=1)) > 1e-2        # neighbours are told apart
+
+
 def test_prefill_f32_cache_head_dim_128():
     """f32 KV cache with head_dim 128 (the tile conversion path of the prompt attention): prompt in one call against
     the same session fed token by token."""

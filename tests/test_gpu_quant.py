@@ -9,7 +9,7 @@ import pytest
 
 import tl_b200 as tl
 from tl_b200 import _lib, synth
-from test_launch_plans_cpu import gemm_form, gemm_plan, gemm_ranges
+from test_launch_plans_cpu import gemm_dispatch, gemm_plan, gemm_ranges
 
 pytestmark = pytest.mark.gpu
 
@@ -262,13 +262,14 @@ def test_qgemm_pairs_of_ctas(orc, t, n, k, m):
 
 
 @pytest.mark.parametrize("t", TYPES)
-@pytest.mark.parametrize("n,k,m,plan", [(9530, 2048, 257, (320, 1)), (9530, 2304, 333, (384, 1)), (11170, 2048, 384, (384, 1)), (6000, 2048, 777, (320, 1)),
-                                        (5000, 2304, 1100, (384, 1)), (5940, 8192, 257, (320, 3)), (5000, 8192, 333, (384, 3))])
-def test_qgemm_wide_tiles_by_pairs(orc, t, n, k, m, plan):
+@pytest.mark.parametrize("n,k,m,plan,cluster", [(9530, 2048, 257, (320, 1), False), (9530, 2304, 333, (384, 1), False), (11170, 2048, 384, (384, 1), False),
+                                                (6000, 2048, 777, (320, 1), False), (5000, 2304, 1100, (384, 1), False), (5940, 8192, 257, (320, 2), True),
+                                                (5000, 8192, 333, (384, 3), True), (3180, 13312, 257, (320, 5), False), (2420, 20480, 333, (384, 7), False)])
+def test_qgemm_wide_tiles_by_pairs(orc, t, n, k, m, plan, cluster):
     """Tiles of 320 and 384 rows by pairs of CTAs, two accumulators: K longer than the activation ring (8 or 9 steps of 64), an
-    odd number of row tiles (9530, 5940) and a ragged last one, token tiles that end inside either CTA's part of either
-    accumulator or leave it empty, and K ranges of unequal length."""
-    assert gemm_plan(m, n, k) == plan
+    odd number of row tiles (9530, 5940, 3180, 2420) and a ragged last one, token tiles that end inside either CTA's part of either
+    accumulator or leave it empty, and K ranges of unequal length, in a cluster and through scratch."""
+    assert gemm_dispatch(m, n, k) == plan + (True, cluster)
     rng = np.random.default_rng(5500 + t + n + m)
     w = synth.random_quant(t, n, k, rng)
     x = rng.standard_normal((m, k), dtype=np.float32)
@@ -283,12 +284,14 @@ def test_qgemm_wide_tiles_by_pairs(orc, t, n, k, m, plan):
         assert relerr(got[i], ref[i]) < GEMM_TOL, i
 
 
-@pytest.mark.parametrize("t,n,k,m,form", [(synth.Q4_K, 14200, 4096, 500, (256, 1, True)), (synth.Q8_0, 4000, 14336, 512, (256, 2, True)), (synth.Q6_K, 10100, 8192, 512, (192, 1, True)),
-                                          (synth.Q4_0, 15000, 4096, 512, (256, 1, True))])
+@pytest.mark.parametrize("t,n,k,m,form", [(synth.Q4_K, 14200, 4096, 500, (256, 2, False, True)), (synth.Q8_0, 4000, 14336, 512, (256, 2, False, True)),
+                                          (synth.Q6_K, 10100, 8192, 512, (256, 2, False, True)), (synth.Q4_0, 15000, 4096, 512, (256, 1, True, False)),
+                                          (synth.Q4_K, 9530, 4096, 700, (256, 1, True, False)), (synth.Q6_K, 4200, 8192, 777, (224, 1, True, False)),
+                                          (synth.Q8_0, 2880, 28672, 500, (256, 3, True, False)), (synth.Q6_K, 2220, 28672, 400, (224, 4, True, False))])
 def test_qgemm_large_launches_by_pairs(t, n, k, m, form):
-    """Tiles of up to 256 rows by pairs: odd numbers of row tiles, ragged last ones and token tiles, two K ranges.  Sampled weight
-    rows, every activation row."""
-    assert gemm_form(m, n, k) == form
+    """Large launches: two K ranges in a cluster; tiles of up to 256 rows by pairs, every format, odd numbers of row tiles, ragged last
+    ones and token tiles; the same with three and four K ranges through scratch.  Sampled weight rows, every activation row."""
+    assert gemm_dispatch(m, n, k) == form
     rng = np.random.default_rng(5600 + t)
     q = tl.QTensor.from_gguf_bytes(t, n, k, synth.random_quant(t, n, k, rng))
     x = rng.standard_normal((m, k), dtype=np.float32)
@@ -418,12 +421,12 @@ def test_mid_row_counts_on_a_wide_weight(orc):
 
 
 @pytest.mark.parametrize("t", TYPES)
-@pytest.mark.parametrize("n,k", [(1000, 512), (4100, 1024), (272, 2304)])
+@pytest.mark.parametrize("n,k", [(1000, 512), (4100, 1024), (272, 2304), (256, 8192)])
 def test_few_rows_kernel_shapes(orc, t, n, k):
     """5 to 16 rows stream through the few-rows kernel: the unit steps (16-tile group x 256-wide unit) are cut evenly over
-    the CTAs, so tile groups are split between CTAs at arbitrary units and summed by a second launch.  1000 rows: a last
-    tile of 8 rows; 4100: a last tile group of one tile; 272 x 2304: 9 units over two tile groups.  Whole result against
-    the oracle, one row 50 times larger than the rest (per-row activation scale)."""
+    the CTAs, so tile groups are split between CTAs at arbitrary units, and one of a tile's CTAs adds its pieces.  1000 rows: a last
+    tile of 8 rows; 4100: a last tile group of one tile; 272 x 2304: 9 units over two tile groups; 256 x 8192: 32 pieces a tile, more
+    than the sixteen warps that fold.  Whole result against the oracle, one row 50 times larger than the rest (per-row activation scale)."""
     rng = np.random.default_rng(7000 + t + n)
     w = synth.random_quant(t, n, k, rng)
     q = tl.QTensor.from_gguf_bytes(t, n, k, w)

@@ -14,7 +14,7 @@ import layered_session as S
 import plain_rukedra as P
 import tl_b200 as tl
 from layered_session import decode, err, greedy, run_portions, toks
-from test_launch_plans_cpu import dense_matvec_plan
+from test_launch_plans_cpu import dense_gemm_ranges, dense_matvec_plan
 from tl_b200 import synth
 
 pytestmark = pytest.mark.gpu
@@ -196,6 +196,25 @@ def test_decoding_with_norms_of_whole_runs(width, groups, ff, shared, f32):
     m = Model(config([(direct(), moe(8, 3, ff, None, 1.3, shared)), (gru(), dense())], width=width, groups=groups), seed=31)
     t, want = m.sure(6)
     assert close(decode(m.dec(f32), t, 0), want, f32)
+
+
+@pytest.mark.parametrize("width,ff,tokens,ranges", [(1100, 610, 140, 2), (1600, 333, 100, 3), (2050, 400, 33, 4)])
+def test_gated_prompt_products_in_ranges(width, ff, tokens, ranges):
+    """The activation of gate and up behind K ranges of one cluster, two to four and of unequal length; a ragged last tile of rows and of tokens."""
+    assert dense_gemm_ranges(tokens, 2 * ff, width, gated=True) == ranges
+    m = Model(config([(gru(20), dense(ff))], width=width, groups=1), seed=13)
+    t = toks(tokens)
+    assert close(m.dec(False, max_seq=tokens).prefill_logits(t), m.ref(t), False)
+
+
+@pytest.mark.parametrize("kv_rank,tokens", [(1024, 140), (970, 70), (1000, 300), (1024, 45)])
+def test_expanded_latents_in_ranges(kv_rank, tokens):
+    """Keys (f16) and values (f16, transposed for tcgen05 and, of 45 tokens, in rows for mma.sync) of two heads, expanded from long latents
+    in two K ranges."""
+    assert dense_gemm_ranges(tokens, 256, kv_rank) == dense_gemm_ranges(tokens, 256, kv_rank, transposed=True) == 2
+    m = Model(config([(direct(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=kv_rank, scale=0.07), None)]), seed=14)
+    t = toks(tokens)
+    assert close(m.dec(False, max_seq=tokens).prefill_logits(t), m.ref(t), False)
 
 
 def test_the_gate_and_the_norms_matter():

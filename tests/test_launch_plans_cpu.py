@@ -35,10 +35,10 @@ def test_matvec_rows_that_go_in_smaller_groups():
 
 
 def test_chains_of_short_launches_as_measured():
-    """Eight warps a CTA where a decode layer was faster with them: rows of 2048 or less, launches of up to 80 units per SM."""
+    """Eight warps a CTA where a decode layer was faster with them: rows of 2048 or less, launches of up to 140 units per SM."""
     f = _lib.lib().tlb_matvec_few
     f.restype, f.argtypes = C.c_int, [C.c_int64, C.c_int64, C.c_int]
-    for d_model, units, few in [(1024, 14, 1), (1536, 21, 1), (2048, 38, 1), (2048, 76, 1), (2048, 194, 0), (2304, 35, 0), (2560, 35, 0), (3072, 83, 0), (4096, 28, 0), (4096, 38, 0)]:
+    for d_model, units, few in [(1024, 14, 1), (1536, 21, 1), (2048, 38, 1), (2048, 76, 1), (2048, 138, 1), (2048, 194, 0), (2304, 35, 0), (2560, 35, 0), (3072, 83, 0), (4096, 28, 0), (4096, 38, 0)]:
         assert f(d_model, units * SMS, SMS) == few, (d_model, units)
     # gate|up of width 1536 (31.9 us a layer unsliced, 34.8 in two slices), down of width 2048 (sliced: 34.8, unsliced: 39)
     assert matvec_slices(synth.Q4_K, 2 * 4096, 1536, 1, few=1) == 1
@@ -65,6 +65,12 @@ def gemm_ranges(m, n, k):
     nt, splits, pair = C.c_int(), C.c_int(), C.c_int()
     found = f(m, (n + 127) // 128, k // 256, n, SMS, C.byref(nt), C.byref(splits), C.byref(pair))
     return (nt.value, splits.value, bool(pair.value)) if found else None
+
+
+def gemm_dispatch(m, n, k):
+    """(rows of a tile, K ranges, by pairs, ranges in one cluster): the form that a product of more than 16 rows runs in"""
+    ranges = gemm_ranges(m, n, k)
+    return (ranges or gemm_form(m, n, k)) + (ranges is not None,)
 
 
 def test_gemm_ranges_are_launchable():
@@ -127,11 +133,11 @@ def dense_matvec_plan(n, k, slots=1):
     return depth, chunks.value, rounds.value
 
 
-def dense_gemm_ranges(T, n, k):
-    """K ranges of a bf16 product without gates or experts, as launch_dense_gemm asks for them"""
+def dense_gemm_ranges(T, n, k, gated=False, transposed=False):
+    """K ranges of a 16-bit product without experts (n: weight rows, gates and ups both), as launch_dense_gemm asks for them"""
     kt = (k + 63) // 64
-    two = kt <= 16                                       # CTAs share an SM
-    nt = min(128 if two else 256, (T + 31) // 32 * 32)
+    two = kt <= 16 or gated                              # CTAs share an SM
+    nt = 128 if transposed else min(128 if two else 256, (T + 31) // 32 * 32)
     stages = min(8, (104 if two else 216) * 1024 // (16384 + nt * 128))
     f = _lib.lib().tlb_dense_gemm_ranges
     f.restype, f.argtypes = C.c_int, [C.c_int] * 7
@@ -144,8 +150,9 @@ def test_dense_gemm_ranges_are_launchable():
     for k in (64, 512, 1024, 1100, 2048, 5632, 14336):
         for n in (128, 1000, 2048, 3072, 5632, 10368, 32768):
             for T in (1, 17, 32, 33, 64, 100, 128, 250, 256, 512, 800, 2048):
-                s = dense_gemm_ranges(T, n, k)
-                assert s in (1, 2, 3, 4) and (s == 1 or (k + 63) // 64 >= 8 * s), (T, n, k)
+                for form in ({}, {"gated": True}, {"transposed": True}):
+                    s = dense_gemm_ranges(T, n, k, **form)
+                    assert s in (1, 2, 3, 4) and (s == 1 or (k + 63) // 64 >= 8 * s), (T, n, k)
 
 
 def test_dense_matvec_rings_fit():

@@ -110,7 +110,7 @@ constexpr int kArgmaxBlocks = 148;
 constexpr int kMaxBatch = 64;      // sequences of a session
 
 // argmax over the logits + advance of the decode state, in one launch.  Tie rule as tlb_argmax.
-__global__ void argmax_advance_kernel(const float *__restrict__ x, int n, int tie_first, float *pv, long long *pi, int *counter,
+__global__ void argmax_advance_kernel(const float *x, int n, int tie_first, float *pv, long long *pi, int *counter,
                                       int *state, int *tokens_out, int tokens_cap, int use_pdl)
 {
     if (use_pdl) {
