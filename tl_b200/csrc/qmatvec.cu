@@ -333,33 +333,31 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
         // go to this warp's slot in shared memory (local mode) or to the item's slot of the slice scratch.
         float *part = local ? segbuf + ((size_t)warp * p.max_seg + seg) * (16 * M)
                             : p.part + ((size_t)ir.slice * p.tiles + ir.tile) * (16 * M);
-        for (int mi = 0; mi < M; mi++) {
-            float v0, v1;                                                   // rows r, r + 8
-            if (ONE) {
-                // The first levels of the two sub-blocks (columns 0 and 4: c == 0 and 2) meet first and the other levels, 1 / 254 of
-                // them, among themselves: two roundings of the size of the result, as with one accumulator.  Sub-block by sub-block
-                // it is three: 2048 x 4096 Q4_K 1.48e-7 of the result off instead of 1.44e-7.
-                const bool lead = !(L.c & 1);
-                auto fold = [&](float a, float b) {
-                    float big = lead ? a : 0.f, rest = lead ? b : a + b;
-                    big += __shfl_xor_sync(0xffffffffu, big, 2);
-                    rest += __shfl_xor_sync(0xffffffffu, rest, 2); rest += __shfl_xor_sync(0xffffffffu, rest, 1);
-                    return big + rest;
-                };
-                v0 = fold(master[0], master[1]);
-                v1 = fold(master[2], master[3]);
-            } else {
+        if constexpr (ONE) {
+            // The first levels of the two sub-blocks (columns 0 and 4: c == 0 and 2) meet first and the other levels, 1 / 254 of
+            // them, among themselves: two roundings of the size of the result, as with one accumulator.  Sub-block by sub-block
+            // it is three: 2048 x 4096 Q4_K 1.48e-7 of the result off instead of 1.44e-7.  Even lanes take row r, odd ones row r + 8.
+            const bool odd = L.c & 1;
+            const float x1 = __shfl_xor_sync(0xffffffffu, odd ? master[0] + master[1] : master[2], 1), x2 = __shfl_xor_sync(0xffffffffu, master[3], 1);
+            float big = odd ? x1 : master[0], rest = odd ? (master[2] + master[3]) + x2 : master[1] + x1;
+            big += __shfl_xor_sync(0xffffffffu, big, 2);
+            rest += __shfl_xor_sync(0xffffffffu, rest, 2);
+            float v = big + rest;
+            if (FMT == TLB_GGML_Q4_K) v -= odd ? mm[2] + mm[3] : mm[0] + mm[1];      // columns 2c, 2c + 1 have the same two terms for every c
+            if (L.c < 2) part[L.r + (odd ? 8 : 0)] = v;
+        } else {
+            for (int mi = 0; mi < M; mi++) {
                 const int lo = mi * NL, hi = lo + NL, cA = 2 * L.c, cB = 2 * L.c + 1;
                 const bool inA = cA >= lo && cA < hi, inB = cB >= lo && cB < hi;
-                v0 = (inA ? master[0] : 0.f) + (inB ? master[1] : 0.f);
-                v1 = (inA ? master[2] : 0.f) + (inB ? master[3] : 0.f);
+                float v0 = (inA ? master[0] : 0.f) + (inB ? master[1] : 0.f);   // row r
+                float v1 = (inA ? master[2] : 0.f) + (inB ? master[3] : 0.f);   // row r + 8
                 v0 += __shfl_xor_sync(0xffffffffu, v0, 1); v0 += __shfl_xor_sync(0xffffffffu, v0, 2);
                 v1 += __shfl_xor_sync(0xffffffffu, v1, 1); v1 += __shfl_xor_sync(0xffffffffu, v1, 2);
-            }
-            if (L.c == mi) {
-                if (FMT == TLB_GGML_Q4_K) { v0 -= mm[0] + mm[1]; v1 -= mm[2] + mm[3]; }
-                part[mi * 16 + L.r] = v0;
-                part[mi * 16 + L.r + 8] = v1;
+                if (L.c == mi) {
+                    if (FMT == TLB_GGML_Q4_K) { v0 -= mm[0] + mm[1]; v1 -= mm[2] + mm[3]; }
+                    part[mi * 16 + L.r] = v0;
+                    part[mi * 16 + L.r + 8] = v1;
+                }
             }
         }
         seg++;
@@ -623,9 +621,9 @@ static double slice_cost(int type, int m, int64_t tiles, int upt, int upi, int s
 }
 
 // Warps of a CTA.  A short launch is bounded by the instructions a warp issues outside its units, and eight warps issue half
-// of them; with one unit or less for each of eight warps the other eight only issue the prologue again: four calls of
-// 2048 x 2048 with norms between them take 49.2 us with sixteen and 46 with eight.  From two units per warp on, a lone launch
-// is faster with sixteen (2048 x 5632: 9.8 against 12.5 us).
+// of them; with one unit or less for each of eight warps the other eight only issue the prologue again.  Calls back to back in Q4_K
+// with sixteen and with eight: 2048 x 2048 5.2 and 5.0 us, 1024 x 1024 5.1 and 4.8.  From two units per warp on, a lone launch
+// is faster with sixteen (2048 x 5632: 5.9 and 6.1, 14336 x 4096: 10.9 and 12.6).
 static int warps_for(const MatvecJob &job, int64_t tiles, int upt, int sm_count)
 {
     return job.m == 1 && (job.few || ((job.lone || !job.pdl) && tiles * upt <= (int64_t)kFewWarps * sm_count)) ? kFewWarps : kWarps;
