@@ -31,11 +31,11 @@ struct Context {
     void *flush_buf = nullptr;
     size_t flush_bytes = 0;
     int *err_flag = nullptr;  // device word set by kernels whose bounded waits ran out
-    // scratch of the streaming matvec (launches are ordered on `stream`, so one set serves all):
-    // partial results per K-slice, and per-tile counts of finished slices (zero between launches)
+    // scratch of the streaming kernels (launches are ordered on `stream`, so one set serves all):
+    // partial results per K-slice, and a word per tile (counts of finished slices, folds left to a late CTA; zero between launches)
     float *mv_part = nullptr;
     size_t mv_part_floats = 0;
-    float *mv_part1 = nullptr;       // one activation row: slice scratch that rests at a sentinel bit pattern between launches
+    float *mv_part1 = nullptr;       // one activation row, and 5 to 16: slices and pieces, at rest at a sentinel bit pattern between launches
     size_t mv_part1_floats = 0;
     int *mv_cnt = nullptr;
     size_t mv_cnt_n = 0;
