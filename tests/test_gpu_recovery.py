@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 import tl_b200 as tl
+from test_launch_plans_cpu import matvec_slices
 from tl_b200 import _lib, build, synth
 
 pytestmark = pytest.mark.gpu
@@ -52,15 +53,19 @@ def hold(tmp_path_factory):
     return C.CDLL(str(d / "hold.so"))
 
 
-@pytest.mark.parametrize("t,k,m", [(synth.Q4_K, 2560, 16), (synth.Q8_0, 2560, 5), (synth.Q6_K, 4096, 11), (synth.Q4_0, 8192, 8)])
-def test_few_rows_beside_a_kernel_that_holds_the_sms(hold, t, k, m):
-    """One group of tiles in 10 to 32 pieces, on six SMs: the CTAs that are there cannot wait for the others, which start when they
-    have ended.  The kernel beside them holds the other SMs for longer than any wait of the library."""
+@pytest.mark.parametrize("t,n,k,m,sms", [(synth.Q4_K, 250, 2560, 16, 6), (synth.Q8_0, 250, 2560, 5, 6), (synth.Q6_K, 250, 4096, 11, 6), (synth.Q4_0, 250, 8192, 8, 6),
+                                         (synth.Q4_K, 2048, 2048, 1, 40), (synth.Q8_0, 2040, 5632, 1, 6), (synth.Q6_K, 4096, 4096, 1, 3), (synth.Q4_0, 4096, 14336, 1, 100),
+                                         (synth.Q4_K, 2048, 4096, 3, 6), (synth.Q8_0, 2048, 2048, 100, 12)])
+def test_beside_a_kernel_that_holds_the_sms(hold, t, n, k, m, sms):
+    """On a few SMs the CTAs that are there cannot wait for the others, which start when they have ended: 5 to 16 rows with one group of
+    tiles in 10 to 32 pieces, one row in K slices, the forms for other rows.  The kernel beside them holds the other SMs for longer
+    than any wait of the library."""
+    assert m != 1 or matvec_slices(t, n, k, 1) > 1
     rng = np.random.default_rng(60 + t)
-    q = tl.QTensor.from_gguf_bytes(t, 250, k, synth.random_quant(t, 250, k, rng))
+    q = tl.QTensor.from_gguf_bytes(t, n, k, synth.random_quant(t, n, k, rng))
     x = tl.Tensor.from_numpy(rng.standard_normal((m, k), dtype=np.float32))
     want = x.matmul_quantized(q).numpy()
-    assert hold.hold_all_but(6, 1500) == 0
+    assert hold.hold_all_but(sms, 1500) == 0
     time.sleep(0.02)
     began = time.monotonic()
     got = [x.matmul_quantized(q) for _ in range(3)]

@@ -424,63 +424,79 @@ __global__ void __launch_bounds__(NW * 32, 1) qmatvec_kernel(const __grid_consta
                 }
             }
         }
-    } else if (ONE && ok && p.fold_poll) {
+    } else if (ONE && ok && wu1 > wu0 && p.fold_poll) {
         // One activation row.  The slice scratch rests at kFoldEmpty between launches, so a value that is not kFoldEmpty is
         // a slice that has arrived: one warp per tile reads the tile's slices (all requested at once, re-read while some are
         // missing; bounded), adds them in slice order, puts kFoldEmpty back and writes the rows.  No fence, counter or atomic:
         // a 4-byte store is indivisible, and the next launch starts after this one is over.
-        // Tiles are dealt to the CTAs one by one, whoever streamed them: their slice 0 lies in the first tenth of the CTAs, where
-        // a warp took over a microsecond for each of two tiles (TinyLlama's ffn_down: 3.1 us from the last unit to the end of the
-        // launch, 1.5 dealt out).  A CTA's last warp begins, since it is never without units: a warp that polls from the start
-        // slows the stores of the slices down (four calls of 2048 x 2048: 48.2 us, 44.1 by the last warp, 46.1 before).
+        // The warp is the one with the tile's last slice, so that CTAs wait for those with lower numbers alone, which start first: a
+        // launch gets through on whatever SMs other streams leave it (dealt to all CTAs, the tiles of a launch on 40 SMs waited for
+        // slices whose CTAs could not start).  Two of its tiles go at once, one in either half of the warp, and the loops are as long as
+        // the slices are many: what bounds the end of a launch here is the instructions of the warps that fold, all sixteen of an SM at a
+        // time.  Eight Llama-3-8B layers and head, 16 tokens: 7.58 ms, 7.81 tile by tile in loops of 16, 7.68 dealt to all CTAs; TinyLlama
+        // shapes, 32 tokens: 20.76, 20.89, 20.60.
         const size_t sstride = (size_t)p.tiles * 16;
-        for (int tile = b + (NW - 1 - warp) * (int)gridDim.x; tile < p.tiles; tile += NW * (int)gridDim.x) {
-            ItemCursor cf;
-            cf.slice = 0;
-            cf.tile = tile;
-            const ItemRef fr = item_ref(p, cf);
-            const float res = residual(fr);
-            float *src = p.part + (size_t)fr.tile * 16 + (lane & 15);
-            unsigned sl[kMaxSlices];
-            bool got = true;
-            if (lane < 16) {
+        const int last0 = (p.kb - 1) * p.tiles, own0 = max(ci0 + it0, last0) - last0, own1 = ci0 + p.div_upi(wu1) - last0;
+        auto fold = [&](auto slots) {                     // slices a launch may have
+            constexpr int S = decltype(slots)::value;
+            for (int t2 = own0; t2 < own1; t2 += 2) {
+                const bool two = t2 + 1 < own1, mine = two || lane < 16;
+                ItemCursor cf;
+                cf.slice = 0;
+                cf.tile = t2;
+                const ItemRef fr0 = item_ref(p, cf);
+                const float res0 = residual(fr0);
+                float *src = p.part + (size_t)t2 * 16 + lane;        // tiles lie one after the other
+                unsigned sl[S];
+                bool got = true;
+                if (mine) {
 #pragma unroll
-                for (int s = 0; s < kMaxSlices; s++) sl[s] = s < p.kb ? ld_volatile_u32(reinterpret_cast<const unsigned *>(src + s * sstride)) : 0u;
-                unsigned long long t0 = 0;
-                for (unsigned it = 0;; it++) {
-                    bool all = true;
+                    for (int s = 0; s < S; s++) sl[s] = s < p.kb ? ld_volatile_u32(reinterpret_cast<const unsigned *>(src + s * sstride)) : 0u;
+                    unsigned long long t0 = 0;
+                    for (unsigned it = 0;; it++) {
+                        bool all = true;
 #pragma unroll
-                    for (int s = 0; s < kMaxSlices; s++)
-                        if (s < p.kb && sl[s] == kFoldEmpty) {
-                            sl[s] = ld_volatile_u32(reinterpret_cast<const unsigned *>(src + s * sstride));
-                            all = all && sl[s] != kFoldEmpty;
+                        for (int s = 0; s < S; s++)
+                            if (s < p.kb && sl[s] == kFoldEmpty) {
+                                sl[s] = ld_volatile_u32(reinterpret_cast<const unsigned *>(src + s * sstride));
+                                all = all && sl[s] != kFoldEmpty;
+                            }
+                        if (all) break;
+                        if ((it & 255) == 255) {
+                            const unsigned long long t = global_ns();
+                            if (!t0) t0 = t;
+                            if (t - t0 > 1000000000ull) { got = false; break; }
                         }
-                    if (all) break;
-                    if ((it & 255) == 255) {
-                        const unsigned long long t = global_ns();
-                        if (!t0) t0 = t;
-                        if (t - t0 > 1000000000ull) { got = false; break; }
                     }
                 }
-            }
-            if (!__all_sync(0xffffffffu, got)) { if (lane == 0) atomicExch(p.err, 3); break; }
-            float a = 0.f;
-            if (lane < 16) {
-                a = __uint_as_float(sl[0]);
+                if (!__all_sync(0xffffffffu, got)) { if (lane == 0) atomicExch(p.err, 3); break; }
+                float a = 0.f;
+                if (mine) {
+                    a = __uint_as_float(sl[0]);
 #pragma unroll
-                for (int s = 1; s < kMaxSlices; s++) a += s < p.kb ? __uint_as_float(sl[s]) : 0.f;
+                    for (int s = 1; s < S; s++) a += s < p.kb ? __uint_as_float(sl[s]) : 0.f;
 #pragma unroll
-                for (int s = 0; s < kMaxSlices; s++)
-                    if (s < p.kb) reinterpret_cast<unsigned *>(src + s * sstride)[0] = kFoldEmpty;
+                    for (int s = 0; s < S; s++)
+                        if (s < p.kb) reinterpret_cast<unsigned *>(src + s * sstride)[0] = kFoldEmpty;
+                }
+                auto finish = [&](const ItemRef &fr, float y, float res) {
+                    if (tpr) {
+                        tp_push_tile(p, tp_seq, fr.row0, p.n_rows[0], y, lane);
+                        y = tp_sum_tile(p, tp_seq, fr.row0, p.n_rows[0], lane, &tp_ok);
+                        tp_finished++;
+                    }
+                    finish_rows(fr, y, res);
+                };
+                finish(fr0, a, res0);
+                if (two) {
+                    cf.tile = t2 + 1;
+                    const ItemRef fr1 = item_ref(p, cf);
+                    finish(fr1, __shfl_down_sync(0xffffffffu, a, 16), residual(fr1));
+                }
             }
-            if (tpr) {
-                tp_push_tile(p, tp_seq, fr.row0, p.n_rows[0], a, lane);
-                finish_rows(fr, tp_sum_tile(p, tp_seq, fr.row0, p.n_rows[0], lane, &tp_ok), res);
-                tp_finished++;
-            } else {
-                finish_rows(fr, a, res);
-            }
-        }
+        };
+        if (p.kb <= 8) fold(std::integral_constant<int, 8>());
+        else fold(std::integral_constant<int, kMaxSlices>());
     } else if (ok && wu1 > wu0) {
         // All partial results of this warp are out.  One fence, then one count per item (lane j counts
         // item j); the warp that completes a tile's last K-slice adds the slices in index order and
